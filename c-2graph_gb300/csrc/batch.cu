@@ -313,6 +313,7 @@ __device__ __forceinline__ void sbatch_pull(const BatchParams& p, int buf, unsig
 __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(const BatchParams p) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1293,6 +1294,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
     ppr_batch_persistent(const PprBatchParams p) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;

@@ -37,7 +37,7 @@ struct TraversalCtl {
     unsigned dctr[3];            // PPR activated vertices without out-edges, per slot
     unsigned farctr[3];          // SSSP far piles (rotating: current, target, free)
     int farmin[3];
-    unsigned bar_count, bar_gen;  // GridBarrier
+    unsigned bar_count, bar_pad;  // GridBarrier
     int flags;                    // C2G_FLAG_*
     int iterations;
     long long popped, relaxed, touched, seeds;

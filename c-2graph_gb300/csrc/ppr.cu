@@ -209,6 +209,7 @@ __device__ __forceinline__ void ppr_pull(const PprParams& p) {
 __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(const PprParams p) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;

@@ -85,7 +85,7 @@ struct PgSssp {
 };
 
 struct PgCtl {
-    unsigned bar_count, bar_gen;  // GridBarrier
+    unsigned bar_count, bar_pad;  // GridBarrier
     int flags;
     unsigned pos;      // the window's first position
     unsigned dmin;     // this round: the first position with an earlier writer of a row it reads
@@ -704,6 +704,7 @@ __global__ void __launch_bounds__(kPgThreads, 3) prune_rounds(const PgParams p) 
     PgRoots& S = s_roots[threadIdx.x >> 5];
     PgCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;

@@ -148,6 +148,7 @@ template <bool kDelta>
 __global__ void __launch_bounds__(512, 2) sssp_persistent(const SsspParams p) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_bits_pers
                                                                                        unsigned* bits) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
+    grid_sync_init();
     int* flags = &ctl->flags;
     const int lane = threadIdx.x & 31;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
