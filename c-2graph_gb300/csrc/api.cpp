@@ -29,6 +29,7 @@ static void graph_release(c2g_graph* g) {
     ppr_batch_free(g);
     ads_free(g);
     if (!g->borrowed) adjoint_free(g);
+    if (!g->borrowed) in_rows_free(g);
     if (!g->borrowed) {
         void* ptrs[] = {g->row, g->adj_w, g->adj_f, g->hv, g->he, g->hw, g->rec_of_vertex};
         for (void* p : ptrs)
@@ -113,6 +114,9 @@ static int records_fill(c2g_graph* g, int32_t R, const int32_t* hv, const int32_
     g->R = R;
     g->H = H;
     g->hw_float = hw_float;
+    g->hw_negative = false;
+    for (int64_t k = 0; k < H && !hw_float; ++k)
+        if (reinterpret_cast<const int32_t*>(hw)[k] < 0) g->hw_negative = true;
     g->h_hv.assign(hv, hv + R + 1);
     g->h_he.assign(he, he + H);
     g->h_hw.assign(reinterpret_cast<const int32_t*>(hw), reinterpret_cast<const int32_t*>(hw) + H);
@@ -220,12 +224,17 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->adj_rw = base->adj_rw;
     g->mark_r = base->mark_r;
     g->mark_f = base->mark_f;
+    g->in_row = base->in_row;
+    g->in_adj = base->in_adj;
+    g->in_edges = base->in_edges;
+    g->in_shift = base->in_shift;
     g->R = base->R;
     g->H = base->H;
     g->hv = base->hv;
     g->he = base->he;
     g->hw = base->hw;
     g->hw_float = base->hw_float;
+    g->hw_negative = base->hw_negative;
     g->rec_of_vertex = base->rec_of_vertex;
     g->h_row = base->h_row;
     g->h_hv = base->h_hv;
@@ -276,7 +285,7 @@ int c2g_graph_create(int device, int32_t V, int64_t E, const int32_t* vlist, con
     c2g_graph* g = nullptr;
     if ((rc = graph_new(device, &g))) return rc;
     DeviceScope ds(device);
-    if ((rc = graph_fill(g, vl, elist, E, wlist, flist))) {
+    if ((rc = graph_fill(g, vl, elist, E, wlist, flist)) || (rc = build_in_rows(g))) {
         graph_release(g);
         return rc;
     }
@@ -339,7 +348,8 @@ int c2g_graph_load(const char* dir, int variant, int device, c2g_graph** out) {
     if ((rc = graph_new(device, &g))) return rc;
     DeviceScope ds(device);
     if ((rc = graph_fill_rows(g, vlist)) ||
-        (rc = stream_graph(g, d + "elist.bin", wpath.empty() ? nullptr : &wpath, fpath.empty() ? nullptr : &fpath))) {
+        (rc = stream_graph(g, d + "elist.bin", wpath.empty() ? nullptr : &wpath, fpath.empty() ? nullptr : &fpath)) ||
+        (rc = build_in_rows(g))) {
         graph_release(g);
         return rc;
     }

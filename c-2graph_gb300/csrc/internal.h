@@ -43,6 +43,7 @@ struct TraversalCtl {
     long long popped, relaxed, touched, seeds;
     int pad[1];
     unsigned long long phase_ns[4];  // block 0's time per phase (see phase_mark)
+    unsigned long long lctr[2];      // SSSP pull rounds: rows left to the whole grid, by round parity
     unsigned long long pcount[3];    // batched PPR: (query, edge) pushes of the frontier per round slot
 };
 
@@ -72,7 +73,8 @@ struct SsspWork {
     int2* q[2] = {nullptr, nullptr};
     int* mark[2] = {nullptr, nullptr};
     int* far = nullptr;  // three far piles of V ids each
-    unsigned* bits = nullptr;  // next-frontier bitmap of the Bellman-Ford kernel (V/32 words)
+    int* pull_mark = nullptr;  // tile owners of a pull round's long rows
+    unsigned* bits = nullptr;  // frontier bitmaps of the Bellman-Ford kernel (2 x V/32 words)
     TraversalCtl* ctl = nullptr;
     StampState* st = nullptr;
     unsigned mark_cap = 0;
@@ -114,6 +116,8 @@ struct PprConfig {
     int dense_div = 16;  // dense push round (red.add, apply sweep over V) when out-edges * dense_div > E
 };
 
+constexpr int kInMaxWeight = 147483648;  // largest weight of in-edge rows: unreachable + weight fits an int32
+
 constexpr int kPullTileLog = 8;  // in-edges per pull tile (reverse-CSR markers)
 
 struct LaunchGeom {
@@ -135,6 +139,11 @@ struct c2g_graph {
     int2* adj_r = nullptr;
     int2* adj_rw = nullptr;     // the same in-edges with int32 weights (batched SSSP pull rounds), on
                                 // demand; adj_r itself when the graph has no float weights
+    // in-edge rows ordered by weight (in_rows.cu), or null: the graph's SSSP queries push only
+    int32_t* in_row = nullptr;  // [V+1], multiples of 4
+    int2* in_adj = nullptr;     // (source, weight), padded with weight INT_MAX
+    int64_t in_edges = 0;       // padded edges
+    int in_shift = 0;           // weights are ordered up to their low in_shift bits
     int32_t* mark_r = nullptr;  // pull-tile owner markers over row_r
     int32_t* mark_f = nullptr;  // pull-tile owner markers over row (pulls on the reverse graph)
     // pruned records
@@ -144,6 +153,7 @@ struct c2g_graph {
     int32_t* he = nullptr;
     int32_t* hw = nullptr;  // int32 or float bits
     bool hw_float = false;
+    bool hw_negative = false;  // some int32 record weight is below 0 (its seeds push only)
     int32_t* rec_of_vertex = nullptr;
     // host copies needed for source rules and seed ranges
     std::vector<int32_t> h_row;
@@ -195,6 +205,8 @@ void batch_free(c2g_graph* g);
 void ppr_batch_free(c2g_graph* g);
 void ads_free(c2g_graph* g);
 int build_reverse_graph(c2g_graph* g);
+int build_in_rows(c2g_graph* g);
+void in_rows_free(c2g_graph* g);
 // The reverse CSR's in-edges with int32 weights (batched SSSP pull rounds).
 int build_reverse_int(c2g_graph* g);
 // Reverse CSR and the weight statistics of the batched pull rounds (once per weights).

@@ -15,6 +15,7 @@
 //     threshold go to a far pile that is filtered into the frontier when the near
 //     frontier runs dry;
 //   * one bounded grid barrier per round instead of four unbounded spins.
+#include <algorithm>
 #include <climits>
 #include <cstring>
 #include <mutex>
@@ -288,20 +289,50 @@ __global__ void __launch_bounds__(512, 2) sssp_persistent(const SsspParams p) {
     }
 }
 
-// Bellman-Ford rounds (delta = 0) with a bitmap next frontier.  A relaxation that
-// improves a distance issues red.min on it and red.or of the vertex's bit into a
-// V-bit map; neither waits for a return value, so the relaxation path has no atomic
-// round trip (the list kernel above needs the atomicMin result and a round-tag exchange
-// per improved vertex).  A sweep over the V/32 map words then builds the next frontier
-// in vertex order (entries, edge-base prefix, tile markers) and clears the words:
-// two grid barriers per round instead of one.
+// Bellman-Ford rounds (delta = 0), each a push or a pull.
+//
+// Push: the frontier is a list; a relaxation that improves a distance issues red.min on it and
+// red.or of the vertex's bit into a V-bit map; neither waits for a return value, so the
+// relaxation path has no atomic round trip (the list kernel above needs the atomicMin result
+// and a round-tag exchange per improved vertex).  A sweep over the V/32 map words builds
+// the next frontier in vertex order (entries, edge-base prefix, tile markers) and clears the
+// words: two grid barriers per round.
+//
+// Pull: every vertex v reads its in-edges, ordered by weight (in_rows.cu), as long as
+// w + (smallest frontier distance) < dist[v]: no later edge can improve v.  A push of a dense
+// frontier is bound by one random L2 read per out-edge of the frontier; in a pull most rows
+// end after one or two groups of 4 edges, hub rows too (their distance is small).  The warp
+// that pulls v is the only writer of dist[v] in the round, so it stores without atomics,
+// writes the map word of its 32 vertices and counts the next frontier: a pull needs no list,
+// and one barrier.
+//
+// Any order of relaxations reaches the same fixed point, so the rounds mix freely.
 constexpr int kSweepGroup = 4;  // map words whose row bounds are loaded together
 constexpr int kBitsThreads = 512;  // block size of the bitmap kernel (its own launch geometry)
 constexpr int kBitsBlocksPerSm = 2;
 // Round-robin tiles in the expansion: a dynamic tile queue measured slower here (2.74 vs
 // 2.20 ms per scale-22 query).
 constexpr bool kBitsDynTiles = false;
+// Swept at scale 22 / 16 (1.05 ms, 133 us): 1, 2 or 3 words at a time, 2 or 4 lane groups, 1.05 - 1.13 ms.
+constexpr int kPullWords = 2;    // map words a warp pulls at a time
+constexpr int kLaneGroups = 2;   // groups of 4 in-edges a lane reads before the warp shares the rest
+constexpr int kWarpGroups = 16;  // rows that need more groups than this go to the whole grid
+constexpr int kPullTile = 6;     // log2 of the groups per warp tile of those rows
 
+// In-edge rows and round rule of the kernel.
+struct SsspPull {
+    const int* row;   // in-edge rows, or nullptr: push only
+    const int2* adj;
+    int shift;           // weights are ordered up to their low `shift` bits
+    unsigned pull_min;   // a round pulls when its frontier has more out-edges (~0: never)
+    int always;          // every round pulls: no map, no list
+    unsigned* bits[2];   // maps of the frontiers of the rounds of each parity
+    double* long_at;     // long rows: (distance << 32) | first group, beside their queue entry
+    int* long_mark;      // tile owners over their groups
+    unsigned long_tiles;
+};
+
+// Warp-collective: the frontier list of a round from its map; the words are cleared.
 __device__ __forceinline__ void bits_sweep(const SsspParams& p, unsigned* bits, const FrontierOut& out,
                                            WarpStage& fst, unsigned gwarp, unsigned nwarps, int lane) {
     const unsigned V = (unsigned)p.V;
@@ -337,8 +368,266 @@ __device__ __forceinline__ void bits_sweep(const SsspParams& p, unsigned* bits, 
     stage_flush(fst, out);
 }
 
-__global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_bits_persistent(const SsspParams p,
-                                                                                       unsigned* bits) {
+// A block's part of a round's totals, added to the round's counters once per block.
+struct RoundShare {
+    unsigned long long count;  // (vertices with out-edges << 32) | out-edges, of the improved vertices
+    int fmin;                  // smallest improved distance
+};
+
+// Add a warp's totals of a round to its block's, and the block's to the round's counters
+// (every warp of the grid adding to one address took longer than a short round).
+__device__ __forceinline__ void round_totals(TraversalCtl* ctl, int slot, RoundShare* share,
+                                             unsigned long long count, int fnew, int lane) {
+    for (int o = 16; o >= 1; o >>= 1) count += __shfl_xor_sync(kFull, count, o);
+    fnew = __reduce_min_sync(kFull, fnew);
+    if (lane == 0) {
+        if (count) atomicAdd(&share->count, count);
+        if (fnew != INT_MAX) atomicMin(&share->fmin, fnew);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (share->count) atomicAdd(&ctl->pcount[slot], share->count);
+        if (share->fmin != INT_MAX) atomicMin(&ctl->farmin[slot], share->fmin);
+        *share = RoundShare{0ull, INT_MAX};
+    }
+}
+
+// A group of 4 in-edges (source, weight): the smallest candidate distance below b among the
+// edges that can improve it (weight below lim).
+__device__ __forceinline__ int pull_edges(const int* dist, const int4& x, const int4& y, int lim, int b) {
+    // Read through L1: other warps lower distances during the round, and either value is a
+    // valid upper bound (a lowered source is in the next frontier); the barrier's acquire
+    // makes the next round read anew.
+    const int d0 = x.y < lim ? __ldca(dist + x.x) : kInfDist;
+    const int d1 = x.w < lim ? __ldca(dist + x.z) : kInfDist;
+    const int d2 = y.y < lim ? __ldca(dist + y.x) : kInfDist;
+    const int d3 = y.w < lim ? __ldca(dist + y.z) : kInfDist;
+    // an edge that cannot improve has weight up to INT_MAX (the padding): no sum of its own
+    if (x.y < lim) b = min(b, d0 + x.y);
+    if (x.w < lim) b = min(b, d1 + x.w);
+    if (y.y < lim) b = min(b, d2 + y.y);
+    if (y.w < lim) b = min(b, d3 + y.w);
+    return b;
+}
+
+__device__ __forceinline__ int pull_group(const SsspPull& in, const int* dist, int i, int lim, int b, int* last) {
+    const int4 x = __ldg(reinterpret_cast<const int4*>(in.adj + i));
+    const int4 y = __ldg(reinterpret_cast<const int4*>(in.adj + i + 2));
+    *last = (y.w >> in.shift) << in.shift;
+    return pull_edges(dist, x, y, lim, b);
+}
+
+// Queue of a pull round's long rows: (vertex, exclusive prefix of the groups to read), with
+// the distance and first group in long_at.  It uses the list buffers, idle in a pull round.
+__device__ __forceinline__ FrontierOut pull_long_out(const SsspParams& p, const SsspPull& in, int parity) {
+    FrontierOut o;
+    o.q = p.q[0];
+    o.val = nullptr;
+    o.vald = in.long_at;
+    o.mark = in.long_mark;
+    o.ctr = &p.ctl->lctr[parity];
+    o.cap = (unsigned)p.V;
+    o.mark_cap = in.long_tiles;
+    o.log_tile = kPullTile;
+    o.flags = &p.ctl->flags;
+    return o;
+}
+
+// What is left of a word's rows after their first group: lanes read on up to kLaneGroups
+// groups; a row that needs more finds by bisection how many groups can still improve it.  Up to
+// kWarpGroups the warp reads together, all rows' groups in one sequence; longer rows are
+// queued for the whole grid.
+__device__ __forceinline__ int pull_rest(const SsspParams& p, const SsspPull& in, int fmin, unsigned v, int b, int i,
+                                      int e, bool more, int* best, WarpStage& lst, const FrontierOut& lout, int lane) {
+    int last = INT_MIN;
+#pragma unroll 1
+    for (int s = 1; s < kLaneGroups; ++s) {
+        if (more) {
+            b = pull_group(in, p.dist, i, b - fmin, b, &last);
+            i += 4;
+        }
+        more = more && i < e && last < b - fmin;
+        if (!__any_sync(kFull, more)) return b;
+    }
+    // groups [0, n) from i on start below the limit (their first weight, rounded down)
+    int n = 0;
+    if (more) {
+        int hi = (e - i) >> 2;
+        while (n < hi) {  // the first group at or above the limit is in [n, hi]: three probes at a time
+            const int q = (hi - n) >> 2, m1 = n + q, m2 = m1 + q, m3 = m2 + q;
+            const bool b1 = ((__ldg(in.adj + i + 4 * m1).y >> in.shift) << in.shift) < b - fmin;
+            const bool b2 = ((__ldg(in.adj + i + 4 * m2).y >> in.shift) << in.shift) < b - fmin;
+            const bool b3 = ((__ldg(in.adj + i + 4 * m3).y >> in.shift) << in.shift) < b - fmin;
+            if (!b1) hi = m1;
+            else if (!b2) { n = m1 + 1; hi = m2; }
+            else if (!b3) { n = m2 + 1; hi = m3; }
+            else n = m3 + 1;
+        }
+    }
+    const bool queued = n > kWarpGroups;
+    stage_push(lst, lout, queued, (int)v, n, 0.f, __longlong_as_double(((long long)b << 32) | (long long)(unsigned)i));
+    if (queued) n = 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const unsigned base = (unsigned)(incl - n), total = (unsigned)__shfl_sync(kFull, incl, 31);
+    best[lane] = b;
+    __syncwarp();
+    for (unsigned g = (unsigned)lane; g - (unsigned)lane < total; g += 32u) {
+        const int k = owner_lane(base, g);
+        const int ki = __shfl_sync(kFull, i, k);
+        const unsigned kb = (unsigned)__shfl_sync(kFull, (int)base, k);
+        if (g < total) {
+            const int bk = *(volatile int*)(best + k);
+            int unused;
+            const int nb = pull_group(in, p.dist, ki + 4 * (int)(g - kb), bk - fmin, bk, &unused);
+            if (nb < bk) atomicMin(best + k, nb);
+        }
+    }
+    __syncwarp();
+    b = best[lane];
+    __syncwarp();
+    return b;
+}
+
+// First part of a pull round.  Each warp takes map words (32 vertices, one per lane),
+// kPullWords at a time so that their first groups' loads are in flight together: at scale 22
+// a pull reads about one group and one source distance per vertex, so it is bound by the chain
+// word -> group -> sources, not by bytes.  Consecutive words go to different blocks and the
+// stride over words is odd: the busiest vertices of a skewed graph have neighbouring ids and
+// ids that are multiples of powers of two (with an even stride 170 of 4,864 warps took
+// 113 us where the average was 42 us).  The rows that need more groups follow in pull_rest.
+__device__ __forceinline__ void sssp_pull(const SsspParams& p, const SsspPull& in, int fmin, unsigned* bits_cur,
+                                          unsigned* bits_next, int* best, WarpStage& lst, const FrontierOut& lout,
+                                          unsigned long long& count, int& fnew, int lane, int wib) {
+    const unsigned V = (unsigned)p.V;
+    const unsigned nw = (V + 31u) >> 5;
+    const unsigned nwarps = (((gridDim.x * blockDim.x) >> 5) - 1u) | 1u;  // odd
+    const unsigned wfirst = (unsigned)wib * gridDim.x + blockIdx.x;
+    for (unsigned w0 = wfirst < nwarps ? wfirst : nw; w0 < nw; w0 += kPullWords * nwarps) {
+        int b0[kPullWords], b[kPullWords], i[kPullWords], e[kPullWords], last[kPullWords], deg[kPullWords];
+        // first groups of all words, their loads in flight together
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            const unsigned v = ((w0 + u * nwarps) << 5) + (unsigned)lane;
+            const bool in_range = w0 + u * nwarps < nw && v < V;
+            b0[u] = in_range ? ldcg(p.dist + v) : INT_MIN;
+            i[u] = in_range ? __ldg(in.row + v) : 0;
+            e[u] = in_range ? __ldg(in.row + v + 1) : 0;
+        }
+        int4 x[kPullWords], y[kPullWords];
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            const bool go = i[u] < e[u] && b0[u] > fmin;
+            x[u] = go ? __ldg(reinterpret_cast<const int4*>(in.adj + i[u])) : make_int4(0, INT_MAX, 0, INT_MAX);
+            y[u] = go ? __ldg(reinterpret_cast<const int4*>(in.adj + i[u] + 2)) : make_int4(0, INT_MAX, 0, INT_MAX);
+            if (!go) e[u] = i[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            b[u] = pull_edges(p.dist, x[u], y[u], b0[u] - fmin, b0[u]);
+            last[u] = (y[u].w >> in.shift) << in.shift;
+            i[u] += 4;
+        }
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            const bool more = i[u] < e[u] && last[u] < b[u] - fmin;
+            if (__any_sync(kFull, more))
+                b[u] = pull_rest(p, in, fmin, ((w0 + u * nwarps) << 5) + (unsigned)lane, b[u], i[u], e[u], more, best,
+                                 lst, lout, lane);
+        }
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            const unsigned v = ((w0 + u * nwarps) << 5) + (unsigned)lane;
+            deg[u] = 0;
+            if (b[u] < b0[u]) {
+                p.dist[v] = b[u];
+                deg[u] = __ldg(p.row + v + 1) - __ldg(p.row + v);
+                fnew = min(fnew, b[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kPullWords; ++u) {
+            if (deg[u] > 0) count += (1ull << 32) | (unsigned)deg[u];
+            if (!in.always && w0 + u * nwarps < nw) {
+                const unsigned m = __ballot_sync(kFull, deg[u] > 0);
+                if (lane == 0) {
+                    bits_next[w0 + u * nwarps] = m;
+                    bits_cur[w0 + u * nwarps] = 0u;  // this round's frontier, if it was not listed
+                }
+            }
+        }
+    }
+    stage_flush(lst, lout);
+}
+
+// Second part, after a barrier, when rows were queued (a hub row that nothing has reached yet needs
+// all its 100,000 edges: read by its warp alone that took 1.07 ms of a scale-22 query): warps
+// take tiles of their groups, and a row's parts meet in atomicMin.  The part that first lowers the queued distance counts the
+// vertex for the next frontier, unless the first part of the round had.
+__device__ __forceinline__ void sssp_pull_long(const SsspParams& p, const SsspPull& in, int fmin, unsigned L,
+                                               unsigned G, unsigned* bits_next, int* best, unsigned long long& count,
+                                               int& fnew, int lane, unsigned gwarp, unsigned nwarps) {
+    const unsigned ntiles = (G + (1u << kPullTile) - 1u) >> kPullTile;
+    if (ntiles > in.long_tiles || L > (unsigned)p.V) {
+        if (lane == 0) atomicOr(&p.ctl->flags, C2G_FLAG_BOUNDS);
+        return;
+    }
+    for (unsigned t = gwarp; t < ntiles; t += nwarps) {
+        unsigned g0 = t << kPullTile;
+        const unsigned g1 = min(g0 + (1u << kPullTile), G);
+        for (unsigned o = (unsigned)ldcg(in.long_mark + t); g0 < g1 && o < L; o += 32) {
+            const unsigned j = o + (unsigned)lane;
+            unsigned base = 0x7fffffffu, next = 0xffffffffu;
+            int v = 0, d = INT_MIN, bq = 0, i = 0;
+            if (j < L) {
+                const int2 ve = ldcg(p.q[0] + j);
+                const long long at = __double_as_longlong(ldcg(in.long_at + j));
+                v = ve.x;
+                base = (unsigned)ve.y;
+                next = j + 1 < L ? (unsigned)ldcg(p.q[0] + j + 1).y : G;
+                bq = (int)(at >> 32);
+                i = (int)(unsigned)at;
+                d = ldcg(p.dist + v);
+            }
+            const unsigned stop = min(g1, (unsigned)__shfl_sync(kFull, (int)next, 31));
+            best[lane] = d;
+            __syncwarp();
+            for (unsigned g = g0 + (unsigned)lane; g - (unsigned)lane < stop; g += 32u) {
+                const int k = owner_lane(base, g);
+                const int ki = __shfl_sync(kFull, i, k);
+                const unsigned kb = (unsigned)__shfl_sync(kFull, (int)base, k);
+                if (g < stop) {
+                    const int bk = *(volatile int*)(best + k);
+                    int unused;
+                    const int nb = pull_group(in, p.dist, ki + 4 * (int)(g - kb), bk - fmin, bk, &unused);
+                    if (nb < bk) atomicMin(best + k, nb);
+                }
+            }
+            __syncwarp();
+            const int nb = best[lane];
+            __syncwarp();
+            if (nb < d) {
+                const int old = atomicMin(p.dist + v, nb);
+                if (nb < old) {
+                    fnew = min(fnew, nb);
+                    const int deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
+                    if (deg > 0) {
+                        if (old == bq) count += (1ull << 32) | (unsigned)deg;
+                        if (!in.always) atomicOr(bits_next + ((unsigned)v >> 5), 1u << (v & 31));
+                    }
+                }
+            }
+            g0 = stop;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_persistent(const SsspParams p,
+                                                                                         const SsspPull in) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
     grid_sync_init();
@@ -348,40 +637,63 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_bits_pers
     const unsigned nthreads = gridDim.x * blockDim.x;
     const unsigned gwarp = gtid >> 5, nwarps = nthreads >> 5;
     const unsigned V = (unsigned)p.V;
-    __shared__ StageSmem sm;
+    __shared__ StageSmemD sm;
+    __shared__ RoundShare share;
     const int wib = threadIdx.x >> 5;
-    WarpStage fst{sm.v0[wib], sm.d0[wib], nullptr, 0};
+    WarpStage fst{sm.v0[wib], sm.d0[wib], nullptr, 0};               // lists (push rounds)
+    WarpStage lst{sm.v0[wib], sm.d0[wib], nullptr, 0, sm.xd0[wib]};  // long rows (pull rounds)
     unsigned long long tph = globaltimer_ns();
 
-    // Init: dis = INF (src/sssp/purn/Main.cu:144-156), empty map.
+    // Init: dis = INF (src/sssp/purn/Main.cu:144-156), empty maps.
     for (unsigned v = gtid; v < V; v += nthreads) p.dist[v] = kInfDist;
-    for (unsigned i = gtid; i < ((V + 31u) >> 5); i += nthreads) bits[i] = 0u;
-    if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
-    // Source and pruned-record seeds (src/sssp/purn/Main.cu:160-181) form round 1.
+    if (!in.always)
+        for (unsigned i = gtid; i < ((V + 31u) >> 5); i += nthreads) in.bits[0][i] = in.bits[1][i] = 0u;
     if (gtid == 0) {
-        atomicMin(p.dist + p.source, 0);
-        atomicOr(bits + ((unsigned)p.source >> 5), 1u << (p.source & 31));
+        // fmin of round 1 is 0 (the source); the next rounds' start empty
+        ctl->farmin[2] = ctl->farmin[0] = INT_MAX;
         ctl->seeds = p.n_seeds;
     }
-    for (unsigned i = gtid; i < (unsigned)p.n_seeds; i += nthreads) {
-        const int v = p.seed_v[i];
-        atomicMin(p.dist + v, p.seed_w[i]);
-        atomicOr(bits + ((unsigned)v >> 5), 1u << (v & 31));
+    if (threadIdx.x == 0) share = RoundShare{0ull, INT_MAX};
+    if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
+    // Source and pruned-record seeds (src/sssp/purn/Main.cu:160-181) form round 1.
+    const int s_row = __ldg(p.row + p.source), s_deg = __ldg(p.row + p.source + 1) - s_row;
+    if (gtid == 0) atomicMin(p.dist + p.source, 0);
+    for (unsigned i = gtid; i < (unsigned)p.n_seeds; i += nthreads) atomicMin(p.dist + p.seed_v[i], p.seed_w[i]);
+    if (!in.always) {
+        if (gtid == 0) atomicOr(in.bits[1] + ((unsigned)p.source >> 5), 1u << (p.source & 31));
+        for (unsigned i = gtid; i < (unsigned)p.n_seeds; i += nthreads) {
+            const int v = p.seed_v[i];
+            atomicOr(in.bits[1] + ((unsigned)v >> 5), 1u << (v & 31));
+        }
+    } else {
+        // Pulls only: no list will hold the source's out-edges, so they are relaxed here
+        // (most of a skewed graph is then one pull away); round 1 counts the same frontier.
+        for (unsigned i = gtid; i < (unsigned)s_deg; i += nthreads) {
+            const int2 ew = __ldg(p.adj + s_row + (int)i);
+            atomicMin(p.dist + ew.x, ew.y);
+        }
+        unsigned long long c = gtid == 0 && s_deg > 0 ? (1ull << 32) | (unsigned)s_deg : 0ull;
+        for (unsigned i = gtid; i < (unsigned)p.n_seeds; i += nthreads) {
+            const int v = p.seed_v[i], deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
+            if (deg > 0) c += (1ull << 32) | (unsigned)deg;
+        }
+        if (c) atomicAdd(&ctl->pcount[1], c);
     }
     if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
     phase_mark(ctl->phase_ns, tph, 0);
 
     int cur = 1, iters = 0;
+    bool counted = in.always != 0;  // this round's frontier is counted (a pull made it), not listed
     for (;;) {
-        const int buf = cur & 1, slot = cur % 3;
-        if (gtid == 0) {
-            ctl->qctr[(cur + 1) % 3] = 0ull;
-            ctl->tilectr[(cur + 1) % 3] = 0u;
+        const int buf = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
+        unsigned long long c = counted ? ldcg(&ctl->pcount[slot]) : 0ull;
+        if (gtid == 0) ctl->qctr[nslot] = 0ull;
+        if (!counted || (c != 0ull && (unsigned)c <= in.pull_min)) {
+            bits_sweep(p, in.bits[buf], sssp_out(p, buf, slot), fst, gwarp, nwarps, lane);
+            if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
+            phase_mark(ctl->phase_ns, tph, 1);
+            c = ldcg(&ctl->qctr[slot]);
         }
-        bits_sweep(p, bits, sssp_out(p, buf, slot), fst, gwarp, nwarps, lane);
-        if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
-        phase_mark(ctl->phase_ns, tph, 1);
-        const unsigned long long c = ldcg(&ctl->qctr[slot]);
         const unsigned F = (unsigned)(c >> 32), T = (unsigned)c;
         if (F == 0) break;
         if (++iters > p.max_iter) {
@@ -391,32 +703,59 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_bits_pers
         if (gtid == 0) {
             ctl->popped += F;
             ctl->relaxed += T;
+            ctl->pcount[fslot] = 0ull;
+            ctl->farmin[fslot] = INT_MAX;
+            ctl->lctr[buf ^ 1] = 0ull;
         }
-        constexpr int U = kSsspUnroll;
-        walk_frontier_edges<U>(
-            p.q[buf], p.mark[buf], p.row, F, T, p.log_tile, p.mark_cap, V, p.E, flags,
-            [&](int v, unsigned) { return ldcg(p.dist + v); },  // the owner's current distance
-            [&](const bool* ok, const unsigned* idx, const int* du) {
-                int c2[U], nd[U], cd[U];
+        unsigned long long count = 0ull;
+        int fnew = INT_MAX;
+        const bool pull = T > in.pull_min;  // grid-uniform
+        const int fmin = ldcg(&ctl->farmin[slot]);
+        if (pull) {
+            sssp_pull(p, in, fmin, in.bits[buf], in.bits[buf ^ 1], sm.v1[wib], lst, pull_long_out(p, in, buf), count,
+                      fnew, lane, wib);
+        } else {
+            constexpr int U = kSsspUnroll;
+            unsigned* bits = in.bits[buf ^ 1];
+            walk_frontier_edges<U>(
+                p.q[buf], p.mark[buf], p.row, F, T, p.log_tile, p.mark_cap, V, p.E, flags,
+                [&](int v, unsigned) { return ldcg(p.dist + v); },  // the owner's current distance
+                [&](const bool* ok, const unsigned* idx, const int* du) {
+                    int c2[U], nd[U], cd[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int2 ew = ok[u] ? __ldg(p.adj + idx[u]) : make_int2(0, 0);
-                    c2[u] = ew.x;
-                    nd[u] = du[u] + ew.y;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) cd[u] = ok[u] ? ldcg(p.dist + c2[u]) : INT_MIN;
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (nd[u] < cd[u]) {  // an L2 read guards the update
-                        atomicMin(p.dist + c2[u], nd[u]);
-                        atomicOr(bits + ((unsigned)c2[u] >> 5), 1u << (c2[u] & 31));
+                    for (int u = 0; u < U; ++u) {
+                        const int2 ew = ok[u] ? __ldg(p.adj + idx[u]) : make_int2(0, 0);
+                        c2[u] = ew.x;
+                        nd[u] = du[u] + ew.y;
                     }
-                }
-            },
-            kBitsDynTiles ? &ctl->tilectr[slot] : nullptr);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) cd[u] = ok[u] ? ldcg(p.dist + c2[u]) : INT_MIN;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        if (nd[u] < cd[u]) {  // an L2 read guards the update
+                            atomicMin(p.dist + c2[u], nd[u]);
+                            atomicOr(bits + ((unsigned)c2[u] >> 5), 1u << (c2[u] & 31));
+                            fnew = min(fnew, nd[u]);
+                        }
+                    }
+                },
+                kBitsDynTiles ? &ctl->tilectr[slot] : nullptr);
+        }
+        round_totals(ctl, nslot, &share, count, fnew, lane);
         if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
+        if (pull) {
+            const unsigned long long lc = ldcg(&ctl->lctr[buf]);  // grid-uniform
+            if (lc) {
+                count = 0ull;
+                fnew = INT_MAX;
+                sssp_pull_long(p, in, fmin, (unsigned)(lc >> 32), (unsigned)lc, in.bits[buf ^ 1], sm.v1[wib], count,
+                               fnew, lane, gwarp, nwarps);
+                round_totals(ctl, nslot, &share, count, fnew, lane);
+                if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
+            }
+        }
         phase_mark(ctl->phase_ns, tph, 2);
+        counted = pull;
         ++cur;
     }
     if (gtid == 0) ctl->iterations = iters;
@@ -433,7 +772,7 @@ static int sssp_geometry(c2g_graph* g) {
     int per_sm_a = 0, per_sm_b = 0, per_sm_c = 0;
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_a, sssp_persistent<false>, 512, 0));
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_b, sssp_persistent<true>, 512, 0));
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, sssp_bits_persistent, kBitsThreads, 0));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, sssp_rounds_persistent, kBitsThreads, 0));
     const int per_sm = per_sm_a < per_sm_b ? per_sm_a : per_sm_b;
     if (per_sm < 1 || per_sm_c < 1) return fail(C2G_ERR_CUDA, "SSSP kernel cannot be resident (occupancy 0)");
     g->geom_sssp.blocks = per_sm * g->num_sms;
@@ -446,7 +785,7 @@ static int sssp_geometry(c2g_graph* g) {
 void sssp_free(c2g_graph* g) {
     SsspWork& w = g->sssp;
     void* ptrs[] = {w.dist, w.stamp, w.farstamp, w.q[0], w.q[1], w.mark[0], w.mark[1],
-                    w.far, w.bits, w.ctl, w.st};
+                    w.far, w.pull_mark, w.bits, w.ctl, w.st};
     for (void* ptr : ptrs)
         if (ptr) cudaFree(ptr);
     w = SsspWork();
@@ -468,7 +807,8 @@ static int sssp_alloc(c2g_graph* g) {
         C2G_CUDA(cudaMalloc(&w.mark[b], sizeof(int) * mark_cap));
     }
     C2G_CUDA(cudaMalloc(&w.far, sizeof(int) * nv * 3));
-    C2G_CUDA(cudaMalloc(&w.bits, sizeof(unsigned) * ((nv + 31) / 32)));
+    C2G_CUDA(cudaMalloc(&w.bits, sizeof(unsigned) * 2 * ((nv + 31) / 32)));
+    if (g->in_adj) C2G_CUDA(cudaMalloc(&w.pull_mark, sizeof(int) * ((size_t)(g->in_edges >> (kPullTile + 2)) + 2)));
     C2G_CUDA(cudaMalloc(&w.ctl, sizeof(TraversalCtl)));
     C2G_CUDA(cudaMalloc(&w.st, sizeof(StampState)));
     C2G_CUDA(cudaMemsetAsync(w.stamp, 0xff, sizeof(int) * nv, g->stream));
@@ -477,6 +817,39 @@ static int sssp_alloc(c2g_graph* g) {
     w.mark_cap = mark_cap;
     w.log_tile = log_tile;
     return C2G_OK;
+}
+
+// Round rule of a launch.  A pull's cost is its pass over the vertices (80 - 110 us at 4.2M),
+// a push's its frontier's out-edges (150 us for 15.6M of 65M) and a second barrier.
+//   * kPullDiv: a round pulls when its frontier holds more than 1/4 of the edges (scale 22:
+//     1.05 ms a query, at 1/10 1.17 ms: the first pull meets rows that nothing has reached).
+//   * kPullAlways*: below these sizes a whole pull is about as short as a barrier (3.5 - 5 us
+//     once most rows are pruned), so every round pulls, without map, list or second barrier
+//     (scale 16, 1M edges: 134 us against 250 us with push rounds; scale 12: 89 against 120).
+//     The vertex bound keeps graphs of few edges and very many rounds on sparse pushes.
+//   * kPullMaxDegree: a warp pulls 32 vertices; with few vertices and very long rows too few
+//     warps would have work.
+constexpr int64_t kPullMaxDegree = 128;
+constexpr int64_t kPullDiv = 4;
+constexpr int64_t kPullAlwaysEdges = 4000000;
+constexpr int32_t kPullAlwaysVertices = 300000;
+
+static void sssp_round_rule(const c2g_graph* g, SsspPull& in) {
+    const SsspWork& w = g->sssp;
+    const size_t nw = ((size_t)g->V + 31) / 32;
+    in.row = g->in_row;
+    in.adj = g->in_adj;
+    in.shift = g->in_shift;
+    in.bits[0] = w.bits;
+    in.bits[1] = w.bits + nw;
+    in.long_at = reinterpret_cast<double*>(w.far);  // the far piles belong to delta > 0
+    in.long_mark = w.pull_mark;
+    in.long_tiles = w.pull_mark ? (unsigned)((g->in_edges >> (kPullTile + 2)) + 2) : 0u;
+    in.pull_min = ~0u;
+    in.always = 0;
+    if (!g->in_adj || g->hw_negative || g->E > kPullMaxDegree * (int64_t)g->V) return;
+    in.always = g->E <= kPullAlwaysEdges && g->V <= kPullAlwaysVertices;
+    in.pull_min = in.always ? 0u : (unsigned)(g->E / kPullDiv);
 }
 
 int sssp_launch(c2g_graph* g, int32_t source, const int32_t* seed_v, const int32_t* seed_w, int32_t n_seeds,
@@ -517,13 +890,17 @@ int sssp_launch(c2g_graph* g, int32_t source, const int32_t* seed_v, const int32
     p.bar_extra = g->stall_next_sssp ? 1u : 0u;
     g->stall_next_sssp = 0;
     C2G_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(TraversalCtl), g->stream));
-    unsigned* bits = w.bits;
-    void* args[] = {&p, &bits};
     const bool delta = p.delta > 0;
-    // delta = 0: Bellman-Ford rounds with the bitmap frontier; delta > 0: near/far buckets
+    SsspPull in;
+    sssp_round_rule(g, in);
+    // delta = 0: Bellman-Ford rounds; delta > 0: near/far buckets
+    void* args[] = {&p, &in};
+    const int blocks = delta ? g->geom_sssp.blocks
+                     : in.always ? std::min(g->geom_bits.blocks, (g->V + kBitsThreads - 1) / kBitsThreads)
+                                 : g->geom_bits.blocks;
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel(delta ? (const void*)sssp_persistent<true> : (const void*)sssp_bits_persistent,
-                                         dim3(delta ? g->geom_sssp.blocks : g->geom_bits.blocks),
+    C2G_CUDA(cudaLaunchCooperativeKernel(delta ? (const void*)sssp_persistent<true> : (const void*)sssp_rounds_persistent,
+                                         dim3(blocks),
                                          dim3(delta ? g->geom_sssp.threads : g->geom_bits.threads), args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     if (ms) {
