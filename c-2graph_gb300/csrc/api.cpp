@@ -221,12 +221,13 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->adj_f = base->adj_f;
     g->row_r = base->row_r;
     g->adj_r = base->adj_r;
-    g->adj_rw = base->adj_rw;
     g->mark_r = base->mark_r;
     g->mark_f = base->mark_f;
     g->in_row = base->in_row;
     g->in_adj = base->in_adj;
     g->in_edges = base->in_edges;
+    g->in_seg = base->in_seg;
+    g->in_segs = base->in_segs;
     g->in_shift = base->in_shift;
     g->R = base->R;
     g->H = base->H;
@@ -476,6 +477,7 @@ int c2g_sssp_batch_set_pull(c2g_graph* g, float frac) {
     if (frac != frac) return fail(C2G_ERR_ARG, "frac is NaN");
     std::lock_guard<std::mutex> lk(g->mu);
     g->sssp_cfg.batch_pull_frac = frac;
+    g->sssp_cfg.batch_pull_set = true;
     return C2G_OK;
 }
 

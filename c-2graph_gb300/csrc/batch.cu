@@ -57,18 +57,21 @@ struct BatchParams {
     int tile_min_log;     // a round walks big tiles when it has >= 2^tile_min_log of them per warp
     int epoch_rounds;     // > 0: an epoch of a resident batch (no initialisation; at most this many rounds)
     RoundTrace* trace;    // [kMaxTraceRounds + 1] per-round trace
-    // pull rounds: reverse CSR with int32 weights and its tile owners; a round pulls when its
+    // pull rounds: in-edge rows ordered by weight (in_rows.cu); a round pulls when its
     // (query, edge) relaxations exceed pull_min (~0: never); amask[b] holds the frontier's lanes per
-    // (vertex, word) of the rounds of parity b (zero elsewhere)
-    const int* row_r;
-    const int2* adj_rw;
-    const int* mark_r;
-    unsigned ntiles_r;
+    // (vertex, word) of the rounds of parity b (zero elsewhere); qmin the smallest distance that
+    // entered each query's frontier, by round slot
+    const int* in_row;
+    const int2* in_adj;
+    const int2* in_seg;
+    unsigned in_segs;
+    int in_shift;
     unsigned long long pull_min;
     unsigned* amask[2];
+    int* qmin;  // [3][Q]
 };
 
-// A warp's chunk of up to 32 in-edges of a pull round (batched SSSP and PPR), staged in shared memory: source, weight bits and
+// A warp's chunk of up to 32 in-edges of a pull round (batched PPR), staged in shared memory: source, weight bits and
 // the source's active lanes in the item's 4 query words.  Each lane loads one in-edge and
 // the live ones (a source with an active lane) are compacted into the chunk; the warp
 // then reads them one by one as broadcasts (two shared loads per in-edge instead of six
@@ -159,7 +162,8 @@ constexpr int kBatchUnroll = 4;  // relaxation items in flight per lane
 // faster than 2 x 512 (32 warps) at the same 4 items per lane (132-135 vs 140 ms for 256
 // sources at scale 22), 1 x 512 with 8-12 items (220 ms) and 6 x 256 (192 ms).
 constexpr int kSsspBatchThreads = 384;
-
+constexpr int kSsspBatchBlocksPerSm = 3;
+constexpr int kQminCap = 1024;  // query slots whose frontier minima are tracked (more: taken as 0)
 
 // Lane compaction of one owner run: the run's work is the items (edge ei, active-query
 // slot j) for ei in [0, len) and j in [0, cnt), numbered i = ei * cnt + j; lane l takes
@@ -193,124 +197,343 @@ __device__ __forceinline__ void owner_items(unsigned cnt, unsigned len, int lane
 
 // Pull round of the batched SSSP.  In a dense round (most (vertex, word) pairs improved in
 // the previous round) the expansion reads a 128-byte distance line per edge-word step and
-// issues red.min for every improvement.  A pull round walks the reverse CSR instead: for
-// each target v and query word it takes the minimum of dist[u] + w over the in-edges
-// u -> v whose source improved in the previous round (amask), lane by lane (lane = query),
-// then compares it with dist[v]: a target whose in-edges lie in one tile gets plain
-// stores of its improved lanes and of its next-round mask word; a target whose in-edges
-// cross a tile boundary gets atomicMin / atomicOr.  Items are (tile of 2^kPullTileLog
-// in-edges, group of 4 query words), in word-group-major order; a warp stages each chunk's
-// live in-edges (a source with an active lane in the item's words) in shared memory, as
-// the PPR pull does, and reads each live in-edge's source lines for the item's words.
+// issues red.min for every improvement.  A pull round reads in-edges instead: for each target
+// v and query word it takes the minimum of dist[u] + w over the in-edges u -> v whose source
+// improved in the previous round (amask), lane by lane (lane = query), and compares it with
+// dist[v].  The rows are ordered by weight, and v's row ends for a group of 4 query words at the
+// first edge whose weight is not below dist[v][q] - qmin[q] for any of its queries q (qmin: the
+// smallest distance in q's frontier): no later edge can improve v.  Without that bound a
+// pull read every live in-edge's lines, 11.3 ms per dense round of 256 queries at scale 22; most
+// rows now end within their first 4 edges: 8.0, 4.6, then 3.0 - 2.1 ms (distances of 4.3 GB
+// read once take 0.65).
+//
+// Items are (16 vertices, word group) and (4 segments of long rows, word group), in
+// word-group-major order.  A warp stages the first 4 in-edges of the 16 rows and their
+// sources' lanes (2 edges per lane, so 16 rows' loads are in flight together); a row that needs
+// more is read on in chunks of 32 edges.  Rows of up to kInHead edges have one writer and get
+// plain stores; longer rows are shared with their segments' warps and get atomics.  A row that
+// few queries have reached needs all its edges: with 32 rows an item and 128 edges before the
+// first segment, a warp that met 32 hubs took longer than the rest of the round (256 queries
+// at scale 19: 15.0 ms a batch, now 8.3; at scale 22 44.8 and 44.3).
 // Any order of relaxations reaches the same fixed point, so the distances are those of
 // the push rounds; pull and push rounds mix freely.
-__device__ __forceinline__ void sbatch_pull(const BatchParams& p, int buf, unsigned* qctr, PullChunk& pc,
-                                            long long& relax, int lane) {
-    const unsigned W = 1u << p.logW;
-    const int lg = p.logW >= 2 ? p.logW - 2 : 0;  // word groups per tile
-    const unsigned nitems = p.ntiles_r << lg;
-    const unsigned* am = p.amask[buf];
-    const unsigned tw = 1u << kPullTileLog;
+//
+// A warp holds 4 (row, word) slots at a time, lane = query: the 4 words of one row, or, with 1
+// or 2 words per vertex (WP), 4 or 2 rows, so that narrow batches have as many lines in
+// flight (31 queries on 685,230 vertices: 0.86 ms a round one row at a time, 0.42 ms four).
+struct SPullChunk {  // shared memory of one warp
+    int2* ed;        // [32] a chunk's live in-edges: source, weight
+    uint4* mk;       // [32] and their sources' active lanes in the item's words
+    int2* red;       // [16][4] first in-edges of 16 rows
+    uint4* rmk;      // [16][4]
+};
+
+template <int WP>
+__device__ __forceinline__ uint4 spull_lanes(const BatchParams& p, const unsigned* am, int u, unsigned w0) {
+    const unsigned* ms = am + ((size_t)(unsigned)u << p.logW) + w0;
+    if (WP == 4) return ldcg(reinterpret_cast<const uint4*>(ms));  // four words, 16-byte aligned
+    return make_uint4(ldcg(ms), WP > 1 ? ldcg(ms + 1) : 0u, 0u, 0u);
+}
+
+__device__ __forceinline__ bool any_lane(const uint4& m) { return (m.x | m.y | m.z | m.w) != 0u; }
+__device__ __forceinline__ unsigned word_of(const uint4& m, int j) {
+    return j == 0 ? m.x : j == 1 ? m.y : j == 2 ? m.z : m.w;
+}
+__device__ __forceinline__ int bucket_floor(int w, int shift) { return (w >> shift) << shift; }
+
+// Weights at or above the returned limit improve none of the warp's queries (cur: this lane's distances).
+template <int WP>
+__device__ __forceinline__ int spull_limit(const int* cur, const int* qm) {
+    int m = cur[0] - qm[0];
+#pragma unroll
+    for (int j = 1; j < WP; ++j) m = max(m, cur[j] - qm[j]);
+    return __reduce_max_sync(kFull, m);
+}
+
+// The source's distances of an in-edge (u, m: its active lanes), unreachable where inactive or !on.
+template <int WP>
+__device__ __forceinline__ void spull_line(const int* dist_w0, unsigned Qu, int u, const uint4& m, bool on, int lane,
+                                           int* d) {
+    const int* line = dist_w0 + (size_t)(unsigned)u * Qu;
+#pragma unroll
+    for (int j = 0; j < WP; ++j)  // L2-coherent: other warps lower distances during the round
+        d[j] = on && ((word_of(m, j) >> lane) & 1u) ? ldcg(line + 32 * j) : kInfDist;
+}
+
+// In-edges [b, e) of a row, 32 at a time, as long as they are below its limit.
+template <int WP>
+__device__ __forceinline__ void spull_chunks(const BatchParams& p, const unsigned* am, const int* dist_w0, unsigned w0,
+                                             const int* qm, int* cur, int lim, const SPullChunk& pc, int b, int e,
+                                             int lane) {
     const unsigned Qu = (unsigned)p.Q;
-    unsigned itn = next_tile(qctr, lane);
-    for (unsigned it = itn; it < nitems; it = itn) {
-        itn = next_tile(qctr, lane);  // the next item, fetched while this one runs
-        const unsigned t = it % p.ntiles_r;
-        const unsigned w0 = (it / p.ntiles_r) * 4u;
-        const unsigned e0 = t << kPullTileLog;
-        const unsigned e1 = min(e0 + tw, p.E);
-        int v = __ldg(p.mark_r + t);  // owner of in-edge e0
-        unsigned vs = (unsigned)__ldg(p.row_r + v);
-        for (;;) {
-            const unsigned ve = (unsigned)__ldg(p.row_r + v + 1);
-            const unsigned ea = max(vs, e0), ez = min(ve, e1);
-            if (ea < ez) {  // warp-uniform: v has in-edges in this tile
-                int mn[4] = {INT_MAX, INT_MAX, INT_MAX, INT_MAX};  // this lane's query in each word
-                for (unsigned b = ea; b < ez; b += 32u) {
-                    const unsigned e = b + (unsigned)lane;
-                    int src = 0, wt = 0;
-                    unsigned mk[4] = {0u, 0u, 0u, 0u};
-                    if (e < ez) {
-                        const int2 ed = __ldg(p.adj_rw + e);
-                        if ((unsigned)ed.x >= (unsigned)p.V) {
-                            atomicOr(&p.ctl->flags, C2G_FLAG_BOUNDS);
-                        } else {
-                            src = ed.x;
-                            wt = ed.y;
-                            const unsigned* ms = am + ((size_t)(unsigned)src << p.logW) + w0;
-                            if (W >= 4u) {  // four words, 16-byte aligned
-                                const uint4 m4 = ldcg(reinterpret_cast<const uint4*>(ms));
-                                mk[0] = m4.x;
-                                mk[1] = m4.y;
-                                mk[2] = m4.z;
-                                mk[3] = m4.w;
-                            } else {
+    for (; b < e; b += 32) {
+        int2 ed = make_int2(0, INT_MAX);
+        if (b + lane < e) ed = __ldg(p.in_adj + b + lane);
+        const unsigned below = __ballot_sync(kFull, bucket_floor(ed.y, p.in_shift) < lim);
+        if (below == 0u) return;
+        uint4 m = make_uint4(0u, 0u, 0u, 0u);
+        if (ed.y < lim) m = spull_lanes<WP>(p, am, ed.x, w0);
+        const bool live = any_lane(m);
+        const unsigned lm = __ballot_sync(kFull, live);
+        const unsigned n = (unsigned)__popc(lm);
+        __syncwarp();  // the previous chunk's reads are done
+        if (live) {
+            const unsigned at = (unsigned)__popc(lm & ((1u << lane) - 1u));
+            pc.ed[at] = ed;
+            pc.mk[at] = m;
+        }
+        __syncwarp();
+        for (unsigned k = 0; k < n; k += 2) {
+            int d[2][WP], w[2];
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    if ((unsigned)j < W) mk[j] = ldcg(ms + j);
-                            }
-                        }
-                    }
-                    // (query, edge) relaxations of the chunk, counted by lane 0
-                    const unsigned nrel = __reduce_add_sync(
-                        kFull, (unsigned)(__popc(mk[0]) + __popc(mk[1]) + __popc(mk[2]) + __popc(mk[3])));
-                    if (lane == 0) relax += (long long)nrel;
-                    const bool live = (mk[0] | mk[1] | mk[2] | mk[3]) != 0u;
-                    const unsigned lm = __ballot_sync(kFull, live);
-                    const unsigned n = (unsigned)__popc(lm);
-                    __syncwarp();  // the previous chunk's reads are done
-                    if (live) {
-                        const unsigned at = (unsigned)__popc(lm & ((1u << lane) - 1u));
-                        pc.ed[at] = make_int2(src, wt);
-                        pc.mk[at] = make_uint4(mk[0], mk[1], mk[2], mk[3]);
-                    }
-                    __syncwarp();
-                    for (unsigned k = 0; k < n; ++k) {
-                        // one in-edge's source lines, then its candidates (two in-edges in
-                        // flight measured slower: 93.8 vs 90.2 ms per 256-query batch)
-                        const int2 ek = pc.ed[k];
-                        const uint4 mq = pc.mk[k];
-                        int dv[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const unsigned mj = j == 0 ? mq.x : j == 1 ? mq.y : j == 2 ? mq.z : mq.w;
-                            // L2-coherent: other warps lower distances during the round
-                            dv[j] = ((mj >> lane) & 1u)
-                                        ? ldcg(p.dist + (size_t)(unsigned)ek.x * Qu + ((w0 + j) << 5) + lane)
-                                        : INT_MAX;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (dv[j] != INT_MAX) mn[j] = min(mn[j], dv[j] + ek.y);
-                    }
-                }
-                const bool whole = vs >= e0 && ve <= e1;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (w0 + j >= W) break;  // warp-uniform
-                    const size_t off = (size_t)(unsigned)v * Qu + ((w0 + j) << 5) + lane;
-                    const unsigned vw = ((unsigned)v << p.logW) + w0 + (unsigned)j;
-                    const bool imp = mn[j] != INT_MAX && mn[j] < ldcg(p.dist + off);
-                    const unsigned bits = __ballot_sync(kFull, imp);
-                    if (bits) {
-                        if (whole) {  // this warp holds all of v's in-edges: no other writer
-                            if (imp) p.dist[off] = mn[j];
-                            if (lane == 0) p.mask[vw] = bits;
-                        } else {
-                            if (imp) atomicMin(p.dist + off, mn[j]);
-                            if (lane == 0) atomicOr(p.mask + vw, bits);
-                        }
-                    }
-                }
+            for (int h = 0; h < 2; ++h) {
+                const unsigned kk = k + h < n ? k + h : k;
+                const int2 ek = pc.ed[kk];
+                w[h] = ek.y;
+                spull_line<WP>(dist_w0, Qu, ek.x, pc.mk[kk], ek.y < lim, lane, d[h]);
             }
-            if (ve >= e1) break;
-            ++v;
-            vs = ve;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int j = 0; j < WP; ++j) cur[j] = min(cur[j], d[h][j] + w[h]);
+            if ((k & 7u) == 6u) lim = spull_limit<WP>(cur, qm);
+        }
+        lim = spull_limit<WP>(cur, qm);
+        if (below != kFull) return;  // the chunk held the first edge beyond the limit
+    }
+}
+
+// The improved lanes of target v's words, d0: its distances when the row was started.
+template <int WP>
+__device__ __forceinline__ void spull_store(const BatchParams& p, int v, unsigned w0, bool whole, const int* d0,
+                                            const int* cur, int* qnew, int lane) {
+#pragma unroll
+    for (int j = 0; j < WP; ++j) {
+        const bool imp = cur[j] < d0[j];
+        const unsigned bits = __ballot_sync(kFull, imp);
+        if (bits == 0u) continue;
+        const size_t off = (size_t)(unsigned)v * (unsigned)p.Q + ((w0 + j) << 5) + lane;
+        const unsigned vw = ((unsigned)v << p.logW) + w0 + (unsigned)j;
+        if (imp) qnew[j] = min(qnew[j], cur[j]);
+        if (whole) {  // this warp reads all of v's in-edges: no other writer
+            if (imp) p.dist[off] = cur[j];
+            if (lane == 0) p.mask[vw] = bits;
+        } else {
+            if (imp) atomicMin(p.dist + off, cur[j]);
+            if (lane == 0) atomicOr(p.mask + vw, bits);
         }
     }
 }
 
-__global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(const BatchParams p) {
+template <int WP>
+__device__ __forceinline__ void sbatch_pull(const BatchParams& p, int buf, int slot, int nslot, unsigned* qctr,
+                                            const SPullChunk& pc, int lane) {
+    constexpr int RP = 4 / WP;  // rows at a time
+    const unsigned Qu = (unsigned)p.Q;
+    const unsigned nblk = ((unsigned)p.V + 15u) / 16u, per_group = nblk + (p.in_segs + 3u) / 4u;
+    const unsigned nitems = per_group << (WP == 4 ? p.logW - 2 : 0);
+    const unsigned* am = p.amask[buf];
+    unsigned w0 = ~0u;  // the word group of qm and qnew
+    int qm[WP], qnew[WP];
+    auto flush = [&]() {  // the group's smallest new distances join the next round's qmin
+        if (w0 == ~0u) return;
+#pragma unroll
+        for (int j = 0; j < WP; ++j) {
+            int* q = p.qmin + nslot * Qu + ((w0 + j) << 5) + lane;
+            if (qnew[j] < ldcg(q)) atomicMin(q, qnew[j]);
+        }
+    };
+    unsigned itn = next_tile(qctr, lane);
+    for (unsigned it = itn; it < nitems; it = itn) {
+        itn = next_tile(qctr, lane);  // the next item, fetched while this one runs
+        const unsigned grp = (it / per_group) * 4u;
+        if (grp != w0) {
+            flush();
+            w0 = grp;
+#pragma unroll
+            for (int j = 0; j < WP; ++j) {
+                const unsigned q = ((w0 + j) << 5) + (unsigned)lane;
+                // a query slot without a query never bounds a row
+                qm[j] = q < (unsigned)p.nq ? ldcg(p.qmin + slot * Qu + q) : INT_MAX;
+                qnew[j] = INT_MAX;
+            }
+        }
+        const int* dist_w0 = p.dist + (w0 << 5) + lane;
+        const unsigned k = it % per_group;
+        if (k >= nblk) {
+            // 4 segments: most hold no weight below their row's limit, so all limits are found first
+            const unsigned s0 = (k - nblk) * 4u;
+            int2 sg = make_int2(0, 0);
+            int w = INT_MAX, se = 0;
+            if (lane < 4 && s0 + lane < p.in_segs) {
+                sg = __ldg(p.in_seg + s0 + lane);
+                w = bucket_floor(__ldg(&p.in_adj[sg.y].y), p.in_shift);
+                se = min(sg.y + kInSegment, __ldg(p.in_row + sg.x + 1));
+            }
+            int d[4][WP];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned v = (unsigned)__shfl_sync(kFull, sg.x, q);
+#pragma unroll
+                for (int j = 0; j < WP; ++j) d[q][j] = ldcg(dist_w0 + (size_t)v * Qu + 32 * j);
+            }
+            unsigned live = 0u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (__shfl_sync(kFull, w, q) < spull_limit<WP>(d[q], qm)) live |= 1u << q;
+            while (live) {
+                const int q = __ffs(live) - 1;
+                live &= live - 1u;
+                const int v = __shfl_sync(kFull, sg.x, q);
+                int d0[WP], cur[WP];
+#pragma unroll
+                for (int j = 0; j < WP; ++j) cur[j] = d0[j] = ldcg(dist_w0 + (size_t)(unsigned)v * Qu + 32 * j);
+                spull_chunks<WP>(p, am, dist_w0, w0, qm, cur, spull_limit<WP>(cur, qm), pc, __shfl_sync(kFull, sg.y, q),
+                                 __shfl_sync(kFull, se, q), lane);
+                spull_store<WP>(p, v, w0, false, d0, cur, qnew, lane);
+            }
+            continue;
+        }
+        const int v0 = (int)(k * 16u);
+        int rs = 0, re = 0;
+        if (lane < 16 && v0 + lane < p.V) {
+            rs = __ldg(p.in_row + v0 + lane);
+            re = __ldg(p.in_row + v0 + lane + 1);
+        }
+        unsigned todo = __ballot_sync(kFull, rs < re);
+        if (todo == 0u) continue;
+        // the first 4 in-edges of 16 rows, two per lane, and their sources' active lanes
+        {
+            const int row = lane >> 1;
+            const int i = __shfl_sync(kFull, rs, row) + 2 * (lane & 1);
+            __syncwarp();
+            if ((todo >> row) & 1u) {
+                const int4 x = __ldg(reinterpret_cast<const int4*>(p.in_adj + i));
+                pc.red[2 * lane] = make_int2(x.x, x.y);
+                pc.red[2 * lane + 1] = make_int2(x.z, x.w);
+                const uint4 none = make_uint4(0u, 0u, 0u, 0u);  // the padding has no source
+                pc.rmk[2 * lane] = x.y != INT_MAX ? spull_lanes<WP>(p, am, x.x, w0) : none;
+                pc.rmk[2 * lane + 1] = x.w != INT_MAX ? spull_lanes<WP>(p, am, x.z, w0) : none;
+            }
+            __syncwarp();
+        }
+        while (todo) {
+            int row[RP], d0[RP][WP], cur[RP][WP], lim[RP];
+            bool valid[RP];
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                valid[r] = todo != 0u;  // warp-uniform
+                row[r] = valid[r] ? __ffs(todo) - 1 : row[0];
+                todo &= todo - 1u;
+#pragma unroll
+                for (int j = 0; j < WP; ++j)
+                    cur[r][j] = d0[r][j] =
+                        ldcg(dist_w0 + (size_t)(unsigned)(v0 + row[r]) * Qu + 32 * j);
+            }
+#pragma unroll
+            for (int r = 0; r < RP; ++r) lim[r] = spull_limit<WP>(cur[r], qm);
+#pragma unroll
+            for (int h0 = 0; h0 < 4; h0 += 2) {  // two in-edges of each row in flight
+                int d[2][RP][WP], w[2][RP];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) {
+                        const int2 e = pc.red[4 * row[r] + h0 + h];
+                        w[h][r] = e.y;
+                        spull_line<WP>(dist_w0, Qu, e.x, pc.rmk[4 * row[r] + h0 + h], e.y < lim[r], lane, d[h][r]);
+                    }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int r = 0; r < RP; ++r)
+#pragma unroll
+                        for (int j = 0; j < WP; ++j)  // (the padding's weight is no summand)
+                            if (d[h][r][j] != kInfDist) cur[r][j] = min(cur[r][j], d[h][r][j] + w[h][r]);
+            }
+            int pos[RP], end[RP];  // what is left of each row (of a long row's head)
+            bool more = false;
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                const int vrs = __shfl_sync(kFull, rs, row[r]), vre = __shfl_sync(kFull, re, row[r]);
+                pos[r] = vrs + 4;
+                end[r] = min(vre, vrs + kInHead);
+                if (!valid[r] || bucket_floor(pc.red[4 * row[r] + 3].y, p.in_shift) >= lim[r]) end[r] = pos[r];
+                more |= pos[r] < end[r];
+            }
+            if (RP == 1) {
+                if (more)
+                    spull_chunks<WP>(p, am, dist_w0, w0, qm, cur[0], spull_limit<WP>(cur[0], qm), pc, pos[0],
+                                     end[0], lane);
+            } else {
+                // the next 32 / RP in-edges of all rows at a time
+                constexpr int EP = 32 / RP;
+                while (more) {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) lim[r] = spull_limit<WP>(cur[r], qm);
+                    int my_pos = pos[0], my_end = end[0], my_lim = lim[0];
+#pragma unroll
+                    for (int r = 1; r < RP; ++r)
+                        if (lane / EP == r) {
+                            my_pos = pos[r];
+                            my_end = end[r];
+                            my_lim = lim[r];
+                        }
+                    int2 ed = make_int2(0, INT_MAX);
+                    if (my_pos + lane % EP < my_end) ed = __ldg(p.in_adj + my_pos + lane % EP);
+                    const unsigned below = __ballot_sync(kFull, bucket_floor(ed.y, p.in_shift) < my_lim);
+                    uint4 m = make_uint4(0u, 0u, 0u, 0u);
+                    if (ed.y < my_lim) m = spull_lanes<WP>(p, am, ed.x, w0);
+                    __syncwarp();  // the previous reads are done
+                    pc.ed[lane] = ed;
+                    pc.mk[lane] = m;
+                    __syncwarp();
+                    int n = 0;  // edges to read: up to the last one below its row's limit
+#pragma unroll
+                    for (int r = 0; r < RP; ++r)
+                        n = max(n, 32 - __clz((int)((below >> (r * EP)) & ((1u << EP) - 1u))));
+                    for (int h0 = 0; h0 < n; h0 += 2) {
+                        int d[2][RP][WP], w[2][RP];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int r = 0; r < RP; ++r) {
+                                const int2 e = pc.ed[r * EP + h0 + h];
+                                w[h][r] = e.y;
+                                spull_line<WP>(dist_w0, Qu, e.x, pc.mk[r * EP + h0 + h], true, lane, d[h][r]);
+                            }
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int r = 0; r < RP; ++r)
+#pragma unroll
+                                for (int j = 0; j < WP; ++j)
+                                    if (d[h][r][j] != kInfDist) cur[r][j] = min(cur[r][j], d[h][r][j] + w[h][r]);
+                    }
+                    more = false;
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) {
+                        pos[r] += EP;
+                        // a row goes on when all its staged edges were below the limit
+                        if (((below >> (r * EP)) & ((1u << EP) - 1u)) != ((1u << EP) - 1u)) end[r] = pos[r];
+                        more |= pos[r] < end[r];
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                if (!valid[r]) break;  // warp-uniform
+                const int len = __shfl_sync(kFull, re, row[r]) - __shfl_sync(kFull, rs, row[r]);
+                spull_store<WP>(p, v0 + row[r], w0, len <= kInHead, d0[r], cur[r], qnew, lane);
+            }
+        }
+    }
+    flush();
+}
+
+// WP: query words a pull takes at a time (1, 2, or 4 of four or more)
+template <int WP>
+__global__ void __launch_bounds__(kSsspBatchThreads, kSsspBatchBlocksPerSm) sssp_batch_persistent(const BatchParams p) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
     grid_sync_init();
@@ -321,12 +544,24 @@ __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(co
     const unsigned gwarp = gtid >> 5, nwarps = nthreads >> 5;
     const int W = 1 << p.logW;
     const unsigned Qu = (unsigned)p.Q;
-    __shared__ StageSmem sm;
+    __shared__ __align__(16) StageSmemN<kSsspBatchThreads / 32> sm;
     const int wib = threadIdx.x >> 5;
     unsigned long long tph = globaltimer_ns();
     WarpStage fst{sm.v0[wib], sm.d0[wib], sm.x0[wib], 0};
     int* qtab = sm.v1[wib];  // slot -> query position table of the owner being expanded
-    __shared__ PullChunk pcs[kSsspBatchThreads / 32];  // pull rounds' in-edge chunks
+    // pull rounds: in-edge chunks in the (empty) stage, 16 rows' first in-edges, new minima
+    __shared__ uint4 rmk[kSsspBatchThreads / 32][64];
+    __shared__ int qlow[kQminCap];
+    const SPullChunk pc{reinterpret_cast<int2*>(sm.v0[wib]), reinterpret_cast<uint4*>(sm.d0[wib]),
+                        reinterpret_cast<int2*>(sm.x0[wib]), rmk[wib]};
+    const bool may_pull = p.pull_min != ~0ull, low = may_pull && p.Q <= kQminCap;
+    if (may_pull && gtid < Qu) {
+        // round 1: no distance is below 0 (seeds and weights are not negative)
+        p.qmin[Qu + gtid] = 0;
+        p.qmin[gtid] = p.qmin[2 * Qu + gtid] = low ? INT_MAX : 0;
+    }
+    if (low)
+        for (unsigned q = threadIdx.x; q < Qu; q += blockDim.x) qlow[q] = INT_MAX;
 
     // An epoch of a resident batch starts from the state the previous epoch left: the
     // distances and the improvement masks (queries that joined since have their column
@@ -372,8 +607,8 @@ __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(co
             ctl->tilectr[(cur + 1) % 3] = 0u;
             ctl->pcount[(cur + 1) % 3] = 0ull;
         }
-        batch_sweep(p, batch_out(p, buf, slot), p.pull_min != ~0ull ? p.amask[buf] : nullptr, &ctl->pcount[slot], fst,
-                    gwarp, nwarps, lane);
+        batch_sweep(p, batch_out(p, buf, slot), may_pull ? p.amask[buf] : nullptr, &ctl->pcount[slot], fst, gwarp,
+                    nwarps, lane);
         if (!grid_sync(bar, flags, p.barrier_ns)) return;
         phase_mark(ctl->phase_ns, tph, 1);
         const unsigned long long c = ldcg(&ctl->qctr[slot]);
@@ -397,15 +632,19 @@ __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(co
             ctl->relaxed += T;
         }
 
-        if (p.pull_min != ~0ull) {
+        if (may_pull) {
             // The previous round's frontier leaves the pull lookup (the lookup of this round,
             // amask[buf], is the one a pull reads; the next round writes amask[buf ^ 1]).
             const unsigned Fp = min((unsigned)(ldcg(&ctl->qctr[(cur + 2) % 3]) >> 32), p.qcap);
             for (unsigned j = gtid; j < Fp; j += nthreads) p.amask[buf ^ 1][ldcg(p.q[buf ^ 1] + j).x] = 0u;
+            if (low && gtid < Qu) p.qmin[((cur + 2) % 3) * Qu + gtid] = INT_MAX;
         }
         if (pull) {
-            if (gtid == 0) steps += T;
-            sbatch_pull(p, buf, &ctl->tilectr[slot], pcs[wib], relax, lane);
+            if (gtid == 0) {
+                steps += T;
+                relax += (long long)ldcg(&ctl->pcount[slot]);
+            }
+            sbatch_pull<WP>(p, buf, slot, (cur + 1) % 3, &ctl->tilectr[slot], pc, lane);
         } else {
         // Phase 2: expand.  Warps take tiles of edge-word steps and walk owner runs: the
         // owner's row of distances is read once; its edges are read 32 at a time (one per
@@ -492,6 +731,7 @@ __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(co
                             if (nd < cd[u]) {
                                 atomicMin(dw + (size_t)(unsigned)ew[u].x * Qu + qq[u], nd);
                                 atomicOr(mrow + ((size_t)(unsigned)ew[u].x << p.logW), 1u << qq[u]);
+                                if (low && nd < qlow[(w << 5) + qq[u]]) atomicMin(&qlow[(w << 5) + qq[u]], nd);
                             }
                         }
                     });
@@ -500,6 +740,15 @@ __global__ void __launch_bounds__(kSsspBatchThreads, 3) sssp_batch_persistent(co
                 }
                 e0 = seg_end;
                 o += 32;
+            }
+        }
+        if (low) {  // the block's smallest new distances join the next round's qmin
+            __syncthreads();
+            int* q = p.qmin + ((cur + 1) % 3) * Qu;
+            for (unsigned i = threadIdx.x; i < Qu; i += blockDim.x) {
+                const int x = qlow[i];
+                if (x < ldcg(q + i)) atomicMin(q + i, x);
+                qlow[i] = INT_MAX;
             }
         }
         }
@@ -586,6 +835,12 @@ static int grid_blocks(const c2g_graph* g, int per_sm) {
     return b < 1 ? 1 : b;
 }
 
+static const void* sssp_batch_kernel(int logW) {
+    return logW == 0 ? (const void*)sssp_batch_persistent<1>
+         : logW == 1 ? (const void*)sssp_batch_persistent<2>
+                     : (const void*)sssp_batch_persistent<4>;
+}
+
 struct BatchWork {
     int* dist = nullptr;
     unsigned* mask = nullptr;
@@ -601,6 +856,7 @@ struct BatchWork {
     int* stage = nullptr;  // caller-layout copy for host output
     RoundTrace* trace = nullptr;
     unsigned* amask[2] = {nullptr, nullptr};  // pull rounds' lookups of the frontier's lanes
+    int* qmin = nullptr;                      // pull rounds: smallest distance of each query's frontier, 3 slots
     size_t seed_cap = 0;
     int Q = 0;
     int V = 0;
@@ -610,7 +866,7 @@ static void batch_free_work(BatchWork* w) {
     if (!w) return;
     void* ptrs[] = {w->dist, w->mask, w->q[0], w->q[1], w->qmask[0], w->qmask[1], w->mark[0], w->mark[1],
                     w->ctl, w->counters, w->src, w->seed_off, w->seed_v, w->seed_w, w->stage, w->trace,
-                    w->amask[0], w->amask[1]};
+                    w->amask[0], w->amask[1], w->qmin};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete w;
@@ -649,31 +905,47 @@ static int batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
     C2G_CUDA(cudaMalloc(&w->seed_w, sizeof(int) * w->seed_cap));
     C2G_CUDA(cudaMalloc(&w->trace, sizeof(RoundTrace) * (kMaxTraceRounds + 1)));
     for (int b = 0; b < 2; ++b) C2G_CUDA(cudaMalloc(&w->amask[b], sizeof(unsigned) * qcap));
+    C2G_CUDA(cudaMalloc(&w->qmin, sizeof(int) * 3 * (size_t)Q));
     w->Q = Q;
     w->V = g->V;
     return C2G_OK;
 }
 
-// The pull rounds of a batched SSSP launch (p.pull_min: (query, edge) relaxations of the
-// frontier above which a round pulls, ~0: never): they need the reverse CSR with int32 weights (a view uses its
-// base's, never builds it), whose arrays are set into p here, after they exist.  The pull
-// lookups start clear; a launch leaves the entries of its last rounds behind.
-static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, BatchParams& p) {
-    p.pull_min = ~0ull;
+// (query, edge) relaxations above which a round pulls: batch_pull_frac * E * Q, times the
+// batch's width factor.  A pull's cost is its pass over the V * W (vertex, word) lines, a push's its
+// relaxations, and a wide batch amortises the pass: measured (push only / 0.3 / 0.1 / 0.03 of
+// E * Q): scale 22, 256 queries 137 / 60.3 / 53.2 / 44.3 ms; 500,003 uniform vertices, 256 queries
+// 27.4 / 22.3 / 21.6 / 21.3; scale 19, 64 queries 5.0 / 3.5 / 3.0 / 3.2; 685,230 uniform vertices, 31
+// queries 5.1 / 5.2 / - / 5.8.  Below a million lines the warps with the longest rows outlast the
+// rest of a pull (60,001 vertices, 128 queries 1.33 / 1.69 / 1.75 / 1.98 ms): those batches expand
+// only, unless the caller set a fraction.
+constexpr size_t kPullMinLines = 1000000;
+
+static unsigned long long sssp_pull_min(const c2g_graph* g, int Q) {
     const float frac = g->sssp_cfg.batch_pull_frac;
-    if (!(frac >= 0.f) || g->E == 0) return C2G_OK;
-    if (!g->adj_rw) {
-        if (g->borrowed) return C2G_OK;
-        int rc = build_reverse_int(g);
-        if (rc) return rc;
-    }
-    if (!g->row_r || !g->adj_rw || !g->mark_r) return C2G_OK;
-    p.row_r = g->row_r;
-    p.adj_rw = g->adj_rw;
-    p.mark_r = g->mark_r;
+    const bool small = !g->sssp_cfg.batch_pull_set && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines;
+    if (!(frac >= 0.f) || small) return ~0ull;
+    const double width = Q <= 32 ? 1.0 : Q <= 64 ? 1.0 / 3.0 : 0.1;
+    return (unsigned long long)((double)frac * width * (double)g->E * (double)Q);
+}
+
+// The pull rounds of a batched SSSP launch (p.pull_min: (query, edge) relaxations of the
+// frontier above which a round pulls, ~0: never): they need the graph's in-edge rows, and
+// seeds that are not below zero (the frontier minima start at 0).  The pull
+// lookups start clear; a launch leaves the entries of its last rounds behind.
+static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchParams& p) {
+    p.pull_min = ~0ull;
+    const unsigned long long pull_min = sssp_pull_min(g, Q);
+    if (pull_min == ~0ull || !g->in_adj || (seeds && g->hw_negative)) return C2G_OK;
+    p.in_row = g->in_row;
+    p.in_adj = g->in_adj;
+    p.in_seg = g->in_seg;
+    p.in_segs = g->in_segs;
+    p.in_shift = g->in_shift;
+    p.qmin = w->qmin;
     for (int b = 0; b < 2; ++b)
         C2G_CUDA(cudaMemsetAsync(w->amask[b], 0, sizeof(unsigned) * (size_t)g->V * (size_t)(Q / 32), g->stream));
-    p.pull_min = (unsigned long long)((double)frac * (double)g->E * (double)Q);
+    p.pull_min = pull_min;
     return C2G_OK;
 }
 
@@ -707,10 +979,12 @@ static void sssp_batch_params(c2g_graph* g, BatchWork* w, int Q, int logW, Batch
     p.epoch_rounds = 0;
     p.trace = w->trace;
     g->last_trace = w->trace;
-    p.row_r = nullptr;  // set by sssp_pull_setup when the launch may pull
-    p.adj_rw = nullptr;
-    p.mark_r = nullptr;
-    p.ntiles_r = (unsigned)(((size_t)g->E + (1u << kPullTileLog) - 1) >> kPullTileLog);
+    p.in_row = nullptr;  // set by sssp_pull_setup when the launch may pull
+    p.in_adj = nullptr;
+    p.in_seg = nullptr;
+    p.in_segs = 0u;
+    p.in_shift = 0;
+    p.qmin = nullptr;
     p.pull_min = ~0ull;
     p.amask[0] = w->amask[0];
     p.amask[1] = w->amask[1];
@@ -760,7 +1034,7 @@ int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const st
     int coop = 0, per_sm = 0;
     C2G_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
     if (!coop) return fail(C2G_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_persistent, kSsspBatchThreads, 0));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(logW), kSsspBatchThreads, 0));
     if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
 
     C2G_CUDA(cudaMemcpyAsync(w->src, sources, sizeof(int) * (size_t)nq, cudaMemcpyHostToDevice, g->stream));
@@ -774,7 +1048,7 @@ int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const st
     }
     BatchParams p;
     sssp_batch_params(g, w, Q, logW, p);
-    if ((rc = sssp_pull_setup(g, w, Q, p))) return rc;
+    if ((rc = sssp_pull_setup(g, w, Q, seed_off != nullptr, p))) return rc;
     p.nq = nq;
     p.seed_off = seed_off ? w->seed_off : nullptr;
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
@@ -782,7 +1056,7 @@ int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const st
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
     const int blocks = grid_blocks(g, per_sm);
-    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_batch_persistent, dim3(blocks), dim3(kSsspBatchThreads),
+    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(logW), dim3(blocks), dim3(kSsspBatchThreads),
                                          args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     return sssp_batch_results(g, w, Q, nq, out, out_on_device, query_major, ms, counters, ctl_out);
@@ -810,18 +1084,18 @@ int sssp_batch_epoch(c2g_graph* g, int Q, int rounds, float* ms, long long* coun
     int logW = 0;
     while ((32 << logW) < Q) ++logW;
     int per_sm = 0;
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_persistent, kSsspBatchThreads, 0));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(logW), kSsspBatchThreads, 0));
     if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
     BatchParams p;
     sssp_batch_params(g, w, Q, logW, p);
     int rc;
-    if ((rc = sssp_pull_setup(g, w, Q, p))) return rc;
+    if ((rc = sssp_pull_setup(g, w, Q, false, p))) return rc;
     p.epoch_rounds = rounds < 1 ? 1 : rounds;
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)sssp_batch_persistent, dim3(grid_blocks(g, per_sm)),
+    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(logW), dim3(grid_blocks(g, per_sm)),
                                          dim3(kSsspBatchThreads), args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     C2G_CUDA(cudaMemcpyAsync(ctl_out, w->ctl, sizeof(TraversalCtl), cudaMemcpyDeviceToHost, g->stream));

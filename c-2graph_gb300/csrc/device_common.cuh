@@ -287,13 +287,15 @@ __device__ __forceinline__ void list_stage_push(WarpStage& st, int* list, unsign
     st.n += cnt;
 }
 
-// Shared-memory backing for two stages per warp (512-thread blocks: 16 warps).
-struct StageSmem {
-    int v0[16][kStageCap];
-    int d0[16][kStageCap];
-    float x0[16][kStageCap];
-    int v1[16][kStageCap];
+// Shared-memory backing for two stages per warp of a block (512-thread blocks: 16 warps).
+template <int kWarps>
+struct StageSmemN {
+    int v0[kWarps][kStageCap];
+    int d0[kWarps][kStageCap];
+    float x0[kWarps][kStageCap];
+    int v1[kWarps][kStageCap];
 };
+using StageSmem = StageSmemN<16>;
 
 // Stage backing for the push kernels: FP64 values instead of 32-bit ones.
 struct StageSmemD {

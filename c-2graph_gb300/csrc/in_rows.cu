@@ -30,6 +30,7 @@ constexpr int kScanItems = 4;  // rows per thread of a scan block
 struct InStats {
     int wmin, wmax;
     unsigned n_long;             // rows longer than a warp
+    unsigned n_seg;              // segments of rows longer than kInHead
     unsigned long long padded;   // padded edges of all rows
 };
 
@@ -131,6 +132,8 @@ __global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restri
     for (int k = 0; k < kScanItems; ++k) {
         const int v = base + k;
         const bool lng = v < V && d[k] > 32;
+        if (v < V && padded4(d[k]) > kInHead)
+            atomicAdd(&st->n_seg, (unsigned)(padded4(d[k]) - kInHead + kInSegment - 1) / kInSegment);
         if (v < V) {
             row[v] = at;
             cursor[v] = at;
@@ -138,6 +141,19 @@ __global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restri
         at += padded4(d[k]);
         if (v == V - 1) row[V] = at;
         list_push(longs, &st->n_long, (unsigned)V, reinterpret_cast<int*>(&st->n_long), lng, v);
+    }
+}
+
+// The parts of long rows behind their first kInHead edges, kInSegment edges each: (vertex, first edge).
+__global__ void in_segments(const int* __restrict__ row, const int* __restrict__ longs, unsigned n_long,
+                            unsigned* __restrict__ ctr, unsigned n_seg, int2* __restrict__ seg) {
+    const unsigned stride = gridDim.x * blockDim.x;
+    for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n_long; r += stride) {
+        const int v = __ldg(longs + r), re = __ldg(row + v + 1);
+        const int first = __ldg(row + v) + kInHead;
+        if (first >= re) continue;
+        unsigned at = atomicAdd(ctr, (unsigned)(re - first + kInSegment - 1) / kInSegment);
+        for (int i = first; i < re && at < n_seg; i += kInSegment) seg[at++] = make_int2(v, i);
     }
 }
 
@@ -246,9 +262,11 @@ __global__ void __launch_bounds__(kInSortThreads) in_sort_long(const int* __rest
 }  // namespace
 
 void in_rows_free(c2g_graph* g) {
-    for (void* p : {(void*)g->in_row, (void*)g->in_adj})
+    for (void* p : {(void*)g->in_row, (void*)g->in_adj, (void*)g->in_seg})
         if (p) cudaFree(p);
     g->in_row = nullptr;
+    g->in_seg = nullptr;
+    g->in_segs = 0;
     g->in_adj = nullptr;
 }
 
@@ -271,7 +289,7 @@ int build_in_rows(c2g_graph* g) {
     InStats* st = reinterpret_cast<InStats*>(tmp);
     int* indeg = reinterpret_cast<int*>(tmp + 256);
     int *cursor = indeg + V, *longs = cursor + V, *sums = longs + V;
-    InStats h{INT_MAX, INT_MIN, 0u, 0ull};
+    InStats h{INT_MAX, INT_MIN, 0u, 0u, 0ull};
     const int blocks = g->num_sms * 8;
     e = cudaMemsetAsync(indeg, 0, sizeof(int) * V, g->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, g->stream);
@@ -304,8 +322,18 @@ int build_in_rows(c2g_graph* g) {
             in_sort_long<<<blocks, kInSortThreads, 0, g->stream>>>(g->in_row, indeg, longs, h.n_long, shift, raw,
                                                                   g->in_adj);
             e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
         }
+        if (e == cudaSuccess && h.n_seg) {
+            fits = cudaMalloc(&g->in_seg, sizeof(int2) * (size_t)h.n_seg) == cudaSuccess;
+            if (!fits) cudaGetLastError();
+            if (fits) e = cudaMemsetAsync(&st->n_long, 0, sizeof(unsigned), g->stream);
+            if (fits && e == cudaSuccess) {
+                in_segments<<<blocks, 256, 0, g->stream>>>(g->in_row, longs, h.n_long, &st->n_long, h.n_seg, g->in_seg);
+                e = cudaGetLastError();
+            }
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+        g->in_segs = h.n_seg;
         g->in_shift = shift;
         g->in_edges = (int64_t)h.padded;
     }

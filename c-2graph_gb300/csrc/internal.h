@@ -105,8 +105,10 @@ struct SsspConfig {
     int max_iter = 1 << 20;
     int batch_tile_big_log = 9;  // batched expansion: 512 edge-word steps per big tile
     int batch_tile_min_log = 4;  // ... in rounds with at least 16 big tiles per warp
-    float batch_pull_frac = 0.3f;  // batched rounds with more (query, edge) relaxations than this * E * Q
-                                   // pull over the reverse CSR (< 0: never)
+    // batched rounds with more (query, edge) relaxations than this * E * Q, scaled by the batch's width
+    // (batch.cu), pull over the in-edge rows (< 0: never); until it is set, small batches never pull
+    float batch_pull_frac = 0.3f;
+    bool batch_pull_set = false;
 };
 
 struct PprConfig {
@@ -117,6 +119,8 @@ struct PprConfig {
 };
 
 constexpr int kInMaxWeight = 147483648;  // largest weight of in-edge rows: unreachable + weight fits an int32
+
+constexpr int kInHead = 32, kInSegment = 256;  // edges; multiples of 32
 
 constexpr int kPullTileLog = 8;  // in-edges per pull tile (reverse-CSR markers)
 
@@ -137,12 +141,12 @@ struct c2g_graph {
     int2* adj_f = nullptr;
     int32_t* row_r = nullptr;  // reverse CSR with float weights (pull rounds, adjoint), on demand
     int2* adj_r = nullptr;
-    int2* adj_rw = nullptr;     // the same in-edges with int32 weights (batched SSSP pull rounds), on
-                                // demand; adj_r itself when the graph has no float weights
     // in-edge rows ordered by weight (in_rows.cu), or null: the graph's SSSP queries push only
     int32_t* in_row = nullptr;  // [V+1], multiples of 4
     int2* in_adj = nullptr;     // (source, weight), padded with weight INT_MAX
     int64_t in_edges = 0;       // padded edges
+    int2* in_seg = nullptr;     // (vertex, first edge): rows behind their first kInHead edges, kInSegment edges each
+    unsigned in_segs = 0;
     int in_shift = 0;           // weights are ordered up to their low in_shift bits
     int32_t* mark_r = nullptr;  // pull-tile owner markers over row_r
     int32_t* mark_f = nullptr;  // pull-tile owner markers over row (pulls on the reverse graph)
@@ -207,8 +211,6 @@ void ads_free(c2g_graph* g);
 int build_reverse_graph(c2g_graph* g);
 int build_in_rows(c2g_graph* g);
 void in_rows_free(c2g_graph* g);
-// The reverse CSR's in-edges with int32 weights (batched SSSP pull rounds).
-int build_reverse_int(c2g_graph* g);
 // Reverse CSR and the weight statistics of the batched pull rounds (once per weights).
 int ppr_pull_prepare(c2g_graph* g);
 int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g_ppr_params& prm,

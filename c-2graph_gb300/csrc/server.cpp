@@ -282,8 +282,6 @@ int c2g_server_create(c2g_graph* g, const float* p_inj, const float* p_cont, con
     {
         std::lock_guard<std::mutex> lk(g->mu);
         if (g->adj_f) rc = ppr_pull_prepare(g);
-        // the batched SSSP's pull rounds: the views share the base's reverse CSR
-        if (!rc && g->adj_w && g->sssp_cfg.batch_pull_frac >= 0.f) rc = build_reverse_int(g);
     }
     for (int k = 0; k < 3 && !rc; ++k) {
         rc = graph_view(g, &s->views[k]);

@@ -217,10 +217,13 @@ int c2g_sssp_batch_get_tile(const c2g_graph* g, int32_t* big_steps, int32_t* min
 
 /* Round shape of the batched SSSP (c2g_sssp_batch and resident SSSP batches; no
  * counterpart in the reference): a round whose frontier makes more than frac * E * Q
- * (query, edge) relaxations (Q = query slots, a multiple of 32) pulls over the reverse
- * CSR with int32 weights (built on first use): each target takes the minimum over its
- * in-edges from sources that improved in the previous round.  frac < 0: expand (push)
- * only; 0: pull every round; default 0.3.  Distances do not depend on the setting. */
+ * (query, edge) relaxations (Q = query slots, a multiple of 32; a third of that for 64
+ * slots, a tenth for more) pulls: each target takes the minimum over its in-edges from
+ * sources that improved in the previous round, in ascending order of weight up to the
+ * first that cannot improve any query of the word.  frac < 0: expand (push) only; 0: pull
+ * every round; default 0.3, and until it is set a batch with fewer than a million (vertex,
+ * 32-query word) pairs expands only.  Graphs with a weight below 0 or above 147483648
+ * always expand.  Distances do not depend on the setting. */
 int c2g_sssp_batch_set_pull(c2g_graph* g, float frac);
 int c2g_sssp_batch_get_pull(const c2g_graph* g, float* frac);
 
