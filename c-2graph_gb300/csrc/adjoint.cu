@@ -18,28 +18,6 @@
 
 namespace c2g {
 
-// In-degree count over the forward CSR.
-__global__ void count_in_kernel(const int2* __restrict__ adj, long long E, int* __restrict__ indeg) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride)
-        atomicAdd(indeg + adj[e].x, 1);
-}
-
-// Scatter every forward edge u->v (weight bits) into v's in-edge row as (u, weight).
-__global__ void scatter_in_kernel(const int* __restrict__ row, const int2* __restrict__ adj, int V,
-                                  int* __restrict__ cursor, int2* __restrict__ adj_r) {
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int u = warp; u < V; u += nwarps) {
-        for (int e = row[u] + lane; e < row[u + 1]; e += 32) {
-            const int2 ew = adj[e];
-            const int pos = atomicAdd(cursor + ew.x, 1);
-            adj_r[pos] = make_int2(u, ew.y);
-        }
-    }
-}
-
 // grad[e] = c * pi[u] * lambda[col[e]] for every forward edge e = (u -> col[e]).  Warps
 // take tiles of 2^kPullTileLog edges; a tile's first owner comes from the forward tile
 // markers (one load), the next 32 owners' row bounds and pi values one per lane, and each
@@ -99,51 +77,6 @@ __global__ void adjoint_grad_kernel(const int* __restrict__ row, const int2* __r
     }
 }
 
-// Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), built once.
-int build_reverse_graph(c2g_graph* g) {
-    if (g->adj_r) return C2G_OK;
-    const int2* fwd = g->adj_f ? g->adj_f : g->adj_w;  // float weights when the graph has them
-    if (!fwd) return fail(C2G_ERR_UNSUPPORTED, "graph has no edge weights");
-    const size_t V = (size_t)g->V, E = (size_t)g->E;
-    int* indeg = nullptr;
-    C2G_CUDA(cudaMalloc(&g->row_r, sizeof(int) * (V + 1)));
-    C2G_CUDA(cudaMalloc(&g->adj_r, sizeof(int2) * (E ? E : 1)));
-    C2G_CUDA(cudaMalloc(&indeg, sizeof(int) * (V ? V : 1)));
-    cudaError_t e = cudaMemsetAsync(indeg, 0, sizeof(int) * V, g->stream);
-    if (e == cudaSuccess && E) {
-        count_in_kernel<<<g->num_sms * 4, 256, 0, g->stream>>>(fwd, (long long)E, indeg);
-        e = cudaGetLastError();
-    }
-    std::vector<int> h(V + 1, 0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h.data() + 1, indeg, sizeof(int) * V, cudaMemcpyDeviceToHost, g->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    for (size_t v = 0; v < V; ++v) h[v + 1] += h[v];
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(g->row_r, h.data(), sizeof(int) * (V + 1), cudaMemcpyHostToDevice, g->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(indeg, h.data(), sizeof(int) * V, cudaMemcpyHostToDevice, g->stream);
-    if (e == cudaSuccess && E) {
-        scatter_in_kernel<<<g->num_sms * 4, 256, 0, g->stream>>>(g->row, fwd, g->V, indeg, g->adj_r);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cudaFree(indeg);
-    C2G_CUDA(e);
-    int rc = build_markers(g, g->row_r, &g->mark_r);
-    if (!rc) rc = build_markers(g, g->row, &g->mark_f);
-    return rc;
-}
-
-void adjoint_free(c2g_graph* g) {
-    void* ptrs[] = {g->row_r, g->adj_r, g->mark_r, g->mark_f};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
-    g->wstat_valid = false;
-    g->row_r = nullptr;
-    g->adj_r = nullptr;
-    g->mark_r = nullptr;
-    g->mark_f = nullptr;
-}
-
 int set_float_weights(c2g_graph* g, const float* w, int on_device);
 
 }  // namespace c2g
@@ -189,7 +122,7 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
         }
     } scope(g->device);
     int rc = build_reverse_graph(g);
-    if (rc) return rc;
+    if (rc || (rc = build_row_lists(g, g->row, g->row_r, &g->rows_out))) return rc;
     const size_t V = (size_t)g->V, E = (size_t)g->E;
     float *pi = nullptr, *lam = nullptr, *dgrad = nullptr, *dtr = nullptr;
     int32_t* dtv = nullptr;
@@ -219,7 +152,7 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
     c2g_ppr_params fp = *params;
     fp.r0 = 1.0f;
     fp.pr0 = fp.alpha;
-    rc = ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->mark_r, source, fp, fp.alpha, 0, nullptr,
+    rc = ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->rows_in, source, fp, fp.alpha, 0, nullptr,
                          nullptr, nullptr, nullptr, 0, pi, nullptr, &ms_f);
     if (!rc && (cudaMemcpyAsync(&cf, g->ppr.ctl, sizeof(cf), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
                 cudaStreamSynchronize(g->stream) != cudaSuccess))
@@ -228,7 +161,7 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
     c2g_ppr_params bp = *params;
     bp.rmax = rmax_backward;
     if (!rc)
-        rc = ppr_launch_view(g, g->row_r, g->adj_r, g->row, g->adj_f, g->mark_f, tv[0], bp, 1.0f, (int32_t)tv.size(),
+        rc = ppr_launch_view(g, g->row_r, g->adj_r, g->row, g->adj_f, g->rows_out, tv[0], bp, 1.0f, (int32_t)tv.size(),
                              dtv, dtr, nullptr, nullptr, 0, lam, nullptr, &ms_b);
     if (!rc && (cudaMemcpyAsync(&cb, g->ppr.ctl, sizeof(cb), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
                 cudaStreamSynchronize(g->stream) != cudaSuccess))

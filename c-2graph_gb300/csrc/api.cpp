@@ -14,7 +14,6 @@ namespace c2g {
 
 int build_adj(c2g_graph* g, const int32_t* col, const int32_t* w, int2** out);
 int stream_graph(c2g_graph* g, const std::string& elist_path, const std::string* w_path, const std::string* f_path);
-void adjoint_free(c2g_graph* g);
 
 static const int kNoSidecar = -2;
 
@@ -28,7 +27,7 @@ static void graph_release(c2g_graph* g) {
     batch_free(g);
     ppr_batch_free(g);
     ads_free(g);
-    if (!g->borrowed) adjoint_free(g);
+    if (!g->borrowed) reverse_free(g);
     if (!g->borrowed) in_rows_free(g);
     if (!g->borrowed) {
         void* ptrs[] = {g->row, g->adj_w, g->adj_f, g->hv, g->he, g->hw, g->rec_of_vertex};
@@ -95,6 +94,14 @@ static int graph_fill(c2g_graph* g, const std::vector<int32_t>& vlist, const int
     if (wlist && (rc = build_adj(g, elist, wlist, &g->adj_w))) return rc;
     if (flist && (rc = build_adj(g, elist, reinterpret_cast<const int32_t*>(flist), &g->adj_f))) return rc;
     return C2G_OK;
+}
+
+// The in-edge structures of the weights the graph has.  A graph made without room for the reverse CSR
+// builds it when a call needs it, and fails there.
+static int build_in_edges(c2g_graph* g) {
+    int rc = build_in_rows(g);
+    if (!rc && g->adj_f && build_reverse_graph(g) == C2G_ERR_CUDA) rc = C2G_ERR_CUDA;
+    return rc;
 }
 
 static int records_fill(c2g_graph* g, int32_t R, const int32_t* hv, const int32_t* he, const void* hw, bool hw_float,
@@ -223,6 +230,7 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->adj_r = base->adj_r;
     g->mark_r = base->mark_r;
     g->mark_f = base->mark_f;
+    g->rows_in = base->rows_in;
     g->in_row = base->in_row;
     g->in_adj = base->in_adj;
     g->in_edges = base->in_edges;
@@ -286,7 +294,7 @@ int c2g_graph_create(int device, int32_t V, int64_t E, const int32_t* vlist, con
     c2g_graph* g = nullptr;
     if ((rc = graph_new(device, &g))) return rc;
     DeviceScope ds(device);
-    if ((rc = graph_fill(g, vl, elist, E, wlist, flist)) || (rc = build_in_rows(g))) {
+    if ((rc = graph_fill(g, vl, elist, E, wlist, flist)) || (rc = build_in_edges(g))) {
         graph_release(g);
         return rc;
     }
@@ -350,7 +358,7 @@ int c2g_graph_load(const char* dir, int variant, int device, c2g_graph** out) {
     DeviceScope ds(device);
     if ((rc = graph_fill_rows(g, vlist)) ||
         (rc = stream_graph(g, d + "elist.bin", wpath.empty() ? nullptr : &wpath, fpath.empty() ? nullptr : &fpath)) ||
-        (rc = build_in_rows(g))) {
+        (rc = build_in_edges(g))) {
         graph_release(g);
         return rc;
     }
@@ -460,6 +468,7 @@ int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div) {
     if (pull_div < 0 || dense_div < 0) return fail(C2G_ERR_ARG, "pull_div and dense_div must be >= 0");
     std::lock_guard<std::mutex> lk(g->mu);
     g->ppr_cfg.pull_div = pull_div;
+    g->ppr_cfg.pull_set = true;
     g->ppr_cfg.dense_div = dense_div;
     return C2G_OK;
 }

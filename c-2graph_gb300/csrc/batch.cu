@@ -57,7 +57,7 @@ struct BatchParams {
     int tile_min_log;     // a round walks big tiles when it has >= 2^tile_min_log of them per warp
     int epoch_rounds;     // > 0: an epoch of a resident batch (no initialisation; at most this many rounds)
     RoundTrace* trace;    // [kMaxTraceRounds + 1] per-round trace
-    // pull rounds: in-edge rows ordered by weight (in_rows.cu); a round pulls when its
+    // pull rounds: in-edge rows ordered by weight (in_edges.cu); a round pulls when its
     // (query, edge) relaxations exceed pull_min (~0: never); amask[b] holds the frontier's lanes per
     // (vertex, word) of the rounds of parity b (zero elsewhere); qmin the smallest distance that
     // entered each query's frontier, by round slot

@@ -72,10 +72,7 @@ __global__ void set_weight_bits_kernel(int2* __restrict__ adj, const int* __rest
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) adj[e].y = w[e];
 }
 
-void adjoint_free(c2g_graph* g);
-
-// Replace the float edge weights (flist order) of a graph in place; the reverse CSR
-// built for the adjoint is dropped and rebuilt on next use.
+// Replace the float edge weights (flist order) of a graph in place, and in its reverse CSR.
 int set_float_weights(c2g_graph* g, const float* w, int on_device) {
     if (!g->adj_f) return fail(C2G_ERR_UNSUPPORTED, "graph has no float weights to replace");
     const size_t E = (size_t)g->E;
@@ -96,8 +93,7 @@ int set_float_weights(c2g_graph* g, const float* w, int on_device) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (tmp) cudaFree(tmp);
     C2G_CUDA(e);
-    adjoint_free(g);
-    return C2G_OK;
+    return refresh_reverse_graph(g);
 }
 
 }  // namespace c2g

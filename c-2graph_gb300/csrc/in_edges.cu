@@ -1,19 +1,21 @@
-// In-edge rows of a graph with int32 weights, ordered by weight: the layout of the SSSP
-// pull rounds (sssp.cu, batch.cu).
+// In-edges of a graph, built on the device: rows ordered by int32 weight for the SSSP pull
+// rounds (sssp.cu, batch.cu), and the reverse CSR with float weights and its rows by length for
+// the push kernels' pull rounds (ppr.cu, batch.cu, adsorption.cu, adjoint.cu).
 //
-// Row v holds v's in-edges (source, weight) in ascending order of weight, padded with
+// Rows ordered by weight: row v holds v's in-edges (source, weight) in ascending order of weight, padded with
 // (0, INT_MAX) to a multiple of 4 edges, so that a row is read in aligned 32-byte groups and
 // a reader can stop at the first group whose weights cannot improve v any more.  The
 // reference has no in-edges; it relaxes out-edges only (src/sssp/purn/Main.cu:236-331).
 //
-// Built on the device when the graph is made (its int32 weights never change): count the
-// in-edges, scan the padded row lengths, scatter the edges into their rows, order each row.
+// They are built when the graph is made (its int32 weights never change): count the in-edges,
+// scan the padded row lengths, scatter the edges into their rows, order each row.
 // Rows of up to 32 edges are ordered by a warp (bitonic network on weight and source), longer
 // ones by a block (counting sort over kInBuckets buckets of weight).  A bucket spans 2^shift
 // weights, where 2^shift * kInBuckets covers the largest weight; inside a bucket the order is
 // free, so a reader compares with the bucket's lower end, (w >> shift) << shift.  Each step is
 // bound by scattered 8-byte accesses: at scale 22 (65M edges) making the graph from host
 // arrays takes 68.2 ms with the rows and 63.5 ms without.
+#include <algorithm>
 #include <climits>
 
 #include "device_common.cuh"
@@ -52,6 +54,7 @@ __global__ void in_count(const int2* __restrict__ adj, unsigned E, int* __restri
 }
 
 __device__ __forceinline__ int padded4(int n) { return (n + 3) & ~3; }
+__device__ __forceinline__ int padded(int n, int pad) { return pad ? padded4(n) : n; }
 
 // Exclusive sum over the block of one int per thread; *total (all threads) gets the block's sum.
 __device__ __forceinline__ int block_exclusive(int x, int* total) {
@@ -84,14 +87,14 @@ __device__ __forceinline__ int block_exclusive(int x, int* total) {
     return r;
 }
 
-// Padded edges of each scan block's rows (their sum may pass 2^31: st->padded).
-__global__ void __launch_bounds__(kScanThreads) in_scan_blocks(const int* __restrict__ indeg, int V,
+// Edges (padded to 4 when pad) of each scan block's rows (the padded sum may pass 2^31: st->padded).
+__global__ void __launch_bounds__(kScanThreads) in_scan_blocks(const int* __restrict__ indeg, int V, int pad,
                                                               int* __restrict__ block_sum, InStats* st) {
     const int base = (int)blockIdx.x * kScanThreads * kScanItems;
     int n = 0;
     for (int k = 0; k < kScanItems; ++k) {
         const int v = base + k * kScanThreads + (int)threadIdx.x;
-        if (v < V) n += padded4(__ldg(indeg + v));
+        if (v < V) n += padded(__ldg(indeg + v), pad);
     }
     int total;
     block_exclusive(n, &total);
@@ -114,8 +117,8 @@ __global__ void __launch_bounds__(kScanThreads) in_scan_sums(int* __restrict__ b
     }
 }
 
-// Row starts, the scatter's cursors and the list of rows longer than a warp.
-__global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restrict__ indeg, int V,
+// Row starts, the scatter's cursors and, when padded, the list of rows longer than a warp.
+__global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restrict__ indeg, int V, int pad,
                                                             const int* __restrict__ block_sum, int* __restrict__ row,
                                                             int* __restrict__ cursor, int* __restrict__ longs,
                                                             InStats* st) {
@@ -124,23 +127,23 @@ __global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restri
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         d[k] = base + k < V ? __ldg(indeg + base + k) : 0;
-        n += padded4(d[k]);
+        n += padded(d[k], pad);
     }
     int total;
     int at = block_sum[blockIdx.x] + block_exclusive(n, &total);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const int v = base + k;
-        const bool lng = v < V && d[k] > 32;
-        if (v < V && padded4(d[k]) > kInHead)
+        const bool lng = pad && v < V && d[k] > 32;
+        if (lng && padded4(d[k]) > kInHead)
             atomicAdd(&st->n_seg, (unsigned)(padded4(d[k]) - kInHead + kInSegment - 1) / kInSegment);
         if (v < V) {
             row[v] = at;
             cursor[v] = at;
         }
-        at += padded4(d[k]);
+        at += padded(d[k], pad);
         if (v == V - 1) row[V] = at;
-        list_push(longs, &st->n_long, (unsigned)V, reinterpret_cast<int*>(&st->n_long), lng, v);
+        if (pad) list_push(longs, &st->n_long, (unsigned)V, reinterpret_cast<int*>(&st->n_long), lng, v);
     }
 }
 
@@ -259,7 +262,193 @@ __global__ void __launch_bounds__(kInSortThreads) in_sort_long(const int* __rest
     }
 }
 
+// Class of a row of n edges (RowLists).
+__device__ __forceinline__ int row_class(int n) {
+    int c = 0;
+#pragma unroll
+    for (int k = 1; k < kRowClasses; ++k)
+        if (n <= ((32 * kLaneEdges) >> (k - 1))) c = k;
+    return c;
+}
+
+struct ClassCount {
+    unsigned n[kRowClasses];  // records
+    unsigned n_long;          // rows of class 0
+};
+
+// Records per class (fill = false), or the records themselves, appended from `at` on.
+template <bool kFill>
+__global__ void __launch_bounds__(256) row_classes(const int* __restrict__ row, const int* __restrict__ other, int V,
+                                                  int segment, ClassCount* count, int4* __restrict__ rec, int2* __restrict__ seg) {
+    __shared__ unsigned s_n[kRowClasses], s_at[kRowClasses];
+    for (int v0 = (int)(blockIdx.x * blockDim.x); v0 < V; v0 += (int)(gridDim.x * blockDim.x)) {
+        if (threadIdx.x < kRowClasses) s_n[threadIdx.x] = 0u;
+        __syncthreads();
+        const int v = v0 + (int)threadIdx.x;
+        const int rs = v < V ? __ldg(row + v) : 0, n = v < V ? __ldg(row + v + 1) - rs : 0;
+        const int c = row_class(n);
+        const unsigned parts = n == 0 ? 0u : c == 0 ? (unsigned)(n + segment - 1) / (unsigned)segment : 1u;
+        unsigned at = 0u;
+        if (parts) at = atomicAdd(&s_n[c], parts);
+        __syncthreads();
+        if (threadIdx.x < kRowClasses && s_n[threadIdx.x])
+            s_at[threadIdx.x] = atomicAdd(&count->n[threadIdx.x], s_n[threadIdx.x]);
+        __syncthreads();
+        if (kFill && parts) {
+            const int out = __ldg(other + v + 1) - __ldg(other + v);
+            at += s_at[c];
+            if (c) {
+                rec[at] = make_int4(v, rs, n, out);
+            } else {
+                const int id = (int)atomicAdd(&count->n_long, 1u);
+                for (unsigned k = 0; k < parts; ++k) {
+                    rec[at + k] = make_int4(v, rs + (int)k * segment, min(segment, n - (int)k * segment), out);
+                    seg[at + k] = make_int2(id, (int)parts);
+                }
+            }
+        } else if (!kFill && parts && c == 0) {
+            atomicAdd(&count->n_long, 1u);
+        }
+        __syncthreads();
+    }
+}
+
 }  // namespace
+
+void row_lists_free(RowLists& r) {
+    for (void* p : {(void*)r.rec, (void*)r.seg})
+        if (p) cudaFree(p);
+    r = RowLists();
+}
+
+// The non-empty rows of a CSR by length; `other` is the CSR of the opposite direction.
+int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* out) {
+    if (out->rec || g->E == 0) return C2G_OK;
+    ClassCount h{};
+    ClassCount* d = nullptr;
+    C2G_CUDA(cudaMalloc(&d, sizeof(ClassCount)));
+    const int blocks = std::min(g->num_sms * 8, (g->V + 255) / 256);
+    RowLists r;
+    // a segment is one step of a warp (256 edges) where every round is latency, two where it is throughput
+    r.segment = g->E <= kPullAlwaysPushEdges ? 32 * kLaneEdges : 64 * kLaneEdges;
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(ClassCount), g->stream);
+    if (e == cudaSuccess) {
+        row_classes<false><<<blocks, 256, 0, g->stream>>>(row, other, g->V, r.segment, d, nullptr, nullptr);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    unsigned total = 0, unit = 0;
+    for (int c = 0; c < kRowClasses; ++c) {
+        const unsigned rows = c <= 1 ? 1u : 1u << (c - 1);  // rows a warp takes at a time
+        r.n[c] = h.n[c];
+        r.off[c] = total;
+        r.unit[c] = unit;
+        total += h.n[c];
+        unit += (h.n[c] + rows - 1) / rows;
+    }
+    r.unit[kRowClasses] = unit;
+    r.n_long = h.n_long;
+    if (e == cudaSuccess) e = cudaMalloc(&r.rec, sizeof(int4) * (total ? total : 1));
+    if (e == cudaSuccess) e = cudaMalloc(&r.seg, sizeof(int2) * (h.n[0] ? h.n[0] : 1));
+    if (e == cudaSuccess) {
+        ClassCount at{};
+        for (int c = 0; c < kRowClasses; ++c) at.n[c] = r.off[c];
+        e = cudaMemcpyAsync(d, &at, sizeof(at), cudaMemcpyHostToDevice, g->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);  // `at` is read
+    }
+    if (e == cudaSuccess) {
+        row_classes<true><<<blocks, 256, 0, g->stream>>>(row, other, g->V, r.segment, d, r.rec, r.seg);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    cudaFree(d);
+    if (e != cudaSuccess) row_lists_free(r);
+    C2G_CUDA(e);
+    *out = r;
+    return C2G_OK;
+}
+
+// Scatter the float-weighted out-edges into the reverse CSR's rows (in any order within a row).
+static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd) {
+    int* cursor = nullptr;
+    const size_t V = (size_t)g->V;
+    cudaError_t e = cudaMalloc(&cursor, sizeof(int) * (V ? V : 1));
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyAsync(cursor, g->row_r, sizeof(int) * V, cudaMemcpyDeviceToDevice, g->stream);
+    if (e == cudaSuccess && g->E) {
+        in_scatter<<<g->num_sms * 8, 256, 0, g->stream>>>(g->row, fwd, g->V, (unsigned)g->E, cursor, g->adj_r);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    cudaFree(cursor);
+    return e;
+}
+
+// Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), its tile owners and its rows by
+// length; built when the graph is made (one with int32 weights only: on first use).
+int build_reverse_graph(c2g_graph* g) {
+    if (g->adj_r) return C2G_OK;
+    const int2* fwd = g->adj_f ? g->adj_f : g->adj_w;  // float weights when the graph has them
+    if (!fwd) return fail(C2G_ERR_UNSUPPORTED, "graph has no edge weights");
+    const size_t V = (size_t)g->V, E = (size_t)g->E;
+    const int scan_blocks = (int)((V + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems));
+    char* tmp = nullptr;  // stats | in-degrees | cursors (unused) | scan block sums
+    C2G_CUDA(cudaMalloc(&tmp, 256 + sizeof(int) * (V * 2 + (size_t)scan_blocks + 1)));
+    InStats* st = reinterpret_cast<InStats*>(tmp);
+    int* indeg = reinterpret_cast<int*>(tmp + 256);
+    int *cursor = indeg + V, *sums = cursor + V;
+    cudaError_t e = cudaMalloc(&g->row_r, sizeof(int) * (V + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&g->adj_r, sizeof(int2) * (E ? E : 1));
+    if (e == cudaSuccess) e = cudaMemsetAsync(tmp, 0, 256 + sizeof(int) * V, g->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(g->row_r, 0, sizeof(int) * (V + 1), g->stream);
+    if (e == cudaSuccess && E) {
+        in_count<<<g->num_sms * 8, 256, 0, g->stream>>>(fwd, (unsigned)E, indeg, st);
+        in_scan_blocks<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, 0, sums, st);
+        in_scan_sums<<<1, kScanThreads, 0, g->stream>>>(sums, scan_blocks);
+        in_scan_rows<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, 0, sums, g->row_r, cursor, nullptr, st);
+        e = cudaGetLastError();
+    }
+    InStats h{};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = scatter_reverse(g, fwd);
+    cudaFree(tmp);
+    if (e == cudaSuccess && g->adj_f) {  // the largest positive weight: positive floats order as integers
+        g->wstat_wmax_bits = (uint32_t)h.wmax;
+        g->wstat_valid = true;
+    }
+    int rc = C2G_OK;
+    if (e != cudaSuccess)
+        rc = fail(e == cudaErrorMemoryAllocation ? C2G_ERR_OOM : C2G_ERR_CUDA, "reverse CSR: %s", cudaGetErrorString(e));
+    if (!rc) rc = build_markers(g, g->row_r, &g->mark_r);
+    if (!rc) rc = build_markers(g, g->row, &g->mark_f);
+    if (!rc) rc = build_row_lists(g, g->row_r, g->row, &g->rows_in);
+    if (rc) {
+        cudaGetLastError();
+        reverse_free(g);
+    }
+    return rc;
+}
+
+// New float weights: the reverse CSR's rows stay, their edges are written anew.
+int refresh_reverse_graph(c2g_graph* g) {
+    g->wstat_valid = false;
+    if (!g->adj_r) return C2G_OK;
+    C2G_CUDA(scatter_reverse(g, g->adj_f));
+    return C2G_OK;
+}
+
+void reverse_free(c2g_graph* g) {
+    for (void* p : {(void*)g->row_r, (void*)g->adj_r, (void*)g->mark_r, (void*)g->mark_f})
+        if (p) cudaFree(p);
+    row_lists_free(g->rows_in);
+    row_lists_free(g->rows_out);
+    g->wstat_valid = false;
+    g->row_r = nullptr;
+    g->adj_r = nullptr;
+    g->mark_r = nullptr;
+    g->mark_f = nullptr;
+}
 
 void in_rows_free(c2g_graph* g) {
     for (void* p : {(void*)g->in_row, (void*)g->in_adj, (void*)g->in_seg})
@@ -295,7 +484,7 @@ int build_in_rows(c2g_graph* g) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, g->stream);
     if (e == cudaSuccess) {
         in_count<<<blocks, 256, 0, g->stream>>>(g->adj_w, (unsigned)E, indeg, st);
-        in_scan_blocks<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, sums, st);
+        in_scan_blocks<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, 1, sums, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
@@ -312,7 +501,7 @@ int build_in_rows(c2g_graph* g) {
         int shift = 0;
         while ((h.wmax >> shift) >= kInBuckets) ++shift;
         in_scan_sums<<<1, kScanThreads, 0, g->stream>>>(sums, scan_blocks);
-        in_scan_rows<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, sums, g->in_row, cursor, longs, st);
+        in_scan_rows<<<scan_blocks, kScanThreads, 0, g->stream>>>(indeg, g->V, 1, sums, g->in_row, cursor, longs, st);
         in_scatter<<<blocks, 256, 0, g->stream>>>(g->row, g->adj_w, g->V, (unsigned)E, cursor, raw);
         in_sort_short<<<blocks, 256, 0, g->stream>>>(g->in_row, indeg, g->V, raw, g->in_adj);
         e = cudaGetLastError();

@@ -85,7 +85,7 @@ struct PprWork {
     float* pr = nullptr;
     double* res = nullptr;
     double* msg = nullptr;
-    double* qd = nullptr;
+    float2* qf[2] = {nullptr, nullptr};
     float* res_f = nullptr;  // residual as float for the caller
     int* stamp = nullptr;
     int2* q[2] = {nullptr, nullptr};
@@ -95,6 +95,8 @@ struct PprWork {
     int* dangle = nullptr;
     TraversalCtl* ctl = nullptr;
     StampState* st = nullptr;
+    unsigned* arrived = nullptr;  // pull rounds: segments of a long row summed so far
+    unsigned arrived_cap = 0;
     unsigned mark_cap = 0;
     int log_tile = -1;
 };
@@ -114,7 +116,8 @@ struct SsspConfig {
 struct PprConfig {
     float batch_pull_ratio = 8.0f;  // batched rounds with more than ratio * E pushes pull (< 0: never)
     int log_tile = 8;
-    int pull_div = 0;   // pull round when frontier out-edges * pull_div > E; 0 = push only (default)
+    int pull_div = 0;   // pull round when frontier out-edges * pull_div > E; 0 = push only
+    bool pull_set = false;  // until it is set, ppr.cu picks the rule by the graph's size
     int dense_div = 16;  // dense push round (red.add, apply sweep over V) when out-edges * dense_div > E
 };
 
@@ -123,6 +126,23 @@ constexpr int kInMaxWeight = 147483648;  // largest weight of in-edge rows: unre
 constexpr int kInHead = 32, kInSegment = 256;  // edges; multiples of 32
 
 constexpr int kPullTileLog = 8;  // in-edges per pull tile (reverse-CSR markers)
+
+// The non-empty rows of a CSR by length (in_edges.cu), for the pull rounds of the single push.  Class 0:
+// rows of more than 256 edges, in segments; class c >= 1: rows of up to 256 >> (c - 1)
+// edges, which 32 >> (c - 1) lanes read, kLaneEdges each.
+constexpr int kRowClasses = 7;
+constexpr int kLaneEdges = 8;
+constexpr int64_t kPullAlwaysPushEdges = 4000000;  // single push: graphs up to this size pull every round (ppr.cu)
+
+struct RowLists {
+    int4* rec = nullptr;           // (row, first edge, edges, out-degree of the row's vertex)
+    int2* seg = nullptr;           // class 0: (index of the row's arrival counter, its segments)
+    unsigned n_long = 0;           // rows of class 0
+    int segment = 0;               // edges per segment
+    unsigned n[kRowClasses] = {};  // records
+    unsigned off[kRowClasses] = {};
+    unsigned unit[kRowClasses + 1] = {};  // first of the class's warp steps
+};
 
 struct LaunchGeom {
     int blocks = 0;
@@ -141,7 +161,7 @@ struct c2g_graph {
     int2* adj_f = nullptr;
     int32_t* row_r = nullptr;  // reverse CSR with float weights (pull rounds, adjoint), on demand
     int2* adj_r = nullptr;
-    // in-edge rows ordered by weight (in_rows.cu), or null: the graph's SSSP queries push only
+    // in-edge rows ordered by weight (in_edges.cu), or null: the graph's SSSP queries push only
     int32_t* in_row = nullptr;  // [V+1], multiples of 4
     int2* in_adj = nullptr;     // (source, weight), padded with weight INT_MAX
     int64_t in_edges = 0;       // padded edges
@@ -149,7 +169,9 @@ struct c2g_graph {
     unsigned in_segs = 0;
     int in_shift = 0;           // weights are ordered up to their low in_shift bits
     int32_t* mark_r = nullptr;  // pull-tile owner markers over row_r
-    int32_t* mark_f = nullptr;  // pull-tile owner markers over row (pulls on the reverse graph)
+    int32_t* mark_f = nullptr;  // pull-tile owner markers over row (the adjoint's gradient pass)
+    c2g::RowLists rows_in;      // rows of row_r by length
+    c2g::RowLists rows_out;     // rows of row by length (the adjoint's push on the reverse graph), on demand
     // pruned records
     int32_t R = -1;
     int64_t H = 0;
@@ -197,7 +219,7 @@ int sssp_launch(c2g_graph* g, int32_t source, const int32_t* seed_v, const int32
 int ppr_launch(c2g_graph* g, int32_t source, const c2g_ppr_params& p, const int32_t* seed_v,
                const float* seed_w, int32_t n_seeds, float* pr_dev, float* res_dev, float* ms);
 int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int32_t* row_rev, const int2* adj_rev,
-                    const int32_t* mark_rev, int32_t source, const c2g_ppr_params& pp, float absorb, int32_t n_src,
+                    const RowLists& rows_rev, int32_t source, const c2g_ppr_params& pp, float absorb, int32_t n_src,
                     const int32_t* src_list, const float* src_r0, const int32_t* seed_v, const float* seed_w,
                     int32_t n_rec, float* pr_dev, float* res_dev, float* ms);
 int build_markers(c2g_graph* g, const int* row, int** out);
@@ -209,6 +231,9 @@ void batch_free(c2g_graph* g);
 void ppr_batch_free(c2g_graph* g);
 void ads_free(c2g_graph* g);
 int build_reverse_graph(c2g_graph* g);
+int refresh_reverse_graph(c2g_graph* g);
+void reverse_free(c2g_graph* g);
+int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* out);
 int build_in_rows(c2g_graph* g);
 void in_rows_free(c2g_graph* g);
 // Reverse CSR and the weight statistics of the batched pull rounds (once per weights).

@@ -14,18 +14,20 @@
 // L1 1e-6 of the FP64 result as graphs grow.  With FP64 residuals the decisions match the
 // FP64 push up to summation order.
 //
-// Two round shapes, chosen per round from the frontier's out-edge count T:
+// Round shapes, chosen per round from the frontier's out-edge count T:
 //   * push (T small): edge-tiled walk over the frontier's out-edges, FP64 atomicAdd into
 //     msg; the add that returns 0 records the target in the touched list and phase B
-//     visits only touched vertices (no O(V) sweep, src/ppr/purn/Main.cu:379-407);
-//   * pull (T * pull_div > E): every vertex sums (1-alpha)*r_u*w(u,v) over its in-edges
-//     (reverse CSR) from a dense array qd of the frontier's pushed residuals, with a
-//     segmented warp reduction (a few atomics per 32 in-edges instead of one per edge),
-//     then a dense apply pass over all V.  Both shapes give the same BSP round.
+//     visits only touched vertices (no O(V) sweep, src/ppr/purn/Main.cu:379-407); with more
+//     edges the adds keep no list and phase B sweeps all vertices;
+//   * pull (T large, or a small graph): every vertex with in-edges gathers the pushed residuals
+//     of its in-neighbours from a dense array qf, sums the messages in registers and
+//     applies them on the spot: no message array, no atomics, one barrier a round.
+// All give the same BSP round.
 // The residual a frontier vertex pushes is captured when it is activated (nothing
 // changes it before its pop).  Activated vertices without out-edges sit in a side list
 // whose residual is cleared at the start of the next round, which is when the reference
 // pops them (when the round cap ends the run first, they keep it).
+#include <algorithm>
 #include <climits>
 
 #include "device_common.cuh"
@@ -41,13 +43,14 @@ struct PprParams {
     int V;
     const int* row_r;   // reverse CSR (in-edges carrying w(u,v)), or nullptr: push only
     const int2* adj_r;
-    const int* mark_r;  // owner of in-edge t * 2^kPullTileLog
-    int pull_div;       // pull when T * pull_div > E (0: never)
+    RowLists rows;      // its rows by length
+    unsigned* arrived;  // class 0: segments of a row summed so far, zero between rounds
+    unsigned pull_min;  // pull when T is larger (~0: never)
     int dense_div;      // dense push round (no touched list) when T * dense_div > E (0: never)
     float* pr;
     double* res;
     double* msg;
-    double* qd;  // (1-alpha)*r of frontier vertices, 0 elsewhere (pull rounds)
+    float2* qf[2];  // (1-alpha)*r of the frontier's vertices as a float pair, 0 elsewhere, by round parity (pulls)
     int* stamp;
     int2* q[2];
     double* qval[2];
@@ -102,14 +105,13 @@ constexpr bool kPprDynTiles = false;
 __device__ __forceinline__ void ppr_push(const PprParams& p, int buf, int slot, unsigned F, unsigned T,
                                          WarpStage& tst, bool track) {
     constexpr int U = kPprUnroll;
-    const double one_m_a = 1.0 - (double)p.alpha;
     const double* qv = p.qval[buf];
     walk_frontier_edges<U>(
         p.q[buf], p.mark[buf], p.row, F, T, p.log_tile, p.mark_cap, (unsigned)p.V, p.E, &p.ctl->flags,
-        // (1-alpha)*r_u (src/ppr/purn/Main.cu:288); the owner is popped, so it leaves qd
+        // (1-alpha)*r_u (src/ppr/purn/Main.cu:288); the owner is popped, so it leaves qf
         [&](int v, unsigned j) {
-            if (p.qd) p.qd[v] = 0.0;
-            return one_m_a * ldcg(qv + j);
+            p.qf[buf][v] = make_float2(0.f, 0.f);
+            return ldcg(qv + j);
         },
         [&](const bool* ok, const unsigned* idx, const double* qu) {
             int c[U];
@@ -150,60 +152,204 @@ __device__ __forceinline__ void ppr_push(const PprParams& p, int buf, int slot, 
     if (track) list_stage_flush(tst, p.touched, &p.ctl->listctr[slot], (unsigned)p.V, &p.ctl->flags);
 }
 
-// Pull round, phase A: msg[v] = sum over in-edges (u, w) of qd[u] * w.  In-edges are
-// walked in tiles of 2^kPullTileLog; 32 consecutive in-edges per step, one per lane; a
-// segmented scan sums each owner's lanes and the segment's last lane adds it to msg.
-__device__ __forceinline__ void ppr_pull(const PprParams& p) {
+// Pulls end when a pushed residual passes 2^60 (float bits): with weights below 2^30 (checked by the host)
+// every sum of up to 2^31 messages then stays a finite float.
+constexpr int kPullMaxQ = (127 + 60) << 23;
+constexpr unsigned kPullMaxWeight = (127 + 30) << 23;
+
+// The float pair of a pushed residual (fp64_mul.h), and its value.
+__device__ __forceinline__ float2 ppr_pair(double q) {
+    if (c2g_split_ok(q)) {
+        const c2g_pair hl = c2g_split_pair(q);
+        return make_float2(c2g_bitsf(hl.hi), c2g_bitsf(hl.lo));
+    }
+    const float hi = __double2float_rz(q);
+    return make_float2(hi, __double2float_rz(q - (double)hi));
+}
+__device__ __forceinline__ double ppr_pair_value(const float2& q) {
+    return c2g_float_bits_to_double(__float_as_uint(q.x)) + c2g_float_bits_to_double(__float_as_uint(q.y));
+}
+
+// Sum of two floats as a rounded sum and its error.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float s = __fadd_rn(a, b), bv = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bv)), __fsub_rn(b, bv));
+    return s;
+}
+
+// Totals of a pull round: activated vertices with out-edges (F << 32 | their out-edges) and without.
+struct PullTotals {
+    unsigned long long count;
+    unsigned dangling;
+    int qmax;  // largest pushed residual (float bits)
+};
+
+// Pull round.  The rows of the reverse CSR are binned by length (RowLists), so that a warp takes 32 / L
+// rows of similar length, L lanes each and at most kLaneEdges in-edges per lane: all its gathers
+// are in flight together, and a row's sum is its lanes' messages and log2(L) shuffles.  Messages
+// are summed as float pairs (products and sums with their errors recovered, about 47 bits
+// relative, as in the batched push): a warp's FP64 instruction holds an SM's FP64 pipe for 16
+// cycles here.  Rows of more than 256 edges are split into segments: each adds its sum to msg, and
+// after one fence for all of a warp's segments the last segment of a row to arrive applies it
+// (a fence per segment of 128 edges held a warp for a quarter of the round).
+// A round over all 16M edges of a scale-20 graph takes 94 us; pushed, 240 us.
+//
+// qf[b] holds the frontier; the new one goes to qf[b ^ 1], for every row, so nothing is cleared.  A vertex
+// that was in the frontier has residual 0 from its pop (its res still holds what it had when it was
+// activated: at the round cap that is what it keeps); one that was not adds its messages to res.
+struct PullSums {
+    float hi, lo;
+};
+
+// Messages of this lane's in-edges first, first + step, ... (up to kLaneEdges of them) below n.
+__device__ __forceinline__ void pull_lane(const int2* __restrict__ adj, const float2* qin, int first, int step, int n,
+                                          PullSums& s) {
+    int2 ew[kLaneEdges];
+    float2 q[kLaneEdges];
+#pragma unroll
+    for (int u = 0; u < kLaneEdges; ++u) {
+        const int i = first + u * step;
+        ew[u] = i < n ? __ldg(adj + i) : make_int2(0, 0);
+    }
+    // through L1: qf[b] does not change during the round
+#pragma unroll
+    for (int u = 0; u < kLaneEdges; ++u) q[u] = ew[u].y > 0 ? __ldca(qin + ew[u].x) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kLaneEdges; ++u) {
+        // message (hi + lo) * w = pm + pe; a source outside the frontier or a weight that is
+        // not positive adds 0
+        const float w = q[u].x != 0.f ? __int_as_float(ew[u].y) : 0.f;
+        const float pm = __fmul_rn(q[u].x, w);
+        const float pe = __fmaf_rn(q[u].y, w, __fmaf_rn(q[u].x, w, -pm));
+        float te;
+        s.hi = two_sum(s.hi, pm, te);
+        s.lo = __fadd_rn(s.lo, __fadd_rn(te, pe));
+    }
+}
+
+// Sum over groups of L lanes; the value as a double (in every lane of the group).
+__device__ __forceinline__ double pull_reduce(PullSums s, int L) {
+    for (int o = 1; o < L; o <<= 1) {
+        const float oh = __shfl_xor_sync(kFull, s.hi, o), ol = __shfl_xor_sync(kFull, s.lo, o);
+        float te;
+        s.hi = two_sum(s.hi, oh, te);
+        s.lo = __fadd_rn(te, __fadd_rn(s.lo, ol));
+    }
+    return ppr_pair_value(make_float2(s.hi, s.lo));
+}
+
+// Vertex v's messages s are complete (q0: the high half of its own pushed residual, r0: its res,
+// pr0: its pr).
+__device__ __forceinline__ void pull_apply(const PprParams& p, float2* qout, int v, int out_degree, double s, float q0,
+                                           double r0, float pr0, PullTotals& tot) {
+    const bool popped = q0 != 0.f;
+    float2 q1 = make_float2(0.f, 0.f);
+    if (c2g_dbits(s) != 0ull) {  // messages are positive
+        const double r = popped ? s : r0 + s;
+        p.res[v] = r;
+        if (c2g_dbits(r) > c2g_dbits((double)p.rmax)) {  // both non-negative
+            p.pr[v] = pr0 + (float)((double)p.absorb * r);
+            q1 = ppr_pair((1.0 - (double)p.alpha) * r);
+            tot.qmax = max(tot.qmax, __float_as_int(q1.x));
+            if (out_degree > 0)
+                tot.count += (1ull << 32) | (unsigned)out_degree;
+            else
+                ++tot.dangling;
+        }
+    } else if (popped) {
+        p.res[v] = 0.0;
+    }
+    qout[v] = q1;
+}
+
+__device__ __forceinline__ void ppr_pull(const PprParams& p, int b, PullTotals& tot) {
     const int lane = threadIdx.x & 31;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
-    const unsigned tw = 1u << kPullTileLog;
-    const unsigned ntiles = (p.E + tw - 1) >> kPullTileLog;
-    const unsigned V = (unsigned)p.V;
-    for (unsigned t = gwarp; t < ntiles; t += nwarps) {
-        unsigned e0 = t << kPullTileLog;
-        const unsigned e1 = min(e0 + tw, p.E);
-        unsigned o = (unsigned)__ldg(p.mark_r + t);
-        while (e0 < e1) {
-            const unsigned j = o + (unsigned)lane;
-            unsigned base = 0x7fffffffu, endv = 0xffffffffu;
-            if (j < V) {
-                base = (unsigned)__ldg(p.row_r + j);
-                endv = (unsigned)__ldg(p.row_r + j + 1);
-            }
-            if (o >= V || (unsigned)__shfl_sync(kFull, (int)base, 0) > e0) {
-                if (lane == 0) atomicOr(&p.ctl->flags, C2G_FLAG_BOUNDS);
-                break;
-            }
-            const unsigned seg_end = min(e1, (unsigned)__shfl_sync(kFull, endv, 31));
-            if (seg_end <= e0) {  // 32 owners without in-edges: move on (o grows to V at most)
-                o += 32;
-                continue;
-            }
-            for (unsigned eb = e0; eb < seg_end; eb += 32) {
-                const unsigned e = eb + (unsigned)lane;
-                const bool valid = e < seg_end;
-                const int k = owner_lane(base, e);  // rows without in-edges share bases: the last one owns e
-                double s = 0.0;
-                if (valid) {
-                    const int2 ew = __ldg(p.adj_r + e);
-                    s = ldcg(p.qd + ew.x) * (double)__int_as_float(ew.y);
-                }
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const double ts = __shfl_up_sync(kFull, s, off);
-                    const int tk = __shfl_up_sync(kFull, k, off);
-                    if (lane >= off && tk == k) s += ts;
-                }
-                const int kn = __shfl_down_sync(kFull, k, 1);
-                const bool vn = __shfl_down_sync(kFull, (int)valid, 1) != 0;
-                const bool tail = valid && (lane == 31 || !vn || kn != k);
-                if (tail && s != 0.0) atomicAdd(p.msg + o + (unsigned)k, s);
-            }
-            e0 = seg_end;
-            o += 32;
+    const float2* qin = p.qf[b];
+    float2* qout = p.qf[b ^ 1];
+    const RowLists& R = p.rows;
+    // segments of long rows
+    for (unsigned r = gwarp; r < R.n[0]; r += nwarps) {
+        const int4 rec = __ldg(R.rec + r);
+        PullSums s{0.f, 0.f};
+        for (int i = 0; i < rec.z; i += 32 * kLaneEdges)
+            pull_lane(p.adj_r + rec.y, qin, i + lane, 32, rec.z, s);
+        const double m = pull_reduce(s, 32);
+        if (lane == 0 && c2g_dbits(m) != 0ull) atomicAdd(p.msg + rec.x, m);
+    }
+    if (gwarp < R.n[0]) {
+        __syncwarp();
+        __threadfence();  // the warp's sums are in msg before it arrives
+        for (unsigned r0 = gwarp; r0 < R.n[0]; r0 += 32u * nwarps) {
+            const unsigned r = r0 + (unsigned)lane * nwarps;
+            if (r >= R.n[0]) continue;
+            const int2 sg = __ldg(R.seg + r);
+            if (atomicAdd(p.arrived + sg.x, 1u) != (unsigned)sg.y - 1u) continue;
+            __threadfence();  // the other segments' sums are seen
+            const int4 rec = __ldg(R.rec + r);
+            const double m = ldcg(p.msg + rec.x);
+            p.msg[rec.x] = 0.0;
+            p.arrived[sg.x] = 0u;
+            pull_apply(p, qout, rec.x, rec.w, m, ldcg(reinterpret_cast<const float*>(qin + rec.x)), ldcg(p.res + rec.x),
+                       ldcg(p.pr + rec.x), tot);
         }
     }
+    // whole rows, starting with the warps that had one segment less
+    const unsigned units = R.unit[kRowClasses], turn = R.n[0] % nwarps;
+    for (unsigned unit = R.unit[1] + (gwarp >= turn ? gwarp - turn : gwarp + nwarps - turn); unit < units;
+         unit += nwarps) {
+        int c = 1;
+        unsigned n = R.n[1], off = R.off[1], first = R.unit[1];
+#pragma unroll
+        for (int k = 2; k < kRowClasses; ++k)
+            if (unit >= R.unit[k]) {
+                c = k;
+                n = R.n[k];
+                off = R.off[k];
+                first = R.unit[k];
+            }
+        const int logL = 6 - c, L = 1 << logL, part = lane & (L - 1);
+        const unsigned r = ((unit - first) << (5 - logL)) + (unsigned)(lane >> logL);
+        const int4 rec = r < n ? __ldg(R.rec + off + r) : make_int4(0, 0, 0, 0);
+        const bool mine = r < n && part == 0;
+        float q0 = 0.f, pr0 = 0.f;
+        double r0 = 0.0;
+        if (mine) {
+            q0 = ldcg(reinterpret_cast<const float*>(qin + rec.x));
+            r0 = ldcg(p.res + rec.x);
+            pr0 = ldcg(p.pr + rec.x);
+        }
+        PullSums s{0.f, 0.f};
+        pull_lane(p.adj_r + rec.y, qin, part, L, rec.z, s);
+        const double m = pull_reduce(s, L);
+        if (mine) pull_apply(p, qout, rec.x, rec.w, m, q0, r0, pr0, tot);
+    }
+}
+
+// The frontier list of a round whose frontier a pull counted: its vertices are popped (those without
+// out-edges for good), and the other parity's qf is cleared for the round's apply.
+__device__ __forceinline__ void ppr_list(const PprParams& p, int b, const FrontierOut& out, WarpStage& fst) {
+    const int lane = threadIdx.x & 31;
+    const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+    const unsigned V = (unsigned)p.V;
+    for (unsigned v0 = gwarp * 32; v0 < V; v0 += nwarps * 32) {
+        const unsigned v = v0 + (unsigned)lane;
+        float2 q = make_float2(0.f, 0.f);
+        int deg = 0;
+        if (v < V) {
+            q = ldcg(p.qf[b] + v);
+            p.qf[b ^ 1][v] = make_float2(0.f, 0.f);
+            if (q.x != 0.f) {
+                p.res[v] = 0.0;
+                deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
+                if (deg == 0) p.qf[b][v] = make_float2(0.f, 0.f);
+            }
+        }
+        stage_push(fst, out, deg > 0, (int)v, deg, 0.f, ppr_pair_value(q));
+    }
+    stage_flush(fst, out);
 }
 
 __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(const PprParams p) {
@@ -222,18 +368,20 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
     const int wib = threadIdx.x >> 5;
     WarpStage fst{sm.v0[wib], sm.d0[wib], nullptr, 0, sm.xd0[wib]};
     WarpStage tst{sm.v1[wib], nullptr, nullptr, 0};
+    __shared__ PullTotals share;
+    if (threadIdx.x == 0) share = PullTotals{0ull, 0u, 0};
     unsigned long long tph = globaltimer_ns();
 
     int sbase = p.st->stamp_base;
     const bool reset = sbase > (1 << 29);
     if (reset) sbase = 0;
 
-    // Init: pr = res = msg = 0 (src/ppr/purn/Main.cu:156-169), qd = 0.
+    // Init: pr = res = msg = 0 (src/ppr/purn/Main.cu:156-169), qf = 0.
     for (unsigned v = gtid; v < V; v += nthreads) {
         p.pr[v] = 0.f;
         p.res[v] = 0.0;
         p.msg[v] = 0.0;
-        if (p.qd) p.qd[v] = 0.0;
+        p.qf[0][v] = p.qf[1][v] = make_float2(0.f, 0.f);
         if (reset) p.stamp[v] = -1;
     }
     if (!grid_sync(bar, flags, p.barrier_ns)) return;
@@ -257,7 +405,8 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                 want = deg > 0;
                 dang = !want;
                 if (dang) p.res[v] = r;
-                if (want && p.qd) p.qd[v] = one_m_a * r;
+                r *= one_m_a;
+                p.qf[1][v] = ppr_pair(r);
             }
             stage_push(fst, out, want, v, deg, 0.f, r);
             list_push(p.dangle, &ctl->dctr[1], (unsigned)p.V, flags, dang, v);
@@ -270,16 +419,15 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
             if (lane == 0) {
                 p.pr[s] = p.pr0;
                 ctl->seeds = 0;
+                p.qf[1][s] = ppr_pair(one_m_a * (double)p.r0);
                 if (s_deg == 0) {
                     p.res[s] = (double)p.r0;
                     p.dangle[0] = s;
                     ctl->dctr[1] = 1;
-                } else if (p.qd) {
-                    p.qd[s] = one_m_a * (double)p.r0;
                 }
             }
             const FrontierOut out = ppr_out(p, 1, 1);
-            stage_push(fst, out, lane == 0 && s_deg > 0, s, s_deg, 0.f, (double)p.r0);
+            stage_push(fst, out, lane == 0 && s_deg > 0, s, s_deg, 0.f, one_m_a * (double)p.r0);
             stage_flush(fst, out);
         }
     } else {
@@ -320,12 +468,10 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                     r = __ldcg(p.res + v);
                     deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
                     want = deg > 0;
-                    if (want) {
-                        p.res[v] = 0.0;
-                        if (p.qd) p.qd[v] = one_m_a * r;
-                    } else {
-                        dang = true;
-                    }
+                    dang = !want;
+                    if (want) p.res[v] = 0.0;
+                    r *= one_m_a;
+                    p.qf[1][v] = ppr_pair(r);
                 }
             }
             stage_push(fst, out, want, v, deg, 0.f, r);
@@ -337,43 +483,95 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
     phase_mark(ctl->phase_ns, tph, 0);
 
     int cur = 1, iters = 0;
+    unsigned F1 = 0;       // entries of round 1's list
+    int qmax = 0;          // largest pushed residual this thread applied in a push round (float bits)
+    bool counted = false;  // this round's frontier is counted (a pull made it), not listed
     for (;;) {
-        const unsigned long long c = ldcg(&ctl->qctr[cur % 3]);
+        const int buf = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
+        const unsigned long long c = counted ? ldcg(&ctl->pcount[slot]) : ldcg(&ctl->qctr[slot]);
         const unsigned F = (unsigned)(c >> 32), T = (unsigned)c;
-        const unsigned D = ldcg(&ctl->dctr[cur % 3]);
+        const unsigned D = ldcg(&ctl->dctr[slot]);
         if (F == 0 && D == 0) break;
+        if (cur == 1) F1 = F;
         if (++iters > p.max_iter) {
             // Round cap (src/ppr/purn/Main.cu:224): the activated vertices keep their
-            // residual, as in the reference where they are never popped.
+            // residual, as in the reference where they are never popped (after a pull
+            // res still holds it).
             if (gtid == 0) atomicOr(flags, C2G_FLAG_ITER_CAP);
-            const int2* q = p.q[cur & 1];
-            const double* qv = p.qval[cur & 1];
-            for (unsigned j = gtid; j < F; j += nthreads) p.res[ldcg(q + j).x] = __ldcg(qv + j);
+            if (!counted)
+                for (unsigned j = gtid; j < F; j += nthreads)
+                    p.res[ldcg(p.q[buf] + j).x] = ldcg(p.qval[buf] + j) / one_m_a;
             break;
         }
-        // Pop the activated vertices without out-edges: their residual is dropped.
-        for (unsigned j = gtid; j < D; j += nthreads) p.res[ldcg(p.dangle + j)] = 0.0;
+        // grid-uniform; float pairs hold the pushed residuals and their sums below kPullMaxQ
+        const bool pull = T > p.pull_min && ldcg(&ctl->farmin[0]) == 0;
+        // Pop the activated vertices without out-edges: their residual is dropped.  A pull does so
+        // for every vertex with in-edges.
+        if (!counted) {
+            for (unsigned j = gtid; j < D; j += nthreads) {
+                const int v = ldcg(p.dangle + j);
+                if (pull && __ldg(p.row_r + v) < __ldg(p.row_r + v + 1)) continue;
+                p.res[v] = 0.0;
+                p.qf[buf][v] = make_float2(0.f, 0.f);
+            }
+        } else if (F == 0) {
+            for (unsigned v = gtid; v < V; v += nthreads)
+                if (ldcg(p.qf[buf] + v).x != 0.f) p.res[v] = 0.0;
+        }
         if (F == 0) {
             if (gtid == 0) ctl->popped += D;
             break;
         }
-        const int slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
-        const bool pull = p.row_r && p.pull_div > 0 && (unsigned long long)T * (unsigned)p.pull_div > p.E;
-        const bool dense = pull || (p.dense_div > 0 && (unsigned long long)T * (unsigned)p.dense_div > p.E);
         if (gtid == 0) {
             ctl->qctr[fslot] = 0ull;
             ctl->tilectr[fslot] = 0u;
             ctl->listctr[fslot] = 0u;
             ctl->dctr[fslot] = 0u;
+            ctl->pcount[fslot] = 0ull;
             ctl->popped += F + D;
-            ctl->relaxed += pull ? p.E : T;
-            if (pull) ctl->pad[0] += 1;  // pull rounds
+            ctl->relaxed += T;
         }
+        if (pull) {
+            // Round 1's frontier may hold vertices without in-edges, which no pull visits: out of qf[1]
+            // before round 3 reads it.
+            if (cur == 2)
+                for (unsigned j = gtid; j < F1; j += nthreads) {
+                    const int v = ldcg(p.q[1] + j).x;
+                    if (__ldg(p.row_r + v) == __ldg(p.row_r + v + 1)) p.qf[1][v] = make_float2(0.f, 0.f);
+                }
+            PullTotals tot{0ull, 0u};
+            ppr_pull(p, buf, tot);
+            for (int o = 16; o >= 1; o >>= 1) tot.count += __shfl_xor_sync(kFull, tot.count, o);
+            tot.dangling = __reduce_add_sync(kFull, tot.dangling);
+            tot.qmax = __reduce_max_sync(kFull, tot.qmax);
+            if (lane == 0) {
+                if (tot.count) atomicAdd(&share.count, tot.count);
+                if (tot.dangling) atomicAdd(&share.dangling, tot.dangling);
+                if (tot.qmax) atomicMax(&share.qmax, tot.qmax);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                if (share.count) atomicAdd(&ctl->pcount[nslot], share.count);
+                if (share.dangling) atomicAdd(&ctl->dctr[nslot], share.dangling);
+                if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], share.qmax);
+                share = PullTotals{0ull, 0u, 0};
+                if (gtid == 0) ctl->touched += V;
+            }
+            if (!grid_sync(bar, flags, p.barrier_ns)) return;
+            phase_mark(ctl->phase_ns, tph, 2);
+            counted = true;
+            ++cur;
+            continue;
+        }
+        if (counted) {
+            ppr_list(p, buf, ppr_out(p, buf, slot), fst);
+            if (!grid_sync(bar, flags, p.barrier_ns)) return;
+            phase_mark(ctl->phase_ns, tph, 1);
+            counted = false;
+        }
+        const bool dense = p.dense_div > 0 && (unsigned long long)T * (unsigned)p.dense_div > p.E;
         const FrontierOut out = ppr_out(p, (cur + 1) & 1, nslot);
-        if (pull)
-            ppr_pull(p);
-        else
-            ppr_push(p, cur & 1, slot, F, T, tst, !dense);
+        ppr_push(p, buf, slot, F, T, tst, !dense);
         if (!grid_sync(bar, flags, p.barrier_ns)) return;
         phase_mark(ctl->phase_ns, tph, 2);
         if (!dense) {
@@ -395,7 +593,10 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                         want = deg > 0;
                         dang = !want;
                         p.res[v] = want ? 0.0 : r;
-                        if (want && p.qd) p.qd[v] = one_m_a * r;
+                        r *= one_m_a;
+                        const float2 q = ppr_pair(r);
+                        p.qf[buf ^ 1][v] = q;
+                        qmax = max(qmax, __float_as_int(q.x));
                     } else {
                         p.res[v] = r;
                     }
@@ -414,7 +615,6 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                 double r = 0.0;
                 if (v < V) {
                     const double m = __ldcg(p.msg + v);
-                    const double q0 = p.qd ? __ldcg(p.qd + v) : 0.0;
                     if (c2g_dbits(m) != 0ull) {  // messages are positive; msg is +0 otherwise
                         p.msg[v] = 0.0;
                         r = __ldcg(p.res + v) + m;
@@ -424,18 +624,21 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                             want = deg > 0;
                             dang = !want;
                             p.res[v] = want ? 0.0 : r;
+                            r *= one_m_a;
+                            const float2 q = ppr_pair(r);
+                            p.qf[buf ^ 1][v] = q;
+                            qmax = max(qmax, __float_as_int(q.x));
                         } else {
                             p.res[v] = r;
                         }
                     }
-                    const double q1 = want ? one_m_a * r : 0.0;
-                    if (p.qd && q1 != q0) p.qd[v] = q1;
                 }
                 stage_push(fst, out, want, (int)v, deg, 0.f, r);
                 list_push(p.dangle, &ctl->dctr[nslot], (unsigned)p.V, flags, dang, (int)v);
             }
         }
         stage_flush(fst, out);
+        if (qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], qmax);
         if (!grid_sync(bar, flags, p.barrier_ns)) return;
         phase_mark(ctl->phase_ns, tph, 1);
         ++cur;
@@ -496,7 +699,7 @@ static int ppr_geometry(c2g_graph* g) {
 
 void ppr_free(c2g_graph* g) {
     PprWork& w = g->ppr;
-    void* ptrs[] = {w.pr, w.res, w.msg, w.qd, w.res_f, w.stamp, w.q[0], w.q[1], w.qval[0], w.qval[1],
+    void* ptrs[] = {w.pr, w.res, w.msg, w.qf[0], w.qf[1], w.arrived, w.res_f, w.stamp, w.q[0], w.q[1], w.qval[0], w.qval[1],
                     w.mark[0], w.mark[1], w.touched, w.dangle, w.ctl, w.st};
     for (void* ptr : ptrs)
         if (ptr) cudaFree(ptr);
@@ -513,7 +716,6 @@ static int ppr_alloc(c2g_graph* g) {
     C2G_CUDA(cudaMalloc(&w.pr, sizeof(float) * nv));
     C2G_CUDA(cudaMalloc(&w.res, sizeof(double) * nv));
     C2G_CUDA(cudaMalloc(&w.msg, sizeof(double) * nv));
-    C2G_CUDA(cudaMalloc(&w.qd, sizeof(double) * nv));
     C2G_CUDA(cudaMalloc(&w.res_f, sizeof(float) * nv));
     C2G_CUDA(cudaMalloc(&w.stamp, sizeof(int) * nv));
     C2G_CUDA(cudaMalloc(&w.touched, sizeof(int) * nv));
@@ -521,6 +723,7 @@ static int ppr_alloc(c2g_graph* g) {
     for (int b = 0; b < 2; ++b) {
         C2G_CUDA(cudaMalloc(&w.q[b], sizeof(int2) * nv));
         C2G_CUDA(cudaMalloc(&w.qval[b], sizeof(double) * nv));
+        C2G_CUDA(cudaMalloc(&w.qf[b], sizeof(float2) * nv));
         C2G_CUDA(cudaMalloc(&w.mark[b], sizeof(int) * mark_cap));
     }
     C2G_CUDA(cudaMalloc(&w.ctl, sizeof(TraversalCtl)));
@@ -532,10 +735,37 @@ static int ppr_alloc(c2g_graph* g) {
     return C2G_OK;
 }
 
-int build_reverse_graph(c2g_graph* g);
+// Out-edges of the frontier above which a round pulls (~0: never).  A pull costs its pass over all
+// in-edges, a push its frontier's out-edges (L2 atomics, 6.6e10 a second) and two barriers: at scale 20
+// (16M edges) a pull takes 94 us, and a query 4.46 ms with pulls above E / 3, 4.49 above E / 2, 4.51
+// above E / 5 and 6.05 with pulls only.  Up to kPullAlwaysPushEdges a pull is about as short as the two
+// barriers and dependent atomics of the emptiest push round (pulls only / both: 1M edges 0.90 / 1.02 ms a
+// query, 3.2M 1.61 / 1.84, 3.9M 1.89 / 1.87), so every round pulls.
+//
+// Pulls sum float pairs, so they need
+// weights below 2^30, a start below 2^60 and rmax of at least 1e-30 (as the batched push's pulls do),
+// and alpha < 1: a residual of 0 pushed at alpha = 1 cannot be told from a vertex outside the
+// frontier.
+constexpr int64_t kPushPullDiv = 3;
+
+static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& rows, unsigned* pull_min) {
+    *pull_min = ~0u;
+    const bool set = g->ppr_cfg.pull_set;
+    if (!rows.rec || !(pp.alpha < 1.f) || !(pp.rmax >= 1e-30f) || !(pp.r0 < 1e18f) || (set && g->ppr_cfg.pull_div <= 0))
+        return C2G_OK;
+    int rc;
+    if (!g->borrowed && (rc = ppr_pull_prepare(g))) return rc;
+    if (!g->wstat_valid || g->wstat_wmax_bits >= kPullMaxWeight) return C2G_OK;
+    if (set) {
+        *pull_min = (unsigned)(g->E / g->ppr_cfg.pull_div);
+        return C2G_OK;
+    }
+    *pull_min = g->E <= kPullAlwaysPushEdges ? 0u : (unsigned)(g->E / kPushPullDiv);
+    return C2G_OK;
+}
 
 int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int32_t* row_rev, const int2* adj_rev,
-                    const int32_t* mark_rev, int32_t source, const c2g_ppr_params& pp, float absorb, int32_t n_src,
+                    const RowLists& rows_rev, int32_t source, const c2g_ppr_params& pp, float absorb, int32_t n_src,
                     const int32_t* src_list, const float* src_r0, const int32_t* seed_v, const float* seed_w,
                     int32_t n_rec, float* pr_dev, float* res_dev, float* ms) {
     int rc;
@@ -550,13 +780,15 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
     p.E = (unsigned)g->E;
     p.row_r = row_rev;
     p.adj_r = adj_rev;
-    p.mark_r = mark_rev;
-    p.pull_div = row_rev ? g->ppr_cfg.pull_div : 0;
+    p.rows = rows_rev;
+    p.arrived = w.arrived;
+    if ((rc = ppr_pull_min(g, pp, rows_rev, &p.pull_min))) return rc;
     p.dense_div = g->ppr_cfg.dense_div;
     p.pr = pr_dev ? pr_dev : w.pr;
     p.res = w.res;
     p.msg = w.msg;
-    p.qd = w.qd;
+    p.qf[0] = w.qf[0];
+    p.qf[1] = w.qf[1];
     p.stamp = w.stamp;
     for (int b = 0; b < 2; ++b) {
         p.q[b] = w.q[b];
@@ -584,10 +816,26 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
     p.log_tile = w.log_tile;
     p.mark_cap = w.mark_cap;
     p.barrier_ns = g->barrier_ns ? g->barrier_ns : 2000000000ull;
+    int blocks = g->geom_ppr.blocks;
+    if (p.pull_min != ~0u) {
+        if (w.arrived_cap < rows_rev.n_long) {
+            if (w.arrived) cudaFree(w.arrived);
+            w.arrived = nullptr;
+            w.arrived_cap = 0;
+            C2G_CUDA(cudaMalloc(&w.arrived, sizeof(unsigned) * rows_rev.n_long));
+            w.arrived_cap = rows_rev.n_long;
+        }
+        p.arrived = w.arrived;
+        if (rows_rev.n_long)
+            C2G_CUDA(cudaMemsetAsync(w.arrived, 0, sizeof(unsigned) * rows_rev.n_long, g->stream));
+        // every round pulls: one warp per step of the row lists is enough
+        if (p.pull_min == 0u)
+            blocks = std::min(blocks, (int)((rows_rev.unit[kRowClasses] + kPprThreads / 32 - 1) / (kPprThreads / 32)));
+    }
     C2G_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(TraversalCtl), g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)ppr_persistent, dim3(g->geom_ppr.blocks),
+    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)ppr_persistent, dim3(blocks),
                                          dim3(g->geom_ppr.threads), args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     // FP64 residuals reach the caller as float.
@@ -602,19 +850,13 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
 
 int ppr_launch(c2g_graph* g, int32_t source, const c2g_ppr_params& pp, const int32_t* seed_v,
                const float* seed_w, int32_t n_rec, float* pr_dev, float* res_dev, float* ms) {
-    const int32_t* row_r = nullptr;
-    const int2* adj_r = nullptr;
-    const int32_t* mark_r = nullptr;
     if (!g->adj_f) return fail(C2G_ERR_UNSUPPORTED, "graph has no float weights (flist)");
-    if (g->ppr_cfg.pull_div > 0) {
+    if (g->ppr_cfg.pull_set && g->ppr_cfg.pull_div > 0) {  // asked for: built now if the graph was made without it
         int rc = build_reverse_graph(g);
         if (rc) return rc;
-        row_r = g->row_r;
-        adj_r = g->adj_r;
-        mark_r = g->mark_r;
     }
-    return ppr_launch_view(g, g->row, g->adj_f, row_r, adj_r, mark_r, source, pp, pp.alpha, 0, nullptr, nullptr,
-                           seed_v, seed_w, n_rec, pr_dev, res_dev, ms);
+    return ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->rows_in, source, pp, pp.alpha, 0, nullptr,
+                           nullptr, seed_v, seed_w, n_rec, pr_dev, res_dev, ms);
 }
 
 }  // namespace c2g

@@ -38,7 +38,6 @@
 #include "internal.h"
 
 namespace c2g {
-int build_reverse_graph(c2g_graph* g);
 void graph_free_view(c2g_graph* g);
 void session_set_grid_share(c2g_session* s, float share);
 }  // namespace c2g

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(512, 2) sssp_persistent(const SsspParams p) {
 // the next frontier in vertex order (entries, edge-base prefix, tile markers) and clears the
 // words: two grid barriers per round.
 //
-// Pull: every vertex v reads its in-edges, ordered by weight (in_rows.cu), as long as
+// Pull: every vertex v reads its in-edges, ordered by weight (in_edges.cu), as long as
 // w + (smallest frontier distance) < dist[v]: no later edge can improve v.  A push of a dense
 // frontier is bound by one random L2 read per out-edge of the frontier; in a pull most rows
 // end after one or two groups of 4 edges, hub rows too (their distance is small).  The warp

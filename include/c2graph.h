@@ -263,11 +263,11 @@ int c2g_ppr_batch(c2g_graph* g, int32_t n, const int32_t* sources, const c2g_ppr
                   float* pr, float* res, int on_device, int layout, c2g_stats* stats);
 
 /* Round shapes of the push kernel.  A round whose frontier has more than E / pull_div
- * out-edges pulls over the reverse CSR (built on first use) instead of pushing
- * (pull_div = 0, the default: never).  A push round whose frontier has more than
- * E / dense_div out-edges adds its messages without tracking first touches and applies
- * them in one sweep over all vertices (dense_div = 0: never; default 16).  Results are
- * the same BSP rounds either way. */
+ * out-edges pulls over the reverse CSR instead of pushing (0: never; until it is set, the
+ * library decides by the graph's size).  Pulls need rmax >= 1e-30 and finite weights.  A
+ * push round whose frontier has more than E / dense_div out-edges adds its messages
+ * without tracking first touches and applies them in one sweep over all vertices
+ * (dense_div = 0: never; default 16).  Results are the same BSP rounds either way. */
 int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div);
 
 /* Round shapes of the batched push (c2g_ppr_batch; no counterpart in the reference, which
