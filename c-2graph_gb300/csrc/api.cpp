@@ -230,6 +230,9 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->adj_r = base->adj_r;
     g->mark_r = base->mark_r;
     g->mark_f = base->mark_f;
+    g->r_bits = base->r_bits;
+    g->r_prefix = base->r_prefix;
+    g->r_rows = base->r_rows;
     g->rows_in = base->rows_in;
     g->in_row = base->in_row;
     g->in_adj = base->in_adj;

@@ -71,16 +71,6 @@ struct BatchParams {
     int* qmin;  // [3][Q]
 };
 
-// A warp's chunk of up to 32 in-edges of a pull round (batched PPR), staged in shared memory: source, weight bits and
-// the source's active lanes in the item's 4 query words.  Each lane loads one in-edge and
-// the live ones (a source with an active lane) are compacted into the chunk; the warp
-// then reads them one by one as broadcasts (two shared loads per in-edge instead of six
-// shuffles, and the chunk's values leave the registers of the gather loop).
-struct PullChunk {
-    int2 ed[32];
-    uint4 mk[32];
-};
-
 // Warp tiles of the expansion: markers are laid every 2^kBatchTileLog edge-word steps; a
 // round with enough work (at least 2^tile_min_log big tiles per warp) walks tiles of
 // 2^tile_big_log steps (every 2^(big - kBatchTileLog)-th marker), a smaller one tiles of
@@ -1151,12 +1141,13 @@ struct PprBatchParams {
     unsigned qcap, mark_cap;
     unsigned long long barrier_ns;
     long long* counters;  // [2] pushes (query, edge), edge-word steps
-    // pull rounds: reverse CSR (source, weight bits) with tile owners; a round pulls when
-    // its pushes exceed pull_min
-    const int* row_r;
+    // pull rounds: reverse CSR (source, weight bits); a round pulls when its pushes exceed
+    // pull_min
     const int2* adj_r;
-    const int* mark_r;
-    unsigned ntiles_r;
+    const unsigned* r_bits;   // per chunk of 32 in-edges: which start a row,
+    const int* r_prefix;      // how many rows start in earlier chunks,
+    const int* r_rows;        // and the rows in order
+    int pull_log;             // log2 of the chunks per pull item
     unsigned long long pull_min;
     int epoch_rounds;  // > 0: an epoch of a resident batch (state at rest in the arrays; at most this many rounds)
     int cur0;          // round index the epoch starts at (its parity picks the frontier buffers)
@@ -1176,11 +1167,10 @@ __device__ __forceinline__ FrontierOut pbatch_out(const PprBatchParams& p, int b
     return o;
 }
 
-// Launch shape of the batched PPR: 2 blocks of 512 threads per SM (64 registers).  With the
-// pull rounds staged through shared memory it beats 3 x 384 (56 registers) by about 1% at
-// 256 sources, scale 22 (766 vs 775 ms: faster pulls, slower pushes) and 4 x 256 (778 ms);
-// before the staging 3 x 384 had been the faster one (962 vs 1,030 ms).
-constexpr int kPprBatchThreads = 512;
+// Launch shape of the batched PPR: 2 blocks of 448 threads per SM (72 registers).  Measured with the
+// pull rounds' chunk streams, 256 queries at scale 21 / 40 at scale 16: 448 threads 368 / 10.0 ms, 512
+// (64 registers, more spills) 383 / 10.8, 384 390 / 9.7; 3 x 384 and 4 x 256 lost before that.
+constexpr int kPprBatchThreads = 448;
 constexpr int kPprBatchBlocksPerSm = 2;
 constexpr int kPprBatchUnroll = 3;  // push items in flight per lane
 
@@ -1319,33 +1309,56 @@ __device__ __forceinline__ unsigned pbatch_sweep(const PprBatchParams& p, bool f
 // (about 47 bits of relative precision): the product is hi*w + lo*w with its rounding
 // error recovered by an FMA, and each add is an error-free two-sum whose error joins lo.
 // Relative precision matters here, not absolute: a message sum decides res > rmax at the
-// scale of rmax, far below the largest sums.  A target whose in-edges lie in one tile is
-// applied by the warp that summed them; only targets whose in-edges cross a tile boundary
-// add their parts to msg (FP64 atomics) for the apply sweep that follows, as after a push.
-// In-edges are cut into tiles of 2^kPullTileLog; warps take (tile, word group) items from
-// the round's queue, kPullWords query words per item.
-constexpr int kPullWords = 4;  // query words per pull item
-constexpr int kPullEdges = 2;  // in-edges whose rq rows are gathered before they are summed
+// scale of rmax, far below the largest sums.
+//
+// In-edges are cut into chunks of 32 and items of 2^pull_log chunks; warps take (item, group of
+// 4 query words) from the round's queue.  Within a warp the chunks form one stream: while a
+// chunk is summed, the next one's activity masks and the one after's in-edges are copied to
+// shared memory (cp.async: no registers held), across rows and items alike; the row
+// boundaries inside a chunk come from one word of start bits, not from the row pointer.
+// (Row by row, each row cost a chain of three dependent loads before its first gather, and
+// narrow batches left most of an item's 4 words empty: 40 queries at scale 16 took 28.0 ms a
+// batch, now 10.0; 256 at scale 21 395, now 368.)  What bounds a dense round of a wide batch is
+// the gathers' bytes, 8 per push, at about 6 TB/s out of L2, and about 60 instructions per
+// (in-edge, item).  A target whose in-edges lie in one item is applied by the warp that summed
+// them; only targets whose in-edges cross an item boundary add their parts to msg (FP64
+// atomics) for the apply sweep that follows, as after a push.
+constexpr int kPullInFlight = 8;  // (in-edge, query word) rows gathered before they are summed
+
+struct PPullSmem {  // one warp's
+    uint4 mk[2][32];  // sources' active lanes of a chunk
+    int2 ed[3][32];   // in-edges (source, weight bits) of a chunk
+};
+
+__device__ __forceinline__ void cp_async4(void* s, const void* g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+__device__ __forceinline__ void cp_async8(void* s, const void* g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+__device__ __forceinline__ void cp_async16(void* s, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Owner v's message sums of the item's words are complete (hi + lo per lane).  An owner
-// whose in-edges lie in this tile has them all: it is applied here, by the pulling warp
+// whose in-edges lie in this item has them all: it is applied here, by the pulling warp
 // (the pullers read the other round parity's rq pairs and activity masks, so this apply
-// does not disturb them).  An owner whose in-edges cross a tile boundary adds its part to
+// does not disturb them).  An owner whose in-edges cross an item boundary adds its part to
 // msg in FP64 (atomics) and marks tmask; the apply after the barrier finishes it.  The
 // first part to mark a (vertex, word) appends it to slist (counter sctr), so that apply
-// visits only the listed words instead of sweeping all V * W (at most one owner straddles
-// each tile boundary, so the list holds at most ntiles_r * W words).
-__device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, int v, unsigned w0, bool whole,
-                                                      const float (&sh)[kPullWords], const float (&sl)[kPullWords],
+// visits only the listed words instead of sweeping all V * W.  dg: v's out-degree.
+template <int WP>
+__device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, int v, int dg, unsigned w0, bool whole,
+                                                      const float (&sh)[WP], const float (&sl)[WP],
                                                       int ob, unsigned long long rmax_bits, WarpStage& fst,
                                                       const FrontierOut& out, unsigned* dctr, unsigned* sctr,
                                                       unsigned long long& psum, int lane) {
-    const unsigned W = 1u << p.logW;
     unsigned cnt = 0;
     if (!whole) {
 #pragma unroll
-        for (int j = 0; j < kPullWords; ++j) {
-            if (w0 + j >= W) break;  // warp-uniform
+        for (int j = 0; j < WP; ++j) {
             const bool nz = sh[j] != 0.f;
             const unsigned bits = __ballot_sync(kFull, nz);
             if (bits) {
@@ -1361,19 +1374,17 @@ __device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, i
         }
         return 0;
     }
-    const int dg = __ldg(p.row + v + 1) - __ldg(p.row + v);
-    double r[kPullWords];
-    float pv[kPullWords];
+    double r[WP];
+    float pv[WP];
 #pragma unroll
-    for (int j = 0; j < kPullWords; ++j) {
+    for (int j = 0; j < WP; ++j) {
         const size_t off = (size_t)v * (size_t)p.Q + ((w0 + j) << 5) + lane;
         const bool nz = sh[j] != 0.f;
         r[j] = nz ? ldcg(p.res + off) : 0.0;
         pv[j] = nz ? ldcg(p.pr + off) : 0.f;
     }
 #pragma unroll
-    for (int j = 0; j < kPullWords; ++j) {
-        if (w0 + j >= W) break;  // warp-uniform
+    for (int j = 0; j < WP; ++j) {
         const bool nz = sh[j] != 0.f;
         if (!__any_sync(kFull, nz)) continue;
         cnt += nz ? 1u : 0u;
@@ -1386,143 +1397,215 @@ __device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, i
     return cnt;
 }
 
-// Phase A of a pull round.  A warp takes (tile, word group) items from the round's queue
-// and walks the tile's owners one by one: for each owner, its in-edges in the tile in
-// chunks of 32 (loaded lane-parallel and staged in pc), the pushed residuals of
-// kPullEdges in-edges gathered before they are summed, two query words per packed
-// instruction (f32x2.h).
+// Position in a warp's stream of chunks.
+struct PPullPos {
+    unsigned c;   // chunk; ~0: beyond the last item
+    unsigned wf;  // first query word of the item's group | kPullFirst | kPullLast (chunk of its item)
+};
+constexpr unsigned kPullFirst = 1u << 31, kPullLast = 1u << 30;
+__device__ __forceinline__ unsigned pull_w0(const PPullPos& q) { return q.wf & ~(kPullFirst | kPullLast); }
+
+// Phase A of a pull round.
+template <int WP>
 __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf, int ob, unsigned* qctr,
-                                                PullChunk& pc, WarpStage& fst, const FrontierOut& out, unsigned* dctr,
+                                                PPullSmem& sm, WarpStage& fst, const FrontierOut& out, unsigned* dctr,
                                                 unsigned* sctr, unsigned long long& psum, int lane, bool& bad) {
-    const unsigned W = 1u << p.logW;
-    const int lg = p.logW >= 2 ? p.logW - 2 : 0;  // word groups per tile = 2^lg (kPullWords = 4)
-    const unsigned nitems = p.ntiles_r << lg;
+    constexpr int EF = kPullInFlight / WP;  // in-edges in flight
+    constexpr int NP = (WP + 1) / 2;        // packed word pairs
+    const unsigned nchunks = (p.E + 31u) >> 5;
+    const unsigned per_group = (nchunks + (1u << p.pull_log) - 1u) >> p.pull_log;
+    const unsigned nitems = per_group << (p.logW - (WP == 4 ? 2 : WP == 2 ? 1 : 0));
     const unsigned* am = p.amask[buf];
-    const float2* rqb = p.rqf[buf];
-    const unsigned tw = 1u << kPullTileLog;
+    const float2* rql = p.rqf[buf] + lane;
+    const unsigned lane_bit = 1u << lane;
     const unsigned long long rmax_bits = c2g_dbits((double)p.rmax);
     unsigned cnt = 0;
-    unsigned itn = next_tile(qctr, lane);
-    for (unsigned it = itn; it < nitems; it = itn) {
-        itn = next_tile(qctr, lane);  // the next item, fetched while this one runs
-        // word group major: all tiles of one word group, then the next, so the residual
-        // rows that L2 holds for the busiest sources are one word group's (1 KB per source,
-        // not 2 at 256 queries): 818 vs 843 ms per 256-query batch at scale 22
-        const unsigned t = it % p.ntiles_r;
-        const unsigned w0 = (it / p.ntiles_r) * (unsigned)kPullWords;
-        const unsigned e0 = t << kPullTileLog;
-        const unsigned e1 = min(e0 + tw, p.E);
-        int v = __ldg(p.mark_r + t);  // owner of in-edge e0
-        unsigned vs = (unsigned)__ldg(p.row_r + v);
-        for (;;) {
-            const unsigned ve = (unsigned)__ldg(p.row_r + v + 1);
-            const unsigned ea = max(vs, e0), ez = min(ve, e1);
-            if (ea < ez) {  // warp-uniform: v has in-edges in this tile
-                // message sums hi + lo of words (0, 1) and (2, 3), packed
-                f32x2 sh2[kPullWords / 2], sl2[kPullWords / 2];
-#pragma unroll
-                for (int j = 0; j < kPullWords / 2; ++j) sh2[j] = sl2[j] = 0ull;
-                for (unsigned b = ea; b < ez; b += 32u) {
-                    const unsigned e = b + (unsigned)lane;
-                    int src = 0;
-                    float wt = 0.f;
-                    unsigned mk[kPullWords];
-#pragma unroll
-                    for (int j = 0; j < kPullWords; ++j) mk[j] = 0u;
-                    if (e < ez) {
-                        const int2 ed = __ldg(p.adj_r + e);
-                        if ((unsigned)ed.x >= (unsigned)p.V) {
-                            bad = true;
-                        } else if (ed.y > 0) {  // positive weights only, as the push
-                            src = ed.x;
-                            wt = __int_as_float(ed.y);
-                            const unsigned* ms = am + ((size_t)(unsigned)src << p.logW) + w0;
-                            if (W >= 4u) {  // four words, 16-byte aligned
-                                const uint4 m4 = ldcg(reinterpret_cast<const uint4*>(ms));
-                                mk[0] = m4.x;
-                                mk[1] = m4.y;
-                                mk[2] = m4.z;
-                                mk[3] = m4.w;
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < kPullWords; ++j)
-                                    if ((unsigned)j < W) mk[j] = ldcg(ms + j);
-                            }
-                        }
-                    }
-                    // only in-edges whose source has an active lane in the item's words are
-                    // staged (in order): the others would add exact zeros
-                    const bool live = (mk[0] | mk[1] | mk[2] | mk[3]) != 0u;
-                    const unsigned lm = __ballot_sync(kFull, live);
-                    const unsigned n = (unsigned)__popc(lm);
-                    __syncwarp();  // the previous chunk's reads are done
-                    if (live) {
-                        const unsigned at = (unsigned)__popc(lm & ((1u << lane) - 1u));
-                        pc.ed[at] = make_int2(src, __float_as_int(wt));
-                        pc.mk[at] = make_uint4(mk[0], mk[1], mk[2], mk[3]);
-                    }
-                    __syncwarp();
-                    for (unsigned k0 = 0; k0 < n; k0 += kPullEdges) {
-                        // gather the pushed residuals of kPullEdges in-edges, then add them
-                        float2 qb[kPullEdges][kPullWords];
-                        float wk[kPullEdges];
-#pragma unroll
-                        for (int h = 0; h < kPullEdges; ++h) {
-                            const unsigned k = k0 + h < n ? k0 + h : n - 1u;
-                            const int2 ek = pc.ed[k];
-                            const uint4 mq = pc.mk[k];
-                            wk[h] = __int_as_float(ek.y);
-                            const int u = ek.x;
-#pragma unroll
-                            for (int j = 0; j < kPullWords; ++j) {
-                                const unsigned mj = j == 0 ? mq.x : j == 1 ? mq.y : j == 2 ? mq.z : mq.w;
-                                const bool on = k0 + h < n && ((mj >> lane) & 1u);
-                                qb[h][j] = on ? ldcg(rqb + ((size_t)(unsigned)u << (p.logW + 5)) + ((w0 + j) << 5) +
-                                                     lane)
-                                              : make_float2(0.f, 0.f);
-                            }
-                        }
-#pragma unroll
-                        for (int h = 0; h < kPullEdges; ++h) {
-                            const f32x2 w2 = f2_pack(wk[h], wk[h]);
-                            const f32x2 nw2 = f2_pack(-wk[h], -wk[h]);
-#pragma unroll
-                            for (int j = 0; j < kPullWords / 2; ++j) {
-                                // message (hi + lo) * w = pm + pe; two-sum of sh + pm, for words
-                                // 2j and 2j+1 at once.  npm = -pm exactly (round-to-nearest is
-                                // symmetric), so every line rounds as the scalar form
-                                //   pm = hi*w, pe = fma(lo, w, fma(hi, w, -pm)), s = sh + pm,
-                                //   bv = s - sh, av = s - bv, te = (sh - av) + (pm - bv),
-                                //   sl += te + pe, sh = s
-                                // does: pm - bv = -(npm + bv).
-                                const f32x2 hi = f2_pack(qb[h][2 * j].x, qb[h][2 * j + 1].x);
-                                const f32x2 lo = f2_pack(qb[h][2 * j].y, qb[h][2 * j + 1].y);
-                                const f32x2 npm = f2_mul(hi, nw2);
-                                const f32x2 pe = f2_fma(lo, w2, f2_fma(hi, w2, npm));
-                                const f32x2 s2 = f2_sub(sh2[j], npm);
-                                const f32x2 bv = f2_sub(s2, sh2[j]);
-                                const f32x2 av = f2_sub(s2, bv);
-                                const f32x2 te = f2_sub(f2_sub(sh2[j], av), f2_add(npm, bv));
-                                sl2[j] = f2_add(sl2[j], f2_add(te, pe));
-                                sh2[j] = s2;
-                            }
-                        }
-                    }
-                }
-                float sh[kPullWords], sl[kPullWords];
-#pragma unroll
-                for (int j = 0; j < kPullWords / 2; ++j) {
-                    f2_unpack(sh2[j], sh[2 * j], sh[2 * j + 1]);
-                    f2_unpack(sl2[j], sl[2 * j], sl[2 * j + 1]);
-                }
-                cnt += pbatch_pull_owner(p, v, w0, vs >= e0 && ve <= e1, sh, sl, ob, rmax_bits, fst, out, dctr,
-                                         sctr, psum, lane);
-            }
-            if (ve >= e1) break;
-            ++v;
-            vs = ve;
+
+    unsigned raw = 0;  // lane 0: the next item, taken from the queue ahead of its use
+    auto take = [&]() {
+        if (lane == 0) raw = atomicAdd(qctr, 1u);
+    };
+    auto item_start = [&]() {
+        unsigned it = (unsigned)__shfl_sync(kFull, (int)raw, 0);
+        PPullPos q{~0u, kPullLast};
+        if (it < nitems) {
+            // from the end of the edge range: items of many short rows cost most (each row is an
+            // apply), and in a skewed graph they lie behind the hubs; first, they do not end the
+            // round alone (dense rounds, 256 queries: scale 18 2.2 -> 1.6 ms, scale 21 11.3 -> 10.4)
+            it = nitems - 1u - it;
+            // word group major: all items of one word group, then the next, so the residual
+            // rows that L2 holds for the busiest sources are one word group's (1 KB per source,
+            // not 2 at 256 queries): 818 vs 843 ms per 256-query batch at scale 22
+            q.c = (it % per_group) << p.pull_log;
+            q.wf = (it / per_group) * (unsigned)WP | kPullFirst;
+            if (p.pull_log == 0 || q.c + 1u == nchunks) q.wf |= kPullLast;
+            take();
         }
+        return q;
+    };
+    auto next = [&](const PPullPos& q) {
+        if (q.c == ~0u) return q;
+        if (q.wf & kPullLast) return item_start();
+        PPullPos r{q.c + 1u, q.wf & ~kPullFirst};
+        if (((r.c + 1u) & ((1u << p.pull_log) - 1u)) == 0u || r.c + 1u == nchunks) r.wf |= kPullLast;
+        return r;
+    };
+    auto load_edges = [&](const PPullPos& q, int slot) {
+        if (q.c == ~0u) return;
+        const unsigned e = (q.c << 5) + (unsigned)lane;
+        if (e < p.E)
+            cp_async8(&sm.ed[slot][lane], p.adj_r + e);
+        else
+            sm.ed[slot][lane] = make_int2(0, 0);
+    };
+    auto load_masks = [&](const PPullPos& q, int eslot, int mslot) {
+        if (q.c == ~0u) return;
+        const int2 e = sm.ed[eslot][lane];
+        uint4* to = &sm.mk[mslot][lane];
+        if ((unsigned)e.x >= (unsigned)p.V) bad = true;
+        if (e.y > 0 && (unsigned)e.x < (unsigned)p.V) {  // positive weights only, as the push
+            const unsigned line = ((unsigned)e.x << p.logW) + pull_w0(q);  // the source's first line of the item
+            sm.ed[eslot][lane].x = (int)line;
+            const unsigned* ms = am + line;
+            if (WP == 4)
+                cp_async16(to, ms);
+            else if (WP == 2)
+                cp_async8(to, ms);
+            else
+                cp_async4(to, ms);
+        } else {
+            *to = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+
+    take();
+    PPullPos q0 = item_start(), q1 = next(q0);
+    load_edges(q0, 0);
+    load_edges(q1, 1);
+    cp_async_commit();
+    cp_async_wait();
+    __syncwarp();
+    load_masks(q0, 0, 0);
+    cp_async_commit();
+    // message sums hi + lo of the words, packed in pairs
+    f32x2 sh2[NP], sl2[NP];
+    bool whole = false, any = false;  // the row started inside the item; it has a live in-edge
+    for (int e0 = 0, m0 = 0; q0.c != ~0u; e0 = e0 == 2 ? 0 : e0 + 1, m0 ^= 1) {
+        const int e1 = e0 == 2 ? 0 : e0 + 1, e2 = e1 == 2 ? 0 : e1 + 1;
+        const PPullPos q2 = next(q1);
+        const unsigned starts = __ldg(p.r_bits + q0.c);
+        const unsigned follow = q0.c + 1u < nchunks ? __ldg(p.r_bits + q0.c + 1u) & 1u : 1u;
+        const unsigned base = (unsigned)__ldg(p.r_prefix + q0.c) + (starts & 1u) - 1u;
+        const unsigned len = min(32u, p.E - (q0.c << 5));
+        // the chunk's rows, one per lane: vertex and out-degree
+        int rv = 0, rdeg = 0;
+        if ((unsigned)lane <= (unsigned)__popc(starts & ~1u)) {
+            rv = __ldg(p.r_rows + base + (unsigned)lane);
+            rdeg = __ldg(p.row + rv + 1) - __ldg(p.row + rv);
+        }
+        cp_async_wait();  // this chunk's masks, the next one's edges
+        __syncwarp();
+        load_edges(q2, e2);
+        load_masks(q1, e1, m0 ^ 1);
+        cp_async_commit();
+        unsigned mine;
+        {
+            const uint4 m = sm.mk[m0][lane];
+            mine = WP == 4 ? m.x | m.y | m.z | m.w : WP == 2 ? m.x | m.y : m.x;
+        }
+        // only in-edges whose source has an active lane in the item's words are visited: the
+        // others would add exact zeros
+        const unsigned lm = __ballot_sync(kFull, mine != 0u);
+        if (q0.wf & kPullFirst) {
+            whole = false;
+            any = false;
+#pragma unroll
+            for (int j = 0; j < NP; ++j) sh2[j] = sl2[j] = 0ull;
+        }
+        unsigned pos = 0u;
+        for (int i = 0; pos < len; ++i) {
+            if ((starts >> pos) & 1u) {
+                whole = true;
+                any = false;
+#pragma unroll
+                for (int j = 0; j < NP; ++j) sh2[j] = sl2[j] = 0ull;
+            }
+            const unsigned after = pos == 31u ? 0u : starts & ~((2u << pos) - 1u);
+            const unsigned nxt = after ? (unsigned)__ffs((int)after) - 1u : len;
+            unsigned l = lm & (nxt == 32u ? ~0u : (1u << nxt) - 1u) & ~((1u << pos) - 1u);
+            any = any || l != 0u;
+            while (l) {
+                // gather the pushed residuals of EF in-edges, then add them
+                float2 qb[EF][WP];
+                float wk[EF];
+#pragma unroll
+                for (int h = 0; h < EF; ++h) {
+                    const bool have = l != 0u;
+                    const int k = __clz((int)__brev(l)) & 31;
+                    l &= l - 1u;
+                    const int2 ek = sm.ed[e0][k];
+                    const uint4 mq = sm.mk[m0][k];
+                    wk[h] = __int_as_float(ek.y);
+                    const float2* line = rql + (size_t)(unsigned)ek.x * 32u;
+                    const unsigned bit = have ? lane_bit : 0u;
+#pragma unroll
+                    for (int j = 0; j < WP; ++j) {
+                        const unsigned mj = j == 0 ? mq.x : j == 1 ? mq.y : j == 2 ? mq.z : mq.w;
+                        qb[h][j] = mj & bit ? ldcg(line + 32 * j) : make_float2(0.f, 0.f);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < EF; ++h) {
+                    const f32x2 w2 = f2_pack(wk[h], wk[h]);
+                    const f32x2 nw2 = f2_pack(-wk[h], -wk[h]);
+#pragma unroll
+                    for (int j = 0; j < NP; ++j) {
+                        // message (hi + lo) * w = pm + pe; two-sum of sh + pm, for words
+                        // 2j and 2j+1 at once.  npm = -pm exactly (round-to-nearest is
+                        // symmetric), so every line rounds as the scalar form
+                        //   pm = hi*w, pe = fma(lo, w, fma(hi, w, -pm)), s = sh + pm,
+                        //   bv = s - sh, av = s - bv, te = (sh - av) + (pm - bv),
+                        //   sl += te + pe, sh = s
+                        // does: pm - bv = -(npm + bv).
+                        const float2 qa = qb[h][2 * j], qc = 2 * j + 1 < WP ? qb[h][(2 * j + 1) % WP] : make_float2(0.f, 0.f);
+                        const f32x2 hi = f2_pack(qa.x, qc.x);
+                        const f32x2 lo = f2_pack(qa.y, qc.y);
+                        const f32x2 npm = f2_mul(hi, nw2);
+                        const f32x2 pe = f2_fma(lo, w2, f2_fma(hi, w2, npm));
+                        const f32x2 s2 = f2_sub(sh2[j], npm);
+                        const f32x2 bv = f2_sub(s2, sh2[j]);
+                        const f32x2 av = f2_sub(s2, bv);
+                        const f32x2 te = f2_sub(f2_sub(sh2[j], av), f2_add(npm, bv));
+                        sl2[j] = f2_add(sl2[j], f2_add(te, pe));
+                        sh2[j] = s2;
+                    }
+                }
+            }
+            const bool ends = nxt < len || follow != 0u;
+            if (any && (ends || (q0.wf & kPullLast))) {
+                float sh[WP], sl[WP];
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    float a, b, c, d;
+                    f2_unpack(sh2[j], a, b);
+                    f2_unpack(sl2[j], c, d);
+                    sh[2 * j] = a;
+                    sl[2 * j] = c;
+                    if (2 * j + 1 < WP) {
+                        sh[(2 * j + 1) % WP] = b;
+                        sl[(2 * j + 1) % WP] = d;
+                    }
+                }
+                cnt += pbatch_pull_owner<WP>(p, __shfl_sync(kFull, rv, i), __shfl_sync(kFull, rdeg, i), pull_w0(q0),
+                                             whole && ends, sh, sl, ob, rmax_bits, fst, out, dctr, sctr, psum, lane);
+            }
+            pos = nxt;
+        }
+        __syncwarp();
+        q0 = q1;
+        q1 = q2;
     }
+    cp_async_wait();
     stage_flush(fst, out);
     return cnt;
 }
@@ -1564,8 +1647,13 @@ __device__ __noinline__ void pbatch_rebuild(const PprBatchParams& p, int b, int 
     if (lane == 0 && ps) atomicAdd(&p.ctl->pcount[slot], ps);
 }
 
+// WP: query words of a pull item (1, 2, or 4 of four or more).  Dynamic shared memory: a PPullSmem per warp.
+constexpr size_t kPprBatchSmem = sizeof(PPullSmem) * (kPprBatchThreads / 32);
+
+template <int WP>
 __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
     ppr_batch_persistent(const PprBatchParams p) {
+    extern __shared__ uint4 pull_smem[];
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
     grid_sync_init();
@@ -1580,7 +1668,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
     const int wib = threadIdx.x >> 5;
     WarpStage fst{sm.v0[wib], sm.d0[wib], sm.x0[wib], 0};
     int* qtab = sm.v1[wib];  // slot -> query position table of the owner being expanded
-    __shared__ PullChunk pcs[kPprBatchThreads / 32];  // pull rounds' in-edge chunks
+    PPullSmem& psm = reinterpret_cast<PPullSmem*>(pull_smem)[wib];
     const double one_m_a = 1.0 - (double)p.alpha;
     unsigned long long tph = globaltimer_ns();
     unsigned long long psum = 0;  // next round's pushes counted by this warp (lane 0)
@@ -1710,7 +1798,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
                 pushes += (long long)P;
                 steps += T;
             }
-            touched += pbatch_pull(p, buf, ob, &ctl->tilectr[cur % 3], pcs[wib], fst, pbatch_out(p, ob, nslot),
+            touched += pbatch_pull<WP>(p, buf, ob, &ctl->tilectr[cur % 3], psm, fst, pbatch_out(p, ob, nslot),
                                    &ctl->dctr[nslot], &ctl->listctr[cur % 3], psum, lane, bad);
         } else {
             // Push round, phase A: push along the frontier's edges (owner runs, as in the
@@ -1891,6 +1979,28 @@ __global__ void batch_transpose_d2f(const double* __restrict__ src, int V, int Q
     }
 }
 
+// The kernel for 2^logW query words, with its shared memory allowed, and its blocks per SM.
+static int ppr_batch_kernel(int logW, const void** kernel, int* per_sm) {
+    *kernel = logW == 0 ? (const void*)ppr_batch_persistent<1>
+            : logW == 1 ? (const void*)ppr_batch_persistent<2>
+                        : (const void*)ppr_batch_persistent<4>;
+    C2G_CUDA(cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPprBatchSmem));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, *kernel, kPprBatchThreads, kPprBatchSmem));
+    if (*per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
+    return C2G_OK;
+}
+
+// log2 of the chunks of 32 in-edges per pull item: 8 chunks (a fourth of the rows then crosses an item
+// boundary), fewer where that leaves the grid's warps less than 16 items each to level the round's
+// end (40 queries at scale 16, 6 chunks per warp: 8-chunk items 14.8 ms a batch, 2 12.8, 1 11.7).
+static int ppr_pull_log(const c2g_graph* g, int logW, int blocks) {
+    const size_t groups = logW >= 2 ? size_t(1) << (logW - 2) : 1;
+    const size_t chunks = ((size_t)g->E + 31) / 32, warps = (size_t)blocks * (kPprBatchThreads / 32);
+    int k = 3;
+    while (k > 0 && (chunks >> k) * groups < 16 * warps) --k;
+    return k;
+}
+
 struct PprBatchWork {
     float* pr = nullptr;
     double* res = nullptr;
@@ -1954,9 +2064,8 @@ static int ppr_batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
     C2G_CUDA(cudaMalloc(&w->rqf[0], sizeof(float2) * VQ));
     C2G_CUDA(cudaMalloc(&w->rqf[1], sizeof(float2) * VQ));
     C2G_CUDA(cudaMalloc(&w->tmask, sizeof(unsigned) * qcap));
-    // pull rounds' straddlers: at most one owner per in-edge tile boundary, W words each
-    const size_t ntiles_r = (((size_t)g->E + (1u << kPullTileLog) - 1) >> kPullTileLog) + 1;
-    w->slist_cap = (unsigned)std::min(qcap, ntiles_r * W);
+    // pull rounds' straddlers: at most one owner per chunk boundary, W words each
+    w->slist_cap = (unsigned)std::min(qcap, (((size_t)g->E >> 5) + 1) * W);
     C2G_CUDA(cudaMalloc(&w->slist, sizeof(unsigned) * w->slist_cap));
     C2G_CUDA(cudaMalloc(&w->dmask, sizeof(unsigned) * qcap));
     C2G_CUDA(cudaMalloc(&w->amask[0], sizeof(unsigned) * qcap));
@@ -2088,10 +2197,11 @@ static void ppr_batch_params(c2g_graph* g, PprBatchWork* w, int Q, int logW, con
     p.mark_cap = (unsigned)((((size_t)g->E * (size_t)(p.Q / 32)) >> kBatchTileLog) + 2);
     p.barrier_ns = g->barrier_ns ? g->barrier_ns : 4000000000ull;
     p.counters = w->counters;
-    p.row_r = g->row_r;
     p.adj_r = g->adj_r;
-    p.mark_r = g->mark_r;
-    p.ntiles_r = (unsigned)(((size_t)g->E + (1u << kPullTileLog) - 1) >> kPullTileLog);
+    p.r_bits = g->r_bits;
+    p.r_prefix = g->r_prefix;
+    p.r_rows = g->r_rows;
+    p.pull_log = 3;
     p.pull_min = pull_min;
     p.trace = w->trace;
     g->last_trace = w->trace;
@@ -2116,10 +2226,10 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     if ((rc = ppr_batch_alloc(g, Q, ns))) return rc;
     PprBatchWork* w = reinterpret_cast<PprBatchWork*>(g->ppr_batch);
     int coop = 0, per_sm = 0;
+    const void* kernel = nullptr;
     C2G_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
     if (!coop) return fail(C2G_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ppr_batch_persistent, kPprBatchThreads, 0));
-    if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
+    if ((rc = ppr_batch_kernel(logW, &kernel, &per_sm))) return rc;
     const size_t VQ = (size_t)g->V * (size_t)w->Q;
     if ((rc = ppr_batch_clean(g, w))) return rc;
     C2G_CUDA(cudaMemcpyAsync(w->src, sources, sizeof(int) * (size_t)nq, cudaMemcpyHostToDevice, g->stream));
@@ -2135,13 +2245,13 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     ppr_batch_params(g, w, Q, logW, prm, pull_min, p);
     p.nq = nq;
     p.seed_off = seed_off ? w->seed_off : nullptr;
+    const int blocks = grid_blocks(g, per_sm);
+    p.pull_log = ppr_pull_log(g, logW, blocks);
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    const int blocks = grid_blocks(g, per_sm);
-    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)ppr_batch_persistent, dim3(blocks), dim3(kPprBatchThreads), args,
-                                         0, g->stream));
+    C2G_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kPprBatchThreads), args, kPprBatchSmem, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     cudaError_t e = cudaSuccess;
     float* outs[2] = {pr_out, res_out};
@@ -2218,10 +2328,12 @@ int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, in
     unsigned long long pull_min = ~0ull;
     if ((rc = ppr_pull_threshold(g, prm, &pull_min))) return rc;
     int per_sm = 0;
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ppr_batch_persistent, kPprBatchThreads, 0));
-    if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
+    const void* kernel = nullptr;
+    if ((rc = ppr_batch_kernel(logW, &kernel, &per_sm))) return rc;
     PprBatchParams p;
     ppr_batch_params(g, w, Q, logW, prm, pull_min, p);
+    const int blocks = grid_blocks(g, per_sm);
+    p.pull_log = ppr_pull_log(g, logW, blocks);
     p.epoch_rounds = rounds < 1 ? 1 : rounds;
     p.cur0 = cur0;
     p.max_iter = 1 << 30;  // the per-query caps are the session's
@@ -2229,8 +2341,7 @@ int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, in
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel((const void*)ppr_batch_persistent, dim3(grid_blocks(g, per_sm)),
-                                         dim3(kPprBatchThreads), args, 0, g->stream));
+    C2G_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kPprBatchThreads), args, kPprBatchSmem, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     C2G_CUDA(cudaMemcpyAsync(ctl_out, w->ctl, sizeof(TraversalCtl), cudaMemcpyDeviceToHost, g->stream));
     C2G_CUDA(cudaMemcpyAsync(counters, w->counters, sizeof(long long) * 2, cudaMemcpyDeviceToHost, g->stream));

@@ -17,6 +17,7 @@
 // arrays takes 68.2 ms with the rows and 63.5 ms without.
 #include <algorithm>
 #include <climits>
+#include <cstdint>
 
 #include "device_common.cuh"
 #include "internal.h"
@@ -262,6 +263,31 @@ __global__ void __launch_bounds__(kInSortThreads) in_sort_long(const int* __rest
     }
 }
 
+// Row starts of a CSR by chunk of 32 edges: bit e % 32 of bits[e / 32] says that edge e starts a row.
+__global__ void start_bits(const int* __restrict__ row, int V, unsigned* __restrict__ bits) {
+    const int stride = gridDim.x * blockDim.x;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += stride) {
+        const int rs = __ldg(row + v);
+        if (__ldg(row + v + 1) > rs) atomicOr(bits + (rs >> 5), 1u << (rs & 31));
+    }
+}
+
+__global__ void start_counts(const unsigned* __restrict__ bits, int n, int* __restrict__ count) {
+    const int stride = gridDim.x * blockDim.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) count[i] = __popc(__ldg(bits + i));
+}
+
+// The non-empty rows in order, from the starts before each chunk.
+__global__ void start_rows(const int* __restrict__ row, int V, const unsigned* __restrict__ bits,
+                           const int* __restrict__ prefix, int* __restrict__ rows) {
+    const int stride = gridDim.x * blockDim.x;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += stride) {
+        const int rs = __ldg(row + v);
+        if (__ldg(row + v + 1) > rs)
+            rows[__ldg(prefix + (rs >> 5)) + __popc(__ldg(bits + (rs >> 5)) & ((1u << (rs & 31)) - 1u))] = v;
+    }
+}
+
 // Class of a row of n edges (RowLists).
 __device__ __forceinline__ int row_class(int n) {
     int c = 0;
@@ -385,6 +411,8 @@ static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd) {
     return e;
 }
 
+static int build_row_starts(c2g_graph* g);
+
 // Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), its tile owners and its rows by
 // length; built when the graph is made (one with int32 weights only: on first use).
 int build_reverse_graph(c2g_graph* g) {
@@ -423,11 +451,41 @@ int build_reverse_graph(c2g_graph* g) {
     if (!rc) rc = build_markers(g, g->row_r, &g->mark_r);
     if (!rc) rc = build_markers(g, g->row, &g->mark_f);
     if (!rc) rc = build_row_lists(g, g->row_r, g->row, &g->rows_in);
+    if (!rc) rc = build_row_starts(g);
     if (rc) {
         cudaGetLastError();
         reverse_free(g);
     }
     return rc;
+}
+
+// Row starts of the reverse CSR by chunk.
+static int build_row_starts(c2g_graph* g) {
+    const size_t V = (size_t)g->V, n = ((size_t)g->E + 31) / 32;
+    if (n == 0) return C2G_OK;
+    const int scan_blocks = (int)((n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems));
+    int* tmp = nullptr;  // counts | cursors (unused) | scan block sums | stats
+    C2G_CUDA(cudaMalloc(&tmp, sizeof(int) * (2 * n + (size_t)scan_blocks) + 256));
+    int *count = tmp, *cursor = tmp + n, *sums = cursor + n;
+    cudaError_t e = cudaMalloc(&g->r_bits, sizeof(unsigned) * n);
+    if (e == cudaSuccess) e = cudaMalloc(&g->r_prefix, sizeof(int) * (n + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&g->r_rows, sizeof(int) * V);
+    if (e == cudaSuccess) e = cudaMemsetAsync(g->r_bits, 0, sizeof(unsigned) * n, g->stream);
+    if (e == cudaSuccess) {
+        InStats* st = reinterpret_cast<InStats*>((reinterpret_cast<uintptr_t>(sums + scan_blocks) + 63) & ~(uintptr_t)63);
+        const int blocks = g->num_sms * 8;
+        start_bits<<<blocks, 256, 0, g->stream>>>(g->row_r, g->V, g->r_bits);
+        start_counts<<<blocks, 256, 0, g->stream>>>(g->r_bits, (int)n, count);
+        in_scan_blocks<<<scan_blocks, kScanThreads, 0, g->stream>>>(count, (int)n, 0, sums, st);
+        in_scan_sums<<<1, kScanThreads, 0, g->stream>>>(sums, scan_blocks);
+        in_scan_rows<<<scan_blocks, kScanThreads, 0, g->stream>>>(count, (int)n, 0, sums, g->r_prefix, cursor, nullptr, st);
+        start_rows<<<blocks, 256, 0, g->stream>>>(g->row_r, g->V, g->r_bits, g->r_prefix, g->r_rows);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    cudaFree(tmp);
+    C2G_CUDA(e);
+    return C2G_OK;
 }
 
 // New float weights: the reverse CSR's rows stay, their edges are written anew.
@@ -439,8 +497,12 @@ int refresh_reverse_graph(c2g_graph* g) {
 }
 
 void reverse_free(c2g_graph* g) {
-    for (void* p : {(void*)g->row_r, (void*)g->adj_r, (void*)g->mark_r, (void*)g->mark_f})
+    for (void* p : {(void*)g->row_r, (void*)g->adj_r, (void*)g->mark_r, (void*)g->mark_f, (void*)g->r_bits,
+                    (void*)g->r_prefix, (void*)g->r_rows})
         if (p) cudaFree(p);
+    g->r_bits = nullptr;
+    g->r_prefix = nullptr;
+    g->r_rows = nullptr;
     row_lists_free(g->rows_in);
     row_lists_free(g->rows_out);
     g->wstat_valid = false;

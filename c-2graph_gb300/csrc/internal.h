@@ -170,6 +170,11 @@ struct c2g_graph {
     int in_shift = 0;           // weights are ordered up to their low in_shift bits
     int32_t* mark_r = nullptr;  // pull-tile owner markers over row_r
     int32_t* mark_f = nullptr;  // pull-tile owner markers over row (the adjoint's gradient pass)
+    // the reverse CSR's row starts by chunk of 32 in-edges (batched push): start bits, rows that start in
+    // earlier chunks, non-empty rows in order
+    unsigned* r_bits = nullptr;
+    int32_t* r_prefix = nullptr;
+    int32_t* r_rows = nullptr;
     c2g::RowLists rows_in;      // rows of row_r by length
     c2g::RowLists rows_out;     // rows of row by length (the adjoint's push on the reverse graph), on demand
     // pruned records
