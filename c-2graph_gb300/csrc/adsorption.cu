@@ -9,18 +9,27 @@
 // fixed number of times from Y = I.  The abandonment share p_abnd(v) goes to the dummy
 // "none" label, which is not stored.
 //
-// One iteration is a pull over the reverse CSR: the in-edges of all vertices form one
-// range [0, E) cut into tiles of 2^kPullTileLog edges; a group of 4 lanes (each holding 4
-// of the 16 labels as a float4) walks a tile from its marker's owner, its in-edges staged
-// through shared memory 32 at a time (16-byte loads, read back as broadcasts: 41.98 vs
-// 42.80 ms per query at scale 22 against shuffling them within the group), accumulating
-// per-owner sums in registers, and writes each owner's row with a plain store when the
-// owner's in-edges lie inside the tile, otherwise with atomicAdd (only owners straddling
-// a tile boundary).  kAdsBatch label rows are gathered before they are used.  A vertex
-// pass then applies p_inj / p_cont.
+// One iteration is one kernel: a pull over the reverse CSR that applies p_inj / p_cont on
+// the spot and writes the next label rows, between two row buffers.  The in-edges of all
+// vertices form one range [0, E) cut into tiles, one per warp, and a tile into eight equal
+// stretches, one per group of 4 lanes (each lane holds 4 of the 16 labels).  A group walks
+// its stretch in order: the in-edges come through shared memory 32 at a time (cp.async, two
+// buffers), the label rows of kAdsBatch in-edges are in flight while those before them are
+// summed, and a bitmap of row starts says where a row ends.  A row that lies inside a
+// stretch is written by its group; one that crosses stretches is summed over the groups by
+// shuffles; one that crosses tiles leaves a partial sum per tile, and the warp that arrives
+// last adds them up, in order.
+// What bounds a large graph is the label-row gathers, 64 bytes per in-edge: 65 M of them
+// take 0.55 ms an iteration at scale 22, 7.6 TB/s into the SMs (a third of the rows from
+// DRAM).  Before, a group found each row's end in the row pointer (a dependent load per
+// row), wrote sums to memory for a vertex pass, and an iteration took 1.40 ms.  30 iterations
+// at scale 22: 16.6 ms with 2 rows ahead and 8 blocks per SM; 17.0 with 7; 18.0 with 4 rows
+// ahead and 8 blocks, 17.8 with 6, 21.5 with 8 rows and 4 blocks: more warps, each with fewer
+// rows in registers.  What bounds a small one is the chain of loads through a stretch.
 // Per iteration: (8 + 64) bytes per edge (in-edge record + source label row) and
-// 64 + 64 + 12 bytes per vertex.  The iteration sequence is captured once per handle
-// (and iteration count) into a CUDA graph and replayed; its buffers stay with the handle.
+// 64 + 16 bytes per vertex with in-edges.  The iteration sequence is captured once per
+// handle (and iteration count) into a CUDA graph and replayed; its buffers stay with the
+// handle.
 #include <cstring>
 #include <vector>
 
@@ -31,122 +40,253 @@ namespace c2g {
 
 constexpr int kAdsL = 16;          // labels per query
 
-constexpr int kAdsBatch = 8;      // in-edges whose label rows a group gathers at once
-constexpr int kAdsMinBlocks = 3;  // launch bounds: resident 256-thread blocks per SM
-constexpr int kAdsThreads = 256;
+constexpr int kAdsBatch = 2;       // in-edges whose label rows a group gathers ahead
+constexpr int kAdsMinBlocks = 8;   // launch bounds: resident 128-thread blocks per SM
+constexpr int kAdsThreads = 128;
+constexpr int kAdsWarps = kAdsThreads / 32;
+constexpr int64_t kAdsFill = 1;    // tiles per resident warp below which tiles get smaller
 constexpr int kAdsChunk = 32;     // in-edges a group stages in shared memory at a time
 
-__global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks) ads_edge_pass(const int* __restrict__ row_r,
-                                                                            const int2* __restrict__ adj_r,
-                              const int* __restrict__ mark_r, int V, unsigned E, const float4* __restrict__ Y,
-                              float* __restrict__ acc) {
-    const int lane = threadIdx.x & 31;
-    const int part = lane & 3;                   // labels 4*part .. 4*part+3 of every row
-    const int g0 = lane & ~3;                    // first lane of this 4-lane group
-    const unsigned gmask = 0xfu << g0;           // the group's lanes (groups diverge)
-    const unsigned ngroups = (gridDim.x * blockDim.x) >> 2;
-    const unsigned tw = 1u << kPullTileLog;
-    const unsigned ntiles = (E + tw - 1) >> kPullTileLog;
-    // each group's staged in-edges; one pad entry per row, so that the 8 groups of a warp,
-    // reading entry k of their rows at once, hit 8 different bank pairs
-    __shared__ int2 staged[kAdsThreads / 4][kAdsChunk + 1];
-    int2* const st = staged[threadIdx.x >> 2];
-    for (unsigned t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; t < ntiles; t += ngroups) {
-        const unsigned e0 = t << kPullTileLog;
-        const unsigned e1 = min(e0 + tw, E);
-        int v = __ldg(mark_r + t);               // owner of in-edge e0
-        unsigned vend = (unsigned)__ldg(row_r + v + 1);
-        bool whole = (unsigned)__ldg(row_r + v) >= e0;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (unsigned c = e0; c < e1; c += kAdsChunk) {
-            // stage the chunk: each lane loads 2 in-edges at a time (16-byte loads; c is even)
-            __syncwarp(gmask);  // the previous chunk's reads are done
+struct AdsPass {
+    const int* row_r;
+    const int2* adj_r;
+    const unsigned* r_bits;   // per chunk of 32 in-edges: which start a row,
+    const int* r_prefix;      // and how many rows start in earlier chunks
+    const int4* coef;         // per row with in-edges, in order: vertex, p_cont, p_inj, seed mask
+    const float* p_inj;
+    const int* seeds;
+    float4* slots;            // per tile: sum of the row that enters it, of the row that leaves it
+    unsigned* arrived;        // per tile: tiles of the row leaving it that have left their sums
+    int V;
+    unsigned E;
+    int tile_log;             // a tile holds 2^tile_log in-edges, eight stretches of whole chunks
+};
+
+__device__ __forceinline__ void ads_apply(float4* __restrict__ out, const int4 c, int part, const float4 s) {
+    const float pc = __int_as_float(c.y), pi = __int_as_float(c.z);
+    const int m = c.w >> (4 * part);
+    float4 y;
+    y.x = fmaf(pc, s.x, m & 1 ? pi : 0.f);
+    y.y = fmaf(pc, s.y, m & 2 ? pi : 0.f);
+    y.z = fmaf(pc, s.z, m & 4 ? pi : 0.f);
+    y.w = fmaf(pc, s.w, m & 8 ? pi : 0.f);
+    out[(size_t)c.x * (kAdsL / 4) + part] = y;
+}
+
+__device__ __forceinline__ float4 ads_add(const float4 a, const float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+__device__ __forceinline__ float4 ads_shfl_up(const float4 a, int d) {
+    return make_float4(__shfl_up_sync(~0u, a.x, d), __shfl_up_sync(~0u, a.y, d), __shfl_up_sync(~0u, a.z, d),
+                       __shfl_up_sync(~0u, a.w, d));
+}
+
+// out = p_cont * (sum over in-edges of w * Y) + p_inj * I for every vertex with in-edges; row V of Y is zero.
+__global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
+    ads_iterate(const AdsPass p, const float4* __restrict__ Y, float4* __restrict__ out) {
+    // each group's staged in-edges, two chunks; 16 bytes of padding per row, so that the 8
+    // groups of a warp, reading 16 bytes of their rows at once, hit different banks
+    __shared__ __align__(16) int2 staged[kAdsWarps][2][8][kAdsChunk + 2];
+    __shared__ float4 heads[kAdsThreads];
+    if (blockIdx.x == 0 && threadIdx.x < kAdsL) {  // a seed without in-edges keeps its injection alone
+        const int v = __ldg(p.seeds + threadIdx.x);
+        if (__ldg(p.row_r + v) == __ldg(p.row_r + v + 1))
+            reinterpret_cast<float*>(out)[(size_t)v * kAdsL + threadIdx.x] = __ldg(p.p_inj + v);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int part = lane & 3, grp = lane >> 2;  // labels 4*part .. 4*part+3 of the group's rows
+    const unsigned t = blockIdx.x * kAdsWarps + warp;
+    const unsigned stretch = 1u << (p.tile_log - 3);
+    const unsigned e0 = (t << p.tile_log) + (unsigned)grp * stretch;
+    if ((t << p.tile_log) >= p.E) return;  // warp-uniform, no block barrier below
+    const unsigned e1 = min(e0 + stretch, p.E);
+    const bool act = e0 < p.E;
+    const unsigned words = (p.E + 31) / 32;
+    unsigned word = e0 >> 5;
+    unsigned bits = act ? __ldg(p.r_bits + word) : 0u;
+    const bool starts = bits & 1u;         // the stretch's first in-edge starts a row
+    const int first = act ? __ldg(p.r_prefix + word) + (int)starts - 1 : 0;  // its row
+    int row = first;
+    int4 coef = act ? __ldg(p.coef + first) : make_int4(0, 0, 0, 0);
+    bits &= ~1u;
+    bool head = !starts;                   // the row being summed began before the stretch
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+
+    const auto stage = [&](unsigned c) {
+        int2* const to = staged[warp][c & 1u][grp];
+        const unsigned base = e0 + c * kAdsChunk;
+        if (base + kAdsChunk <= p.E) {
 #pragma unroll
-            for (int r = 0; r < kAdsChunk / 8; ++r) {
-                const unsigned idx = c + 2u * part + 8u * r;
-                int4 two = make_int4(0, 0, 0, 0);
-                if (idx + 1 < e1) {
-                    two = __ldg(reinterpret_cast<const int4*>(adj_r + idx));
-                } else if (idx < e1) {
-                    const int2 one = __ldg(adj_r + idx);
-                    two.x = one.x;
-                    two.y = one.y;
-                }
-                st[2 * part + 8 * r] = make_int2(two.x, two.y);
-                st[2 * part + 8 * r + 1] = make_int2(two.z, two.w);
-            }
-            __syncwarp(gmask);
-            const unsigned cend = min(c + kAdsChunk, e1);
-            for (unsigned b = c; b < cend; b += kAdsBatch) {
-                // kAdsBatch in-edges read from the stage (broadcast within the group), their
-                // label rows gathered together, then consumed in order
-                float4 y[kAdsBatch];
-                float wt[kAdsBatch];
-#pragma unroll
-                for (int k = 0; k < kAdsBatch; ++k) {
-                    const int2 ek = st[b - c + k];
-                    wt[k] = __int_as_float(ek.y);
-                    y[k] = b + k < e1 ? __ldg(Y + (size_t)ek.x * (kAdsL / 4) + part) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int k = 0; k < kAdsBatch; ++k) {
-                    const unsigned e = b + k;
-                    if (e >= e1) break;  // group-uniform
-                    while (e >= vend) {  // owner changes: write the finished owner's row part
-                        float* o = acc + (size_t)v * kAdsL + 4 * part;
-                        if (whole) {
-                            *reinterpret_cast<float4*>(o) = s;
-                        } else {
-                            atomicAdd(o, s.x);
-                            atomicAdd(o + 1, s.y);
-                            atomicAdd(o + 2, s.z);
-                            atomicAdd(o + 3, s.w);
-                        }
-                        s = make_float4(0.f, 0.f, 0.f, 0.f);
-                        ++v;
-                        whole = true;  // rows starting inside the tile
-                        vend = (unsigned)__ldg(row_r + v + 1);
-                    }
-                    s.x = fmaf(wt[k], y[k].x, s.x);
-                    s.y = fmaf(wt[k], y[k].y, s.y);
-                    s.z = fmaf(wt[k], y[k].z, s.z);
-                    s.w = fmaf(wt[k], y[k].w, s.w);
-                }
-            }
+            for (int r = 0; r < kAdsChunk / 8; ++r)
+                cp_async16(to + 2 * part + 8 * r, p.adj_r + base + 2 * part + 8 * r);
+        } else {  // beyond the last in-edge: the zero row
+#pragma unroll 1
+            for (unsigned i = part; i < kAdsChunk; i += 4)
+                to[i] = base + i < p.E ? __ldg(p.adj_r + base + i) : make_int2(p.V, 0);
         }
-        float* o = acc + (size_t)v * kAdsL + 4 * part;
-        if (whole && vend <= e1) {
-            *reinterpret_cast<float4*>(o) = s;
-        } else {
-            atomicAdd(o, s.x);
-            atomicAdd(o + 1, s.y);
-            atomicAdd(o + 2, s.z);
-            atomicAdd(o + 3, s.w);
+    };
+    float4 y[2][kAdsBatch];
+    float w[2][kAdsBatch];
+    const auto gather = [&](int b, const int2* from) {
+#pragma unroll
+        for (int k = 0; k < kAdsBatch; k += 2) {
+            const int4 two = *reinterpret_cast<const int4*>(from + k);
+            w[b][k] = __int_as_float(two.y);
+            w[b][k + 1] = __int_as_float(two.w);
+            y[b][k] = __ldg(Y + (size_t)two.x * (kAdsL / 4) + part);
+            y[b][k + 1] = __ldg(Y + (size_t)two.z * (kAdsL / 4) + part);
         }
+    };
+    const auto consume = [&](int b) {
+#pragma unroll
+        for (int k = 0; k < kAdsBatch; ++k) {
+            if (bits & (1u << k)) {  // a new row: the one before is complete
+                if (head) {
+                    heads[threadIdx.x] = s;
+                    head = false;
+                } else {
+                    ads_apply(out, coef, part, s);
+                }
+                s = make_float4(0.f, 0.f, 0.f, 0.f);
+                ++row;
+                coef = __ldg(p.coef + row);
+            }
+            s.x = fmaf(w[b][k], y[b][k].x, s.x);
+            s.y = fmaf(w[b][k], y[b][k].y, s.y);
+            s.z = fmaf(w[b][k], y[b][k].z, s.z);
+            s.w = fmaf(w[b][k], y[b][k].w, s.w);
+        }
+        bits >>= kAdsBatch;
+    };
+
+    const unsigned chunks = stretch / kAdsChunk;
+    stage(0);
+    cp_async_commit();
+    if (chunks > 1) stage(1);
+    cp_async_commit();
+    cp_async_wait_but<1>();
+    __syncwarp();
+    gather(0, staged[warp][0][grp]);
+    for (unsigned c = 0; c < chunks; ++c) {
+        const int2* const st = staged[warp][c & 1u][grp];
+        const unsigned next_bits = c + 1 < chunks && word + 1 < words ? __ldg(p.r_bits + word + 1) : 0u;
+        ++word;
+#pragma unroll 1
+        for (int b = 0; b < kAdsChunk - 2 * kAdsBatch; b += 2 * kAdsBatch) {
+            gather(1, st + b + kAdsBatch);
+            consume(0);
+            gather(0, st + b + 2 * kAdsBatch);
+            consume(1);
+        }
+        gather(1, st + kAdsChunk - kAdsBatch);
+        consume(0);
+        if (c + 1 < chunks) {
+            cp_async_wait_but<0>();
+            __syncwarp();  // the next chunk is there, and this one is read
+            if (c + 2 < chunks) stage(c + 2);
+            cp_async_commit();
+            gather(0, staged[warp][(c + 1) & 1u][grp]);
+        }
+        consume(1);
+        bits = next_bits;
+    }
+    __syncwarp();
+
+    // the row at the end of each stretch, summed over the stretches that it crosses
+    const bool had_head = !starts && !head;  // a row that began before the stretch ended in it
+    const bool done = act && (e1 == p.E || (__ldg(p.r_bits + (e1 >> 5)) & 1u));
+    int f = starts || had_head;              // it began in the tile
+#pragma unroll
+    for (int d = 1; d < 8; d *= 2) {
+        const float4 ps = ads_shfl_up(s, 4 * d);
+        const int pf = __shfl_up_sync(~0u, f, 4 * d);
+        if (grp >= d) {
+            if (!f) s = ads_add(s, ps);
+            f |= pf;
+        }
+    }
+    float4 enter = ads_shfl_up(s, 4);
+    int enter_f = __shfl_up_sync(~0u, f, 4);
+    if (grp == 0) {
+        enter = make_float4(0.f, 0.f, 0.f, 0.f);
+        enter_f = 0;
+    }
+    if (had_head) {
+        enter = ads_add(enter, heads[threadIdx.x]);
+        if (enter_f) ads_apply(out, __ldg(p.coef + first), part, enter);
+    }
+    if (done && f) ads_apply(out, coef, part, s);
+    // rows that cross tiles: at most one enters the tile (its group: in), one leaves it (out)
+    const bool in_row = act && ((had_head && !enter_f) || (!f && (done || grp == 7)));
+    const bool out_row = act && grp == 7 && !done && f;
+    const unsigned any_in = __ballot_sync(~0u, in_row), any_out = __ballot_sync(~0u, out_row);
+    if (!(any_in | any_out)) return;
+    if (in_row) p.slots[(size_t)t * 8 + part] = had_head ? enter : s;
+    if (out_row) p.slots[(size_t)t * 8 + 4 + part] = s;
+    __threadfence();
+    __syncwarp();
+    unsigned ts[2] = {0, 0}, te[2] = {0, 0};
+    int rows[2] = {0, 0};
+    int last[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const unsigned any = k ? any_out : any_in;
+        if (!any) continue;  // warp-uniform
+        const int src = __ffs(any) - 1;
+        rows[k] = __shfl_sync(~0u, k ? row : first, src);
+        const int v = __ldg(&p.coef[rows[k]].x);
+        ts[k] = (unsigned)__ldg(p.row_r + v) >> p.tile_log;
+        te[k] = (unsigned)(__ldg(p.row_r + v + 1) - 1) >> p.tile_log;
+        if (lane == 0) {
+            last[k] = atomicAdd(p.arrived + ts[k], 1u) == te[k] - ts[k];
+            if (last[k]) p.arrived[ts[k]] = 0u;  // for the next iteration
+        }
+    }
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (!__shfl_sync(~0u, last[k], 0)) continue;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (grp == 0) sum = __ldcg(p.slots + (size_t)ts[k] * 8 + 4 + part);
+#pragma unroll 4
+        for (unsigned i = ts[k] + 1 + (unsigned)grp; i <= te[k]; i += 8)
+            sum = ads_add(sum, __ldcg(p.slots + (size_t)i * 8 + part));
+#pragma unroll
+        for (int d = 4; d < 32; d *= 2) {
+            sum.x += __shfl_xor_sync(~0u, sum.x, d);
+            sum.y += __shfl_xor_sync(~0u, sum.y, d);
+            sum.z += __shfl_xor_sync(~0u, sum.z, d);
+            sum.w += __shfl_xor_sync(~0u, sum.w, d);
+        }
+        if (grp == 0) ads_apply(out, __ldg(p.coef + rows[k]), part, sum);
     }
 }
 
-// Y[v][l] = p_cont(v) * acc[v][l] + (label l seeded at v ? p_inj(v) : 0); acc = 0.
-__global__ void ads_vertex_pass(int V, const float* __restrict__ p_inj, const float* __restrict__ p_cont,
-                                const unsigned* __restrict__ seedmask, float* __restrict__ acc, float* __restrict__ Y) {
-    const size_t n = (size_t)V * kAdsL;
+// Y0 = I (seed labels) and its zero row, Y1 = p_inj * I for the rows that no iteration writes,
+// and the coefficients of the rows with in-edges, in their order.
+__global__ void ads_init(const AdsPass p, const float* __restrict__ p_cont, const unsigned* __restrict__ seedmask,
+                         float4* __restrict__ Y0, float4* __restrict__ Y1, int4* __restrict__ coef) {
+    const size_t n = ((size_t)p.V + 1) * (kAdsL / 4);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const size_t v = i / kAdsL;
-        const int l = (int)(i % kAdsL);
-        const float inj = ((seedmask[v] >> l) & 1u) ? p_inj[v] : 0.f;
-        Y[i] = fmaf(p_cont[v], acc[i], inj);
-        acc[i] = 0.f;
-    }
-}
-
-// Y = I (seed labels), acc = 0.
-__global__ void ads_init(int V, const unsigned* __restrict__ seedmask, float* __restrict__ acc, float* __restrict__ Y) {
-    const size_t n = (size_t)V * kAdsL;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        Y[i] = ((seedmask[i / kAdsL] >> (i % kAdsL)) & 1u) ? 1.f : 0.f;
-        acc[i] = 0.f;
+        const int v = (int)(i / (kAdsL / 4)), part = (int)(i % (kAdsL / 4));
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v == p.V) {
+            Y0[i] = zero;
+            Y1[i] = zero;
+            continue;
+        }
+        const unsigned mask = seedmask[v], m = mask >> (4 * part);
+        Y0[i] = make_float4(m & 1u, (m >> 1) & 1u, (m >> 2) & 1u, (m >> 3) & 1u);
+        const int r0 = __ldg(p.row_r + v);
+        if (r0 == __ldg(p.row_r + v + 1)) {
+            ads_apply(Y1, make_int4(v, 0, __float_as_int(p.p_inj[v]), (int)mask), part, zero);
+        } else if (part == 0) {
+            const unsigned before = __ldg(p.r_bits + (r0 >> 5)) & ((1u << (r0 & 31)) - 1u);
+            coef[__ldg(p.r_prefix + (r0 >> 5)) + __popc(before)] =
+                make_int4(v, __float_as_int(p_cont[v]), __float_as_int(p.p_inj[v]), (int)mask);
+        }
     }
 }
 
@@ -161,25 +301,38 @@ __global__ void ads_seed_mask(const int* __restrict__ seeds, int n, unsigned* __
 // cudaFree synchronise the device and would stall the other kinds' batches), with the
 // iteration sequence captured once into a CUDA graph and replayed.
 struct AdsWork {
-    float* Y = nullptr;    // [V][16]
-    float* acc = nullptr;  // [V][16]
+    float* Y[2] = {nullptr, nullptr};  // [V + 1][16], row V zero
+    int4* coef = nullptr;              // [V]
+    float4* slots = nullptr;           // [tiles][2][16 floats]
+    unsigned* arrived = nullptr;       // [tiles], zero between iterations
     unsigned* mask = nullptr;
     float* pi = nullptr;
     float* pc = nullptr;
     int* seeds = nullptr;  // [16]
     cudaGraphExec_t exec = nullptr;
     int iterations = -1;
+    int tile_log = 0;
 };
 
 void ads_free(c2g_graph* g) {
     AdsWork* w = reinterpret_cast<AdsWork*>(g->ads);
     if (!w) return;
     if (w->exec) cudaGraphExecDestroy(w->exec);
-    void* ptrs[] = {w->Y, w->acc, w->mask, w->pi, w->pc, w->seeds};
+    void* ptrs[] = {w->Y[0], w->Y[1], w->coef, w->slots, w->arrived, w->mask, w->pi, w->pc, w->seeds};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     delete w;
     g->ads = nullptr;
+}
+
+// In-edges per tile (log2): eight stretches of 128, shorter ones where that leaves the SMs short of
+// warps.  30 iterations at scale 22: 16.6 ms with 1024-edge tiles, 20.4 with 512, 25.8 with 256 (a
+// tile's start and end are chains of loads); at scale 18 1.25 ms with 512, 1.36 with 256.
+static int ads_tile_log(const c2g_graph* g) {
+    const int64_t warps = (int64_t)g->num_sms * kAdsMinBlocks * kAdsWarps;
+    int log = 10;
+    while (log > 8 && ((int64_t)g->E >> log) < kAdsFill * warps) --log;
+    return log;
 }
 
 static int ads_alloc(c2g_graph* g, AdsWork** out) {
@@ -188,35 +341,43 @@ static int ads_alloc(c2g_graph* g, AdsWork** out) {
         w = new AdsWork();
         g->ads = w;
         const size_t V = g->V ? (size_t)g->V : 1;
-        C2G_CUDA(cudaMalloc(&w->Y, sizeof(float) * V * kAdsL));
-        C2G_CUDA(cudaMalloc(&w->acc, sizeof(float) * V * kAdsL));
-        C2G_CUDA(cudaMalloc(&w->mask, sizeof(unsigned) * V));
-        C2G_CUDA(cudaMalloc(&w->pi, sizeof(float) * V));
-        C2G_CUDA(cudaMalloc(&w->pc, sizeof(float) * V));
-        C2G_CUDA(cudaMalloc(&w->seeds, sizeof(int) * kAdsL));
+        w->tile_log = ads_tile_log(g);
+        const size_t tiles = ((size_t)g->E >> w->tile_log) + 1;
+        cudaError_t e = cudaMalloc(&w->Y[0], sizeof(float) * (V + 1) * kAdsL);
+        if (e == cudaSuccess) e = cudaMalloc(&w->Y[1], sizeof(float) * (V + 1) * kAdsL);
+        if (e == cudaSuccess) e = cudaMalloc(&w->coef, sizeof(int4) * V);
+        if (e == cudaSuccess) e = cudaMalloc(&w->slots, sizeof(float) * tiles * 2 * kAdsL);
+        if (e == cudaSuccess) e = cudaMalloc(&w->arrived, sizeof(unsigned) * tiles);
+        if (e == cudaSuccess) e = cudaMemsetAsync(w->arrived, 0, sizeof(unsigned) * tiles, g->stream);
+        if (e == cudaSuccess) e = cudaMalloc(&w->mask, sizeof(unsigned) * V);
+        if (e == cudaSuccess) e = cudaMalloc(&w->pi, sizeof(float) * V);
+        if (e == cudaSuccess) e = cudaMalloc(&w->pc, sizeof(float) * V);
+        if (e == cudaSuccess) e = cudaMalloc(&w->seeds, sizeof(int) * kAdsL);
+        if (e != cudaSuccess) ads_free(g);
+        C2G_CUDA(e);
     }
     *out = w;
     return C2G_OK;
 }
 
-// Capture init + `iterations` x (edge pass, vertex pass) on the handle's stream.
+// Capture init + `iterations` passes on the handle's stream; the result is in Y[iterations & 1].
 static int ads_capture(c2g_graph* g, AdsWork* w, int iterations) {
     if (w->exec && w->iterations == iterations) return C2G_OK;
     if (w->exec) {
         cudaGraphExecDestroy(w->exec);
         w->exec = nullptr;
     }
+    const AdsPass p{g->row_r, g->adj_r, g->r_bits, g->r_prefix, w->coef, w->pi, w->seeds, w->slots, w->arrived,
+                    g->V,     (unsigned)g->E, w->tile_log};
+    const unsigned tile_edges = kAdsWarps << w->tile_log;
+    const int blocks = (int)(((size_t)g->E + tile_edges - 1) / tile_edges);
+    float4* const Y[2] = {reinterpret_cast<float4*>(w->Y[0]), reinterpret_cast<float4*>(w->Y[1])};
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const int eb = g->num_sms * 8, vb = g->num_sms * 8;
-        ads_init<<<vb, 256, 0, g->stream>>>(g->V, w->mask, w->acc, w->Y);
-        for (int it = 0; it < iterations; ++it) {
-            if (g->E)
-                ads_edge_pass<<<eb, kAdsThreads, 0, g->stream>>>(g->row_r, g->adj_r, g->mark_r, g->V, (unsigned)g->E,
-                                                          reinterpret_cast<const float4*>(w->Y), w->acc);
-            ads_vertex_pass<<<vb, 256, 0, g->stream>>>(g->V, w->pi, w->pc, w->mask, w->acc, w->Y);
-        }
+        ads_init<<<g->num_sms * 8, 256, 0, g->stream>>>(p, w->pc, w->mask, Y[0], Y[1], w->coef);
+        for (int it = 0; it < iterations; ++it)  // without in-edges one block writes the seeds' rows
+            ads_iterate<<<blocks ? blocks : 1, kAdsThreads, 0, g->stream>>>(p, Y[it & 1], Y[(it + 1) & 1]);
         e = cudaStreamEndCapture(g->stream, &graph);
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&w->exec, graph, 0);
@@ -272,7 +433,7 @@ extern "C" int c2g_adsorption(c2g_graph* g, int32_t n_labels, const int32_t* see
     if (e == cudaSuccess) e = cudaGraphLaunch(w->exec, g->stream);
     if (e == cudaSuccess) e = cudaEventRecord(g->ev1, g->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(Y_out, w->Y, sizeof(float) * V * kAdsL,
+        e = cudaMemcpyAsync(Y_out, w->Y[iterations & 1], sizeof(float) * V * kAdsL,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, g->ev0, g->ev1);

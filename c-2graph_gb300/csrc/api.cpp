@@ -228,7 +228,6 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->adj_f = base->adj_f;
     g->row_r = base->row_r;
     g->adj_r = base->adj_r;
-    g->mark_r = base->mark_r;
     g->mark_f = base->mark_f;
     g->r_bits = base->r_bits;
     g->r_prefix = base->r_prefix;

@@ -1330,18 +1330,6 @@ struct PPullSmem {  // one warp's
     int2 ed[3][32];   // in-edges (source, weight bits) of a chunk
 };
 
-__device__ __forceinline__ void cp_async4(void* s, const void* g) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
-}
-__device__ __forceinline__ void cp_async8(void* s, const void* g) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
-}
-__device__ __forceinline__ void cp_async16(void* s, const void* g) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
 // Owner v's message sums of the item's words are complete (hi + lo per lane).  An owner
 // whose in-edges lie in this item has them all: it is applied here, by the pulling warp
 // (the pullers read the other round parity's rq pairs and activity masks, so this apply
@@ -1483,7 +1471,7 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
     load_edges(q0, 0);
     load_edges(q1, 1);
     cp_async_commit();
-    cp_async_wait();
+    cp_async_wait_but<0>();
     __syncwarp();
     load_masks(q0, 0, 0);
     cp_async_commit();
@@ -1503,7 +1491,7 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
             rv = __ldg(p.r_rows + base + (unsigned)lane);
             rdeg = __ldg(p.row + rv + 1) - __ldg(p.row + rv);
         }
-        cp_async_wait();  // this chunk's masks, the next one's edges
+        cp_async_wait_but<0>();  // this chunk's masks, the next one's edges
         __syncwarp();
         load_edges(q2, e2);
         load_masks(q1, e1, m0 ^ 1);
@@ -1605,7 +1593,7 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
         q0 = q1;
         q1 = q2;
     }
-    cp_async_wait();
+    cp_async_wait_but<0>();
     stage_flush(fst, out);
     return cnt;
 }

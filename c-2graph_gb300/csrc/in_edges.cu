@@ -413,8 +413,8 @@ static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd) {
 
 static int build_row_starts(c2g_graph* g);
 
-// Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), its tile owners and its rows by
-// length; built when the graph is made (one with int32 weights only: on first use).
+// Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), its rows by length and by
+// chunk, the forward CSR's tile owners; built when the graph is made (one with int32 weights only: on first use).
 int build_reverse_graph(c2g_graph* g) {
     if (g->adj_r) return C2G_OK;
     const int2* fwd = g->adj_f ? g->adj_f : g->adj_w;  // float weights when the graph has them
@@ -448,7 +448,6 @@ int build_reverse_graph(c2g_graph* g) {
     int rc = C2G_OK;
     if (e != cudaSuccess)
         rc = fail(e == cudaErrorMemoryAllocation ? C2G_ERR_OOM : C2G_ERR_CUDA, "reverse CSR: %s", cudaGetErrorString(e));
-    if (!rc) rc = build_markers(g, g->row_r, &g->mark_r);
     if (!rc) rc = build_markers(g, g->row, &g->mark_f);
     if (!rc) rc = build_row_lists(g, g->row_r, g->row, &g->rows_in);
     if (!rc) rc = build_row_starts(g);
@@ -497,7 +496,7 @@ int refresh_reverse_graph(c2g_graph* g) {
 }
 
 void reverse_free(c2g_graph* g) {
-    for (void* p : {(void*)g->row_r, (void*)g->adj_r, (void*)g->mark_r, (void*)g->mark_f, (void*)g->r_bits,
+    for (void* p : {(void*)g->row_r, (void*)g->adj_r, (void*)g->mark_f, (void*)g->r_bits,
                     (void*)g->r_prefix, (void*)g->r_rows})
         if (p) cudaFree(p);
     g->r_bits = nullptr;
@@ -508,7 +507,6 @@ void reverse_free(c2g_graph* g) {
     g->wstat_valid = false;
     g->row_r = nullptr;
     g->adj_r = nullptr;
-    g->mark_r = nullptr;
     g->mark_f = nullptr;
 }
 

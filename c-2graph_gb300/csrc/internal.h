@@ -168,10 +168,9 @@ struct c2g_graph {
     int2* in_seg = nullptr;     // (vertex, first edge): rows behind their first kInHead edges, kInSegment edges each
     unsigned in_segs = 0;
     int in_shift = 0;           // weights are ordered up to their low in_shift bits
-    int32_t* mark_r = nullptr;  // pull-tile owner markers over row_r
     int32_t* mark_f = nullptr;  // pull-tile owner markers over row (the adjoint's gradient pass)
-    // the reverse CSR's row starts by chunk of 32 in-edges (batched push): start bits, rows that start in
-    // earlier chunks, non-empty rows in order
+    // the reverse CSR's row starts by chunk of 32 in-edges (batched push, label propagation): start
+    // bits, rows that start in earlier chunks, non-empty rows in order
     unsigned* r_bits = nullptr;
     int32_t* r_prefix = nullptr;
     int32_t* r_rows = nullptr;
