@@ -5,7 +5,8 @@
 // query's state to a CPU thread through a pinned ring of snapshots.  Here:
 //   * one worker thread per query kind (SSSP, PPR, adsorption), each on its own CUDA
 //     stream; the three kinds run on the device at the same time, each batched launch on
-//     a third of the SMs so the persistent kernels are co-resident;
+//     a third of the SMs so the persistent kernels are co-resident (a kind alone at work
+//     has them all);
 //   * SSSP and PPR requests run in a resident batch (c2g_session): the worker runs epochs
 //     of a few rounds, and between epochs it admits waiting requests into free slots, so a
 //     request that arrives while others run starts at the next epoch, not after the
@@ -71,11 +72,14 @@ struct c2g_server {
     int64_t bytes_per_query[3] = {0, 0, 0};
     int64_t budget_per_kind = 0;
     std::mutex mu;
-    std::condition_variable cv_work, cv_done;
+    std::condition_variable cv_work, cv_done, cv_epoch;
     std::deque<Pending> queue[3];
     std::map<int64_t, Done> done;
     std::vector<double> latencies;
     int64_t next_ticket = 1;
+    bool busy[3] = {false, false, false};    // the kind has requests (queued for its epoch or running)
+    bool in_epoch[3] = {false, false, false};  // SSSP, PPR: its kernels may be on the GPU
+    bool whole = false;                      // that epoch has the whole GPU
     int64_t batches[3] = {0, 0, 0};
     int64_t evictions = 0;
     int64_t completed = 0;
@@ -120,6 +124,33 @@ struct Parked {
     Pending p;
     c2g_snapshot* snap;
 };
+
+constexpr float kShare = 1.0f / 3.0f;
+
+// The SMs of a kind's next epoch.  A third each is what lets two persistent kernels and the
+// label propagation's run side by side: the blocks of other splits need not fit together, and a
+// grid that waits at its barrier for blocks without room would hold what the other needs.  A kind
+// with no other at work takes the whole GPU, and then an epoch of another waits for its end
+// (11 PPR queries alone on a scale-18 graph: 28.3 ms on a third, 18.7 on all; a wave of 32 mixed
+// requests 29.9 -> 27.3 ms, its last third being PPR alone.  Two thirds beside the label
+// propagation gave the wave nothing, 27.1 to 27.9.)
+float epoch_begin(c2g_server* s, int kind) {
+    std::unique_lock<std::mutex> lk(s->mu);
+    s->busy[kind] = true;
+    const int other = kind == C2G_REQ_SSSP ? C2G_REQ_PPR : C2G_REQ_SSSP;
+    s->cv_epoch.wait(lk, [&] { return !(s->in_epoch[other] && s->whole); });
+    s->whole = !s->busy[other] && !s->busy[C2G_REQ_ADSORPTION] && !s->in_epoch[other];
+    s->in_epoch[kind] = true;
+    return s->whole ? 1.0f : kShare;
+}
+
+void epoch_end(c2g_server* s, int kind, bool more) {
+    std::lock_guard<std::mutex> lk(s->mu);
+    s->in_epoch[kind] = false;
+    s->whole = false;
+    s->busy[kind] = more;
+    s->cv_epoch.notify_all();
+}
 
 // SSSP / PPR: a resident batch run in epochs; waiting requests (evicted ones first) take
 // free slots between epochs.
@@ -204,7 +235,9 @@ void session_worker(c2g_server* s, int kind) {
         if (running == 0) continue;
         int32_t nf = 0;
         c2g_stats st;
+        session_set_grid_share(ss, epoch_begin(s, kind));
         int rc = c2g_session_step(ss, rounds, finished.data(), cap, &nf, &st);
+        epoch_end(s, kind, rc == C2G_OK && running > nf);
         {
             std::lock_guard<std::mutex> lk(s->mu);
             s->batches[kind] += 1;
@@ -249,8 +282,13 @@ void worker(c2g_server* s, int kind) {
                 batch.push_back(std::move(s->queue[kind].front()));
                 s->queue[kind].pop_front();
             }
+            s->busy[kind] = true;
         }
         run_adsorption(s, batch);
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            s->busy[kind] = false;
+        }
     }
 }
 
@@ -284,13 +322,13 @@ int c2g_server_create(c2g_graph* g, const float* p_inj, const float* p_cont, con
     }
     for (int k = 0; k < 3 && !rc; ++k) {
         rc = graph_view(g, &s->views[k]);
-        if (!rc) s->views[k]->grid_scale = 1.0f / 3.0f;
+        if (!rc) s->views[k]->grid_scale = kShare;
     }
     // Per-query device state (bytes) and the admission budget.  Per (vertex, query): SSSP
     // distance 4 B plus 28 B per 32 queries (mask, two frontier entries and masks, two pull
     // lookups); PPR
     // pr 4, res 8, msg 8, two pushed residuals 16 and their float pairs 16, plus 32 B per
-    // 32 queries of masks and frontier entries; adsorption 16 labels x (Y, accumulator,
+    // 32 queries of masks and frontier entries; adsorption 16 labels x (two row buffers,
     // host stage).
     s->bytes_per_query[C2G_REQ_SSSP] = (int64_t)V * 4 + (int64_t)V * 28 / 32;
     s->bytes_per_query[C2G_REQ_PPR] = (int64_t)V * 52 + (int64_t)V * 32 / 32;
@@ -312,7 +350,6 @@ int c2g_server_create(c2g_graph* g, const float* p_inj, const float* p_cont, con
         prm.pr0 = cfg->alpha;
         prm.seeded = 0;
         rc = c2g_session_create(g, k, (int32_t)cap, k == C2G_REQ_PPR ? &prm : nullptr, &s->sessions[k]);
-        if (!rc) session_set_grid_share(s->sessions[k], 1.0f / 3.0f);
     }
     if (prev >= 0) cudaSetDevice(prev);
     if (rc) {

@@ -601,7 +601,7 @@ void c2g_snapshot_free(c2g_snapshot* snap) { delete snap; }
 }  // extern "C"
 
 // The share of the SMs a session's launches take (the serving loop runs three kinds side
-// by side, each on a third, so their persistent kernels are co-resident).
+// by side, each on a third unless it is alone, so their persistent kernels are co-resident).
 void c2g::session_set_grid_share(c2g_session* s, float share) {
     std::lock_guard<std::mutex> lk(s->mu);
     s->g->grid_scale = share;
