@@ -77,6 +77,64 @@ __global__ void adjoint_grad_kernel(const int* __restrict__ row, const int2* __r
     }
 }
 
+// out[i] = pi[v[i]]: what the loss needs of pi.
+__global__ void adjoint_at_targets(const float* __restrict__ pi, const int* __restrict__ v, int n, float* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = __ldg(pi + __ldg(v + i));
+}
+
+// Per-handle workspace of the gradient, kept across calls: a training loop calls it every step, and
+// allocating and freeing its arrays each time (cudaFree waits for the device) took 0.9 ms of a call at
+// scale 20.
+struct AdjointWork {
+    float *pi = nullptr, *lam = nullptr;  // [V]
+    float* grad = nullptr;                // [E], once a gradient goes to the host
+    int32_t* tv = nullptr;                // distinct targets,
+    float *tr = nullptr, *tpi = nullptr;  // their multiplicities, and pi there
+    size_t targets = 0;                   // allocated
+    TraversalCtl* ctl = nullptr;          // the backward push's status, before the gradient pass adds its own
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+};
+
+void adjoint_free(c2g_graph* g) {
+    AdjointWork* w = reinterpret_cast<AdjointWork*>(g->adjoint);
+    if (!w) return;
+    for (void* p : {(void*)w->pi, (void*)w->lam, (void*)w->grad, (void*)w->tv, (void*)w->tr, (void*)w->tpi,
+                    (void*)w->ctl})
+        if (p) cudaFree(p);
+    for (cudaEvent_t ev : {w->ev0, w->ev1})
+        if (ev) cudaEventDestroy(ev);
+    delete w;
+    g->adjoint = nullptr;
+}
+
+static int adjoint_alloc(c2g_graph* g, size_t targets, bool host_grad, AdjointWork** out) {
+    AdjointWork* w = reinterpret_cast<AdjointWork*>(g->adjoint);
+    if (!w) g->adjoint = w = new AdjointWork();
+    const size_t V = (size_t)g->V, E = (size_t)g->E;
+    cudaError_t e = cudaSuccess;
+    if (!w->ctl) e = cudaMalloc(&w->ctl, sizeof(TraversalCtl));
+    if (e == cudaSuccess && !w->ev0) e = cudaEventCreate(&w->ev0);
+    if (e == cudaSuccess && !w->ev1) e = cudaEventCreate(&w->ev1);
+    if (e == cudaSuccess && !w->pi) e = cudaMalloc(&w->pi, sizeof(float) * V);
+    if (e == cudaSuccess && !w->lam) e = cudaMalloc(&w->lam, sizeof(float) * V);
+    if (e == cudaSuccess && host_grad && !w->grad) e = cudaMalloc(&w->grad, sizeof(float) * (E ? E : 1));
+    if (e == cudaSuccess && w->targets < targets) {
+        for (void* p : {(void*)w->tv, (void*)w->tr, (void*)w->tpi})
+            if (p) cudaFree(p);
+        w->tv = nullptr;
+        w->tr = w->tpi = nullptr;
+        w->targets = 0;
+        e = cudaMalloc(&w->tv, sizeof(int32_t) * targets);
+        if (e == cudaSuccess) e = cudaMalloc(&w->tr, sizeof(float) * targets);
+        if (e == cudaSuccess) e = cudaMalloc(&w->tpi, sizeof(float) * targets);
+        if (e == cudaSuccess) w->targets = targets;
+    }
+    if (e != cudaSuccess) adjoint_free(g);
+    C2G_CUDA(e);
+    *out = w;
+    return C2G_OK;
+}
+
 int set_float_weights(c2g_graph* g, const float* w, int on_device);
 
 }  // namespace c2g
@@ -124,30 +182,15 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
     int rc = build_reverse_graph(g);
     if (rc || (rc = build_row_lists(g, g->row, g->row_r, &g->rows_out))) return rc;
     const size_t V = (size_t)g->V, E = (size_t)g->E;
-    float *pi = nullptr, *lam = nullptr, *dgrad = nullptr, *dtr = nullptr;
-    int32_t* dtv = nullptr;
-    C2G_CUDA(cudaMalloc(&pi, sizeof(float) * V));
-    C2G_CUDA(cudaMalloc(&lam, sizeof(float) * V));
-    C2G_CUDA(cudaMalloc(&dtv, sizeof(int32_t) * tv.size()));
-    C2G_CUDA(cudaMalloc(&dtr, sizeof(float) * tr.size()));
-    dgrad = on_device ? grad : nullptr;
-    if (!dgrad) C2G_CUDA(cudaMalloc(&dgrad, sizeof(float) * (E ? E : 1)));
-    auto cleanup = [&]() {
-        cudaFree(pi);
-        cudaFree(lam);
-        cudaFree(dtv);
-        cudaFree(dtr);
-        if (!on_device) cudaFree(dgrad);
-    };
+    AdjointWork* w = nullptr;
+    if ((rc = adjoint_alloc(g, tv.size(), !on_device, &w))) return rc;
+    float *const pi = w->pi, *const lam = w->lam, *const dgrad = on_device ? grad : w->grad;
     float ms_f = 0.f, ms_b = 0.f, ms_g = 0.f;
     TraversalCtl cf, cb;
-    cudaError_t e = cudaMemcpyAsync(dtv, tv.data(), sizeof(int32_t) * tv.size(), cudaMemcpyHostToDevice, g->stream);
+    cudaError_t e = cudaMemcpyAsync(w->tv, tv.data(), sizeof(int32_t) * tv.size(), cudaMemcpyHostToDevice, g->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(dtr, tr.data(), sizeof(float) * tr.size(), cudaMemcpyHostToDevice, g->stream);
-    if (e != cudaSuccess) {
-        cleanup();
-        C2G_CUDA(e);
-    }
+        e = cudaMemcpyAsync(w->tr, tr.data(), sizeof(float) * tr.size(), cudaMemcpyHostToDevice, g->stream);
+    C2G_CUDA(e);
     // forward: pi
     c2g_ppr_params fp = *params;
     fp.r0 = 1.0f;
@@ -162,30 +205,30 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
     bp.rmax = rmax_backward;
     if (!rc)
         rc = ppr_launch_view(g, g->row_r, g->adj_r, g->row, g->adj_f, g->rows_out, tv[0], bp, 1.0f, (int32_t)tv.size(),
-                             dtv, dtr, nullptr, nullptr, 0, lam, nullptr, &ms_b);
-    if (!rc && (cudaMemcpyAsync(&cb, g->ppr.ctl, sizeof(cb), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
-                cudaStreamSynchronize(g->stream) != cudaSuccess))
-        rc = fail(C2G_ERR_CUDA, "adjoint: reading the backward push status failed");
-    if (rc) {
-        cleanup();
-        return rc;
-    }
-    if ((cf.flags | cb.flags) & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS)) {
-        cleanup();
-        return fail(C2G_ERR_OVERFLOW, "adjoint push reported device errors (flags %d/%d)", cf.flags, cb.flags);
-    }
+                             w->tv, w->tr, nullptr, nullptr, 0, lam, nullptr, nullptr);
+    if (rc) return rc;
+    // The gradient pass and the copies follow the push at once: a copy to pageable memory that is issued while
+    // the stream is busy makes its pages ready beside the kernels (67 MB: 3 ms when issued after them).
+    e = cudaMemcpyAsync(w->ctl, g->ppr.ctl, sizeof(cb), cudaMemcpyDeviceToDevice, g->stream);
+    C2G_CUDA(e);
     // gradient pass
-    cudaEventRecord(g->ev0, g->stream);
+    cudaEventRecord(w->ev0, g->stream);
     if (E)
         adjoint_grad_kernel<<<g->num_sms * 8, 256, 0, g->stream>>>(g->row, g->adj_f, g->mark_f, g->V, (unsigned)E, pi,
                                                                    lam, 1.0f - params->alpha, dgrad,
                                                                    &g->ppr.ctl->flags);
-    cudaEventRecord(g->ev1, g->stream);
+    cudaEventRecord(w->ev1, g->stream);
     e = cudaGetLastError();
     if (e == cudaSuccess && !on_device)
         e = cudaMemcpyAsync(grad, dgrad, sizeof(float) * E, cudaMemcpyDeviceToHost, g->stream);
-    std::vector<float> hpi(V);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hpi.data(), pi, sizeof(float) * V, cudaMemcpyDeviceToHost, g->stream);
+    std::vector<float> tpi(loss ? tv.size() : 0);
+    if (e == cudaSuccess && loss) {
+        adjoint_at_targets<<<(int)std::min<size_t>((tv.size() + 255) / 256, 1024), 256, 0, g->stream>>>(
+            pi, w->tv, (int)tv.size(), w->tpi);
+        e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(tpi.data(), w->tpi, sizeof(float) * tv.size(), cudaMemcpyDeviceToHost, g->stream);
+    }
     if (e == cudaSuccess && pi_out)
         e = cudaMemcpyAsync(pi_out, pi, sizeof(float) * V, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                             g->stream);
@@ -193,16 +236,20 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
         e = cudaMemcpyAsync(lambda_out, lam, sizeof(float) * V,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, g->stream);
     int gflags = 0;  // the gradient pass's bounds checks report into the push's control block
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&cb, w->ctl, sizeof(cb), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&gflags, &g->ppr.ctl->flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    if (e == cudaSuccess) cudaEventElapsedTime(&ms_g, g->ev0, g->ev1);
-    cleanup();
     C2G_CUDA(e);
+    if ((cf.flags | cb.flags) & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS))
+        return fail(C2G_ERR_OVERFLOW, "adjoint push reported device errors (flags %d/%d)", cf.flags, cb.flags);
+    C2G_CUDA(cudaEventElapsedTime(&ms_b, g->ev0, g->ev1));
+    C2G_CUDA(cudaEventElapsedTime(&ms_g, w->ev0, w->ev1));
     if (gflags & C2G_FLAG_BOUNDS) return fail(C2G_ERR_OVERFLOW, "adjoint gradient pass: device index check failed");
     if (loss) {
         double L = 0.0;
-        for (int32_t t = 0; t < n_targets; ++t) L += (double)hpi[targets[t]];
+        for (int32_t t = 0; t < n_targets; ++t)
+            L += (double)tpi[(size_t)(std::lower_bound(tv.begin(), tv.end(), targets[t]) - tv.begin())];
         *loss = L;
     }
     if (stats) {

@@ -27,6 +27,7 @@ static void graph_release(c2g_graph* g) {
     batch_free(g);
     ppr_batch_free(g);
     ads_free(g);
+    adjoint_free(g);
     if (!g->borrowed) reverse_free(g);
     if (!g->borrowed) in_rows_free(g);
     if (!g->borrowed) {

@@ -193,6 +193,7 @@ struct c2g_graph {
     void* batch = nullptr;            // batched-query workspaces (batch.cu)
     void* ppr_batch = nullptr;
     void* ads = nullptr;              // label-propagation workspace (adsorption.cu)
+    void* adjoint = nullptr;          // gradient workspace (adjoint.cu)
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -227,6 +228,7 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
                     const int32_t* src_list, const float* src_r0, const int32_t* seed_v, const float* seed_w,
                     int32_t n_rec, float* pr_dev, float* res_dev, float* ms);
 int build_markers(c2g_graph* g, const int* row, int** out);
+void adjoint_free(c2g_graph* g);
 void sssp_free(c2g_graph* g);
 void ppr_free(c2g_graph* g);
 // A handle sharing `base`'s device graph arrays with its own stream, workspaces and lock.
