@@ -1248,10 +1248,16 @@ __device__ __forceinline__ unsigned pbatch_sweep(const PprBatchParams& p, bool f
     const unsigned nm = list ? nlist : (unsigned)p.V << p.logW;
     const unsigned long long rmax_bits = c2g_dbits((double)p.rmax);
     unsigned cnt = 0;
-    for (unsigned b = gwarp * 32u; b < nm; b += nwarps * 32u) {
+    // words a warp takes at a time: every listed word costs an apply, so a list is spread over all warps
+    // (50,000 words on 4,256 warps, 40 queries at scale 16: 65 us a round at 32 each, 23 so; a mask word
+    // of a whole sweep is mostly empty)
+    const unsigned rounds = (nm + nwarps * 32u - 1u) / (nwarps * 32u);
+    const unsigned take = list ? (nm + nwarps * rounds - 1u) / max(1u, nwarps * rounds) : 32u;
+    for (unsigned b = gwarp * take; b < nm; b += nwarps * take) {
         const unsigned pos = b + (unsigned)lane;
-        const unsigned i = pos < nm ? (list ? ldcg(list + pos) : pos) : 0u;  // this lane's (vertex, word)
-        const unsigned tm = pos < nm ? ldcg(p.tmask + i) : 0u;
+        const bool in = (unsigned)lane < take && pos < nm;
+        const unsigned i = in ? (list ? ldcg(list + pos) : pos) : 0u;  // this lane's (vertex, word)
+        const unsigned tm = in ? ldcg(p.tmask + i) : 0u;
         int dg = 0;
         if (tm) {
             p.tmask[i] = 0u;
@@ -1318,7 +1324,7 @@ __device__ __forceinline__ unsigned pbatch_sweep(const PprBatchParams& p, bool f
 // boundaries inside a chunk come from one word of start bits, not from the row pointer.
 // (Row by row, each row cost a chain of three dependent loads before its first gather, and
 // narrow batches left most of an item's 4 words empty: 40 queries at scale 16 took 28.0 ms a
-// batch, now 10.0; 256 at scale 21 395, now 368.)  What bounds a dense round of a wide batch is
+// batch, now 8.4; 256 at scale 21 395, now 368.)  What bounds a dense round of a wide batch is
 // the gathers' bytes, 8 per push, at about 6 TB/s out of L2, and about 60 instructions per
 // (in-edge, item).  A target whose in-edges lie in one item is applied by the warp that summed
 // them; only targets whose in-edges cross an item boundary add their parts to msg (FP64
