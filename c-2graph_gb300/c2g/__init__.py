@@ -333,8 +333,8 @@ class Graph:
 
     def sssp_batch_pull(self, frac=0.5):
         """Batched SSSP rounds with more than frac * E * Q (query, edge) relaxations pull over
-        the in-edges (Q: query slots; a third of that for 64, a tenth for more; frac < 0:
-        expand only; 0: every round)."""
+        the in-edges (Q: query slots; a third of that for 64, a tenth for more and after
+        the first pull; frac < 0: expand only; 0: every round)."""
         _check(lib().c2g_sssp_batch_set_pull(self._h, float(frac)))
 
     def sssp_batch_pull_frac(self):

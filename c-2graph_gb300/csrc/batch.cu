@@ -67,6 +67,7 @@ struct BatchParams {
     unsigned in_segs;
     int in_shift;
     unsigned long long pull_min;
+    unsigned long long pull_next;  // the same, once a round of the launch has pulled (batches of one or two words)
     unsigned* amask[2];
     int* qmin;  // [3][Q]
 };
@@ -608,6 +609,7 @@ __global__ void __launch_bounds__(kSsspBatchThreads, kSsspBatchBlocksPerSm) sssp
 
     long long relax = 0, steps = 0;
     int cur = 1, iters = 0;
+    bool pulled = false;  // a round of this launch has pulled
     for (;;) {
         const int buf = cur & 1, slot = cur % 3;
         // Phase 1: this round's frontier from the masks of the previous one.
@@ -625,7 +627,8 @@ __global__ void __launch_bounds__(kSsspBatchThreads, kSsspBatchBlocksPerSm) sssp
         // pull when the frontier's (query, edge) relaxations exceed pull_min: the dense rounds
         // in which most active words have most of their queries active (the push pays a
         // red.min per improvement there), not every round with many edge-word steps
-        const bool pull = ldcg(&ctl->pcount[slot]) > p.pull_min;  // grid-uniform
+        const bool pull = ldcg(&ctl->pcount[slot]) > (WP < 4 && pulled ? p.pull_next : p.pull_min);  // grid-uniform
+        pulled = pull || pulled;
         if (gtid == 0) trace_round(p.trace, iters, (long long)T, pull ? 1 : 0);
         if (F == 0) break;
         if (++iters > p.max_iter) {
@@ -927,15 +930,20 @@ static int batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
 // 27.4 / 22.3 / 21.6 / 21.3; scale 19, 64 queries 5.0 / 3.5 / 3.0 / 3.2; 685,230 uniform vertices, 31
 // queries 5.1 / 5.2 / - / 5.8.  Below a million lines the warps with the longest rows outlast the
 // rest of a pull (60,001 vertices, 128 queries 1.33 / 1.69 / 1.75 / 1.98 ms): those batches expand
-// only, unless the caller set a fraction.
+// only, unless the caller set a fraction.  After a launch's first pull the distances bound the rows
+// of the next ones, whose passes get shorter (scale 22, 256 queries: 7.8 ms, then 4.0, 2.9, 2.6), so a
+// batch of one or two words goes on pulling down to the wide one's limit: scale 21, 64 queries 9.15 -> 7.95
+// ms, 32 6.60 -> 5.91; for 256 a lower limit is no gain (500,003 uniform vertices 25.0, a third of it 26.6).
 constexpr size_t kPullMinLines = 1000000;
 
-static unsigned long long sssp_pull_min(const c2g_graph* g, int Q) {
+static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, unsigned long long* next) {
+    *first = *next = ~0ull;
     const float frac = g->sssp_cfg.batch_pull_frac;
     const bool small = !g->sssp_cfg.batch_pull_set && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines;
-    if (!(frac >= 0.f) || small) return ~0ull;
-    const double width = Q <= 32 ? 1.0 : Q <= 64 ? 1.0 / 3.0 : 0.1;
-    return (unsigned long long)((double)frac * width * (double)g->E * (double)Q);
+    if (!(frac >= 0.f) || small) return;
+    const double width = Q <= 32 ? 1.0 : Q <= 64 ? 1.0 / 3.0 : 0.1, all = (double)frac * (double)g->E * (double)Q;
+    *first = (unsigned long long)(width * all);
+    *next = (unsigned long long)(0.1 * all);
 }
 
 // The pull rounds of a batched SSSP launch (p.pull_min: (query, edge) relaxations of the
@@ -944,7 +952,8 @@ static unsigned long long sssp_pull_min(const c2g_graph* g, int Q) {
 // lookups start clear; a launch leaves the entries of its last rounds behind.
 static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchParams& p) {
     p.pull_min = ~0ull;
-    const unsigned long long pull_min = sssp_pull_min(g, Q);
+    unsigned long long pull_min, pull_next;
+    sssp_pull_min(g, Q, &pull_min, &pull_next);
     if (pull_min == ~0ull || !g->in_adj || (seeds && g->hw_negative)) return C2G_OK;
     p.in_row = g->in_row;
     p.in_adj = g->in_adj;
@@ -955,6 +964,7 @@ static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchP
     for (int b = 0; b < 2; ++b)
         C2G_CUDA(cudaMemsetAsync(w->amask[b], 0, sizeof(unsigned) * (size_t)g->V * (size_t)(Q / 32), g->stream));
     p.pull_min = pull_min;
+    p.pull_next = pull_next;
     return C2G_OK;
 }
 

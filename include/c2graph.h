@@ -218,7 +218,7 @@ int c2g_sssp_batch_get_tile(const c2g_graph* g, int32_t* big_steps, int32_t* min
 /* Round shape of the batched SSSP (c2g_sssp_batch and resident SSSP batches; no
  * counterpart in the reference): a round whose frontier makes more than frac * E * Q
  * (query, edge) relaxations (Q = query slots, a multiple of 32; a third of that for 64
- * slots, a tenth for more) pulls: each target takes the minimum over its in-edges from
+ * slots, a tenth for more and for every round after a launch's first pull) pulls: each target takes the minimum over its in-edges from
  * sources that improved in the previous round, in ascending order of weight up to the
  * first that cannot improve any query of the word.  frac < 0: expand (push) only; 0: pull
  * every round; default 0.3, and until it is set a batch with fewer than a million (vertex,
