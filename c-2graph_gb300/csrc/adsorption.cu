@@ -13,9 +13,9 @@
 // the spot and writes the next label rows, between two row buffers.  The in-edges of all
 // vertices form one range [0, E) cut into tiles, one per warp, and a tile into eight equal
 // stretches, one per group of 4 lanes (each lane holds 4 of the 16 labels).  A group walks
-// its stretch in order: the in-edges come through shared memory 32 at a time (cp.async, two
-// buffers), the label rows of kAdsBatch in-edges are in flight while those before them are
-// summed, and a bitmap of row starts says where a row ends.  A row that lies inside a
+// its stretch in order: the in-edges come through shared memory 32 (small graphs: 8) at a
+// time (cp.async, two buffers), the label rows of kAdsBatch in-edges are in flight while those
+// before them are summed, and a bitmap of row starts says where a row ends.  A row that lies inside a
 // stretch is written by its group; one that crosses stretches is summed over the groups by
 // shuffles; one that crosses tiles leaves a partial sum per tile, and the warp that arrives
 // last adds them up, in order.
@@ -44,8 +44,6 @@ constexpr int kAdsBatch = 2;       // in-edges whose label rows a group gathers 
 constexpr int kAdsMinBlocks = 8;   // launch bounds: resident 128-thread blocks per SM
 constexpr int kAdsThreads = 128;
 constexpr int kAdsWarps = kAdsThreads / 32;
-constexpr int64_t kAdsFill = 1;    // tiles per resident warp below which tiles get smaller
-constexpr int kAdsChunk = 32;     // in-edges a group stages in shared memory at a time
 
 struct AdsPass {
     const int* row_r;
@@ -83,11 +81,13 @@ __device__ __forceinline__ float4 ads_shfl_up(const float4 a, int d) {
 }
 
 // out = p_cont * (sum over in-edges of w * Y) + p_inj * I for every vertex with in-edges; row V of Y is zero.
+// C: in-edges a group stages in shared memory at a time.
+template <int C>
 __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
     ads_iterate(const AdsPass p, const float4* __restrict__ Y, float4* __restrict__ out) {
     // each group's staged in-edges, two chunks; 16 bytes of padding per row, so that the 8
     // groups of a warp, reading 16 bytes of their rows at once, hit different banks
-    __shared__ __align__(16) int2 staged[kAdsWarps][2][8][kAdsChunk + 2];
+    __shared__ __align__(16) int2 staged[kAdsWarps][2][8][C + 2];
     __shared__ float4 heads[kAdsThreads];
     if (blockIdx.x == 0 && threadIdx.x < kAdsL) {  // a seed without in-edges keeps its injection alone
         const int v = __ldg(p.seeds + threadIdx.x);
@@ -102,11 +102,14 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
     if ((t << p.tile_log) >= p.E) return;  // warp-uniform, no block barrier below
     const unsigned e1 = min(e0 + stretch, p.E);
     const bool act = e0 < p.E;
-    const unsigned words = (p.E + 31) / 32;
-    unsigned word = e0 >> 5;
-    unsigned bits = act ? __ldg(p.r_bits + word) : 0u;
+    const auto start_bits = [&](unsigned e) { return __ldg(p.r_bits + (e >> 5)) >> (e & 31u) & (~0u >> (32 - C)); };
+    unsigned bits = act ? start_bits(e0) : 0u;
     const bool starts = bits & 1u;         // the stretch's first in-edge starts a row
-    const int first = act ? __ldg(p.r_prefix + word) + (int)starts - 1 : 0;  // its row
+    int first = 0;                         // its row
+    if (act) {
+        const unsigned before = C < 32 ? __ldg(p.r_bits + (e0 >> 5)) & ((1u << (e0 & 31u)) - 1u) : 0u;
+        first = __ldg(p.r_prefix + (e0 >> 5)) + __popc(before) + (int)starts - 1;
+    }
     int row = first;
     int4 coef = act ? __ldg(p.coef + first) : make_int4(0, 0, 0, 0);
     bits &= ~1u;
@@ -115,14 +118,14 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
 
     const auto stage = [&](unsigned c) {
         int2* const to = staged[warp][c & 1u][grp];
-        const unsigned base = e0 + c * kAdsChunk;
-        if (base + kAdsChunk <= p.E) {
+        const unsigned base = e0 + c * C;
+        if (base + C <= p.E) {
 #pragma unroll
-            for (int r = 0; r < kAdsChunk / 8; ++r)
+            for (int r = 0; r < C / 8; ++r)
                 cp_async16(to + 2 * part + 8 * r, p.adj_r + base + 2 * part + 8 * r);
         } else {  // beyond the last in-edge: the zero row
 #pragma unroll 1
-            for (unsigned i = part; i < kAdsChunk; i += 4)
+            for (unsigned i = part; i < C; i += 4)
                 to[i] = base + i < p.E ? __ldg(p.adj_r + base + i) : make_int2(p.V, 0);
         }
     };
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
         bits >>= kAdsBatch;
     };
 
-    const unsigned chunks = stretch / kAdsChunk;
+    const unsigned chunks = stretch / C;
     stage(0);
     cp_async_commit();
     if (chunks > 1) stage(1);
@@ -170,16 +173,16 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
     gather(0, staged[warp][0][grp]);
     for (unsigned c = 0; c < chunks; ++c) {
         const int2* const st = staged[warp][c & 1u][grp];
-        const unsigned next_bits = c + 1 < chunks && word + 1 < words ? __ldg(p.r_bits + word + 1) : 0u;
-        ++word;
+        const unsigned next = e0 + (c + 1) * C;
+        const unsigned next_bits = c + 1 < chunks && next < p.E ? start_bits(next) : 0u;
 #pragma unroll 1
-        for (int b = 0; b < kAdsChunk - 2 * kAdsBatch; b += 2 * kAdsBatch) {
+        for (int b = 0; b < C - 2 * kAdsBatch; b += 2 * kAdsBatch) {
             gather(1, st + b + kAdsBatch);
             consume(0);
             gather(0, st + b + 2 * kAdsBatch);
             consume(1);
         }
-        gather(1, st + kAdsChunk - kAdsBatch);
+        gather(1, st + C - kAdsBatch);
         consume(0);
         if (c + 1 < chunks) {
             cp_async_wait_but<0>();
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
 
     // the row at the end of each stretch, summed over the stretches that it crosses
     const bool had_head = !starts && !head;  // a row that began before the stretch ended in it
-    const bool done = act && (e1 == p.E || (__ldg(p.r_bits + (e1 >> 5)) & 1u));
+    const bool done = act && (e1 == p.E || (start_bits(e1) & 1u));
     int f = starts || had_head;              // it began in the tile
 #pragma unroll
     for (int d = 1; d < 8; d *= 2) {
@@ -327,11 +330,15 @@ void ads_free(c2g_graph* g) {
 
 // In-edges per tile (log2): eight stretches of 128, shorter ones where that leaves the SMs short of
 // warps.  30 iterations at scale 22: 16.6 ms with 1024-edge tiles, 20.4 with 512, 25.8 with 256 (a
-// tile's start and end are chains of loads); at scale 18 1.25 ms with 512, 1.36 with 256.
+// tile's start and end are chains of loads); at scale 18 1.25 ms with 512, 1.36 with 256.  64-edge
+// tiles, staged 8 in-edges at a time, where all of them are resident at once: there the walk along a
+// stretch is what an iteration takes (scale 10 0.34 -> 0.20 ms, scale 14 0.40 -> 0.26, against 256; scale 15
+// 0.42 either way, scale 16 0.48 -> 0.69).
 static int ads_tile_log(const c2g_graph* g) {
     const int64_t warps = (int64_t)g->num_sms * kAdsMinBlocks * kAdsWarps;
     int log = 10;
-    while (log > 8 && ((int64_t)g->E >> log) < kAdsFill * warps) --log;
+    while (log > 8 && ((int64_t)g->E >> log) < warps) --log;
+    if (((int64_t)g->E >> 6) < warps) log = 6;
     return log;
 }
 
@@ -377,7 +384,7 @@ static int ads_capture(c2g_graph* g, AdsWork* w, int iterations) {
     if (e == cudaSuccess) {
         ads_init<<<g->num_sms * 8, 256, 0, g->stream>>>(p, w->pc, w->mask, Y[0], Y[1], w->coef);
         for (int it = 0; it < iterations; ++it)  // without in-edges one block writes the seeds' rows
-            ads_iterate<<<blocks ? blocks : 1, kAdsThreads, 0, g->stream>>>(p, Y[it & 1], Y[(it + 1) & 1]);
+            (w->tile_log < 8 ? ads_iterate<8> : ads_iterate<32>)<<<blocks ? blocks : 1, kAdsThreads, 0, g->stream>>>(p, Y[it & 1], Y[(it + 1) & 1]);
         e = cudaStreamEndCapture(g->stream, &graph);
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&w->exec, graph, 0);

@@ -1,8 +1,8 @@
-"""Label propagation over rows that start, end and cross at the edges of chunks (32 in-edges), stretches
-(32 to 128) and tiles (256 to 1024), both result buffers, seeds without in-edges, no edges at all.
+"""Label propagation over rows that start, end and cross at the edges of chunks (8 or 32 in-edges), stretches
+(8 to 128) and tiles (64 to 1024), both result buffers, seeds without in-edges, no edges at all.
 
 Weights and start values are not negative, so a row's sum is off by at most its additions in sequence:
-128 in a stretch, 3 over a tile's stretches, a row's tiles in eighths (20000 / 256 / 8 = 10) and 3 more,
+128 in a stretch, 3 over a tile's stretches, a row's tiles in eighths (20000 / 64 / 8 = 40) and 3 more,
 and each iteration multiplies and adds once more.  Per entry: (150 k) 2^-24 of the FP64 value after k
 iterations, and 1e-38 for what lies below the normal range."""
 import numpy as np
@@ -46,7 +46,7 @@ def _check(csr, seed, iterations=(3,)):
             assert st.iterations == k and st.edges_relaxed == k * len(csr[1])
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 31, 32, 33, 63, 64, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 5000])
 def test_edge_counts_around_a_tile(gpu_available, n):
     _check(_graph([3, n, 1], 9, n), n)
 
@@ -58,7 +58,7 @@ def test_rows_across_tiles(gpu_available, lengths):
     _check(_graph(lengths, 50, len(lengths)), 3, (0, 1, 2, 3, 10, 3))
 
 
-@pytest.mark.parametrize("extra", [3000000, 9000000])
+@pytest.mark.parametrize("extra", [500000, 3000000, 9000000])
 def test_longer_stretches(gpu_available, extra):
     """Graphs large enough for the longer stretches, with rows of many tiles among the short ones."""
     rng = np.random.default_rng(extra)
