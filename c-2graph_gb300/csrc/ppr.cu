@@ -46,6 +46,7 @@ struct PprParams {
     RowLists rows;      // its rows by length
     unsigned* arrived;  // class 0: segments of a row summed so far, zero between rounds
     unsigned pull_min;  // pull when T is larger (~0: never)
+    bool one_step;      // every round pulls, and its row lists are at most one step per warp
     int dense_div;      // dense push round (no touched list) when T * dense_div > E (0: never)
     float* pr;
     double* res;
@@ -92,6 +93,7 @@ __device__ __forceinline__ FrontierOut ppr_out(const PprParams& p, int buf, int 
 constexpr int kPprUnroll = 8;  // edges in flight per lane
 constexpr int kPprThreads = 512;  // launch shape of the persistent push
 constexpr int kPprBlocksPerSm = 2;
+constexpr unsigned kStepsPerBlock = 2;  // steps of a small graph's pull that are worth another block
 // Round-robin tiles in push rounds (a dynamic tile queue measured no faster: 20.2 vs 20.4 ms
 // per scale-22 query).
 constexpr bool kPprDynTiles = false;
@@ -201,6 +203,17 @@ struct PullSums {
     float hi, lo;
 };
 
+// s += q * w, exactly up to the last bits of lo; a source outside the frontier (q = 0) or a weight that is
+// not positive adds 0.
+__device__ __forceinline__ void pull_add(const float2& q, int wbits, PullSums& s) {
+    const float w = q.x != 0.f ? __int_as_float(wbits) : 0.f;
+    const float pm = __fmul_rn(q.x, w);
+    const float pe = __fmaf_rn(q.y, w, __fmaf_rn(q.x, w, -pm));
+    float te;
+    s.hi = two_sum(s.hi, pm, te);
+    s.lo = __fadd_rn(s.lo, __fadd_rn(te, pe));
+}
+
 // Messages of this lane's in-edges first, first + step, ... (up to kLaneEdges of them) below n.
 __device__ __forceinline__ void pull_lane(const int2* __restrict__ adj, const float2* qin, int first, int step, int n,
                                           PullSums& s) {
@@ -215,16 +228,7 @@ __device__ __forceinline__ void pull_lane(const int2* __restrict__ adj, const fl
 #pragma unroll
     for (int u = 0; u < kLaneEdges; ++u) q[u] = ew[u].y > 0 ? __ldca(qin + ew[u].x) : make_float2(0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < kLaneEdges; ++u) {
-        // message (hi + lo) * w = pm + pe; a source outside the frontier or a weight that is
-        // not positive adds 0
-        const float w = q[u].x != 0.f ? __int_as_float(ew[u].y) : 0.f;
-        const float pm = __fmul_rn(q[u].x, w);
-        const float pe = __fmaf_rn(q[u].y, w, __fmaf_rn(q[u].x, w, -pm));
-        float te;
-        s.hi = two_sum(s.hi, pm, te);
-        s.lo = __fadd_rn(s.lo, __fadd_rn(te, pe));
-    }
+    for (int u = 0; u < kLaneEdges; ++u) pull_add(q[u], ew[u].y, s);
 }
 
 // Sum over groups of L lanes; the value as a double (in every lane of the group).
@@ -324,6 +328,139 @@ __device__ __forceinline__ void ppr_pull(const PprParams& p, int b, PullTotals& 
         pull_lane(p.adj_r + rec.y, qin, part, L, rec.z, s);
         const double m = pull_reduce(s, L);
         if (mine) pull_apply(p, qout, rec.x, rec.w, m, q0, r0, pr0, tot);
+    }
+}
+
+// A block's totals of a pull round join the next round's counts.
+__device__ __forceinline__ void pull_totals(TraversalCtl* ctl, int nslot, PullTotals tot, PullTotals& share) {
+    for (int o = 16; o >= 1; o >>= 1) tot.count += __shfl_xor_sync(kFull, tot.count, o);
+    tot.dangling = __reduce_add_sync(kFull, tot.dangling);
+    tot.qmax = __reduce_max_sync(kFull, tot.qmax);
+    if ((threadIdx.x & 31) == 0) {
+        if (tot.count) atomicAdd(&share.count, tot.count);
+        if (tot.dangling) atomicAdd(&share.dangling, tot.dangling);
+        if (tot.qmax) atomicMax(&share.qmax, tot.qmax);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (share.count) atomicAdd(&ctl->pcount[nslot], share.count);
+        if (share.dangling) atomicAdd(&ctl->dctr[nslot], share.dangling);
+        if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], share.qmax);
+        share = PullTotals{0ull, 0u, 0};
+    }
+}
+
+// Pull rounds of a graph whose row lists are at most one step per warp, from round `cur` (2 or later)
+// until one that is not a pull with a frontier (the caller's).  A small graph's round is a chain of loads: the
+// counts, the warp's row record, its in-edges, their sources' residuals.  Here the record and
+// the in-edges (in shared memory, in the list stages that only push rounds use) stay with the warp for all
+// rounds, and the gathers go out before the round's counts are known.  A query at scale 14 (8 edges per
+// vertex) 0.449 -> 0.331 ms, scale 10 0.444 -> 0.293, scale 15 (16 per vertex) 0.746 -> 0.622; what is left
+// of a round's 5 us is the barrier, one gather and the apply's FP64.
+// false: the grid barrier gave up.
+__device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur, int& iters, unsigned F1,
+                                                    StageSmemD& sm, PullTotals& share, GridBarrier* bar,
+                                                    unsigned long long& tph) {
+    TraversalCtl* ctl = p.ctl;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const unsigned gwarp = (unsigned)wib * gridDim.x + blockIdx.x;  // the warp's step: over all SMs first
+    const RowLists& R = p.rows;
+    const auto edge = [&](int u) {  // 8 x 32 in-edges: 4 x 32 in xd0, 2 x 32 each in v0 and d0
+        int2* const at = u < 4   ? reinterpret_cast<int2*>(sm.xd0[wib]) + 32 * u
+                         : u < 6 ? reinterpret_cast<int2*>(sm.v0[wib]) + 32 * (u - 4)
+                                 : reinterpret_cast<int2*>(sm.d0[wib]) + 32 * (u - 6);
+        return at + lane;
+    };
+    const bool seg = gwarp < R.n[0];
+    int L = 32;
+    int4 rec = make_int4(0, 0, 0, 0);
+    int2 sg = make_int2(0, 0);
+    bool mine = false;
+    if (seg) {
+        rec = __ldg(R.rec + gwarp);
+        sg = __ldg(R.seg + gwarp);
+    } else if (gwarp < R.unit[kRowClasses]) {
+        int c = 1;
+        unsigned n = R.n[1], off = R.off[1], first = R.unit[1];
+#pragma unroll
+        for (int k = 2; k < kRowClasses; ++k)
+            if (gwarp >= R.unit[k]) {
+                c = k;
+                n = R.n[k];
+                off = R.off[k];
+                first = R.unit[k];
+            }
+        const int logL = 6 - c;
+        L = 1 << logL;
+        const unsigned row = ((gwarp - first) << (5 - logL)) + (unsigned)(lane >> logL);
+        if (row < n) rec = __ldg(R.rec + off + row);
+        mine = row < n && (lane & (L - 1)) == 0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kLaneEdges; ++u) {
+        const int i = (lane & (L - 1)) + u * L;
+        *edge(u) = i < rec.z ? __ldg(p.adj_r + rec.y + i) : make_int2(0, 0);
+    }
+    for (;;) {
+        const int b = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
+        const float2* qin = p.qf[b];
+        float2 q[kLaneEdges];
+        int wb[kLaneEdges];
+#pragma unroll
+        for (int u = 0; u < kLaneEdges; ++u) {
+            const int2 e = *edge(u);
+            wb[u] = e.y;
+            q[u] = e.y > 0 ? __ldca(qin + e.x) : make_float2(0.f, 0.f);
+        }
+        float q0 = 0.f, pr0 = 0.f;
+        double r0 = 0.0;
+        if (mine || (seg && lane == 0)) {
+            q0 = ldcg(reinterpret_cast<const float*>(qin + rec.x));
+            r0 = ldcg(p.res + rec.x);
+            pr0 = ldcg(p.pr + rec.x);
+        }
+        const unsigned long long c = ldcg(&ctl->pcount[slot]);
+        const unsigned F = (unsigned)(c >> 32), T = (unsigned)c, D = ldcg(&ctl->dctr[slot]);
+        if (F == 0 || T == 0 || iters >= p.max_iter || ldcg(&ctl->farmin[0]) != 0) return true;  // grid-uniform
+        ++iters;
+        if (gtid == 0) {
+            ctl->qctr[fslot] = 0ull;
+            ctl->tilectr[fslot] = 0u;
+            ctl->listctr[fslot] = 0u;
+            ctl->dctr[fslot] = 0u;
+            ctl->pcount[fslot] = 0ull;
+            ctl->popped += F + D;
+            ctl->relaxed += T;
+            ctl->touched += (unsigned)p.V;
+        }
+        if (cur == 2)  // as in ppr_persistent
+            for (unsigned j = gtid; j < F1; j += nthreads) {
+                const int v = ldcg(p.q[1] + j).x;
+                if (__ldg(p.row_r + v) == __ldg(p.row_r + v + 1)) p.qf[1][v] = make_float2(0.f, 0.f);
+            }
+        PullTotals tot{0ull, 0u, 0};
+        PullSums s{0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < kLaneEdges; ++u) pull_add(q[u], wb[u], s);
+        const double m = pull_reduce(s, L);
+        if (mine) pull_apply(p, p.qf[b ^ 1], rec.x, rec.w, m, q0, r0, pr0, tot);
+        if (seg && lane == 0) {
+            if (c2g_dbits(m) != 0ull) atomicAdd(p.msg + rec.x, m);
+            __threadfence();  // the sum is in msg before the segment arrives
+            if (atomicAdd(p.arrived + sg.x, 1u) == (unsigned)sg.y - 1u) {
+                __threadfence();  // the other segments' sums are seen
+                const double all = ldcg(p.msg + rec.x);
+                p.msg[rec.x] = 0.0;
+                p.arrived[sg.x] = 0u;
+                pull_apply(p, p.qf[b ^ 1], rec.x, rec.w, all, q0, r0, pr0, tot);
+            }
+        }
+        pull_totals(ctl, nslot, tot, share);
+        if (!grid_sync(bar, &ctl->flags, p.barrier_ns)) return false;
+        phase_mark(ctl->phase_ns, tph, 2);
+        ++cur;
     }
 }
 
@@ -486,6 +623,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
     unsigned F1 = 0;       // entries of round 1's list
     int qmax = 0;          // largest pushed residual this thread applied in a push round (float bits)
     bool counted = false;  // this round's frontier is counted (a pull made it), not listed
+    bool kept = false;     // ppr_rounds_one_step has run
     for (;;) {
         const int buf = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
         const unsigned long long c = counted ? ldcg(&ctl->pcount[slot]) : ldcg(&ctl->qctr[slot]);
@@ -541,26 +679,16 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                 }
             PullTotals tot{0ull, 0u};
             ppr_pull(p, buf, tot);
-            for (int o = 16; o >= 1; o >>= 1) tot.count += __shfl_xor_sync(kFull, tot.count, o);
-            tot.dangling = __reduce_add_sync(kFull, tot.dangling);
-            tot.qmax = __reduce_max_sync(kFull, tot.qmax);
-            if (lane == 0) {
-                if (tot.count) atomicAdd(&share.count, tot.count);
-                if (tot.dangling) atomicAdd(&share.dangling, tot.dangling);
-                if (tot.qmax) atomicMax(&share.qmax, tot.qmax);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                if (share.count) atomicAdd(&ctl->pcount[nslot], share.count);
-                if (share.dangling) atomicAdd(&ctl->dctr[nslot], share.dangling);
-                if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], share.qmax);
-                share = PullTotals{0ull, 0u, 0};
-                if (gtid == 0) ctl->touched += V;
-            }
+            pull_totals(ctl, nslot, tot, share);
+            if (gtid == 0) ctl->touched += V;
             if (!grid_sync(bar, flags, p.barrier_ns)) return;
             phase_mark(ctl->phase_ns, tph, 2);
             counted = true;
             ++cur;
+            if (p.one_step && !kept) {
+                kept = true;
+                if (!ppr_rounds_one_step(p, cur, iters, F1, sm, share, bar, tph)) return;
+            }
             continue;
         }
         if (counted) {
@@ -783,6 +911,7 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
     p.rows = rows_rev;
     p.arrived = w.arrived;
     if ((rc = ppr_pull_min(g, pp, rows_rev, &p.pull_min))) return rc;
+    p.one_step = false;
     p.dense_div = g->ppr_cfg.dense_div;
     p.pr = pr_dev ? pr_dev : w.pr;
     p.res = w.res;
@@ -828,9 +957,14 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
         p.arrived = w.arrived;
         if (rows_rev.n_long)
             C2G_CUDA(cudaMemsetAsync(w.arrived, 0, sizeof(unsigned) * rows_rev.n_long, g->stream));
-        // every round pulls: one warp per step of the row lists is enough
-        if (p.pull_min == 0u)
-            blocks = std::min(blocks, (int)((rows_rev.unit[kRowClasses] + kPprThreads / 32 - 1) / (kPprThreads / 32)));
+        // every round pulls: one warp per step of the row lists is enough, over all SMs (the applies of
+        // an SM's warps share its FP64 pipe: scale 14 0.368 ms a query on 82 full blocks, 0.331 so)
+        if (p.pull_min == 0u) {
+            const unsigned units = rows_rev.unit[kRowClasses], warps = kPprThreads / 32;
+            blocks = std::min(blocks, std::max((int)((units + warps - 1) / warps),
+                                               std::min(g->num_sms, (int)((units + kStepsPerBlock - 1) / kStepsPerBlock))));
+            p.one_step = units <= (unsigned)blocks * warps && rows_rev.segment <= 32 * kLaneEdges;
+        }
     }
     C2G_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(TraversalCtl), g->stream));
     void* args[] = {&p};
