@@ -564,6 +564,66 @@ __device__ __forceinline__ void sssp_pull(const SsspParams& p, const SsspPull& i
     stage_flush(lst, lout);
 }
 
+// What a warp keeps of its word for all rounds (sssp_pull_kept).
+struct KeptWord {
+    int4 x[32], y[32];  // the rows' first groups
+    int2 rest[32];      // first in-edge behind them, end
+    int deg[32];        // out-degrees
+};
+
+__device__ __forceinline__ void kept_load(const SsspParams& p, const SsspPull& in, KeptWord& k, int lane, int wib) {
+    const unsigned v = (((unsigned)wib * gridDim.x + blockIdx.x) << 5) + (unsigned)lane;
+    int i = 0, e = 0, deg = 0;
+    int4 x = make_int4(0, INT_MAX, 0, INT_MAX), y = x;
+    if (v < (unsigned)p.V) {
+        i = __ldg(in.row + v);
+        e = __ldg(in.row + v + 1);
+        deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
+        if (i < e) {
+            x = __ldg(reinterpret_cast<const int4*>(in.adj + i));
+            y = __ldg(reinterpret_cast<const int4*>(in.adj + i + 2));
+        }
+    }
+    k.x[lane] = x;
+    k.y[lane] = y;
+    k.rest[lane] = make_int2(i + 4, e);
+    k.deg[lane] = deg;
+}
+
+// The first part on a graph with at most one word per warp.  Its rounds are chains of loads (counts, distances
+// and row bounds, first groups, sources, out-degrees) between barriers, so the word's first groups and
+// degrees stay in shared memory, and its distances, which only this warp and the second part write, in b (read
+// anew where stale: rows that may have been queued).  A query at scale 12 (8 edges per vertex) 89.6 -> 74.6 us,
+// scale 16 pruned 133 -> 122, 100,003 uniform vertices 207 -> 178; what is left of a round's 6 us is the
+// barrier, the counts, one gather and the rows that need more than a group.
+__device__ __forceinline__ void sssp_pull_kept(const SsspParams& p, const SsspPull& in, int fmin, const KeptWord& k,
+                                               int& b, bool& stale, int* best, WarpStage& lst,
+                                               const FrontierOut& lout, unsigned long long& count, int& fnew,
+                                               int lane, int wib) {
+    const unsigned w = (unsigned)wib * gridDim.x + blockIdx.x;
+    const unsigned v = (w << 5) + (unsigned)lane;
+    if ((w << 5) < (unsigned)p.V) {
+        if (stale) b = v < (unsigned)p.V ? ldcg(p.dist + v) : INT_MIN;
+        const int b0 = b;
+        const int4 x = k.x[lane], y = k.y[lane];
+        const int2 rest = k.rest[lane];
+        // (a row that is done, or empty, has nothing below the limit)
+        const bool go = b0 > fmin;
+        if (go) b = pull_edges(p.dist, x, y, b0 - fmin, b0);
+        const int last = (y.w >> in.shift) << in.shift;
+        const bool more = go && rest.x < rest.y && last < b - fmin;
+        stale = more && rest.y - rest.x > 4 * kWarpGroups;
+        if (__any_sync(kFull, more)) b = pull_rest(p, in, fmin, v, b, rest.x, rest.y, more, best, lst, lout, lane);
+        if (b < b0) {
+            p.dist[v] = b;
+            fnew = min(fnew, b);
+            const int deg = k.deg[lane];
+            if (deg > 0) count += (1ull << 32) | (unsigned)deg;
+        }
+    }
+    stage_flush(lst, lout);
+}
+
 // Second part, after a barrier, when rows were queued (a hub row that nothing has reached yet needs
 // all its 100,000 edges: read by its warp alone that took 1.07 ms of a scale-22 query): warps
 // take tiles of their groups, and a row's parts meet in atomicMin.  The part that first lowers the queued distance counts the
@@ -626,8 +686,10 @@ __device__ __forceinline__ void sssp_pull_long(const SsspParams& p, const SsspPu
     }
 }
 
-__global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_persistent(const SsspParams p,
-                                                                                         const SsspPull in) {
+// kKept: every round pulls, and the map has at most one word per warp (sssp_pull_kept).
+template <bool kKept>
+__global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm)
+    sssp_rounds_persistent(const SsspParams p, const SsspPull in) {
     TraversalCtl* ctl = p.ctl;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(&ctl->bar_count);
     grid_sync_init();
@@ -682,13 +744,22 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_pe
     if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
     phase_mark(ctl->phase_ns, tph, 0);
 
+    extern __shared__ int4 kept_smem[];
+    KeptWord* const kept = reinterpret_cast<KeptWord*>(kept_smem) + wib;  // kKept
+    if (kKept) kept_load(p, in, *kept, lane, wib);
+    int kept_b = 0;
+    bool kept_stale = true;
+
     int cur = 1, iters = 0;
     bool counted = in.always != 0;  // this round's frontier is counted (a pull made it), not listed
+    // kKept: the coming round's count and smallest frontier distance, loaded together after each barrier
+    unsigned long long next_count = kKept ? ldcg(&ctl->pcount[1]) : 0ull;
+    int next_fmin = kKept ? ldcg(&ctl->farmin[1]) : 0;
     for (;;) {
         const int buf = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
-        unsigned long long c = counted ? ldcg(&ctl->pcount[slot]) : 0ull;
+        unsigned long long c = kKept ? next_count : counted ? ldcg(&ctl->pcount[slot]) : 0ull;
         if (gtid == 0) ctl->qctr[nslot] = 0ull;
-        if (!counted || (c != 0ull && (unsigned)c <= in.pull_min)) {
+        if (!kKept && (!counted || (c != 0ull && (unsigned)c <= in.pull_min))) {
             bits_sweep(p, in.bits[buf], sssp_out(p, buf, slot), fst, gwarp, nwarps, lane);
             if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
             phase_mark(ctl->phase_ns, tph, 1);
@@ -709,9 +780,12 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_pe
         }
         unsigned long long count = 0ull;
         int fnew = INT_MAX;
-        const bool pull = T > in.pull_min;  // grid-uniform
-        const int fmin = ldcg(&ctl->farmin[slot]);
-        if (pull) {
+        const bool pull = kKept || T > in.pull_min;  // grid-uniform
+        const int fmin = kKept ? next_fmin : ldcg(&ctl->farmin[slot]);
+        if (kKept) {
+            sssp_pull_kept(p, in, fmin, *kept, kept_b, kept_stale, sm.v1[wib], lst, pull_long_out(p, in, buf), count, fnew,
+                           lane, wib);
+        } else if (pull) {
             sssp_pull(p, in, fmin, in.bits[buf], in.bits[buf ^ 1], sm.v1[wib], lst, pull_long_out(p, in, buf), count,
                       fnew, lane, wib);
         } else {
@@ -745,6 +819,10 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_pe
         if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
         if (pull) {
             const unsigned long long lc = ldcg(&ctl->lctr[buf]);  // grid-uniform
+            if (kKept) {
+                next_count = ldcg(&ctl->pcount[nslot]);
+                next_fmin = ldcg(&ctl->farmin[nslot]);
+            }
             if (lc) {
                 count = 0ull;
                 fnew = INT_MAX;
@@ -752,6 +830,10 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_pe
                                fnew, lane, gwarp, nwarps);
                 round_totals(ctl, nslot, &share, count, fnew, lane);
                 if (!grid_sync(bar, flags, p.barrier_ns, p.bar_extra)) return;
+                if (kKept) {
+                    next_count = ldcg(&ctl->pcount[nslot]);
+                    next_fmin = ldcg(&ctl->farmin[nslot]);
+                }
             }
         }
         phase_mark(ctl->phase_ns, tph, 2);
@@ -764,6 +846,8 @@ __global__ void __launch_bounds__(kBitsThreads, kBitsBlocksPerSm) sssp_rounds_pe
 // ---------------------------------------------------------------------------------------
 // host side
 
+constexpr size_t kKeptSmem = sizeof(KeptWord) * (kBitsThreads / 32);
+
 static int sssp_geometry(c2g_graph* g) {
     if (g->geom_sssp.blocks > 0) return C2G_OK;
     int coop = 0;
@@ -772,7 +856,12 @@ static int sssp_geometry(c2g_graph* g) {
     int per_sm_a = 0, per_sm_b = 0, per_sm_c = 0;
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_a, sssp_persistent<false>, 512, 0));
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_b, sssp_persistent<true>, 512, 0));
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, sssp_rounds_persistent, kBitsThreads, 0));
+    C2G_CUDA(cudaFuncSetAttribute(sssp_rounds_persistent<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kKeptSmem));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, sssp_rounds_persistent<false>, kBitsThreads, 0));
+    int per_sm_d = 0;
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_d, sssp_rounds_persistent<true>, kBitsThreads, kKeptSmem));
+    per_sm_c = std::min(per_sm_c, per_sm_d);
     const int per_sm = per_sm_a < per_sm_b ? per_sm_a : per_sm_b;
     if (per_sm < 1 || per_sm_c < 1) return fail(C2G_ERR_CUDA, "SSSP kernel cannot be resident (occupancy 0)");
     g->geom_sssp.blocks = per_sm * g->num_sms;
@@ -895,13 +984,18 @@ int sssp_launch(c2g_graph* g, int32_t source, const int32_t* seed_v, const int32
     sssp_round_rule(g, in);
     // delta = 0: Bellman-Ford rounds; delta > 0: near/far buckets
     void* args[] = {&p, &in};
+    const int words = (g->V + 31) / 32, warps = kBitsThreads / 32;
     const int blocks = delta ? g->geom_sssp.blocks
-                     : in.always ? std::min(g->geom_bits.blocks, (g->V + kBitsThreads - 1) / kBitsThreads)
+                     : in.always ? std::min(g->geom_bits.blocks, (words + warps - 1) / warps)
                                  : g->geom_bits.blocks;
+    const bool kept = !delta && in.always && words <= blocks * warps;
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel(delta ? (const void*)sssp_persistent<true> : (const void*)sssp_rounds_persistent,
+    C2G_CUDA(cudaLaunchCooperativeKernel(delta  ? (const void*)sssp_persistent<true>
+                                         : kept ? (const void*)sssp_rounds_persistent<true>
+                                                : (const void*)sssp_rounds_persistent<false>,
                                          dim3(blocks),
-                                         dim3(delta ? g->geom_sssp.threads : g->geom_bits.threads), args, 0, g->stream));
+                                         dim3(delta ? g->geom_sssp.threads : g->geom_bits.threads), args, kept ? kKeptSmem : 0,
+                                         g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     if (ms) {
         C2G_CUDA(cudaEventSynchronize(g->ev1));
