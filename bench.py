@@ -269,8 +269,8 @@ def run_ours(args, rank, world, local_rank):
     sssp_tile = {"big_steps": big, "min_tiles_per_warp": mn,
                  "rule": "rounds with >= min_tiles_per_warp big tiles per warp walk big tiles, else 128 steps",
                  "pull_frac": gs.sssp_batch_pull_frac(),
-                 "pull_rule": "rounds with more than pull_frac * E * Q (query, edge) relaxations pull over the "
-                              "reverse CSR"}
+                 "pull_rule": "rounds with more than a tenth of pull_frac * E * Q (query, edge) relaxations pull over "
+                              "the in-edges, each row in weight order"}
     dist_d = torch.empty((nS, V), dtype=torch.int32, device=dev)
     pr_d = torch.empty((nP, V), dtype=torch.float32, device=dev)
     dist_h = torch.empty((nS, V), dtype=torch.int32).pin_memory().numpy()
@@ -351,9 +351,9 @@ def run_ours(args, rank, world, local_rank):
     kernel_name = "sssp_batch_persistent" if dominant == "s" else "ppr_batch_persistent"
     # DRAM bytes (read + write) per unit processed (push or relaxation), from an ncu
     # capture of the kernel, scaled to this run's average launch.
-    # Full-size step (the autotuners' picks): 2,422 GB per 371.46 G pushes for the PPR
-    # launch, 290.4 GB per 61.37 G relaxations for the SSSP launch.
-    traffic_per_unit = {"p": 2.422e12 / 371.46e9, "s": 290.4e9 / 61.37e9}[dominant]
+    # Full-size step (the autotuners' picks): 2,574.5 GB per 371.46 G pushes for the PPR
+    # launch, 115.3 GB per 61.14 G relaxations for the SSSP launch.
+    traffic_per_unit = {"p": 2.5745e12 / 371.46e9, "s": 115.3e9 / 61.14e9}[dominant]
     units = tot["p_push"] if dominant == "p" else tot["s_rel"]
     traffic = traffic_per_unit * units / args.steps
 
