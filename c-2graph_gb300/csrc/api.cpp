@@ -102,6 +102,7 @@ static int graph_fill(c2g_graph* g, const std::vector<int32_t>& vlist, const int
 static int build_in_edges(c2g_graph* g) {
     int rc = build_in_rows(g);
     if (!rc && g->adj_f && build_reverse_graph(g) == C2G_ERR_CUDA) rc = C2G_ERR_CUDA;
+    if (!rc) cudaGetLastError();  // rows that did not fit leave no error behind
     return rc;
 }
 
