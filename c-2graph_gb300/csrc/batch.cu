@@ -1420,6 +1420,47 @@ __device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, i
     return cnt;
 }
 
+// Two queries' sums s = sh + sl take the messages (hi + lo) * w: the message is pm + pe, then a two-sum of
+// sh + pm.  npm = -pm exactly (round-to-nearest is symmetric), so every line rounds as the scalar form
+//   pm = hi*w, pe = fma(lo, w, fma(hi, w, -pm)), s = sh + pm,
+//   bv = s - sh, av = s - bv, te = (sh - av) + (pm - bv),
+//   sl += te + pe, sh = s
+// does: pm - bv = -(npm + bv).
+__device__ __forceinline__ void pull_pair_add(f32x2 hi, f32x2 lo, f32x2 w, f32x2 nw, f32x2& sh, f32x2& sl) {
+    const f32x2 npm = f2_mul(hi, nw);
+    const f32x2 pe = f2_fma(lo, w, f2_fma(hi, w, npm));
+    const f32x2 s = f2_sub(sh, npm);
+    const f32x2 bv = f2_sub(s, sh);
+    const f32x2 av = f2_sub(s, bv);
+    const f32x2 te = f2_sub(f2_sub(sh, av), f2_add(npm, bv));
+    sl = f2_add(sl, f2_add(te, pe));
+    sh = s;
+}
+
+// The sums of the warp's 32 / LG groups of lanes, two queries per lane, to one query per lane.
+template <int LG>
+__device__ __forceinline__ void pull_pair_reduce(f32x2 h, f32x2 l, int lane, float& sh, float& sl) {
+    float hx, hy, lx, ly;
+    f2_unpack(h, hx, hy);
+    f2_unpack(l, lx, ly);
+#pragma unroll
+    for (int o = LG; o < 32; o <<= 1) {
+        const f32x2 a = f2_pack(hx, hy);
+        const f32x2 b = f2_pack(__shfl_xor_sync(kFull, hx, o), __shfl_xor_sync(kFull, hy, o));
+        const f32x2 ol = f2_pack(__shfl_xor_sync(kFull, lx, o), __shfl_xor_sync(kFull, ly, o));
+        const f32x2 s = f2_add(a, b), bv = f2_sub(s, a);
+        const f32x2 te = f2_add(f2_sub(a, f2_sub(s, bv)), f2_sub(b, bv));
+        f2_unpack(s, hx, hy);
+        f2_unpack(f2_add(f2_add(f2_pack(lx, ly), ol), te), lx, ly);
+    }
+    const int src = lane >> 1;
+    const float h0 = __shfl_sync(kFull, hx, src), h1 = __shfl_sync(kFull, hy, src);
+    const float l0 = __shfl_sync(kFull, lx, src), l1 = __shfl_sync(kFull, ly, src);
+    const bool has = lane < 2 * LG;
+    sh = has ? (lane & 1 ? h1 : h0) : 0.f;
+    sl = has ? (lane & 1 ? l1 : l0) : 0.f;
+}
+
 // Position in a warp's stream of chunks.
 struct PPullPos {
     unsigned c;   // chunk; ~0: beyond the last item
@@ -1428,8 +1469,11 @@ struct PPullPos {
 constexpr unsigned kPullFirst = 1u << 31, kPullLast = 1u << 30;
 __device__ __forceinline__ unsigned pull_w0(const PPullPos& q) { return q.wf & ~(kPullFirst | kPullLast); }
 
-// Phase A of a pull round.
-template <int WP>
+// Phase A of a pull round.  LG < 32: a batch of one query word, at most 2 LG queries; LG lanes of two queries each
+// take an in-edge, so that a warp takes 32 / LG in-edges at a time and its packed pairs are full (with one query
+// per lane a round cost 66 instructions per in-edge for any number of queries: 11 queries at scale 18
+// 14.3 -> 11.2 ms a batch, 32 16.6 -> 14.0, 12 at scale 20 42.5 -> 32.0).
+template <int WP, int LG>
 __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf, int ob, unsigned* qctr,
                                                 PPullSmem& sm, WarpStage& fst, const FrontierOut& out, unsigned* dctr,
                                                 unsigned* sctr, unsigned long long& psum, int lane, bool& bad) {
@@ -1439,7 +1483,8 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
     const unsigned per_group = (nchunks + (1u << p.pull_log) - 1u) >> p.pull_log;
     const unsigned nitems = per_group << (p.logW - (WP == 4 ? 2 : WP == 2 ? 1 : 0));
     const unsigned* am = p.amask[buf];
-    const float2* rql = p.rqf[buf] + lane;
+    const float2* rqf = p.rqf[buf];
+    const float2* rql = rqf + lane;
     const unsigned lane_bit = 1u << lane;
     const unsigned long long rmax_bits = c2g_dbits((double)p.rmax);
     unsigned cnt = 0;
@@ -1539,6 +1584,14 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
         // only in-edges whose source has an active lane in the item's words are visited: the
         // others would add exact zeros
         const unsigned lm = __ballot_sync(kFull, mine != 0u);
+        if constexpr (LG < 32) {  // they move to the front, in order: (lanes, line, weight)
+            const int2 my = sm.ed[e0][lane];
+            const unsigned below = lane_bit - 1u;
+            const int at = (lm >> lane) & 1u ? __popc(lm & below) : __popc(lm) + __popc(~lm & below);
+            __syncwarp();
+            sm.mk[m0][at] = make_uint4(mine, (unsigned)my.x, (unsigned)my.y, 0u);
+            __syncwarp();
+        }
         if (q0.wf & kPullFirst) {
             whole = false;
             any = false;
@@ -1557,6 +1610,32 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
             const unsigned nxt = after ? (unsigned)__ffs((int)after) - 1u : len;
             unsigned l = lm & (nxt == 32u ? ~0u : (1u << nxt) - 1u) & ~((1u << pos) - 1u);
             any = any || l != 0u;
+            if constexpr (LG < 32) {
+                constexpr int G = 32 / LG;          // in-edges at a time,
+                constexpr int U = G >= 4 ? 2 : 4;   // times U in flight
+                const unsigned first = (unsigned)__popc(lm & ((1u << pos) - 1u)), end = first + (unsigned)__popc(l);
+                const unsigned q2 = 2u * (unsigned)(lane & (LG - 1));  // this lane's queries q2, q2 + 1
+                for (unsigned i0 = first + (unsigned)(lane / LG); i0 - (unsigned)(lane / LG) < end; i0 += G * U) {
+                    float4 v[U];
+                    float wa[U], wb[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const unsigned i = i0 + (unsigned)(u * G);
+                        const uint4 e = i < end ? sm.mk[m0][i] : make_uint4(0u, 0u, 0u, 0u);
+                        const unsigned on = (e.x >> q2) & 3u;
+                        v[u] = on ? __ldcg(reinterpret_cast<const float4*>(rqf + (size_t)e.y * 32u + q2))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+                        // a query at rest adds exact zeros
+                        wa[u] = on & 1u ? __uint_as_float(e.z) : 0.f;
+                        wb[u] = on & 2u ? __uint_as_float(e.z) : 0.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        pull_pair_add(f2_pack(v[u].x, v[u].z), f2_pack(v[u].y, v[u].w), f2_pack(wa[u], wb[u]),
+                                      f2_pack(-wa[u], -wb[u]), sh2[0], sl2[0]);
+                }
+                l = 0u;
+            }
             while (l) {
                 // gather the pushed residuals of EF in-edges, then add them
                 float2 qb[EF][WP];
@@ -1583,32 +1662,17 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
                     const f32x2 nw2 = f2_pack(-wk[h], -wk[h]);
 #pragma unroll
                     for (int j = 0; j < NP; ++j) {
-                        // message (hi + lo) * w = pm + pe; two-sum of sh + pm, for words
-                        // 2j and 2j+1 at once.  npm = -pm exactly (round-to-nearest is
-                        // symmetric), so every line rounds as the scalar form
-                        //   pm = hi*w, pe = fma(lo, w, fma(hi, w, -pm)), s = sh + pm,
-                        //   bv = s - sh, av = s - bv, te = (sh - av) + (pm - bv),
-                        //   sl += te + pe, sh = s
-                        // does: pm - bv = -(npm + bv).
                         const float2 qa = qb[h][2 * j], qc = 2 * j + 1 < WP ? qb[h][(2 * j + 1) % WP] : make_float2(0.f, 0.f);
-                        const f32x2 hi = f2_pack(qa.x, qc.x);
-                        const f32x2 lo = f2_pack(qa.y, qc.y);
-                        const f32x2 npm = f2_mul(hi, nw2);
-                        const f32x2 pe = f2_fma(lo, w2, f2_fma(hi, w2, npm));
-                        const f32x2 s2 = f2_sub(sh2[j], npm);
-                        const f32x2 bv = f2_sub(s2, sh2[j]);
-                        const f32x2 av = f2_sub(s2, bv);
-                        const f32x2 te = f2_sub(f2_sub(sh2[j], av), f2_add(npm, bv));
-                        sl2[j] = f2_add(sl2[j], f2_add(te, pe));
-                        sh2[j] = s2;
+                        pull_pair_add(f2_pack(qa.x, qc.x), f2_pack(qa.y, qc.y), w2, nw2, sh2[j], sl2[j]);
                     }
                 }
             }
             const bool ends = nxt < len || follow != 0u;
             if (any && (ends || (q0.wf & kPullLast))) {
                 float sh[WP], sl[WP];
+                if constexpr (LG < 32) pull_pair_reduce<LG>(sh2[0], sl2[0], lane, sh[0], sl[0]);
 #pragma unroll
-                for (int j = 0; j < NP; ++j) {
+                for (int j = 0; j < NP && LG == 32; ++j) {
                     float a, b, c, d;
                     f2_unpack(sh2[j], a, b);
                     f2_unpack(sl2[j], c, d);
@@ -1673,7 +1737,8 @@ __device__ __noinline__ void pbatch_rebuild(const PprBatchParams& p, int b, int 
 // WP: query words of a pull item (1, 2, or 4 of four or more).  Dynamic shared memory: a PPullSmem per warp.
 constexpr size_t kPprBatchSmem = sizeof(PPullSmem) * (kPprBatchThreads / 32);
 
-template <int WP>
+// WP: query words a pull takes at a time (1, 2, or 4 of four or more); LG: lanes of a pulled in-edge (pbatch_pull)
+template <int WP, int LG>
 __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
     ppr_batch_persistent(const PprBatchParams p) {
     extern __shared__ uint4 pull_smem[];
@@ -1821,7 +1886,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
                 pushes += (long long)P;
                 steps += T;
             }
-            touched += pbatch_pull<WP>(p, buf, ob, &ctl->tilectr[cur % 3], psm, fst, pbatch_out(p, ob, nslot),
+            touched += pbatch_pull<WP, LG>(p, buf, ob, &ctl->tilectr[cur % 3], psm, fst, pbatch_out(p, ob, nslot),
                                    &ctl->dctr[nslot], &ctl->listctr[cur % 3], psum, lane, bad);
         } else {
             // Push round, phase A: push along the frontier's edges (owner runs, as in the
@@ -2002,11 +2067,13 @@ __global__ void batch_transpose_d2f(const double* __restrict__ src, int V, int Q
     }
 }
 
-// The kernel for 2^logW query words, with its shared memory allowed, and its blocks per SM.
-static int ppr_batch_kernel(int logW, const void** kernel, int* per_sm) {
-    *kernel = logW == 0 ? (const void*)ppr_batch_persistent<1>
-            : logW == 1 ? (const void*)ppr_batch_persistent<2>
-                        : (const void*)ppr_batch_persistent<4>;
+// The kernel for nq queries in 2^logW words, with its shared memory allowed, and its blocks per SM.
+static int ppr_batch_kernel(int logW, int nq, const void** kernel, int* per_sm) {
+    *kernel = logW == 0 ? nq <= 8    ? (const void*)ppr_batch_persistent<1, 4>
+                          : nq <= 16 ? (const void*)ppr_batch_persistent<1, 8>
+                                     : (const void*)ppr_batch_persistent<1, 16>
+            : logW == 1 ? (const void*)ppr_batch_persistent<2, 32>
+                        : (const void*)ppr_batch_persistent<4, 32>;
     C2G_CUDA(cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPprBatchSmem));
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, *kernel, kPprBatchThreads, kPprBatchSmem));
     if (*per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
@@ -2252,7 +2319,7 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     const void* kernel = nullptr;
     C2G_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
     if (!coop) return fail(C2G_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    if ((rc = ppr_batch_kernel(logW, &kernel, &per_sm))) return rc;
+    if ((rc = ppr_batch_kernel(logW, nq, &kernel, &per_sm))) return rc;
     const size_t VQ = (size_t)g->V * (size_t)w->Q;
     if ((rc = ppr_batch_clean(g, w))) return rc;
     C2G_CUDA(cudaMemcpyAsync(w->src, sources, sizeof(int) * (size_t)nq, cudaMemcpyHostToDevice, g->stream));
@@ -2352,7 +2419,7 @@ int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, in
     if ((rc = ppr_pull_threshold(g, prm, &pull_min))) return rc;
     int per_sm = 0;
     const void* kernel = nullptr;
-    if ((rc = ppr_batch_kernel(logW, &kernel, &per_sm))) return rc;
+    if ((rc = ppr_batch_kernel(logW, Q, &kernel, &per_sm))) return rc;
     PprBatchParams p;
     ppr_batch_params(g, w, Q, logW, prm, pull_min, p);
     const int blocks = grid_blocks(g, per_sm);

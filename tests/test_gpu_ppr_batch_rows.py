@@ -49,7 +49,7 @@ def _check(csr, n, seed):
                 assert np.abs(res[i].astype(np.float64) - rr).sum() <= 1e-6, (n, ratio, i)
 
 
-@pytest.mark.parametrize("n", [1, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("n", [1, 2, 8, 9, 16, 17, 31, 32, 33, 64, 65, 200])
 def test_rows_across_chunks(gpu_available, n):
     lengths = [1, 31, 32, 33, 63, 64, 65, 1, 1, 1, 255, 256, 257, 30, 2, 500] * 2 + [1] * 70
     _check(_rows_graph(lengths, 600, n, 700), n, n)
