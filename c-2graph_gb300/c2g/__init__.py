@@ -411,7 +411,7 @@ class Graph:
 
     def ppr_batch_pull(self, ratio=8.0):
         """Batched rounds with more than ratio * E pushes pull over the reverse CSR
-        (ratio < 0: push only; 0: every round)."""
+        (ratio < 0: push only; 0: every round; until set: at most 8, by queries and edges)."""
         _check(lib().c2g_ppr_batch_set_pull(self._h, float(ratio)))
 
     def ppr_batch_autotune(self, sources, params, reps=1, json_path=None):

@@ -482,6 +482,7 @@ int c2g_ppr_batch_set_pull(c2g_graph* g, float ratio) {
     if (ratio != ratio) return fail(C2G_ERR_ARG, "ratio is NaN");
     std::lock_guard<std::mutex> lk(g->mu);
     g->ppr_cfg.batch_pull_ratio = ratio;
+    g->ppr_cfg.batch_ratio_set = true;
     return C2G_OK;
 }
 

@@ -2216,9 +2216,20 @@ int ppr_pull_prepare(c2g_graph* g) {
 // reverse CSR (a view uses its base's, never builds it) and finite weights; with rmax
 // below 1e-30 pushed residuals may leave the FP32 range of the pull's float pairs, so such
 // launches push only.
-static int ppr_pull_threshold(c2g_graph* g, const c2g_ppr_params& prm, unsigned long long* pull_min) {
+//
+// Until the caller sets a ratio: 8 E, but for a batch of nq queries (0: a resident batch, whose slots say little
+// about the queries at work) half an E per query for fewer than 16, and E / 4 for up to 64 on
+// graphs up to kSmallPullEdges, where a round is latency and a pull saves the push's atomics and its sweep.  ms a batch
+// at 8 E / this: 5 queries at scale 14 7.39 / 3.95, 2 6.74 / 3.74, 20 4.82 / 4.57, 3 on 3,000 uniform
+// vertices 5.48 / 2.30, 4 at scale 18 10.4 / 9.5, 8 11.6 / 10.1, 3 at scale 20 27.5 / 25.2; 11 or more at scale
+// 18 are within 1%; 250 on 100,003 uniform vertices 35.9 at 8 E, 37.4 at E / 4.
+constexpr int64_t kSmallPullEdges = 1 << 20;
+
+static int ppr_pull_threshold(c2g_graph* g, const c2g_ppr_params& prm, int nq, unsigned long long* pull_min) {
     *pull_min = ~0ull;
-    const float ratio = g->ppr_cfg.batch_pull_ratio;
+    float ratio = g->ppr_cfg.batch_pull_ratio;
+    if (!g->ppr_cfg.batch_ratio_set && nq > 0)
+        ratio = nq <= 64 && g->E <= kSmallPullEdges ? 0.25f : std::min(ratio, 0.5f * (float)nq);
     if (ratio >= 0.f && g->E > 0 && prm.rmax >= 1e-30f && (g->wstat_valid || !g->borrowed)) {
         int rc;
         if (!g->borrowed && (rc = ppr_pull_prepare(g))) return rc;
@@ -2312,7 +2323,7 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     int rc;
     const size_t ns = seed_v ? seed_v->size() : 0;
     unsigned long long pull_min = ~0ull;
-    if ((rc = ppr_pull_threshold(g, prm, &pull_min))) return rc;
+    if ((rc = ppr_pull_threshold(g, prm, nq, &pull_min))) return rc;
     if ((rc = ppr_batch_alloc(g, Q, ns))) return rc;
     PprBatchWork* w = reinterpret_cast<PprBatchWork*>(g->ppr_batch);
     int coop = 0, per_sm = 0;
@@ -2416,7 +2427,7 @@ int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, in
     while ((32 << logW) < Q) ++logW;
     int rc;
     unsigned long long pull_min = ~0ull;
-    if ((rc = ppr_pull_threshold(g, prm, &pull_min))) return rc;
+    if ((rc = ppr_pull_threshold(g, prm, 0, &pull_min))) return rc;  // slots, not queries
     int per_sm = 0;
     const void* kernel = nullptr;
     if ((rc = ppr_batch_kernel(logW, Q, &kernel, &per_sm))) return rc;

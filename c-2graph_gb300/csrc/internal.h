@@ -115,6 +115,7 @@ struct SsspConfig {
 
 struct PprConfig {
     float batch_pull_ratio = 8.0f;  // batched rounds with more than ratio * E pushes pull (< 0: never)
+    bool batch_ratio_set = false;   // the caller's; else ppr_pull_threshold lowers it for few queries
     int log_tile = 8;
     int pull_div = 0;   // pull round when frontier out-edges * pull_div > E; 0 = push only
     bool pull_set = false;  // until it is set, ppr.cu picks the rule by the graph's size

@@ -275,9 +275,10 @@ int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div);
  * than ratio * E (query, edge) pushes pulls over the reverse CSR (built on first use):
  * each target gathers its in-neighbours' pushed residuals and sums the messages as FP32
  * pairs (about 47 bits of relative precision) before they meet the FP64 residual.
- * ratio < 0: push only; 0: pull every round; default 8.  Pull rounds need finite weights
- * and rmax >= 1e-30.  Results are the same BSP rounds either way, within summation
- * order. */
+ * ratio < 0: push only; 0: pull every round; default 8, and until it is set, in
+ * c2g_ppr_batch, half the number of queries where that is less, 1/4 for up to 64 queries on
+ * graphs up to 2^20 edges.  Pull rounds need finite weights and rmax >= 1e-30.  Results are
+ * the same BSP rounds either way, within summation order. */
 int c2g_ppr_batch_set_pull(c2g_graph* g, float ratio);
 
 /* Autotuner of that round shape (no counterpart in the reference): times ratios {push only, 1, 2, 4, 8, 16, 32} on this

@@ -39,8 +39,9 @@ def _check(csr, n, seed):
     src = np.random.default_rng(seed).integers(0, V, n).astype(np.int32)
     with c2g.Graph.create(csr[0], csr[1], flist=csr[2]) as g:
         prm = g.ppr_params(alpha=0.15, rmax=1e-7, seeded=0, pr0=0.15, r0=1.0, max_iter=500)
-        for ratio in (0.0, 4.0):
-            g.ppr_batch_pull(ratio)
+        for ratio in (None, 0.0, 4.0):  # None: the library's own
+            if ratio is not None:
+                g.ppr_batch_pull(ratio)
             pr, res, st = g.ppr_batch(src, prm)
             assert st.status_flags == 0
             for i in range(0, n, max(1, n // 12)):
