@@ -1177,6 +1177,7 @@ struct PprBatchParams {
     const int* r_prefix;      // how many rows start in earlier chunks,
     const int* r_rows;        // and the rows in order
     int pull_log;             // log2 of the chunks per pull item
+    unsigned pull_groups;     // groups of WP query words with queries
     unsigned long long pull_min;
     int epoch_rounds;  // > 0: an epoch of a resident batch (state at rest in the arrays; at most this many rounds)
     int cur0;          // round index the epoch starts at (its parity picks the frontier buffers)
@@ -1481,7 +1482,7 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
     constexpr int NP = (WP + 1) / 2;        // packed word pairs
     const unsigned nchunks = (p.E + 31u) >> 5;
     const unsigned per_group = (nchunks + (1u << p.pull_log) - 1u) >> p.pull_log;
-    const unsigned nitems = per_group << (p.logW - (WP == 4 ? 2 : WP == 2 ? 1 : 0));
+    const unsigned nitems = per_group * p.pull_groups;
     const unsigned* am = p.amask[buf];
     const float2* rqf = p.rqf[buf];
     const float2* rql = rqf + lane;
@@ -2067,13 +2068,17 @@ __global__ void batch_transpose_d2f(const double* __restrict__ src, int V, int Q
     }
 }
 
-// The kernel for nq queries in 2^logW words, with its shared memory allowed, and its blocks per SM.
-static int ppr_batch_kernel(int logW, int nq, const void** kernel, int* per_sm) {
-    *kernel = logW == 0 ? nq <= 8    ? (const void*)ppr_batch_persistent<1, 4>
-                          : nq <= 16 ? (const void*)ppr_batch_persistent<1, 8>
-                                     : (const void*)ppr_batch_persistent<1, 16>
-            : logW == 1 ? (const void*)ppr_batch_persistent<2, 32>
-                        : (const void*)ppr_batch_persistent<4, 32>;
+// The kernel for queries in the first nq of 32 * 2^logW slots, with its shared memory allowed, its groups of query
+// words and its blocks per SM.  Pulls take as many words at a time as hold queries: a resident batch of 64 slots
+// with 11 queries at work pulls one word, not two (a wave of 32 mixed requests, scale 18: 27.5 -> 24.2 ms).
+static int ppr_batch_kernel(int nq, const void** kernel, unsigned* groups, int* per_sm) {
+    const unsigned words = ((unsigned)nq + 31u) / 32u;
+    *groups = words <= 2u ? 1u : (words + 3u) / 4u;
+    *kernel = words <= 1u ? nq <= 8    ? (const void*)ppr_batch_persistent<1, 4>
+                            : nq <= 16 ? (const void*)ppr_batch_persistent<1, 8>
+                                       : (const void*)ppr_batch_persistent<1, 16>
+            : words == 2u ? (const void*)ppr_batch_persistent<2, 32>
+                          : (const void*)ppr_batch_persistent<4, 32>;
     C2G_CUDA(cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPprBatchSmem));
     C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, *kernel, kPprBatchThreads, kPprBatchSmem));
     if (*per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
@@ -2083,8 +2088,7 @@ static int ppr_batch_kernel(int logW, int nq, const void** kernel, int* per_sm) 
 // log2 of the chunks of 32 in-edges per pull item: 8 chunks (a fourth of the rows then crosses an item
 // boundary), fewer where that leaves the grid's warps less than 16 items each to level the round's
 // end (40 queries at scale 16, 6 chunks per warp: 8-chunk items 14.8 ms a batch, 2 12.8, 1 11.7).
-static int ppr_pull_log(const c2g_graph* g, int logW, int blocks) {
-    const size_t groups = logW >= 2 ? size_t(1) << (logW - 2) : 1;
+static int ppr_pull_log(const c2g_graph* g, unsigned groups, int blocks) {
     const size_t chunks = ((size_t)g->E + 31) / 32, warps = (size_t)blocks * (kPprBatchThreads / 32);
     int k = 3;
     while (k > 0 && (chunks >> k) * groups < 16 * warps) --k;
@@ -2330,7 +2334,8 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     const void* kernel = nullptr;
     C2G_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
     if (!coop) return fail(C2G_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    if ((rc = ppr_batch_kernel(logW, nq, &kernel, &per_sm))) return rc;
+    unsigned groups = 0;
+    if ((rc = ppr_batch_kernel(nq, &kernel, &groups, &per_sm))) return rc;
     const size_t VQ = (size_t)g->V * (size_t)w->Q;
     if ((rc = ppr_batch_clean(g, w))) return rc;
     C2G_CUDA(cudaMemcpyAsync(w->src, sources, sizeof(int) * (size_t)nq, cudaMemcpyHostToDevice, g->stream));
@@ -2347,7 +2352,8 @@ int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g
     p.nq = nq;
     p.seed_off = seed_off ? w->seed_off : nullptr;
     const int blocks = grid_blocks(g, per_sm);
-    p.pull_log = ppr_pull_log(g, logW, blocks);
+    p.pull_groups = groups;
+    p.pull_log = ppr_pull_log(g, groups, blocks);
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
@@ -2419,7 +2425,7 @@ int ppr_batch_reserve(c2g_graph* g, int Q, PprBatchArrays* a) {
     return C2G_OK;
 }
 
-int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, int rounds, float* ms,
+int ppr_batch_epoch(c2g_graph* g, int Q, int used, const c2g_ppr_params& prm, int cur0, int rounds, float* ms,
                     long long* counters, TraversalCtl* ctl_out) {
     PprBatchWork* w = reinterpret_cast<PprBatchWork*>(g->ppr_batch);
     if (!w || w->Q < Q) return fail(C2G_ERR_ARG, "resident PPR batch has no workspace");
@@ -2430,11 +2436,13 @@ int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, in
     if ((rc = ppr_pull_threshold(g, prm, 0, &pull_min))) return rc;  // slots, not queries
     int per_sm = 0;
     const void* kernel = nullptr;
-    if ((rc = ppr_batch_kernel(logW, Q, &kernel, &per_sm))) return rc;
+    unsigned groups = 0;
+    if ((rc = ppr_batch_kernel(used, &kernel, &groups, &per_sm))) return rc;
     PprBatchParams p;
     ppr_batch_params(g, w, Q, logW, prm, pull_min, p);
     const int blocks = grid_blocks(g, per_sm);
-    p.pull_log = ppr_pull_log(g, logW, blocks);
+    p.pull_groups = groups;
+    p.pull_log = ppr_pull_log(g, groups, blocks);
     p.epoch_rounds = rounds < 1 ? 1 : rounds;
     p.cur0 = cur0;
     p.max_iter = 1 << 30;  // the per-query caps are the session's

@@ -263,7 +263,7 @@ void session_set_grid_share(c2g_session* s, float share);
 int sssp_batch_reserve(c2g_graph* g, int Q, int** dist, unsigned** mask);
 int sssp_batch_epoch(c2g_graph* g, int Q, int rounds, float* ms, long long* counters, TraversalCtl* ctl_out);
 int ppr_batch_reserve(c2g_graph* g, int Q, PprBatchArrays* a);
-int ppr_batch_epoch(c2g_graph* g, int Q, const c2g_ppr_params& prm, int cur0, int rounds, float* ms,
+int ppr_batch_epoch(c2g_graph* g, int Q, int used, const c2g_ppr_params& prm, int cur0, int rounds, float* ms,
                     long long* counters, TraversalCtl* ctl_out);
 int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const std::vector<int32_t>* seed_off,
                       const std::vector<int32_t>* seed_v, const std::vector<int32_t>* seed_w, int32_t* out,

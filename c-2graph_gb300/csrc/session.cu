@@ -415,11 +415,12 @@ int c2g_session_step(c2g_session* s, int32_t rounds, int32_t* finished, int32_t 
     if (stats) std::memset(stats, 0, sizeof(*stats));
     int rc;
     if ((rc = apply_pending(s))) return rc;
-    int running = 0;
+    int running = 0, used = 0;  // used: slots up to the last running one
     int room = rounds;
     for (int i = 0; i < s->Q; ++i)
         if (s->state[i] == kRunning) {
             ++running;
+            used = i + 1;
             if (s->kind == C2G_REQ_PPR) room = std::min(room, s->prm.max_iter - s->rounds[i]);
         }
     int iters = 0;
@@ -428,7 +429,7 @@ int c2g_session_step(c2g_session* s, int32_t rounds, int32_t* finished, int32_t 
         long long counters[2] = {0, 0};
         TraversalCtl ctl;
         rc = s->kind == C2G_REQ_SSSP ? sssp_batch_epoch(g, s->Q, room, &ms, counters, &ctl)
-                                     : ppr_batch_epoch(g, s->Q, s->prm, s->cur, room, &ms, counters, &ctl);
+                                     : ppr_batch_epoch(g, s->Q, used, s->prm, s->cur, room, &ms, counters, &ctl);
         if (rc) return rc;
         if (ctl.flags & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS))
             return fail(ctl.flags & C2G_FLAG_BARRIER_TIMEOUT ? C2G_ERR_TIMEOUT : C2G_ERR_OVERFLOW,
