@@ -155,7 +155,10 @@ __device__ __forceinline__ void ppr_push(const PprParams& p, int buf, int slot, 
 }
 
 // Pulls end when a pushed residual passes 2^60 (float bits): with weights below 2^30 (checked by the host)
-// every sum of up to 2^31 messages then stays a finite float.
+// every sum of up to 2^31 messages then stays a finite float.  The rounds' word for it is ctl->farmin[slot],
+// kept by round slot like the counts: a round reads its own slot's and whoever finds such a residual writes the
+// next round's, so nothing that a round reads is written while it runs (a pull round has one barrier, at its
+// end).  A round that finds it set hands it on, so that it stays.
 constexpr int kPullMaxQ = (127 + 60) << 23;
 constexpr unsigned kPullMaxWeight = (127 + 30) << 23;
 
@@ -345,7 +348,7 @@ __device__ __forceinline__ void pull_totals(TraversalCtl* ctl, int nslot, PullTo
     if (threadIdx.x == 0) {
         if (share.count) atomicAdd(&ctl->pcount[nslot], share.count);
         if (share.dangling) atomicAdd(&ctl->dctr[nslot], share.dangling);
-        if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], share.qmax);
+        if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[nslot], share.qmax);
         share = PullTotals{0ull, 0u, 0};
     }
 }
@@ -423,7 +426,7 @@ __device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur
         }
         const unsigned long long c = ldcg(&ctl->pcount[slot]);
         const unsigned F = (unsigned)(c >> 32), T = (unsigned)c, D = ldcg(&ctl->dctr[slot]);
-        if (F == 0 || T == 0 || iters >= p.max_iter || ldcg(&ctl->farmin[0]) != 0) return true;  // grid-uniform
+        if (F == 0 || T == 0 || iters >= p.max_iter || ldcg(&ctl->farmin[slot]) != 0) return true;  // grid-uniform
         ++iters;
         if (gtid == 0) {
             ctl->qctr[fslot] = 0ull;
@@ -431,6 +434,7 @@ __device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur
             ctl->listctr[fslot] = 0u;
             ctl->dctr[fslot] = 0u;
             ctl->pcount[fslot] = 0ull;
+            ctl->farmin[fslot] = 0;
             ctl->popped += F + D;
             ctl->relaxed += T;
             ctl->touched += (unsigned)p.V;
@@ -642,7 +646,8 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
             break;
         }
         // grid-uniform; float pairs hold the pushed residuals and their sums below kPullMaxQ
-        const bool pull = T > p.pull_min && ldcg(&ctl->farmin[0]) == 0;
+        const bool large = ldcg(&ctl->farmin[slot]) != 0;
+        const bool pull = T > p.pull_min && !large;
         // Pop the activated vertices without out-edges: their residual is dropped.  A pull does so
         // for every vertex with in-edges.
         if (!counted) {
@@ -666,6 +671,8 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
             ctl->listctr[fslot] = 0u;
             ctl->dctr[fslot] = 0u;
             ctl->pcount[fslot] = 0ull;
+            ctl->farmin[fslot] = 0;
+            if (large) atomicMax(&ctl->farmin[nslot], 1);
             ctl->popped += F + D;
             ctl->relaxed += T;
         }
@@ -766,7 +773,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
             }
         }
         stage_flush(fst, out);
-        if (qmax > kPullMaxQ) atomicMax(&ctl->farmin[0], qmax);
+        if (qmax > kPullMaxQ) atomicMax(&ctl->farmin[nslot], qmax);
         if (!grid_sync(bar, flags, p.barrier_ns)) return;
         phase_mark(ctl->phase_ns, tph, 1);
         ++cur;

@@ -1,0 +1,40 @@
+"""Single push whose residuals pass 2^60 on the way: the round after, every block leaves the pulls together and
+the rounds push in FP64.  Weights that multiply the mass by 34 to 255,000 a round, so that the limit is passed
+after few or many pulls; graphs of one row step per warp, of several, and above the size where every round pulls.
+
+Tolerance: pr is FP32 and a vertex takes at most one rounding of 2^-24 per round, so L1 within rounds * 2^-24 of
+the mass; the residuals are FP64 and come back rounded once."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(V, ef, scale, seed):
+    rng = np.random.default_rng(seed)
+    key = np.unique(rng.integers(0, V, V * ef) * V + rng.integers(0, V, V * ef))
+    src, dst = key // V, (key % V).astype(np.int32)
+    vl = np.zeros(V + 1, np.int32)
+    np.cumsum(np.bincount(src, minlength=V), out=vl[1:])
+    w = rng.random(len(src)) + 0.01
+    return vl, dst, (w * scale / np.bincount(src, weights=w, minlength=V)[src]).astype(np.float32)
+
+
+@pytest.mark.parametrize("V,ef", [(3000, 8), (120000, 12), (400000, 11)])
+@pytest.mark.parametrize("scale,cap", [(40.0, 18), (4000.0, 9), (3e5, 6)])
+def test_all_blocks_leave_the_pulls_together(gpu_available, V, ef, scale, cap):
+    import c2g
+    import oracle
+
+    vl, el, w = _graph(V, ef, scale, V + cap)
+    rng = np.random.default_rng(cap)
+    with c2g.Graph.create(vl, el, flist=w) as g:
+        prm = g.ppr_params(alpha=0.15, rmax=1e-7, seeded=0, pr0=0.15, r0=1.0, max_iter=cap)
+        for s in rng.choice(np.flatnonzero(np.diff(vl) > 0), 2):
+            rp, rr, _, _ = oracle.ppr_push(vl, el, w, int(s), 0.15, 1e-7, max_iter=cap)
+            assert np.abs(rr).max() > 2.0 ** 60  # passed on the way
+            for _ in range(6):
+                pr, res, st = g.ppr(int(s), prm)
+                assert st.status_flags == c2g.FLAG_ITER_CAP
+                for got, want in ((pr, rp), (res, rr)):
+                    assert np.abs(got.astype(np.float64) - want).sum() <= cap * 2.0 ** -24 * np.abs(want).sum()
