@@ -527,6 +527,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
     }
     if (!grid_sync(bar, flags, p.barrier_ns)) return;
 
+    int qmax = 0;  // largest pushed residual this thread set outside a pull (float bits)
     const int s = p.source;
     const int s_deg = __ldg(p.row + s + 1) - __ldg(p.row + s);
     if (p.src_list) {
@@ -612,12 +613,15 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
                     dang = !want;
                     if (want) p.res[v] = 0.0;
                     r *= one_m_a;
-                    p.qf[1][v] = ppr_pair(r);
+                    const float2 q = ppr_pair(r);
+                    p.qf[1][v] = q;
+                    qmax = max(qmax, __float_as_int(q.x));  // a record's weight may be as large as a float
                 }
             }
             stage_push(fst, out, want, v, deg, 0.f, r);
             list_push(p.dangle, &ctl->dctr[1], (unsigned)p.V, flags, dang, v);
         }
+        if (qmax > kPullMaxQ) atomicMax(&ctl->farmin[1], qmax);
         stage_flush(fst, out);
     }
     if (!grid_sync(bar, flags, p.barrier_ns)) return;
@@ -625,7 +629,6 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
 
     int cur = 1, iters = 0;
     unsigned F1 = 0;       // entries of round 1's list
-    int qmax = 0;          // largest pushed residual this thread applied in a push round (float bits)
     bool counted = false;  // this round's frontier is counted (a pull made it), not listed
     bool kept = false;     // ppr_rounds_one_step has run
     for (;;) {

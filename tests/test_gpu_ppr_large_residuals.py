@@ -38,3 +38,40 @@ def test_all_blocks_leave_the_pulls_together(gpu_available, V, ef, scale, cap):
                 assert st.status_flags == c2g.FLAG_ITER_CAP
                 for got, want in ((pr, rp), (res, rr)):
                     assert np.abs(got.astype(np.float64) - want).sum() <= cap * 2.0 ** -24 * np.abs(want).sum()
+
+
+def _heavy_records():
+    """Vertex 0 has 40 records of weight 3e38; their vertices send all to a hub (weight 1), the hub to 64 leaves
+    (1/64), the leaves to one tail (1e-30): the hub's residual is beyond FP32, what comes after it is not."""
+    n, hub = 40, 41
+    leaf = np.arange(42, 106)
+    src = np.concatenate([np.arange(1, n + 1), np.full(64, hub), leaf])
+    dst = np.concatenate([np.full(n, hub), leaf, np.full(64, 106)]).astype(np.int32)
+    w = np.concatenate([np.ones(n), np.full(64, 1 / 64), np.full(64, 1e-30)]).astype(np.float32)
+    V = 107
+    vl = np.zeros(V + 1, np.int32)
+    np.cumsum(np.bincount(src, minlength=V), out=vl[1:])
+    hv = np.full(V + 1, n, np.int32)
+    hv[0] = 0
+    return (vl, dst, w), (hv, np.arange(1, n + 1, dtype=np.int32), np.full(n, 3e38, np.float32))
+
+
+def _check_heavy(got, want, rounds):
+    fits = np.abs(want) < 3e38
+    assert np.isinf(got[~fits]).all() and np.count_nonzero(~fits) <= 1
+    assert np.all(np.abs(got[fits].astype(np.float64) - want[fits]) <= rounds * 2.0 ** -24 * np.abs(want[fits]))
+
+
+def test_records_beyond_the_limit(gpu_available):
+    """The first round's residuals are the records': a sum of them overflows FP32, not FP64."""
+    import c2g
+    import oracle
+
+    csr, (hv, he, hw) = _heavy_records()
+    with c2g.Graph.create(csr[0], csr[1], flist=csr[2]) as g:
+        g.set_records(hv, he, hw)
+        pr, res, st = g.ppr(0, g.ppr_params(alpha=0.15, rmax=1e-7, seeded=1, max_iter=500))
+        rp, rr, rounds, _ = oracle.ppr_push(*csr, 0, 0.15, 1e-7, seeded=True, seed_v=he, seed_w=hw)
+        assert st.status_flags == 0
+        _check_heavy(pr, rp, rounds)
+        _check_heavy(res, rr, rounds)
