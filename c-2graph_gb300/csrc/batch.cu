@@ -1618,7 +1618,7 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
                 const unsigned q2 = 2u * (unsigned)(lane & (LG - 1));  // this lane's queries q2, q2 + 1
                 for (unsigned i0 = first + (unsigned)(lane / LG); i0 - (unsigned)(lane / LG) < end; i0 += G * U) {
                     float4 v[U];
-                    float wa[U], wb[U];
+                    float w[U];
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const unsigned i = i0 + (unsigned)(u * G);
@@ -1626,14 +1626,16 @@ __device__ __forceinline__ unsigned pbatch_pull(const PprBatchParams& p, int buf
                         const unsigned on = (e.x >> q2) & 3u;
                         v[u] = on ? __ldcg(reinterpret_cast<const float4*>(rqf + (size_t)e.y * 32u + q2))
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-                        // a query at rest adds exact zeros
-                        wa[u] = on & 1u ? __uint_as_float(e.z) : 0.f;
-                        wb[u] = on & 2u ? __uint_as_float(e.z) : 0.f;
+                        // a query at rest adds exact zeros: its pair here may hold anything (an earlier
+                        // query's residual, infinity or NaN), so it is dropped, not weighted with 0
+                        if (!(on & 1u)) v[u].x = v[u].y = 0.f;
+                        if (!(on & 2u)) v[u].z = v[u].w = 0.f;
+                        w[u] = __uint_as_float(e.z);
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u)
-                        pull_pair_add(f2_pack(v[u].x, v[u].z), f2_pack(v[u].y, v[u].w), f2_pack(wa[u], wb[u]),
-                                      f2_pack(-wa[u], -wb[u]), sh2[0], sl2[0]);
+                        pull_pair_add(f2_pack(v[u].x, v[u].z), f2_pack(v[u].y, v[u].w), f2_pack(w[u], w[u]),
+                                      f2_pack(-w[u], -w[u]), sh2[0], sl2[0]);
                 }
                 l = 0u;
             }
