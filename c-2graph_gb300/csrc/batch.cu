@@ -1203,6 +1203,7 @@ __device__ __forceinline__ FrontierOut pbatch_out(const PprBatchParams& p, int b
 constexpr int kPprBatchThreads = 448;
 constexpr int kPprBatchBlocksPerSm = 2;
 constexpr int kPprBatchUnroll = 3;  // push items in flight per lane
+constexpr unsigned long long kPullMaxQBits = (unsigned long long)((kPullMaxQ >> 23) - 127 + 1023) << 52;  // as a double
 
 // Apply of one (vertex, word) to the lanes that received messages: res += m; a lane whose
 // residual exceeds rmax adds alpha * res to pr and activates.  An activated lane with
@@ -1210,7 +1211,11 @@ constexpr int kPprBatchUnroll = 3;  // push items in flight per lane
 // zeroes res; one without out-edges keeps res until the next round pops it.  The word's
 // activated lanes go to the next frontier (and to amask[ob], the pull rounds' lookup),
 // or to the dangling list.  force = true: the seeded first hop (activate every touched
-// lane, no messages).  psum (lane 0) accumulates the next round's pushes.
+// lane, no messages).  psum (lane 0) accumulates the next round's pushes.  WP < 4: a residual too large for the
+// pulls' float pairs makes the next round and those after it push, as in ppr.cu.  Batches of up to 64 queries need
+// that, which pull from few pushes on (ppr_pull_threshold); in the kernel of wider ones, which pull above 8 E
+// pushes as they always have, the test took 1% of a batch (256 queries at scale 21: 372 -> 377 ms).
+template <int WP>
 __device__ __forceinline__ void pbatch_apply_word(const PprBatchParams& p, bool force, int ob, int vw, int dg,
                                                   size_t off, bool mine, double r, double m, float pv,
                                                   unsigned long long rmax_bits, WarpStage& fst, const FrontierOut& out,
@@ -1226,12 +1231,14 @@ __device__ __forceinline__ void pbatch_apply_word(const PprBatchParams& p, bool 
             if (dg > 0) {
                 const double q = (1.0 - (double)p.alpha) * rr;  // (1-alpha)*r_u (src/ppr/purn/Main.cu:288)
                 p.rq[ob][off] = q;
-                if (c2g_split_ok(q)) {  // float pair for pull rounds (fp64_mul.h)
+                if (c2g_split_ok(q) && (WP == 4 || c2g_dbits(q) < kPullMaxQBits)) {  // float pair for pull rounds (fp64_mul.h)
                     const c2g_pair hl = c2g_split_pair(q);
                     p.rqf[ob][off] = make_float2(c2g_bitsf(hl.hi), c2g_bitsf(hl.lo));
                 } else {
                     const float hi = __double2float_rz(q);
                     p.rqf[ob][off] = make_float2(hi, __double2float_rz(q - (double)hi));
+                    // too large for the pairs' sums: the next round and those after it push (ppr.cu)
+                    if (WP < 4 && c2g_dbits(q) >= kPullMaxQBits) atomicMax(&p.ctl->farmin[dctr - p.ctl->dctr], 1);
                 }
                 p.res[off] = 0.0;
             } else {
@@ -1271,6 +1278,7 @@ __device__ __forceinline__ void pbatch_apply_word(const PprBatchParams& p, bool 
 // measured slower: 852 and 870 ms.)
 constexpr int kApplyGroup = 3;  // 4 spills at 64 registers
 
+template <int WP>
 __device__ __forceinline__ unsigned pbatch_sweep(const PprBatchParams& p, bool force, int ob, const unsigned* list,
                                                  unsigned nlist, WarpStage& fst, const FrontierOut& out,
                                                  unsigned* dctr, unsigned long long& psum, unsigned gwarp,
@@ -1326,7 +1334,7 @@ __device__ __forceinline__ unsigned pbatch_sweep(const PprBatchParams& p, bool f
                 const size_t off = ((size_t)(unsigned)vw << 5) + lane;
                 const bool mine = (ln >> lane) & 1u;
                 if (mine && !force) p.msg[off] = 0.0;
-                pbatch_apply_word(p, force, ob, vw, dgu, off, mine, r[u], m[u], pv[u], rmax_bits, fst, out, dctr,
+                pbatch_apply_word<WP>(p, force, ob, vw, dgu, off, mine, r[u], m[u], pv[u], rmax_bits, fst, out, dctr,
                                   psum, lane);
             }
         }
@@ -1415,8 +1423,8 @@ __device__ __forceinline__ unsigned pbatch_pull_owner(const PprBatchParams& p, i
         const size_t off = (size_t)v * (size_t)p.Q + ((w0 + j) << 5) + lane;
         const double m = c2g_float_bits_to_double(__float_as_uint(sh[j])) +
                          c2g_float_bits_to_double(__float_as_uint(sl[j]));
-        pbatch_apply_word(p, false, ob, (int)(((unsigned)v << p.logW) + w0 + j), dg, off, nz, r[j], m, pv[j],
-                          rmax_bits, fst, out, dctr, psum, lane);
+        pbatch_apply_word<WP>(p, false, ob, (int)(((unsigned)v << p.logW) + w0 + j), dg, off, nz, r[j], m, pv[j],
+                              rmax_bits, fst, out, dctr, psum, lane);
     }
     return cnt;
 }
@@ -1816,7 +1824,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
     }
     if (!grid_sync(bar, flags, p.barrier_ns)) return;
     // Round-1 frontier: every touched (vertex, word) activates its touched lanes.
-    pbatch_sweep(p, true, 1, nullptr, 0u, fst, pbatch_out(p, 1, 1), &ctl->dctr[1], psum, gwarp, nwarps, lane);
+    pbatch_sweep<WP>(p, true, 1, nullptr, 0u, fst, pbatch_out(p, 1, 1), &ctl->dctr[1], psum, gwarp, nwarps, lane);
     if (lane == 0 && psum) atomicAdd(&ctl->pcount[1], psum);
     psum = 0;
     if (!grid_sync(bar, flags, p.barrier_ns)) return;
@@ -1836,8 +1844,11 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
         const unsigned F = (unsigned)(c >> 32), T = (unsigned)c;
         const unsigned D = min(ldcg(&ctl->dctr[cur % 3]), p.qcap);
         const unsigned long long P = ldcg(&ctl->pcount[cur % 3]);  // this round's (query, edge) pushes
+        const bool large = WP < 4 && ldcg(&ctl->farmin[cur % 3]) != 0;
+        if (gtid == 0 && large) atomicMax(&ctl->farmin[(cur + 1) % 3], 1);
+        const bool pull = P > p.pull_min && !large;  // grid-uniform
         const int buf = cur & 1, ob = (cur + 1) & 1;
-        if (gtid == 0) trace_round(p.trace, iters, (long long)P, P > p.pull_min ? 1 : 0);
+        if (gtid == 0) trace_round(p.trace, iters, (long long)P, pull ? 1 : 0);
         if (F == 0 && D == 0) break;
         // end of an epoch: the state rests in the arrays for the next one
         if (p.epoch_rounds > 0 && iters >= p.epoch_rounds) break;
@@ -1864,7 +1875,6 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
             if (lane == 0) p.dmask[dv.x] = 0u;
         }
         if (F == 0) break;
-        const bool pull = P > p.pull_min;  // grid-uniform
         // A pull round applies targets while it pulls: the pops above (residuals) and the
         // dangling list they read (which the applies refill) must be done first.
         if (pull && D > 0 && !grid_sync(bar, flags, p.barrier_ns)) return;
@@ -1879,6 +1889,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
             ctl->tilectr[fslot] = 0u;
             ctl->listctr[fslot] = 0u;
             ctl->pcount[fslot] = 0ull;
+            if (WP < 4) ctl->farmin[fslot] = 0;
             ctl->popped += F;
             ctl->relaxed += T;
         }
@@ -2015,7 +2026,7 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
         // listed straddlers (unless the list overflowed); after a push, every touched word.
         const unsigned nl = pull ? ldcg(&ctl->listctr[cur % 3]) : 0u;
         const bool listed = pull && nl <= p.slist_cap;  // grid-uniform
-        touched += pbatch_sweep(p, false, ob, listed ? p.slist : nullptr, nl, fst, pbatch_out(p, ob, nslot),
+        touched += pbatch_sweep<WP>(p, false, ob, listed ? p.slist : nullptr, nl, fst, pbatch_out(p, ob, nslot),
                                 &ctl->dctr[nslot], psum, gwarp, nwarps, lane);
         if (lane == 0 && psum) atomicAdd(&ctl->pcount[nslot], psum);
         psum = 0;
@@ -2186,7 +2197,7 @@ static int ppr_batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
 }
 
 // Largest positive weight of the reverse CSR (its bits: positive floats order as
-// integers).  A non-finite weight makes it non-finite, which disables pull rounds.
+// integers).  From 2^30 on, infinity and NaN included, pull rounds are off.
 __global__ void weight_stats_kernel(const int2* __restrict__ adj_r, long long E, unsigned* wmax_bits) {
     unsigned wm = 0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < E; e += (long long)gridDim.x * blockDim.x) {
@@ -2219,7 +2230,7 @@ int ppr_pull_prepare(c2g_graph* g) {
 }
 
 // Push count above which a round pulls (c2g_ppr_batch_set_pull): pull rounds need the
-// reverse CSR (a view uses its base's, never builds it) and finite weights; with rmax
+// reverse CSR (a view uses its base's, never builds it) and weights below 2^30; with rmax
 // below 1e-30 pushed residuals may leave the FP32 range of the pull's float pairs, so such
 // launches push only.
 //
@@ -2239,9 +2250,7 @@ static int ppr_pull_threshold(c2g_graph* g, const c2g_ppr_params& prm, int nq, u
     if (ratio >= 0.f && g->E > 0 && prm.rmax >= 1e-30f && (g->wstat_valid || !g->borrowed)) {
         int rc;
         if (!g->borrowed && (rc = ppr_pull_prepare(g))) return rc;
-        float wmax;
-        std::memcpy(&wmax, &g->wstat_wmax_bits, sizeof(float));
-        if (std::isfinite(wmax)) *pull_min = (unsigned long long)((double)ratio * (double)g->E);
+        if (g->wstat_wmax_bits < kPullMaxWeight) *pull_min = (unsigned long long)((double)ratio * (double)g->E);
     }
     return C2G_OK;
 }

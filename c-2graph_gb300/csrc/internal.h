@@ -36,7 +36,7 @@ struct TraversalCtl {
     unsigned listctr[3];         // PPR touched-list counters per round slot
     unsigned dctr[3];            // PPR activated vertices without out-edges, per slot
     unsigned farctr[3];          // SSSP far piles (rotating: current, target, free)
-    int farmin[3];  // by slot; single PPR: not 0 when a residual pushed in the slot's round is too large for pulls
+    int farmin[3];  // by slot; PPR: not 0 when a residual pushed in the slot's round is too large for pulls
     unsigned bar_count, bar_pad;  // GridBarrier
     int flags;                    // C2G_FLAG_*
     int iterations;
@@ -125,6 +125,12 @@ struct PprConfig {
 constexpr int kInMaxWeight = 147483648;  // largest weight of in-edge rows: unreachable + weight fits an int32
 
 constexpr int kInHead = 32, kInSegment = 256;  // edges; multiples of 32
+
+// Pulls of the push (ppr.cu, batch.cu) sum messages as float pairs: with weights below 2^30 and pushed residuals
+// up to 2^60 every sum of up to 2^31 messages stays a finite float.  Other weights, and the rounds after a larger
+// residual, push in FP64.
+constexpr unsigned kPullMaxWeight = (127 + 30) << 23;  // float bits
+constexpr int kPullMaxQ = (127 + 60) << 23;
 
 constexpr int kPullTileLog = 8;  // in-edges per pull tile (reverse-CSR markers)
 

@@ -154,13 +154,10 @@ __device__ __forceinline__ void ppr_push(const PprParams& p, int buf, int slot, 
     if (track) list_stage_flush(tst, p.touched, &p.ctl->listctr[slot], (unsigned)p.V, &p.ctl->flags);
 }
 
-// Pulls end when a pushed residual passes 2^60 (float bits): with weights below 2^30 (checked by the host)
-// every sum of up to 2^31 messages then stays a finite float.  The rounds' word for it is ctl->farmin[slot],
-// kept by round slot like the counts: a round reads its own slot's and whoever finds such a residual writes the
+// Pulls end when a pushed residual passes kPullMaxQ.  The rounds' word for it is ctl->farmin[slot], kept by
+// round slot like the counts: a round reads its own slot's and whoever finds such a residual writes the
 // next round's, so nothing that a round reads is written while it runs (a pull round has one barrier, at its
 // end).  A round that finds it set hands it on, so that it stays.
-constexpr int kPullMaxQ = (127 + 60) << 23;
-constexpr unsigned kPullMaxWeight = (127 + 30) << 23;
 
 // The float pair of a pushed residual (fp64_mul.h), and its value.
 __device__ __forceinline__ float2 ppr_pair(double q) {

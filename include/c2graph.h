@@ -277,8 +277,9 @@ int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div);
  * pairs (about 47 bits of relative precision) before they meet the FP64 residual.
  * ratio < 0: push only; 0: pull every round; default 8, and until it is set, in
  * c2g_ppr_batch, half the number of queries where that is less, 1/4 for up to 64 queries on
- * graphs up to 2^20 edges.  Pull rounds need finite weights and rmax >= 1e-30.  Results are
- * the same BSP rounds either way, within summation order. */
+ * graphs up to 2^20 edges.  Pull rounds need weights below 2^30 and rmax >= 1e-30; in
+ * batches of up to 64 queries they end when a pushed residual passes 2^60.  Results are the same BSP rounds either way, within
+ * summation order. */
 int c2g_ppr_batch_set_pull(c2g_graph* g, float ratio);
 
 /* Autotuner of that round shape (no counterpart in the reference): times ratios {push only, 1, 2, 4, 8, 16, 32} on this

@@ -75,3 +75,31 @@ def test_records_beyond_the_limit(gpu_available):
         assert st.status_flags == 0
         _check_heavy(pr, rp, rounds)
         _check_heavy(res, rr, rounds)
+
+
+@pytest.mark.parametrize("n", [1, 3, 40])
+@pytest.mark.parametrize("records", [True, False])
+def test_batches_beyond_the_limit(gpu_available, n, records):
+    """The same in batches, which pull from few pushes on when the library decides; and a path whose weights, not
+    its records, pass the limit: 1e20, 1e20, 1e-30, 1."""
+    import c2g
+    import oracle
+
+    csr, (hv, he, hw) = _heavy_records()
+    if not records:
+        csr = (np.arange(6, dtype=np.int32).clip(0, 4), np.array([1, 2, 3, 4], np.int32),
+               np.array([1e20, 1e20, 1e-30, 1.0], np.float32))
+        he, hw = [], []
+    with c2g.Graph.create(csr[0], csr[1], flist=csr[2]) as g:
+        if records:
+            g.set_records(hv, he, hw)
+        prm = g.ppr_params(alpha=0.15, rmax=1e-7, pr0=0.15, seeded=int(records), max_iter=500)
+        rp, rr, rounds, _ = oracle.ppr_push(*csr, 0, 0.15, 1e-7, seeded=records, seed_v=he, seed_w=hw)
+        for ratio in (None, 0.0):
+            if ratio is not None:
+                g.ppr_batch_pull(ratio)
+            pr, res, st = g.ppr_batch(np.zeros(n, np.int32), prm)
+            assert st.status_flags == 0
+            for q in range(n):
+                _check_heavy(pr[q], rp, rounds)
+                _check_heavy(res[q], rr, rounds)
