@@ -356,7 +356,7 @@ int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* ou
     const int blocks = std::min(g->num_sms * 8, (g->V + 255) / 256);
     RowLists r;
     // a segment is one step of a warp (256 edges) where every round is latency, two where it is throughput
-    r.segment = g->E <= kPullAlwaysPushEdges ? 32 * kLaneEdges : 64 * kLaneEdges;
+    r.segment = g->E <= kShortSegmentEdges ? 32 * kLaneEdges : 64 * kLaneEdges;
     cudaError_t e = cudaMemsetAsync(d, 0, sizeof(ClassCount), g->stream);
     if (e == cudaSuccess) {
         row_classes<false><<<blocks, 256, 0, g->stream>>>(row, other, g->V, r.segment, d, nullptr, nullptr);

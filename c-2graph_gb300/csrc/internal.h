@@ -139,7 +139,7 @@ constexpr int kPullTileLog = 8;  // in-edges per pull tile (reverse-CSR markers)
 // edges, which 32 >> (c - 1) lanes read, kLaneEdges each.
 constexpr int kRowClasses = 7;
 constexpr int kLaneEdges = 8;
-constexpr int64_t kPullAlwaysPushEdges = 4000000;  // single push: graphs up to this size pull every round (ppr.cu)
+constexpr int64_t kShortSegmentEdges = 4000000;  // graphs up to this size have segments of one warp step
 
 struct RowLists {
     int4* rec = nullptr;           // (row, first edge, edges, out-degree of the row's vertex)

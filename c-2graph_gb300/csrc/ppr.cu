@@ -45,7 +45,8 @@ struct PprParams {
     const int2* adj_r;
     RowLists rows;      // its rows by length
     unsigned* arrived;  // class 0: segments of a row summed so far, zero between rounds
-    unsigned pull_min;  // pull when T is larger (~0: never)
+    unsigned pull_min;   // pull when T is larger (~0: never),
+    unsigned pull_next;  // after a pull when it is larger than this
     bool one_step;      // every round pulls, and its row lists are at most one step per warp
     int dense_div;      // dense push round (no touched list) when T * dense_div > E (0: never)
     float* pr;
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
         }
         // grid-uniform; float pairs hold the pushed residuals and their sums below kPullMaxQ
         const bool large = ldcg(&ctl->farmin[slot]) != 0;
-        const bool pull = T > p.pull_min && !large;
+        const bool pull = T > (counted ? p.pull_next : p.pull_min) && !large;
         // Pop the activated vertices without out-edges: their residual is dropped.  A pull does so
         // for every vertex with in-edges.
         if (!counted) {
@@ -873,18 +874,25 @@ static int ppr_alloc(c2g_graph* g) {
 // Out-edges of the frontier above which a round pulls (~0: never).  A pull costs its pass over all
 // in-edges, a push its frontier's out-edges (L2 atomics, 6.6e10 a second) and two barriers: at scale 20
 // (16M edges) a pull takes 94 us, and a query 4.46 ms with pulls above E / 3, 4.49 above E / 2, 4.51
-// above E / 5 and 6.05 with pulls only.  Up to kPullAlwaysPushEdges a pull is about as short as the two
-// barriers and dependent atomics of the emptiest push round (pulls only / both: 1M edges 0.90 / 1.02 ms a
-// query, 3.2M 1.61 / 1.84, 3.9M 1.89 / 1.87), so every round pulls.
+// above E / 5 and 6.05 with pulls only.  On small graphs a pull is about as short as the two
+// barriers and dependent atomics of the emptiest push round: up to kPullAlwaysEdges every round pulls, and up to
+// kPullMostEdges every round but those of a few thousand edges, which are all there is of a local query (large
+// rmax); the last ones of any other pull on up to kPullTailEdges.  us a query, pulls above E / 3, E / 200, always:
+// 1.2M edges (100,000 uniform vertices), rmax 1e-3 102 / 102 / 75, 1e-7 1273 / 1043 / 900; 2.1M (150,000) 90 /
+// 90 / 80, 1358 / 1198 / 1132; 3.7M (scale 18) 110 / 106 / 124, 1770 / 1747 / 1798; 3.9M (299,999) 92 / 93 /
+// 118, 1553 / 1460 / 1518; rmax 0.1 37 / 37 / 34, 32 / 32 / 36, 38 / 38 / 57, 38 / 38 / 58.
 //
 // Pulls sum float pairs, so they need
 // weights below 2^30, a start below 2^60 and rmax of at least 1e-30 (as the batched push's pulls do),
 // and alpha < 1: a residual of 0 pushed at alpha = 1 cannot be told from a vertex outside the
 // frontier.
 constexpr int64_t kPushPullDiv = 3;
+constexpr int64_t kPullAlwaysEdges = 1600000, kPullTailEdges = 2500000, kPullMostEdges = 4000000;
+constexpr int64_t kMostPullDiv = 200;
 
-static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& rows, unsigned* pull_min) {
-    *pull_min = ~0u;
+static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& rows, unsigned* pull_min,
+                        unsigned* pull_next) {
+    *pull_min = *pull_next = ~0u;
     const bool set = g->ppr_cfg.pull_set;
     if (!rows.rec || !(pp.alpha < 1.f) || !(pp.rmax >= 1e-30f) || !(pp.r0 < 1e18f) || (set && g->ppr_cfg.pull_div <= 0))
         return C2G_OK;
@@ -892,10 +900,12 @@ static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& 
     if (!g->borrowed && (rc = ppr_pull_prepare(g))) return rc;
     if (!g->wstat_valid || g->wstat_wmax_bits >= kPullMaxWeight) return C2G_OK;
     if (set) {
-        *pull_min = (unsigned)(g->E / g->ppr_cfg.pull_div);
+        *pull_min = *pull_next = (unsigned)(g->E / g->ppr_cfg.pull_div);
         return C2G_OK;
     }
-    *pull_min = g->E <= kPullAlwaysPushEdges ? 0u : (unsigned)(g->E / kPushPullDiv);
+    const unsigned min = (unsigned)(g->E / (g->E <= kPullMostEdges ? kMostPullDiv : kPushPullDiv));
+    *pull_min = g->E <= kPullAlwaysEdges ? 0u : min;
+    *pull_next = g->E <= kPullTailEdges ? 0u : min;
     return C2G_OK;
 }
 
@@ -917,7 +927,7 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
     p.adj_r = adj_rev;
     p.rows = rows_rev;
     p.arrived = w.arrived;
-    if ((rc = ppr_pull_min(g, pp, rows_rev, &p.pull_min))) return rc;
+    if ((rc = ppr_pull_min(g, pp, rows_rev, &p.pull_min, &p.pull_next))) return rc;
     p.one_step = false;
     p.dense_div = g->ppr_cfg.dense_div;
     p.pr = pr_dev ? pr_dev : w.pr;
