@@ -327,7 +327,7 @@ struct SsspPull {
     unsigned pull_min;   // a round pulls when its frontier has more out-edges (~0: never)
     int always;          // every round pulls: no map, no list
     unsigned* bits[2];   // maps of the frontiers of the rounds of each parity
-    double* long_at;     // long rows: (distance << 32) | first group, beside their queue entry
+    double* long_at;     // long rows: (distance to count from << 32) | first group, beside their queue entry
     int* long_mark;      // tile owners over their groups
     unsigned long_tiles;
 };
@@ -417,8 +417,9 @@ __device__ __forceinline__ int pull_group(const SsspPull& in, const int* dist, i
     return pull_edges(dist, x, y, lim, b);
 }
 
-// Queue of a pull round's long rows: (vertex, exclusive prefix of the groups to read), with
-// the distance and first group in long_at.  It uses the list buffers, idle in a pull round.
+// Queue of a pull round's long rows: (vertex, exclusive prefix of the groups to read), with the first group in
+// long_at beside the distance that the second part may count the vertex from (-1: the first part lowered the
+// distance and has counted it).  It uses the list buffers, idle in a pull round.
 __device__ __forceinline__ FrontierOut pull_long_out(const SsspParams& p, const SsspPull& in, int parity) {
     FrontierOut o;
     o.q = p.q[0];
@@ -433,12 +434,12 @@ __device__ __forceinline__ FrontierOut pull_long_out(const SsspParams& p, const 
     return o;
 }
 
-// What is left of a word's rows after their first group: lanes read on up to kLaneGroups
+// What is left of a word's rows after their first group (b0: the distances before it): lanes read on up to kLaneGroups
 // groups; a row that needs more finds by bisection how many groups can still improve it.  Up to
 // kWarpGroups the warp reads together, all rows' groups in one sequence; longer rows are
 // queued for the whole grid.
-__device__ __forceinline__ int pull_rest(const SsspParams& p, const SsspPull& in, int fmin, unsigned v, int b, int i,
-                                      int e, bool more, int* best, WarpStage& lst, const FrontierOut& lout, int lane) {
+__device__ __forceinline__ int pull_rest(const SsspParams& p, const SsspPull& in, int fmin, unsigned v, int b0, int b,
+                                      int i, int e, bool more, int* best, WarpStage& lst, const FrontierOut& lout, int lane) {
     int last = INT_MIN;
 #pragma unroll 1
     for (int s = 1; s < kLaneGroups; ++s) {
@@ -465,7 +466,9 @@ __device__ __forceinline__ int pull_rest(const SsspParams& p, const SsspPull& in
         }
     }
     const bool queued = n > kWarpGroups;
-    stage_push(lst, lout, queued, (int)v, n, 0.f, __longlong_as_double(((long long)b << 32) | (long long)(unsigned)i));
+    const unsigned from = b < b0 ? ~0u : (unsigned)b;
+    stage_push(lst, lout, queued, (int)v, n, 0.f,
+               __longlong_as_double((long long)(((unsigned long long)from << 32) | (unsigned)i)));
     if (queued) n = 0;
     int incl = n;
 #pragma unroll
@@ -536,8 +539,8 @@ __device__ __forceinline__ void sssp_pull(const SsspParams& p, const SsspPull& i
         for (int u = 0; u < kPullWords; ++u) {
             const bool more = i[u] < e[u] && last[u] < b[u] - fmin;
             if (__any_sync(kFull, more))
-                b[u] = pull_rest(p, in, fmin, ((w0 + u * nwarps) << 5) + (unsigned)lane, b[u], i[u], e[u], more, best,
-                                 lst, lout, lane);
+                b[u] = pull_rest(p, in, fmin, ((w0 + u * nwarps) << 5) + (unsigned)lane, b0[u], b[u], i[u], e[u], more,
+                                 best, lst, lout, lane);
         }
 #pragma unroll
         for (int u = 0; u < kPullWords; ++u) {
@@ -613,7 +616,7 @@ __device__ __forceinline__ void sssp_pull_kept(const SsspParams& p, const SsspPu
         const int last = (y.w >> in.shift) << in.shift;
         const bool more = go && rest.x < rest.y && last < b - fmin;
         stale = more && rest.y - rest.x > 4 * kWarpGroups;
-        if (__any_sync(kFull, more)) b = pull_rest(p, in, fmin, v, b, rest.x, rest.y, more, best, lst, lout, lane);
+        if (__any_sync(kFull, more)) b = pull_rest(p, in, fmin, v, b0, b, rest.x, rest.y, more, best, lst, lout, lane);
         if (b < b0) {
             p.dist[v] = b;
             fnew = min(fnew, b);
@@ -626,8 +629,8 @@ __device__ __forceinline__ void sssp_pull_kept(const SsspParams& p, const SsspPu
 
 // Second part, after a barrier, when rows were queued (a hub row that nothing has reached yet needs
 // all its 100,000 edges: read by its warp alone that took 1.07 ms of a scale-22 query): warps
-// take tiles of their groups, and a row's parts meet in atomicMin.  The part that first lowers the queued distance counts the
-// vertex for the next frontier, unless the first part of the round had.
+// take tiles of their groups, and a row's parts meet in atomicMin.  The part that first lowers the queued distance
+// counts the vertex for the next frontier, unless the first part of the round has (it then queued no distance).
 __device__ __forceinline__ void sssp_pull_long(const SsspParams& p, const SsspPull& in, int fmin, unsigned L,
                                                unsigned G, unsigned* bits_next, int* best, unsigned long long& count,
                                                int& fnew, int lane, unsigned gwarp, unsigned nwarps) {
