@@ -20,13 +20,16 @@
 
 namespace c2g {
 
-#define C2G_CUDA(call)                                                                       \
-    do {                                                                                     \
-        cudaError_t e_ = (call);                                                             \
-        if (e_ != cudaSuccess)                                                               \
-            return ::c2g::fail(e_ == cudaErrorMemoryAllocation ? C2G_ERR_OOM : C2G_ERR_CUDA, \
-                               "%s in %s at line %d", cudaGetErrorString(e_), __FILE__,      \
-                               __LINE__);                                                    \
+// Returns the status of a failed call.  The runtime's own record of it is cleared: the next call's launch checks
+// (cudaGetLastError) would find it there.
+#define C2G_CUDA(call)                                                                           \
+    do {                                                                                         \
+        cudaError_t e_ = (call);                                                                 \
+        if (e_ != cudaSuccess) {                                                                 \
+            cudaGetLastError();                                                                  \
+            return ::c2g::fail(e_ == cudaErrorMemoryAllocation ? C2G_ERR_OOM : C2G_ERR_CUDA,     \
+                               "%s in %s at line %d", cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                        \
     } while (0)
 
 // Control block of one persistent traversal launch; zeroed before every launch.

@@ -1,0 +1,64 @@
+"""Failures on the library's host side, made by a CUDA runtime without a device (fake_cudart.cpp): allocations that
+do not fit and launches that are refused or end with status flags.  Device memory is host memory and kernels do
+nothing, so these tests read status codes, the kernels that were launched and what the caller's arrays hold.
+No GPU."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import PKG, REPO
+
+
+@pytest.fixture(scope="module")
+def fake_lib(built, tmp_path_factory):
+    """The library's objects linked against the fake runtime."""
+    d = str(tmp_path_factory.mktemp("fake"))
+    csrc = os.path.join(PKG, "csrc")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    objs = [os.path.join(PKG, "lib", "obj", f + ".o") for f in os.listdir(csrc) if f.endswith((".cu", ".cpp"))]
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-I", os.path.join(cuda, "include"), "-I", csrc, "-c",
+                    os.path.join(REPO, "tests", "fake_cudart.cpp"), "-o", d + "/fake.o"], check=True)
+    subprocess.run(["g++", "-shared", "-fopenmp", "-Wl,-Bsymbolic", "-o", d + "/libfake.so", d + "/fake.o"] + objs +
+                   ["-lpthread"], check=True)
+    return d + "/libfake.so"
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    import c2g
+
+    monkeypatch.setattr(c2g, "LIB_PATH", fake_lib)
+    monkeypatch.setattr(c2g, "_lib", None)
+    L = c2g.lib()
+    L.fake_budget.argtypes = [ctypes.c_size_t]
+    L.fake_in_use.restype = ctypes.c_size_t
+    L.fake_launched.restype = ctypes.c_char_p
+    L.fake_reset()
+    yield L
+    L.fake_reset()
+
+
+def _graph(V=4096, ef=16, **kw):
+    import c2g
+
+    rng = np.random.default_rng(3)
+    src = np.sort(rng.integers(0, V, V * ef))
+    vl = np.zeros(V + 1, np.int32)
+    np.cumsum(np.bincount(src, minlength=V), out=vl[1:])
+    E = len(src)
+    return c2g.Graph.create(vl, rng.integers(0, V, E).astype(np.int32), wlist=rng.integers(1, 9, E).astype(np.int32),
+                            flist=rng.random(E).astype(np.float32), **kw)
+
+
+def test_a_call_that_does_not_fit_leaves_no_error_behind(fake):
+    import c2g
+
+    with _graph() as g:
+        fake.fake_fail_malloc(2)
+        with pytest.raises(c2g.C2GError) as e:
+            g.ppr(0)
+        assert e.value.code == c2g.ERR_OOM
+        g.ppr(0)  # its launches are checked for errors
