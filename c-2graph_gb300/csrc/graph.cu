@@ -78,22 +78,26 @@ int set_float_weights(c2g_graph* g, const float* w, int on_device) {
     const size_t E = (size_t)g->E;
     if (E == 0) return C2G_OK;
     const int* src = reinterpret_cast<const int*>(w);
-    int* tmp = nullptr;
-    if (!on_device) {
-        C2G_CUDA(cudaMalloc(&tmp, sizeof(int) * E));
-        cudaError_t e = cudaMemcpyAsync(tmp, w, sizeof(int) * E, cudaMemcpyHostToDevice, g->stream);
-        if (e != cudaSuccess) {
-            cudaFree(tmp);
-            C2G_CUDA(e);
-        }
+    // All memory first: a call that does not fit leaves the old weights in both directions.
+    int *tmp = nullptr, *cursor = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (g->adj_r) e = cudaMalloc(&cursor, sizeof(int) * (size_t)g->V);
+    if (e == cudaSuccess && !on_device) e = cudaMalloc(&tmp, sizeof(int) * E);
+    if (e == cudaSuccess && tmp) {
+        e = cudaMemcpyAsync(tmp, w, sizeof(int) * E, cudaMemcpyHostToDevice, g->stream);
         src = tmp;
     }
-    set_weight_bits_kernel<<<g->num_sms * 4, 256, 0, g->stream>>>(g->adj_f, src, (long long)E);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    if (tmp) cudaFree(tmp);
+    int rc = C2G_OK;
+    if (e == cudaSuccess) {
+        set_weight_bits_kernel<<<g->num_sms * 4, 256, 0, g->stream>>>(g->adj_f, src, (long long)E);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+        rc = refresh_reverse_graph(g, cursor);
+    }
+    for (int* p : {tmp, cursor})
+        if (p) cudaFree(p);
     C2G_CUDA(e);
-    return refresh_reverse_graph(g);
+    return rc;
 }
 
 }  // namespace c2g

@@ -395,19 +395,15 @@ int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* ou
     return C2G_OK;
 }
 
-// Scatter the float-weighted out-edges into the reverse CSR's rows (in any order within a row).
-static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd) {
-    int* cursor = nullptr;
+// Scatter the float-weighted out-edges into the reverse CSR's rows (in any order within a row); cursor: V ints.
+static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd, int* cursor) {
     const size_t V = (size_t)g->V;
-    cudaError_t e = cudaMalloc(&cursor, sizeof(int) * (V ? V : 1));
-    if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(cursor, g->row_r, sizeof(int) * V, cudaMemcpyDeviceToDevice, g->stream);
+    cudaError_t e = cudaMemcpyAsync(cursor, g->row_r, sizeof(int) * V, cudaMemcpyDeviceToDevice, g->stream);
     if (e == cudaSuccess && g->E) {
         in_scatter<<<g->num_sms * 8, 256, 0, g->stream>>>(g->row, fwd, g->V, (unsigned)g->E, cursor, g->adj_r);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cudaFree(cursor);
     return e;
 }
 
@@ -421,7 +417,7 @@ int build_reverse_graph(c2g_graph* g) {
     if (!fwd) return fail(C2G_ERR_UNSUPPORTED, "graph has no edge weights");
     const size_t V = (size_t)g->V, E = (size_t)g->E;
     const int scan_blocks = (int)((V + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems));
-    char* tmp = nullptr;  // stats | in-degrees | cursors (unused) | scan block sums
+    char* tmp = nullptr;  // stats | in-degrees | cursors | scan block sums
     C2G_CUDA(cudaMalloc(&tmp, 256 + sizeof(int) * (V * 2 + (size_t)scan_blocks + 1)));
     InStats* st = reinterpret_cast<InStats*>(tmp);
     int* indeg = reinterpret_cast<int*>(tmp + 256);
@@ -439,7 +435,7 @@ int build_reverse_graph(c2g_graph* g) {
     }
     InStats h{};
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
-    if (e == cudaSuccess) e = scatter_reverse(g, fwd);
+    if (e == cudaSuccess) e = scatter_reverse(g, fwd, cursor);
     cudaFree(tmp);
     if (e == cudaSuccess && g->adj_f) {  // the largest positive weight: positive floats order as integers
         g->wstat_wmax_bits = (uint32_t)h.wmax;
@@ -487,11 +483,17 @@ static int build_row_starts(c2g_graph* g) {
     return C2G_OK;
 }
 
-// New float weights: the reverse CSR's rows stay, their edges are written anew.
-int refresh_reverse_graph(c2g_graph* g) {
+// New float weights: the reverse CSR's rows stay, their edges are written anew (cursor: V ints, where there is a
+// reverse CSR).  If that fails it goes, and with it what holds its addresses; the next call that needs it builds it.
+int refresh_reverse_graph(c2g_graph* g, int* cursor) {
     g->wstat_valid = false;
     if (!g->adj_r) return C2G_OK;
-    C2G_CUDA(scatter_reverse(g, g->adj_f));
+    const cudaError_t e = scatter_reverse(g, g->adj_f, cursor);
+    if (e != cudaSuccess) {
+        ads_free(g);
+        reverse_free(g);
+    }
+    C2G_CUDA(e);
     return C2G_OK;
 }
 

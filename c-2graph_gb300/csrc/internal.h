@@ -247,7 +247,7 @@ void batch_free(c2g_graph* g);
 void ppr_batch_free(c2g_graph* g);
 void ads_free(c2g_graph* g);
 int build_reverse_graph(c2g_graph* g);
-int refresh_reverse_graph(c2g_graph* g);
+int refresh_reverse_graph(c2g_graph* g, int* cursor);
 void reverse_free(c2g_graph* g);
 int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* out);
 int build_in_rows(c2g_graph* g);

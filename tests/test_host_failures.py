@@ -62,3 +62,20 @@ def test_a_call_that_does_not_fit_leaves_no_error_behind(fake):
             g.ppr(0)
         assert e.value.code == c2g.ERR_OOM
         g.ppr(0)  # its launches are checked for errors
+
+
+@pytest.mark.parametrize("on_device", [0, 1])
+def test_set_weights_that_do_not_fit_change_nothing(fake, on_device):
+    import c2g
+
+    with _graph() as g:
+        w = np.ones(g.E, np.float32)
+        for n in range(2 - on_device):  # each of the call's allocations
+            fake.fake_reset()
+            fake.fake_fail_malloc(n)
+            held = fake.fake_in_use()
+            assert fake.c2g_graph_set_weights(g._h, c2g._ptr(w), on_device) == c2g.ERR_OOM
+            assert fake.fake_launched() == b"" and fake.fake_in_use() == held
+        fake.fake_reset()
+        g.set_weights(w)
+        assert b"set_weight_bits" in fake.fake_launched() and b"in_scatter" in fake.fake_launched()
