@@ -467,7 +467,8 @@ __device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur
 }
 
 // The frontier list of a round whose frontier a pull counted: its vertices are popped (those without
-// out-edges for good), and the other parity's qf is cleared for the round's apply.
+// out-edges for good), with the FP64 residual that res still holds (qf only says who is in it: its pair is cut),
+// and the other parity's qf is cleared for the round's apply.
 __device__ __forceinline__ void ppr_list(const PprParams& p, int b, const FrontierOut& out, WarpStage& fst) {
     const int lane = threadIdx.x & 31;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -475,18 +476,19 @@ __device__ __forceinline__ void ppr_list(const PprParams& p, int b, const Fronti
     const unsigned V = (unsigned)p.V;
     for (unsigned v0 = gwarp * 32; v0 < V; v0 += nwarps * 32) {
         const unsigned v = v0 + (unsigned)lane;
-        float2 q = make_float2(0.f, 0.f);
+        double r = 0.0;
         int deg = 0;
         if (v < V) {
-            q = ldcg(p.qf[b] + v);
+            const float2 q = ldcg(p.qf[b] + v);
             p.qf[b ^ 1][v] = make_float2(0.f, 0.f);
             if (q.x != 0.f) {
+                r = ldcg(p.res + v);
                 p.res[v] = 0.0;
                 deg = __ldg(p.row + v + 1) - __ldg(p.row + v);
                 if (deg == 0) p.qf[b][v] = make_float2(0.f, 0.f);
             }
         }
-        stage_push(fst, out, deg > 0, (int)v, deg, 0.f, ppr_pair_value(q));
+        stage_push(fst, out, deg > 0, (int)v, deg, 0.f, (1.0 - (double)p.alpha) * r);
     }
     stage_flush(fst, out);
 }
