@@ -334,7 +334,8 @@ class Graph:
     def sssp_batch_pull(self, frac=0.5):
         """Batched SSSP rounds with more than frac * E * Q (query, edge) relaxations pull over
         the in-edges (Q: query slots; a third of that for 64, a tenth for more and after
-        the first pull; frac < 0: expand only; 0: every round)."""
+        the first pull; frac < 0: expand only; 0: every round; 0.3, the library's default: small
+        batches expand only)."""
         _check(lib().c2g_sssp_batch_set_pull(self._h, float(frac)))
 
     def sssp_batch_pull_frac(self):
@@ -406,12 +407,14 @@ class Graph:
     def watchdog(self, barrier_timeout_ms=0, stall_next_sssp=False):
         _check(lib().c2g_graph_set_watchdog(self._h, barrier_timeout_ms, int(bool(stall_next_sssp))))
 
-    def ppr_config(self, pull_div=0, dense_div=16):
+    def ppr_config(self, pull_div=-1, dense_div=16):
+        """Round shapes of the push: see c2g_ppr_set_config (the defaults: the library decides)."""
         _check(lib().c2g_ppr_set_config(self._h, pull_div, dense_div))
 
     def ppr_batch_pull(self, ratio=8.0):
         """Batched rounds with more than ratio * E pushes pull over the reverse CSR
-        (ratio < 0: push only; 0: every round; until set: at most 8, by queries and edges)."""
+        (ratio < 0: push only; 0: every round; 8: the library decides, at most 8, by queries and
+        edges)."""
         _check(lib().c2g_ppr_batch_set_pull(self._h, float(ratio)))
 
     def ppr_batch_autotune(self, sources, params, reps=1, json_path=None):

@@ -469,10 +469,9 @@ int c2g_graph_set_watchdog(c2g_graph* g, int32_t barrier_timeout_ms, int32_t sta
 
 int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div) {
     if (!g) return fail(C2G_ERR_ARG, "graph is NULL");
-    if (pull_div < 0 || dense_div < 0) return fail(C2G_ERR_ARG, "pull_div and dense_div must be >= 0");
+    if (pull_div < -1 || dense_div < 0) return fail(C2G_ERR_ARG, "pull_div must be >= -1 and dense_div >= 0");
     std::lock_guard<std::mutex> lk(g->mu);
     g->ppr_cfg.pull_div = pull_div;
-    g->ppr_cfg.pull_set = true;
     g->ppr_cfg.dense_div = dense_div;
     return C2G_OK;
 }
@@ -482,7 +481,6 @@ int c2g_ppr_batch_set_pull(c2g_graph* g, float ratio) {
     if (ratio != ratio) return fail(C2G_ERR_ARG, "ratio is NaN");
     std::lock_guard<std::mutex> lk(g->mu);
     g->ppr_cfg.batch_pull_ratio = ratio;
-    g->ppr_cfg.batch_ratio_set = true;
     return C2G_OK;
 }
 
@@ -491,7 +489,6 @@ int c2g_sssp_batch_set_pull(c2g_graph* g, float frac) {
     if (frac != frac) return fail(C2G_ERR_ARG, "frac is NaN");
     std::lock_guard<std::mutex> lk(g->mu);
     g->sssp_cfg.batch_pull_frac = frac;
-    g->sssp_cfg.batch_pull_set = true;
     return C2G_OK;
 }
 

@@ -214,7 +214,6 @@ extern "C" int c2g_ppr_batch_autotune(c2g_graph* g, int32_t n, const int32_t* so
     }
     std::vector<float> ref(rows * V), got(rows * V);
     const float saved = g->ppr_cfg.batch_pull_ratio;
-    const bool saved_set = g->ppr_cfg.batch_ratio_set;
     double best_ms = 1e300;
     float best = saved;
     std::string json = "{\"candidates\": [";
@@ -256,7 +255,6 @@ extern "C" int c2g_ppr_batch_autotune(c2g_graph* g, int32_t n, const int32_t* so
     cudaFree(dpr);
     if (rc) {
         c2g_ppr_batch_set_pull(g, saved);
-        g->ppr_cfg.batch_ratio_set = saved_set;
         return rc;
     }
     char tail[128];

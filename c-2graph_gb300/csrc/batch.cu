@@ -930,7 +930,7 @@ static int batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
 // 27.4 / 22.3 / 21.6 / 21.3; scale 19, 64 queries 5.0 / 3.5 / 3.0 / 3.2; 685,230 uniform vertices, 31
 // queries 5.1 / 5.2 / - / 5.8.  Below a million lines the warps with the longest rows outlast the
 // rest of a pull (60,001 vertices, 128 queries 1.33 / 1.69 / 1.75 / 1.98 ms): those batches expand
-// only, unless the caller set a fraction.  After a launch's first pull the distances bound the rows
+// only, unless the caller set another fraction.  After a launch's first pull the distances bound the rows
 // of the next ones, whose passes get shorter (scale 22, 256 queries: 7.8 ms, then 4.0, 2.9, 2.6), so a
 // batch of one or two words goes on pulling down to the wide one's limit: scale 21, 64 queries 9.15 -> 7.95
 // ms, 32 6.60 -> 5.91; for 256 a lower limit is no gain (500,003 uniform vertices 25.0, a third of it 26.6).
@@ -939,7 +939,7 @@ constexpr size_t kPullMinLines = 1000000;
 static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, unsigned long long* next) {
     *first = *next = ~0ull;
     const float frac = g->sssp_cfg.batch_pull_frac;
-    const bool small = !g->sssp_cfg.batch_pull_set && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines;
+    const bool small = frac == kDefaultPullFrac && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines;
     if (!(frac >= 0.f) || small) return;
     const double width = Q <= 32 ? 1.0 : Q <= 64 ? 1.0 / 3.0 : 0.1, all = (double)frac * (double)g->E * (double)Q;
     *first = (unsigned long long)(width * all);
@@ -2234,7 +2234,7 @@ int ppr_pull_prepare(c2g_graph* g) {
 // below 1e-30 pushed residuals may leave the FP32 range of the pull's float pairs, so such
 // launches push only.
 //
-// Until the caller sets a ratio: 8 E, but for a batch of nq queries (0: a resident batch, whose slots say little
+// At the default ratio: 8 E, but for a batch of nq queries (0: a resident batch, whose slots say little
 // about the queries at work) half an E per query for fewer than 16, and E / 4 for up to 64 on
 // graphs up to kSmallPullEdges, where a round is latency and a pull saves the push's atomics and its sweep.  ms a batch
 // at 8 E / this: 5 queries at scale 14 7.39 / 3.95, 2 6.74 / 3.74, 20 4.82 / 4.57, 3 on 3,000 uniform
@@ -2245,7 +2245,7 @@ constexpr int64_t kSmallPullEdges = 1 << 20;
 static int ppr_pull_threshold(c2g_graph* g, const c2g_ppr_params& prm, int nq, unsigned long long* pull_min) {
     *pull_min = ~0ull;
     float ratio = g->ppr_cfg.batch_pull_ratio;
-    if (!g->ppr_cfg.batch_ratio_set && nq > 0)
+    if (ratio == kDefaultPullRatio && nq > 0)
         ratio = nq <= 64 && g->E <= kSmallPullEdges ? 0.25f : std::min(ratio, 0.5f * (float)nq);
     if (ratio >= 0.f && g->E > 0 && prm.rmax >= 1e-30f && (g->wstat_valid || !g->borrowed)) {
         int rc;

@@ -104,6 +104,9 @@ struct PprWork {
     int log_tile = -1;
 };
 
+// The defaults of the batched round shapes, at which the library decides by the batch and the graph.
+constexpr float kDefaultPullFrac = 0.3f, kDefaultPullRatio = 8.0f;
+
 struct SsspConfig {
     int delta = 0;       // <= 0: no near/far split
     int log_tile = 8;    // 256 edges per warp tile
@@ -111,17 +114,16 @@ struct SsspConfig {
     int batch_tile_big_log = 9;  // batched expansion: 512 edge-word steps per big tile
     int batch_tile_min_log = 4;  // ... in rounds with at least 16 big tiles per warp
     // batched rounds with more (query, edge) relaxations than this * E * Q, scaled by the batch's width
-    // (batch.cu), pull over the in-edge rows (< 0: never); until it is set, small batches never pull
-    float batch_pull_frac = 0.3f;
-    bool batch_pull_set = false;
+    // (batch.cu), pull over the in-edge rows (< 0: never); at the default small batches never pull
+    float batch_pull_frac = kDefaultPullFrac;
 };
 
 struct PprConfig {
-    float batch_pull_ratio = 8.0f;  // batched rounds with more than ratio * E pushes pull (< 0: never)
-    bool batch_ratio_set = false;   // the caller's; else ppr_pull_threshold lowers it for few queries
+    // batched rounds with more than ratio * E pushes pull (< 0: never); the default is lowered for few
+    // queries (ppr_pull_threshold)
+    float batch_pull_ratio = kDefaultPullRatio;
     int log_tile = 8;
-    int pull_div = 0;   // pull round when frontier out-edges * pull_div > E; 0 = push only
-    bool pull_set = false;  // until it is set, ppr.cu picks the rule by the graph's size
+    int pull_div = -1;  // pull round when frontier out-edges * pull_div > E; 0: never; -1: by the graph's size (ppr.cu)
     int dense_div = 16;  // dense push round (red.add, apply sweep over V) when out-edges * dense_div > E
 };
 

@@ -895,14 +895,14 @@ constexpr int64_t kMostPullDiv = 200;
 static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& rows, unsigned* pull_min,
                         unsigned* pull_next) {
     *pull_min = *pull_next = ~0u;
-    const bool set = g->ppr_cfg.pull_set;
-    if (!rows.rec || !(pp.alpha < 1.f) || !(pp.rmax >= 1e-30f) || !(pp.r0 < 1e18f) || (set && g->ppr_cfg.pull_div <= 0))
+    const int div = g->ppr_cfg.pull_div;
+    if (!rows.rec || !(pp.alpha < 1.f) || !(pp.rmax >= 1e-30f) || !(pp.r0 < 1e18f) || div == 0)
         return C2G_OK;
     int rc;
     if (!g->borrowed && (rc = ppr_pull_prepare(g))) return rc;
     if (!g->wstat_valid || g->wstat_wmax_bits >= kPullMaxWeight) return C2G_OK;
-    if (set) {
-        *pull_min = *pull_next = (unsigned)(g->E / g->ppr_cfg.pull_div);
+    if (div > 0) {
+        *pull_min = *pull_next = (unsigned)(g->E / div);
         return C2G_OK;
     }
     const unsigned min = (unsigned)(g->E / (g->E <= kPullMostEdges ? kMostPullDiv : kPushPullDiv));
@@ -1004,7 +1004,7 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
 int ppr_launch(c2g_graph* g, int32_t source, const c2g_ppr_params& pp, const int32_t* seed_v,
                const float* seed_w, int32_t n_rec, float* pr_dev, float* res_dev, float* ms) {
     if (!g->adj_f) return fail(C2G_ERR_UNSUPPORTED, "graph has no float weights (flist)");
-    if (g->ppr_cfg.pull_set && g->ppr_cfg.pull_div > 0) {  // asked for: built now if the graph was made without it
+    if (g->ppr_cfg.pull_div > 0) {  // asked for: built now if the graph was made without it
         int rc = build_reverse_graph(g);
         if (rc) return rc;
     }

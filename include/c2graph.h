@@ -221,8 +221,8 @@ int c2g_sssp_batch_get_tile(const c2g_graph* g, int32_t* big_steps, int32_t* min
  * slots, a tenth for more and for every round after a launch's first pull) pulls: each target takes the minimum over its in-edges from
  * sources that improved in the previous round, in ascending order of weight up to the
  * first that cannot improve any query of the word.  frac < 0: expand (push) only; 0: pull
- * every round; default 0.3, and until it is set a batch with fewer than a million (vertex,
- * 32-query word) pairs expands only.  Graphs with a weight below 0 or above 147483648
+ * every round; 0.3, the default: the library decides, as for any fraction but that a batch
+ * with fewer than a million (vertex, 32-query word) pairs expands only.  Graphs with a weight below 0 or above 147483648
  * always expand.  Distances do not depend on the setting. */
 int c2g_sssp_batch_set_pull(c2g_graph* g, float frac);
 int c2g_sssp_batch_get_pull(const c2g_graph* g, float* frac);
@@ -263,7 +263,7 @@ int c2g_ppr_batch(c2g_graph* g, int32_t n, const int32_t* sources, const c2g_ppr
                   float* pr, float* res, int on_device, int layout, c2g_stats* stats);
 
 /* Round shapes of the push kernel.  A round whose frontier has more than E / pull_div
- * out-edges pulls over the reverse CSR instead of pushing (0: never; until it is set, the
+ * out-edges pulls over the reverse CSR instead of pushing (0: never; -1, the default: the
  * library decides by the graph's size).  Pulls need rmax >= 1e-30 and finite weights.  A
  * push round whose frontier has more than E / dense_div out-edges adds its messages
  * without tracking first touches and applies them in one sweep over all vertices
@@ -275,8 +275,8 @@ int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div);
  * than ratio * E (query, edge) pushes pulls over the reverse CSR (built on first use):
  * each target gathers its in-neighbours' pushed residuals and sums the messages as FP32
  * pairs (about 47 bits of relative precision) before they meet the FP64 residual.
- * ratio < 0: push only; 0: pull every round; default 8, and until it is set, in
- * c2g_ppr_batch, half the number of queries where that is less, 1/4 for up to 64 queries on
+ * ratio < 0: push only; 0: pull every round; 8, the default: the library decides, 8 but in
+ * c2g_ppr_batch half the number of queries where that is less, 1/4 for up to 64 queries on
  * graphs up to 2^20 edges.  Pull rounds need weights below 2^30 and rmax >= 1e-30; in
  * batches of up to 64 queries they end when a pushed residual passes 2^60.  Results are the same BSP rounds either way, within
  * summation order. */
