@@ -9,6 +9,9 @@
 // computed by a transposed push: the same BSP push kernel, run on the reverse CSR
 // (in-edges carrying w(u,v)) from the target set, absorbing 1*r instead of alpha*r.
 // The gradient pass reads each forward edge once: 12 bytes per edge + 8 per vertex.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -91,15 +94,13 @@ struct AdjointWork {
     int32_t* tv = nullptr;                // distinct targets,
     float *tr = nullptr, *tpi = nullptr;  // their multiplicities, and pi there
     size_t targets = 0;                   // allocated
-    TraversalCtl* ctl = nullptr;          // the backward push's status, before the gradient pass adds its own
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
 void adjoint_free(c2g_graph* g) {
     AdjointWork* w = reinterpret_cast<AdjointWork*>(g->adjoint);
     if (!w) return;
-    for (void* p : {(void*)w->pi, (void*)w->lam, (void*)w->grad, (void*)w->tv, (void*)w->tr, (void*)w->tpi,
-                    (void*)w->ctl})
+    for (void* p : {(void*)w->pi, (void*)w->lam, (void*)w->grad, (void*)w->tv, (void*)w->tr, (void*)w->tpi})
         if (p) cudaFree(p);
     for (cudaEvent_t ev : {w->ev0, w->ev1})
         if (ev) cudaEventDestroy(ev);
@@ -112,8 +113,7 @@ static int adjoint_alloc(c2g_graph* g, size_t targets, bool host_grad, AdjointWo
     if (!w) g->adjoint = w = new AdjointWork();
     const size_t V = (size_t)g->V, E = (size_t)g->E;
     cudaError_t e = cudaSuccess;
-    if (!w->ctl) e = cudaMalloc(&w->ctl, sizeof(TraversalCtl));
-    if (e == cudaSuccess && !w->ev0) e = cudaEventCreate(&w->ev0);
+    if (!w->ev0) e = cudaEventCreate(&w->ev0);
     if (e == cudaSuccess && !w->ev1) e = cudaEventCreate(&w->ev1);
     if (e == cudaSuccess && !w->pi) e = cudaMalloc(&w->pi, sizeof(float) * V);
     if (e == cudaSuccess && !w->lam) e = cudaMalloc(&w->lam, sizeof(float) * V);
@@ -136,6 +136,18 @@ static int adjoint_alloc(c2g_graph* g, size_t targets, bool host_grad, AdjointWo
 }
 
 int set_float_weights(c2g_graph* g, const float* w, int on_device);
+
+// Maps the pages inside a host array that a copy will fill, without writing to it (where the system cannot, the copy
+// maps them).
+static void map_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = ((uintptr_t)p + page - 1) & ~(page - 1),
+                    b = ((uintptr_t)p + bytes) & ~(page - 1);
+    if (p && a < b) madvise(reinterpret_cast<void*>(a), b - a, MADV_POPULATE_WRITE);
+#else
+    (void)p, (void)bytes;
+#endif
+}
 
 }  // namespace c2g
 
@@ -207,10 +219,19 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
         rc = ppr_launch_view(g, g->row_r, g->adj_r, g->row, g->adj_f, g->rows_out, tv[0], bp, 1.0f, (int32_t)tv.size(),
                              w->tv, w->tr, nullptr, nullptr, 0, lam, nullptr, nullptr);
     if (rc) return rc;
-    // The gradient pass and the copies follow the push at once: a copy to pageable memory that is issued while
-    // the stream is busy makes its pages ready beside the kernels (67 MB: 3 ms when issued after them).
-    e = cudaMemcpyAsync(w->ctl, g->ppr.ctl, sizeof(cb), cudaMemcpyDeviceToDevice, g->stream);
+    // Nothing is written to the caller's arrays before both pushes have ended well; their pages are mapped
+    // meanwhile, beside the backward push (67 MB: 3 ms of a copy to pages that are not).
+    if (!on_device) {
+        map_pages(grad, sizeof(float) * E);
+        map_pages(pi_out, sizeof(float) * V);
+        map_pages(lambda_out, sizeof(float) * V);
+    }
+    e = cudaMemcpyAsync(&cb, g->ppr.ctl, sizeof(cb), cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms_b, g->ev0, g->ev1);
     C2G_CUDA(e);
+    if ((cf.flags | cb.flags) & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS))
+        return fail(C2G_ERR_OVERFLOW, "adjoint push reported device errors (flags %d/%d)", cf.flags, cb.flags);
     // gradient pass
     cudaEventRecord(w->ev0, g->stream);
     if (E)
@@ -236,14 +257,10 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
         e = cudaMemcpyAsync(lambda_out, lam, sizeof(float) * V,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, g->stream);
     int gflags = 0;  // the gradient pass's bounds checks report into the push's control block
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&cb, w->ctl, sizeof(cb), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&gflags, &g->ppr.ctl->flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     C2G_CUDA(e);
-    if ((cf.flags | cb.flags) & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS))
-        return fail(C2G_ERR_OVERFLOW, "adjoint push reported device errors (flags %d/%d)", cf.flags, cb.flags);
-    C2G_CUDA(cudaEventElapsedTime(&ms_b, g->ev0, g->ev1));
     C2G_CUDA(cudaEventElapsedTime(&ms_g, w->ev0, w->ev1));
     if (gflags & C2G_FLAG_BOUNDS) return fail(C2G_ERR_OVERFLOW, "adjoint gradient pass: device index check failed");
     if (loss) {

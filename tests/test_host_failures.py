@@ -79,3 +79,22 @@ def test_set_weights_that_do_not_fit_change_nothing(fake, on_device):
         fake.fake_reset()
         g.set_weights(w)
         assert b"set_weight_bits" in fake.fake_launched() and b"in_scatter" in fake.fake_launched()
+
+
+@pytest.mark.parametrize("push", [0, 1])
+def test_a_failed_adjoint_leaves_the_results_alone(fake, push):
+    """A push that ends with an error (here: its grid barrier gave up) returns it before anything is written."""
+    import c2g
+
+    with _graph() as g:
+        prm = g.ppr_params(alpha=0.15, rmax=1e-7, seeded=0)
+        targets = np.array([5, 7], np.int32)
+        out = [np.full(n, 7.0, np.float32) for n in (g.E, g.V, g.V)]
+        loss = ctypes.c_double(7.0)
+        call = lambda: fake.c2g_ppr_adjoint(  # noqa: E731
+            g._h, 1, ctypes.byref(prm), 2, c2g._ptr(targets), 1e-7, *(c2g._ptr(a) for a in out), ctypes.byref(loss), 0, None)
+        fake.fake_flag_launch(push, c2g.FLAG_BARRIER_TIMEOUT)
+        assert call() == c2g.ERR_OVERFLOW
+        assert all((a == 7.0).all() for a in out) and loss.value == 7.0
+        fake.fake_reset()
+        assert call() == c2g.OK and not any((a == 7.0).any() for a in out)
