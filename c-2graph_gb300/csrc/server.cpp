@@ -126,12 +126,13 @@ struct Parked {
 };
 
 constexpr float kShare = 1.0f / 3.0f;
+constexpr int kWholeRounds = 4;  // rounds of an epoch that has the whole GPU, at most: another kind waits for its end
 
 // The SMs of a kind's next epoch.  A third each is what lets two persistent kernels and the
 // label propagation's run side by side: the blocks of other splits need not fit together, and a
 // grid that waits at its barrier for blocks without room would hold what the other needs.  A kind
-// with no other at work takes the whole GPU, and then an epoch of another waits for its end
-// (11 PPR queries alone on a scale-18 graph: 28.3 ms on a third, 18.7 on all; a wave of 32 mixed
+// with no other at work takes the whole GPU, and then an epoch of another waits for its end, kWholeRounds rounds at
+// most however long the server's epochs are (11 PPR queries alone on a scale-18 graph: 28.3 ms on a third, 18.7 on all; a wave of 32 mixed
 // requests 29.9 -> 27.3 ms, its last third being PPR alone.  Two thirds beside the label
 // propagation gave the wave nothing, 27.1 to 27.9.)
 float epoch_begin(c2g_server* s, int kind) {
@@ -235,8 +236,9 @@ void session_worker(c2g_server* s, int kind) {
         if (running == 0) continue;
         int32_t nf = 0;
         c2g_stats st;
-        session_set_grid_share(ss, epoch_begin(s, kind));
-        int rc = c2g_session_step(ss, rounds, finished.data(), cap, &nf, &st);
+        const float share = epoch_begin(s, kind);
+        session_set_grid_share(ss, share);
+        int rc = c2g_session_step(ss, share < 1.0f ? rounds : std::min(rounds, kWholeRounds), finished.data(), cap, &nf, &st);
         epoch_end(s, kind, rc == C2G_OK && running > nf);
         {
             std::lock_guard<std::mutex> lk(s->mu);

@@ -343,7 +343,8 @@ typedef struct c2g_server_config {
     int32_t ads_iterations;   /* adsorption iterations                                 */
     float   alpha, rmax;      /* PPR parameters (base mode)                            */
     int64_t hbm_budget_bytes; /* admission budget for per-query state, 0 = 80% of free */
-    int32_t epoch_rounds;     /* rounds per epoch of the SSSP / PPR batches (0: 4)     */
+    int32_t epoch_rounds;     /* rounds per epoch of the SSSP / PPR batches (0: 4); at
+                               * most 4 while a kind is alone and has the whole GPU   */
     int32_t preempt_rounds;   /* evict queries past this many rounds when requests wait
                                  and no slot is free (0: never)                         */
 } c2g_server_config;
