@@ -44,15 +44,16 @@ constexpr int kAdsBatch = 2;       // in-edges whose label rows a group gathers 
 constexpr int kAdsMinBlocks = 8;   // launch bounds: resident 128-thread blocks per SM
 constexpr int kAdsThreads = 128;
 constexpr int kAdsWarps = kAdsThreads / 32;
+constexpr unsigned kAdsBareBlocks = 64;  // blocks that write the listed rows without in-edges
 
 struct AdsPass {
     const int* row_r;
     const int2* adj_r;
     const unsigned* r_bits;   // per chunk of 32 in-edges: which start a row,
     const int* r_prefix;      // and how many rows start in earlier chunks
-    const int4* coef;         // per row with in-edges, in order: vertex, p_cont, p_inj, seed mask
+    const int4* coef;         // per row with in-edges, in order: vertex, p_cont, p_inj, seed mask; from the
+    const unsigned* n_bare;   // end, this many rows without in-edges whose labels are not 0 after an iteration
     const float* p_inj;
-    const int* seeds;
     float4* slots;            // per tile: sum of the row that enters it, of the row that leaves it
     unsigned* arrived;        // per tile: tiles of the row leaving it that have left their sums
     int V;
@@ -89,10 +90,10 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
     // groups of a warp, reading 16 bytes of their rows at once, hit different banks
     __shared__ __align__(16) int2 staged[kAdsWarps][2][8][C + 2];
     __shared__ float4 heads[kAdsThreads];
-    if (blockIdx.x == 0 && threadIdx.x < kAdsL) {  // a seed without in-edges keeps its injection alone
-        const int v = __ldg(p.seeds + threadIdx.x);
-        if (__ldg(p.row_r + v) == __ldg(p.row_r + v + 1))
-            reinterpret_cast<float*>(out)[(size_t)v * kAdsL + threadIdx.x] = __ldg(p.p_inj + v);
+    if (blockIdx.x < kAdsBareBlocks) {
+        const unsigned n = 4u * __ldg(p.n_bare), step = min(gridDim.x, kAdsBareBlocks) * kAdsThreads;
+        for (unsigned i = blockIdx.x * kAdsThreads + threadIdx.x; i < n; i += step)
+            ads_apply(out, __ldg(p.coef + (p.V - 1 - (int)(i >> 2))), (int)(i & 3u), make_float4(0.f, 0.f, 0.f, 0.f));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int part = lane & 3, grp = lane >> 2;  // labels 4*part .. 4*part+3 of the group's rows
@@ -266,10 +267,13 @@ __global__ void __launch_bounds__(kAdsThreads, kAdsMinBlocks)
     }
 }
 
-// Y0 = I (seed labels) and its zero row, Y1 = p_inj * I for the rows that no iteration writes,
-// and the coefficients of the rows with in-edges, in their order.
+// Y0 = I (seed labels) and its zero row, Y1 = 0 for the rows that no iteration writes, and the coefficients of the
+// rows with in-edges, in their order.  Of those without, the ones that an iteration leaves with other labels than 0
+// are listed from coef's end: the seeds, which keep their injection alone, and those whose p_cont is not finite (it
+// times an empty sum is NaN).
 __global__ void ads_init(const AdsPass p, const float* __restrict__ p_cont, const unsigned* __restrict__ seedmask,
-                         float4* __restrict__ Y0, float4* __restrict__ Y1, int4* __restrict__ coef) {
+                         float4* __restrict__ Y0, float4* __restrict__ Y1, int4* __restrict__ coef,
+                         unsigned* __restrict__ n_bare) {
     const size_t n = ((size_t)p.V + 1) * (kAdsL / 4);
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -283,19 +287,25 @@ __global__ void ads_init(const AdsPass p, const float* __restrict__ p_cont, cons
         const unsigned mask = seedmask[v], m = mask >> (4 * part);
         Y0[i] = make_float4(m & 1u, (m >> 1) & 1u, (m >> 2) & 1u, (m >> 3) & 1u);
         const int r0 = __ldg(p.row_r + v);
-        if (r0 == __ldg(p.row_r + v + 1)) {
-            ads_apply(Y1, make_int4(v, 0, __float_as_int(p.p_inj[v]), (int)mask), part, zero);
-        } else if (part == 0) {
-            const unsigned before = __ldg(p.r_bits + (r0 >> 5)) & ((1u << (r0 & 31)) - 1u);
-            coef[__ldg(p.r_prefix + (r0 >> 5)) + __popc(before)] =
-                make_int4(v, __float_as_int(p_cont[v]), __float_as_int(p.p_inj[v]), (int)mask);
+        const bool bare = r0 == __ldg(p.row_r + v + 1);
+        if (bare) Y1[i] = zero;
+        if (part == 0) {
+            const float pc = p_cont[v];
+            const int4 c = make_int4(v, __float_as_int(pc), __float_as_int(p.p_inj[v]), (int)mask);
+            if (!bare) {
+                const unsigned before = __ldg(p.r_bits + (r0 >> 5)) & ((1u << (r0 & 31)) - 1u);
+                coef[__ldg(p.r_prefix + (r0 >> 5)) + __popc(before)] = c;
+            } else if (mask != 0u || !isfinite(pc)) {
+                coef[p.V - 1 - (int)atomicAdd(n_bare, 1u)] = c;
+            }
         }
     }
 }
 
 // Seed mask from the 16 seed vertices: bit l of mask[v] says label l is seeded at v.
-__global__ void ads_seed_mask(const int* __restrict__ seeds, int n, unsigned* __restrict__ mask) {
+__global__ void ads_seed_mask(const int* __restrict__ seeds, int n, unsigned* __restrict__ mask, unsigned* n_bare) {
     const int l = threadIdx.x;
+    if (l == 0) *n_bare = 0u;
     if (l < n) atomicOr(mask + seeds[l], 1u << l);
 }
 
@@ -311,7 +321,7 @@ struct AdsWork {
     unsigned* mask = nullptr;
     float* pi = nullptr;
     float* pc = nullptr;
-    int* seeds = nullptr;  // [16]
+    int* seeds = nullptr;  // [16], and the number of listed rows without in-edges behind them
     cudaGraphExec_t exec = nullptr;
     int iterations = -1;
     int tile_log = 0;
@@ -359,7 +369,7 @@ static int ads_alloc(c2g_graph* g, AdsWork** out) {
         if (e == cudaSuccess) e = cudaMalloc(&w->mask, sizeof(unsigned) * V);
         if (e == cudaSuccess) e = cudaMalloc(&w->pi, sizeof(float) * V);
         if (e == cudaSuccess) e = cudaMalloc(&w->pc, sizeof(float) * V);
-        if (e == cudaSuccess) e = cudaMalloc(&w->seeds, sizeof(int) * kAdsL);
+        if (e == cudaSuccess) e = cudaMalloc(&w->seeds, sizeof(int) * (kAdsL + 1));
         if (e != cudaSuccess) ads_free(g);
         C2G_CUDA(e);
     }
@@ -374,7 +384,8 @@ static int ads_capture(c2g_graph* g, AdsWork* w, int iterations) {
         cudaGraphExecDestroy(w->exec);
         w->exec = nullptr;
     }
-    const AdsPass p{g->row_r, g->adj_r, g->r_bits, g->r_prefix, w->coef, w->pi, w->seeds, w->slots, w->arrived,
+    unsigned* const n_bare = reinterpret_cast<unsigned*>(w->seeds) + kAdsL;
+    const AdsPass p{g->row_r, g->adj_r, g->r_bits, g->r_prefix, w->coef, n_bare, w->pi, w->slots, w->arrived,
                     g->V,     (unsigned)g->E, w->tile_log};
     const unsigned tile_edges = kAdsWarps << w->tile_log;
     const int blocks = (int)(((size_t)g->E + tile_edges - 1) / tile_edges);
@@ -382,8 +393,8 @@ static int ads_capture(c2g_graph* g, AdsWork* w, int iterations) {
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        ads_init<<<g->num_sms * 8, 256, 0, g->stream>>>(p, w->pc, w->mask, Y[0], Y[1], w->coef);
-        for (int it = 0; it < iterations; ++it)  // without in-edges one block writes the seeds' rows
+        ads_init<<<g->num_sms * 8, 256, 0, g->stream>>>(p, w->pc, w->mask, Y[0], Y[1], w->coef, n_bare);
+        for (int it = 0; it < iterations; ++it)  // without in-edges one block writes the listed rows
             (w->tile_log < 8 ? ads_iterate<8> : ads_iterate<32>)<<<blocks ? blocks : 1, kAdsThreads, 0, g->stream>>>(p, Y[it & 1], Y[(it + 1) & 1]);
         e = cudaStreamEndCapture(g->stream, &graph);
     }
@@ -431,7 +442,7 @@ extern "C" int c2g_adsorption(c2g_graph* g, int32_t n_labels, const int32_t* see
     if (e == cudaSuccess) e = cudaMemcpyAsync(w->pc, p_cont, sizeof(float) * V, in_kind, g->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(w->mask, 0, sizeof(unsigned) * V, g->stream);
     if (e == cudaSuccess) {
-        ads_seed_mask<<<1, 32, 0, g->stream>>>(w->seeds, kAdsL, w->mask);
+        ads_seed_mask<<<1, 32, 0, g->stream>>>(w->seeds, kAdsL, w->mask, reinterpret_cast<unsigned*>(w->seeds) + kAdsL);
         e = cudaGetLastError();
     }
     C2G_CUDA(e);
