@@ -191,11 +191,14 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
             if (prev >= 0) cudaSetDevice(prev);
         }
     } scope(g->device);
-    int rc = build_reverse_graph(g);
-    if (rc || (rc = build_row_lists(g, g->row, g->row_r, &g->rows_out))) return rc;
     const size_t V = (size_t)g->V, E = (size_t)g->E;
     AdjointWork* w = nullptr;
-    if ((rc = adjoint_alloc(g, tv.size(), !on_device, &w))) return rc;
+    int rc = with_room_of_rows(g, [&] {
+        int r = build_reverse_graph(g);
+        if (!r) r = build_row_lists(g, g->row, g->row_r, &g->rows_out);
+        return r ? r : adjoint_alloc(g, tv.size(), !on_device, &w);
+    });
+    if (rc) return rc;
     float *const pi = w->pi, *const lam = w->lam, *const dgrad = on_device ? grad : w->grad;
     float ms_f = 0.f, ms_b = 0.f, ms_g = 0.f;
     TraversalCtl cf, cb;
@@ -207,8 +210,10 @@ extern "C" int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_param
     c2g_ppr_params fp = *params;
     fp.r0 = 1.0f;
     fp.pr0 = fp.alpha;
-    rc = ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->rows_in, source, fp, fp.alpha, 0, nullptr,
-                         nullptr, nullptr, nullptr, 0, pi, nullptr, &ms_f);
+    rc = with_room_of_rows(g, [&] {
+        return ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->rows_in, source, fp, fp.alpha, 0, nullptr,
+                               nullptr, nullptr, nullptr, 0, pi, nullptr, &ms_f);
+    });
     if (!rc && (cudaMemcpyAsync(&cf, g->ppr.ctl, sizeof(cf), cudaMemcpyDeviceToHost, g->stream) != cudaSuccess ||
                 cudaStreamSynchronize(g->stream) != cudaSuccess))
         rc = fail(C2G_ERR_CUDA, "adjoint: reading the forward push status failed");

@@ -430,10 +430,12 @@ extern "C" int c2g_adsorption(c2g_graph* g, int32_t n_labels, const int32_t* see
             if (d >= 0) cudaSetDevice(d);
         }
     } restore{prev};
-    int rc = build_reverse_graph(g);
-    if (rc) return rc;
     AdsWork* w = nullptr;
-    if ((rc = ads_alloc(g, &w))) return rc;
+    int rc = with_room_of_rows(g, [&] {
+        const int r = build_reverse_graph(g);
+        return r ? r : ads_alloc(g, &w);
+    });
+    if (rc) return rc;
     const size_t V = (size_t)g->V;
     const cudaMemcpyKind in_kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     float ms = 0.f;

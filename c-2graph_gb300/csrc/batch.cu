@@ -954,6 +954,8 @@ static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchP
     p.pull_min = ~0ull;
     unsigned long long pull_min, pull_next;
     sssp_pull_min(g, Q, &pull_min, &pull_next);
+    int rc;
+    if (pull_min != ~0ull && (rc = ensure_in_rows(g))) return rc;
     if (pull_min == ~0ull || !g->in_adj || (seeds && g->hw_negative)) return C2G_OK;
     p.in_row = g->in_row;
     p.in_adj = g->in_adj;

@@ -7,8 +7,8 @@
 // a reader can stop at the first group whose weights cannot improve v any more.  The
 // reference has no in-edges; it relaxes out-edges only (src/sssp/purn/Main.cu:236-331).
 //
-// They are built when the graph is made (its int32 weights never change): count the in-edges,
-// scan the padded row lengths, scatter the edges into their rows, order each row.
+// They are built when the graph is made, or by its first SSSP call where it has both kinds of weights (int32 weights
+// never change): count the in-edges, scan the padded row lengths, scatter the edges into their rows, order each row.
 // Rows of up to 32 edges are ordered by a warp (bitonic network on weight and source), longer
 // ones by a block (counting sort over kInBuckets buckets of weight).  A bucket spans 2^shift
 // weights, where 2^shift * kInBuckets covers the largest weight; inside a bucket the order is
@@ -410,7 +410,7 @@ static cudaError_t scatter_reverse(c2g_graph* g, const int2* fwd, int* cursor) {
 static int build_row_starts(c2g_graph* g);
 
 // Reverse CSR of the float-weighted graph (in-edges carrying w(u,v)), its rows by length and by
-// chunk, the forward CSR's tile owners; built when the graph is made (one with int32 weights only: on first use).
+// chunk, the forward CSR's tile owners; built when the graph is made, where it has float weights only, else on first use.
 int build_reverse_graph(c2g_graph* g) {
     if (g->adj_r) return C2G_OK;
     const int2* fwd = g->adj_f ? g->adj_f : g->adj_w;  // float weights when the graph has them
@@ -510,6 +510,33 @@ void reverse_free(c2g_graph* g) {
     g->row_r = nullptr;
     g->adj_r = nullptr;
     g->mark_f = nullptr;
+}
+
+int ensure_reverse(c2g_graph* g) {
+    if (g->borrowed || g->reverse_tried || g->adj_r) return C2G_OK;
+    g->reverse_tried = true;
+    const int rc = build_reverse_graph(g);
+    return rc == C2G_ERR_OOM ? C2G_OK : rc;
+}
+
+int ensure_in_rows(c2g_graph* g) {
+    if (g->borrowed || g->in_rows_tried || g->in_adj) return C2G_OK;
+    g->in_rows_tried = true;
+    return build_in_rows(g);
+}
+
+// Free them where no view shares them; false: there was nothing to free.
+bool in_rows_drop(c2g_graph* g) {
+    if (g->borrowed || !g->in_adj || *g->views > 0) return false;
+    in_rows_free(g);
+    return true;
+}
+
+bool reverse_drop(c2g_graph* g) {
+    if (g->borrowed || !g->adj_r || *g->views > 0) return false;
+    ads_free(g);  // its captured launches hold the addresses
+    reverse_free(g);
+    return true;
 }
 
 void in_rows_free(c2g_graph* g) {

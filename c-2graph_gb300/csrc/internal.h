@@ -11,7 +11,9 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -186,6 +188,8 @@ struct c2g_graph {
     unsigned* r_bits = nullptr;
     int32_t* r_prefix = nullptr;
     int32_t* r_rows = nullptr;
+    bool in_rows_tried = false, reverse_tried = false;  // built, or found not to fit: no call tries again by itself
+    std::shared_ptr<std::atomic<int>> views = std::make_shared<std::atomic<int>>(0);  // handles that share the arrays
     c2g::RowLists rows_in;      // rows of row_r by length
     c2g::RowLists rows_out;     // rows of row by length (the adjoint's push on the reverse graph), on demand
     // pruned records
@@ -254,6 +258,25 @@ void reverse_free(c2g_graph* g);
 int build_row_lists(c2g_graph* g, const int* row, const int* other, RowLists* out);
 int build_in_rows(c2g_graph* g);
 void in_rows_free(c2g_graph* g);
+// The in-edges of a kind of call, built by the first one where the graph was made without them.  Those that do not fit
+// are no error: the calls push.
+int ensure_in_rows(c2g_graph* g);
+int ensure_reverse(c2g_graph* g);
+bool in_rows_drop(c2g_graph* g);
+bool reverse_drop(c2g_graph* g);
+
+// A call whose workspace does not fit beside the in-edges runs without those that it can do without: the rows that
+// only SSSP reads, and the reverse CSR.
+template <typename F>
+int with_room_of_rows(c2g_graph* g, F call) {
+    const int rc = call();
+    return rc == C2G_ERR_OOM && in_rows_drop(g) ? call() : rc;
+}
+template <typename F>
+int with_room(c2g_graph* g, F call) {
+    const int rc = with_room_of_rows(g, call);
+    return rc == C2G_ERR_OOM && reverse_drop(g) ? call() : rc;
+}
 // Reverse CSR and the weight statistics of the batched pull rounds (once per weights).
 int ppr_pull_prepare(c2g_graph* g);
 int ppr_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const c2g_ppr_params& prm,

@@ -848,7 +848,7 @@ static int ppr_alloc(c2g_graph* g) {
     PprWork& w = g->ppr;
     const int log_tile = g->ppr_cfg.log_tile;
     if (w.msg && w.log_tile == log_tile) return C2G_OK;
-    if (w.msg) ppr_free(g);
+    if (w.pr) ppr_free(g);
     const size_t nv = g->V ? (size_t)g->V : 1;
     const unsigned mark_cap = (unsigned)(((size_t)g->E >> log_tile) + 2);
     C2G_CUDA(cudaMalloc(&w.pr, sizeof(float) * nv));
@@ -1004,10 +1004,9 @@ int ppr_launch_view(c2g_graph* g, const int32_t* row, const int2* adj, const int
 int ppr_launch(c2g_graph* g, int32_t source, const c2g_ppr_params& pp, const int32_t* seed_v,
                const float* seed_w, int32_t n_rec, float* pr_dev, float* res_dev, float* ms) {
     if (!g->adj_f) return fail(C2G_ERR_UNSUPPORTED, "graph has no float weights (flist)");
-    if (g->ppr_cfg.pull_div > 0) {  // asked for: built now if the graph was made without it
-        int rc = build_reverse_graph(g);
-        if (rc) return rc;
-    }
+    int rc = C2G_OK;
+    if (g->ppr_cfg.pull_div != 0) rc = g->ppr_cfg.pull_div > 0 ? build_reverse_graph(g) : ensure_reverse(g);
+    if (rc) return rc;
     return ppr_launch_view(g, g->row, g->adj_f, g->row_r, g->adj_r, g->rows_in, source, pp, pp.alpha, 0, nullptr,
                            nullptr, seed_v, seed_w, n_rec, pr_dev, res_dev, ms);
 }

@@ -321,10 +321,11 @@ int c2g_server_create(c2g_graph* g, const float* p_inj, const float* p_cont, con
     {
         std::lock_guard<std::mutex> lk(g->mu);
         if (g->adj_f) rc = ppr_pull_prepare(g);
-    }
-    for (int k = 0; k < 3 && !rc; ++k) {
-        rc = graph_view(g, &s->views[k]);
-        if (!rc) s->views[k]->grid_scale = kShare;
+        if (!rc && g->adj_w && g->sssp_cfg.batch_pull_frac >= 0.f) rc = ensure_in_rows(g);
+        for (int k = 0; k < 3 && !rc; ++k) {
+            rc = graph_view(g, &s->views[k]);
+            if (!rc) s->views[k]->grid_scale = kShare;
+        }
     }
     // Per-query device state (bytes) and the admission budget.  Per (vertex, query): SSSP
     // distance 4 B plus 28 B per 32 queries (mask, two frontier entries and masks, two pull

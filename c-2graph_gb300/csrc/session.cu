@@ -342,16 +342,19 @@ int c2g_session_create(c2g_graph* g, int kind, int32_t slots, const c2g_ppr_para
         ++s->logW;
     }
     int rc = C2G_OK;
-    if (kind == C2G_REQ_PPR && g->adj_f && g->ppr_cfg.batch_pull_ratio >= 0.f && !g->borrowed) {
-        // pull rounds read the base graph's reverse CSR; the view takes it as it is now
+    {
+        // pull rounds read the base graph's in-edges; the view takes them as they are now
         std::lock_guard<std::mutex> lk(g->mu);
         int prev = -1;
         cudaGetDevice(&prev);
         cudaSetDevice(g->device);
-        rc = ppr_pull_prepare(g);
+        if (kind == C2G_REQ_SSSP && g->sssp_cfg.batch_pull_frac >= 0.f)
+            rc = ensure_in_rows(g);
+        else if (kind == C2G_REQ_PPR && g->adj_f && g->ppr_cfg.batch_pull_ratio >= 0.f && !g->borrowed)
+            rc = ppr_pull_prepare(g);
+        if (!rc) rc = graph_view(g, &s->g);
         if (prev >= 0) cudaSetDevice(prev);
     }
-    if (!rc) rc = graph_view(g, &s->g);
     if (!rc) {
         std::lock_guard<std::mutex> lk(s->g->mu);
         int prev = -1;

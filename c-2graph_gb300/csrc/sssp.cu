@@ -883,10 +883,18 @@ void sssp_free(c2g_graph* g) {
     w = SsspWork();
 }
 
+static int pull_mark_alloc(c2g_graph* g) {
+    C2G_CUDA(cudaMalloc(&g->sssp.pull_mark, sizeof(int) * ((size_t)(g->in_edges >> (kPullTile + 2)) + 2)));
+    return C2G_OK;
+}
+
 static int sssp_alloc(c2g_graph* g) {
     SsspWork& w = g->sssp;
     const int log_tile = g->sssp_cfg.log_tile;
-    if (w.dist && w.log_tile == log_tile) return C2G_OK;
+    if (w.dist && w.log_tile == log_tile) {
+        if (g->in_adj && !w.pull_mark) return pull_mark_alloc(g);
+        return C2G_OK;
+    }
     if (w.dist) sssp_free(g);
     const size_t V = (size_t)g->V;
     const size_t nv = V ? V : 1;
@@ -900,7 +908,8 @@ static int sssp_alloc(c2g_graph* g) {
     }
     C2G_CUDA(cudaMalloc(&w.far, sizeof(int) * nv * 3));
     C2G_CUDA(cudaMalloc(&w.bits, sizeof(unsigned) * 2 * ((nv + 31) / 32)));
-    if (g->in_adj) C2G_CUDA(cudaMalloc(&w.pull_mark, sizeof(int) * ((size_t)(g->in_edges >> (kPullTile + 2)) + 2)));
+    int rc;
+    if (g->in_adj && (rc = pull_mark_alloc(g))) return rc;
     C2G_CUDA(cudaMalloc(&w.ctl, sizeof(TraversalCtl)));
     C2G_CUDA(cudaMalloc(&w.st, sizeof(StampState)));
     C2G_CUDA(cudaMemsetAsync(w.stamp, 0xff, sizeof(int) * nv, g->stream));
@@ -948,6 +957,7 @@ int sssp_launch(c2g_graph* g, int32_t source, const int32_t* seed_v, const int32
                 int32_t* dist_dev, float* ms) {
     int rc;
     if ((rc = sssp_geometry(g))) return rc;
+    if (g->sssp_cfg.delta == 0 && (rc = ensure_in_rows(g))) return rc;
     if ((rc = sssp_alloc(g))) return rc;
     if (!g->adj_w) return fail(C2G_ERR_UNSUPPORTED, "graph has no int32 weights (wlist)");
     SsspWork& w = g->sssp;

@@ -41,7 +41,7 @@ def fake(fake_lib, monkeypatch):
     L.fake_reset()
 
 
-def _graph(V=4096, ef=16, **kw):
+def _graph(V=4096, ef=16, kinds="wf"):
     import c2g
 
     rng = np.random.default_rng(3)
@@ -49,14 +49,16 @@ def _graph(V=4096, ef=16, **kw):
     vl = np.zeros(V + 1, np.int32)
     np.cumsum(np.bincount(src, minlength=V), out=vl[1:])
     E = len(src)
-    return c2g.Graph.create(vl, rng.integers(0, V, E).astype(np.int32), wlist=rng.integers(1, 9, E).astype(np.int32),
-                            flist=rng.random(E).astype(np.float32), **kw)
+    return c2g.Graph.create(vl, rng.integers(0, V, E).astype(np.int32),
+                            wlist=rng.integers(1, 9, E).astype(np.int32) if "w" in kinds else None,
+                            flist=rng.random(E).astype(np.float32) if "f" in kinds else None)
 
 
 def test_a_call_that_does_not_fit_leaves_no_error_behind(fake):
     import c2g
 
     with _graph() as g:
+        g.ppr_config(pull_div=0)  # no in-edges, which the call could do without
         fake.fake_fail_malloc(2)
         with pytest.raises(c2g.C2GError) as e:
             g.ppr(0)
@@ -68,7 +70,7 @@ def test_a_call_that_does_not_fit_leaves_no_error_behind(fake):
 def test_set_weights_that_do_not_fit_change_nothing(fake, on_device):
     import c2g
 
-    with _graph() as g:
+    with _graph(kinds="f") as g:
         w = np.ones(g.E, np.float32)
         for n in range(2 - on_device):  # each of the call's allocations
             fake.fake_reset()
@@ -98,3 +100,54 @@ def test_a_failed_adjoint_leaves_the_results_alone(fake, push):
         assert all((a == 7.0).all() for a in out) and loss.value == 7.0
         fake.fake_reset()
         assert call() == c2g.OK and not any((a == 7.0).any() for a in out)
+
+
+def test_each_kind_of_call_builds_its_own_in_edges(fake):
+    """A graph with both kinds of weights is made without in-edges; one with a single kind with that kind's."""
+    with _graph() as g:
+        assert b"in_count" not in fake.fake_launched()
+        for call, rows, lists in ((lambda: g.sssp(0), 1, 0), (lambda: g.ppr(0), 1, 1), (lambda: g.sssp(1), 1, 1),
+                                  (lambda: g.ppr(1), 1, 1)):
+            call()
+            log = fake.fake_launched()
+            assert log.count(b"in_sort_short") == rows and (b"row_classes" in log) == bool(lists)
+    fake.fake_reset()
+    with _graph(kinds="w") as g:
+        assert b"in_sort_short" in fake.fake_launched() and b"row_classes" not in fake.fake_launched()
+    fake.fake_reset()
+    with _graph(kinds="f") as g:
+        assert b"in_sort_short" not in fake.fake_launched() and b"row_classes" in fake.fake_launched()
+
+
+_SOURCES = np.arange(3, dtype=np.int32)
+_CALLS = {"sssp": ("w", lambda g: g.sssp(0)), "sssp_batch": ("w", lambda g: g.sssp_batch(_SOURCES)),
+          "ppr": ("f", lambda g: g.ppr(0)), "ppr after sssp": ("wf", lambda g: (g.sssp(0), g.ppr(0))),
+          "ppr_batch after sssp": ("wf", lambda g: (g.sssp(0), g.ppr_batch(_SOURCES))),
+          "adsorption after sssp": ("wf", lambda g: (g.sssp(0), g.adsorption(np.arange(16), *np.ones((3, g.V), np.float32)))),
+          "adjoint after sssp": ("wf", lambda g: (g.sssp(0), g.ppr_adjoint(0, _SOURCES)))}
+
+
+@pytest.mark.parametrize("name", sorted(_CALLS))
+def test_workspaces_that_fit_only_without_in_edges(fake, name):
+    """In-edges that leave too little room for a call's workspace go, where no session shares them."""
+    import c2g
+
+    kinds, call = _CALLS[name]
+    before = fake.fake_in_use()
+    with _graph(kinds=kinds) as g:
+        call(g)
+        held = fake.fake_in_use()
+    assert fake.fake_in_use() == before
+    with _graph(kinds=kinds) as g:
+        fake.fake_budget(held - 1000)
+        call(g)
+        assert fake.fake_in_use() <= held - 1000
+        call(g)
+    assert fake.fake_in_use() == before
+    if name == "sssp_batch":  # a session's view keeps them
+        fake.fake_reset()
+        with _graph(kinds=kinds) as g, c2g.Session(g, c2g.REQ_SSSP, 32):
+            fake.fake_budget(fake.fake_in_use() + 1000)
+            with pytest.raises(c2g.C2GError) as e:
+                call(g)
+            assert e.value.code == c2g.ERR_OOM
