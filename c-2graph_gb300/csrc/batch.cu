@@ -37,7 +37,8 @@ struct BatchParams {
     int V;
     int logW;  // words per vertex = 1 << logW
     int Q;     // padded query count = 32 << logW
-    int nq;    // real queries
+    int nq;    // real queries (a resident batch: slots up to the last running one)
+    unsigned live[32];  // of those, by query word: the queries (slots) at work
     int* dist;          // [V][Q]
     unsigned* mask;     // [V][W] next-round masks
     int2* q[2];         // entries (v*W + w, edge base)
@@ -68,6 +69,7 @@ struct BatchParams {
     int in_shift;
     unsigned long long pull_min;
     unsigned long long pull_next;  // the same, once a round of the launch has pulled (batches of one or two words)
+    unsigned pull_groups;          // groups of WP query words with queries
     unsigned* amask[2];
     int* qmin;  // [3][Q]
 };
@@ -341,7 +343,7 @@ __device__ __forceinline__ void sbatch_pull(const BatchParams& p, int buf, int s
     constexpr int RP = 4 / WP;  // rows at a time
     const unsigned Qu = (unsigned)p.Q;
     const unsigned nblk = ((unsigned)p.V + 15u) / 16u, per_group = nblk + (p.in_segs + 3u) / 4u;
-    const unsigned nitems = per_group << (WP == 4 ? p.logW - 2 : 0);
+    const unsigned nitems = WP == 4 ? per_group * p.pull_groups : per_group;
     const unsigned* am = p.amask[buf];
     unsigned w0 = ~0u;  // the word group of qm and qnew
     int qm[WP], qnew[WP];
@@ -566,8 +568,9 @@ __global__ void __launch_bounds__(kSsspBatchThreads, kSsspBatchBlocksPerSm) sssp
                         reinterpret_cast<int2*>(sm.x0[wib]), rmk[wib]};
     const bool may_pull = p.pull_min != ~0ull, low = may_pull && p.Q <= kQminCap;
     if (may_pull && gtid < Qu) {
-        // round 1: no distance is below 0 (seeds and weights are not negative)
-        p.qmin[Qu + gtid] = 0;
+        // round 1: no distance is below 0 (seeds and weights are not negative); a slot without a query at work
+        // bounds no row in any round (its distances may be anything)
+        p.qmin[Qu + gtid] = !low || ((p.live[gtid >> 5] >> (gtid & 31u)) & 1u) ? 0 : INT_MAX;
         p.qmin[gtid] = p.qmin[2 * Qu + gtid] = low ? INT_MAX : 0;
     }
     if (low)
@@ -847,10 +850,11 @@ static int grid_blocks(const c2g_graph* g, int per_sm) {
     return b < 1 ? 1 : b;
 }
 
-static const void* sssp_batch_kernel(int logW) {
-    return logW == 0 ? (const void*)sssp_batch_persistent<1>
-         : logW == 1 ? (const void*)sssp_batch_persistent<2>
-                     : (const void*)sssp_batch_persistent<4>;
+// The kernel for queries in the first nq slots: pulls take as many words at a time as hold queries.
+static const void* sssp_batch_kernel(int nq) {
+    return nq <= 32 ? (const void*)sssp_batch_persistent<1>
+         : nq <= 64 ? (const void*)sssp_batch_persistent<2>
+                    : (const void*)sssp_batch_persistent<4>;
 }
 
 struct BatchWork {
@@ -936,6 +940,9 @@ static int batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
 // ms, 32 6.60 -> 5.91; for 256 a lower limit is no gain (500,003 uniform vertices 25.0, a third of it 26.6).
 constexpr size_t kPullMinLines = 1000000;
 
+// A resident batch goes by the words up to its last running slot, not by its slots (Q here): with all slots' pull
+// limits and words 11 queries in 256 slots pulled 8 words of which one was at work (scale 18: 0.92 ms with expansion
+// only, 1.46 so).
 static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, unsigned long long* next) {
     *first = *next = ~0ull;
     const float frac = g->sssp_cfg.batch_pull_frac;
@@ -949,11 +956,13 @@ static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, 
 // The pull rounds of a batched SSSP launch (p.pull_min: (query, edge) relaxations of the
 // frontier above which a round pulls, ~0: never): they need the graph's in-edge rows, and
 // seeds that are not below zero (the frontier minima start at 0).  The pull
-// lookups start clear; a launch leaves the entries of its last rounds behind.
-static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchParams& p) {
+// lookups start clear; a launch leaves the entries of its last rounds behind.  Qrule: the queries the limits go by;
+// queries: those at work, which all together cannot pass the limit when they are few: such a launch keeps no lookup.
+static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, int Qrule, int queries, bool seeds, BatchParams& p) {
     p.pull_min = ~0ull;
     unsigned long long pull_min, pull_next;
-    sssp_pull_min(g, Q, &pull_min, &pull_next);
+    sssp_pull_min(g, Qrule, &pull_min, &pull_next);
+    if ((unsigned long long)queries * (unsigned long long)g->E <= pull_min) pull_min = ~0ull;
     int rc;
     if (pull_min != ~0ull && (rc = ensure_in_rows(g))) return rc;
     if (pull_min == ~0ull || !g->in_adj || (seeds && g->hw_negative)) return C2G_OK;
@@ -967,6 +976,8 @@ static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, bool seeds, BatchP
         C2G_CUDA(cudaMemsetAsync(w->amask[b], 0, sizeof(unsigned) * (size_t)g->V * (size_t)(Q / 32), g->stream));
     p.pull_min = pull_min;
     p.pull_next = pull_next;
+    const unsigned words = ((unsigned)p.nq + 31u) / 32u;
+    p.pull_groups = words <= 2u ? 1u : (words + 3u) / 4u;
     return C2G_OK;
 }
 
@@ -978,6 +989,7 @@ static void sssp_batch_params(c2g_graph* g, BatchWork* w, int Q, int logW, Batch
     p.logW = logW;
     p.Q = Q;
     p.nq = Q;
+    for (unsigned& live : p.live) live = ~0u;
     p.dist = w->dist;
     p.mask = w->mask;
     for (int b = 0; b < 2; ++b) {
@@ -1005,6 +1017,7 @@ static void sssp_batch_params(c2g_graph* g, BatchWork* w, int Q, int logW, Batch
     p.in_seg = nullptr;
     p.in_segs = 0u;
     p.in_shift = 0;
+    p.pull_groups = 0u;
     p.qmin = nullptr;
     p.pull_min = ~0ull;
     p.amask[0] = w->amask[0];
@@ -1055,7 +1068,7 @@ int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const st
     int coop = 0, per_sm = 0;
     C2G_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device));
     if (!coop) return fail(C2G_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(logW), kSsspBatchThreads, 0));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(nq), kSsspBatchThreads, 0));
     if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
 
     C2G_CUDA(cudaMemcpyAsync(w->src, sources, sizeof(int) * (size_t)nq, cudaMemcpyHostToDevice, g->stream));
@@ -1069,15 +1082,15 @@ int sssp_batch_launch(c2g_graph* g, int32_t nq, const int32_t* sources, const st
     }
     BatchParams p;
     sssp_batch_params(g, w, Q, logW, p);
-    if ((rc = sssp_pull_setup(g, w, Q, seed_off != nullptr, p))) return rc;
     p.nq = nq;
+    if ((rc = sssp_pull_setup(g, w, Q, Q, nq, seed_off != nullptr, p))) return rc;
     p.seed_off = seed_off ? w->seed_off : nullptr;
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
     const int blocks = grid_blocks(g, per_sm);
-    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(logW), dim3(blocks), dim3(kSsspBatchThreads),
+    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(nq), dim3(blocks), dim3(kSsspBatchThreads),
                                          args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     return sssp_batch_results(g, w, Q, nq, out, out_on_device, query_major, ms, counters, ctl_out);
@@ -1099,24 +1112,27 @@ int sssp_batch_reserve(c2g_graph* g, int Q, int** dist, unsigned** mask) {
     return C2G_OK;
 }
 
-int sssp_batch_epoch(c2g_graph* g, int Q, int rounds, float* ms, long long* counters, TraversalCtl* ctl_out) {
+int sssp_batch_epoch(c2g_graph* g, int Q, int used, int running, const unsigned* live, int rounds, float* ms,
+                     long long* counters, TraversalCtl* ctl_out) {
     BatchWork* w = reinterpret_cast<BatchWork*>(g->batch);
     if (!w || w->Q < Q) return fail(C2G_ERR_ARG, "resident SSSP batch has no workspace");
     int logW = 0;
     while ((32 << logW) < Q) ++logW;
     int per_sm = 0;
-    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(logW), kSsspBatchThreads, 0));
+    C2G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_batch_kernel(used), kSsspBatchThreads, 0));
     if (per_sm < 1) return fail(C2G_ERR_CUDA, "batch kernel cannot be resident");
     BatchParams p;
     sssp_batch_params(g, w, Q, logW, p);
     int rc;
-    if ((rc = sssp_pull_setup(g, w, Q, false, p))) return rc;
+    p.nq = used;
+    std::memcpy(p.live, live, sizeof(p.live));
+    if ((rc = sssp_pull_setup(g, w, Q, std::max(32, (used + 31) / 32 * 32), running, false, p))) return rc;
     p.epoch_rounds = rounds < 1 ? 1 : rounds;
     C2G_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(TraversalCtl), g->stream));
     C2G_CUDA(cudaMemsetAsync(w->counters, 0, sizeof(long long) * 2, g->stream));
     void* args[] = {&p};
     C2G_CUDA(cudaEventRecord(g->ev0, g->stream));
-    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(logW), dim3(grid_blocks(g, per_sm)),
+    C2G_CUDA(cudaLaunchCooperativeKernel(sssp_batch_kernel(used), dim3(grid_blocks(g, per_sm)),
                                          dim3(kSsspBatchThreads), args, 0, g->stream));
     C2G_CUDA(cudaEventRecord(g->ev1, g->stream));
     C2G_CUDA(cudaMemcpyAsync(ctl_out, w->ctl, sizeof(TraversalCtl), cudaMemcpyDeviceToHost, g->stream));

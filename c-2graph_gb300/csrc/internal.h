@@ -295,7 +295,9 @@ struct PprBatchArrays {
 };
 void session_set_grid_share(c2g_session* s, float share);
 int sssp_batch_reserve(c2g_graph* g, int Q, int** dist, unsigned** mask);
-int sssp_batch_epoch(c2g_graph* g, int Q, int rounds, float* ms, long long* counters, TraversalCtl* ctl_out);
+// live: the running slots, a bit each; used: slots up to the last of them
+int sssp_batch_epoch(c2g_graph* g, int Q, int used, int running, const unsigned* live, int rounds, float* ms,
+                     long long* counters, TraversalCtl* ctl_out);
 int ppr_batch_reserve(c2g_graph* g, int Q, PprBatchArrays* a);
 int ppr_batch_epoch(c2g_graph* g, int Q, int used, const c2g_ppr_params& prm, int cur0, int rounds, float* ms,
                     long long* counters, TraversalCtl* ctl_out);

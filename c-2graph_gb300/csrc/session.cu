@@ -419,11 +419,13 @@ int c2g_session_step(c2g_session* s, int32_t rounds, int32_t* finished, int32_t 
     int rc;
     if ((rc = apply_pending(s))) return rc;
     int running = 0, used = 0;  // used: slots up to the last running one
+    unsigned live[32] = {};     // running slots
     int room = rounds;
     for (int i = 0; i < s->Q; ++i)
         if (s->state[i] == kRunning) {
             ++running;
             used = i + 1;
+            live[i >> 5] |= 1u << (i & 31);
             if (s->kind == C2G_REQ_PPR) room = std::min(room, s->prm.max_iter - s->rounds[i]);
         }
     int iters = 0;
@@ -431,7 +433,7 @@ int c2g_session_step(c2g_session* s, int32_t rounds, int32_t* finished, int32_t 
         float ms = 0.f;
         long long counters[2] = {0, 0};
         TraversalCtl ctl;
-        rc = s->kind == C2G_REQ_SSSP ? sssp_batch_epoch(g, s->Q, room, &ms, counters, &ctl)
+        rc = s->kind == C2G_REQ_SSSP ? sssp_batch_epoch(g, s->Q, used, running, live, room, &ms, counters, &ctl)
                                      : ppr_batch_epoch(g, s->Q, used, s->prm, s->cur, room, &ms, counters, &ctl);
         if (rc) return rc;
         if (ctl.flags & (C2G_FLAG_BARRIER_TIMEOUT | C2G_FLAG_QUEUE_OVERFLOW | C2G_FLAG_BOUNDS))
