@@ -2118,11 +2118,15 @@ static int ppr_batch_kernel(int nq, const void** kernel, unsigned* groups, int* 
 
 // log2 of the chunks of 32 in-edges per pull item: 8 chunks (a fourth of the rows then crosses an item
 // boundary), fewer where that leaves the grid's warps less than 16 items each to level the round's
-// end (40 queries at scale 16, 6 chunks per warp: 8-chunk items 14.8 ms a batch, 2 12.8, 1 11.7).
+// end (40 queries at scale 16, 6 chunks per warp: 8-chunk items 14.8 ms a batch, 2 12.8, 1 11.7).  What
+// is uneven is the chunks of a skewed graph: 32 rows of one in-edge, each an apply, or part of one hub's.  Where no row
+// has more than 256 in-edges (no segments) 3 items per warp are enough, and shorter items would only cut rows: 4M
+// edges on 100,000 uniform vertices, 70 queries 14.0 ms a batch with 1 chunk per item, 9.6 with 4 or 8, 250 queries
+// 41.8 / 23.4 / 21.6; 2M on 250,000, 130 queries 30.8 / 26.7 / 26.9.
 static int ppr_pull_log(const c2g_graph* g, unsigned groups, int blocks) {
     const size_t chunks = ((size_t)g->E + 31) / 32, warps = (size_t)blocks * (kPprBatchThreads / 32);
     int k = 3;
-    while (k > 0 && (chunks >> k) * groups < 16 * warps) --k;
+    while (k > 0 && (chunks >> k) * groups < (g->rows_in.n[0] ? 16 : 3) * warps) --k;
     return k;
 }
 
