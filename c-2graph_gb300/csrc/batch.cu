@@ -1221,6 +1221,7 @@ __device__ __forceinline__ FrontierOut pbatch_out(const PprBatchParams& p, int b
 constexpr int kPprBatchThreads = 448;
 constexpr int kPprBatchBlocksPerSm = 2;
 constexpr int kPprBatchUnroll = 3;  // push items in flight per lane
+constexpr unsigned long long kPullsEnd = 1ull << 63;  // beside a round's push count: a residual too large for pulls
 constexpr unsigned long long kPullMaxQBits = (unsigned long long)((kPullMaxQ >> 23) - 127 + 1023) << 52;  // as a double
 
 // Apply of one (vertex, word) to the lanes that received messages: res += m; a lane whose
@@ -1256,7 +1257,7 @@ __device__ __forceinline__ void pbatch_apply_word(const PprBatchParams& p, bool 
                     const float hi = __double2float_rz(q);
                     p.rqf[ob][off] = make_float2(hi, __double2float_rz(q - (double)hi));
                     // too large for the pairs' sums: the next round and those after it push (ppr.cu)
-                    if (WP < 4 && c2g_dbits(q) >= kPullMaxQBits) atomicMax(&p.ctl->farmin[dctr - p.ctl->dctr], 1);
+                    if (WP < 4 && c2g_dbits(q) >= kPullMaxQBits) atomicOr(&p.ctl->pcount[dctr - p.ctl->dctr], kPullsEnd);
                 }
                 p.res[off] = 0.0;
             } else {
@@ -1861,9 +1862,10 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
         const unsigned long long c = ldcg(&ctl->qctr[cur % 3]);
         const unsigned F = (unsigned)(c >> 32), T = (unsigned)c;
         const unsigned D = min(ldcg(&ctl->dctr[cur % 3]), p.qcap);
-        const unsigned long long P = ldcg(&ctl->pcount[cur % 3]);  // this round's (query, edge) pushes
-        const bool large = WP < 4 && ldcg(&ctl->farmin[cur % 3]) != 0;
-        if (gtid == 0 && large) atomicMax(&ctl->farmin[(cur + 1) % 3], 1);
+        const unsigned long long pc = ldcg(&ctl->pcount[cur % 3]);
+        const unsigned long long P = pc & ~kPullsEnd;  // this round's (query, edge) pushes
+        const bool large = WP < 4 && pc != P;
+        if (gtid == 0 && large) atomicOr(&ctl->pcount[(cur + 1) % 3], kPullsEnd);
         const bool pull = P > p.pull_min && !large;  // grid-uniform
         const int buf = cur & 1, ob = (cur + 1) & 1;
         if (gtid == 0) trace_round(p.trace, iters, (long long)P, pull ? 1 : 0);
@@ -1907,7 +1909,6 @@ __global__ void __launch_bounds__(kPprBatchThreads, kPprBatchBlocksPerSm)
             ctl->tilectr[fslot] = 0u;
             ctl->listctr[fslot] = 0u;
             ctl->pcount[fslot] = 0ull;
-            if (WP < 4) ctl->farmin[fslot] = 0;
             ctl->popped += F;
             ctl->relaxed += T;
         }
