@@ -241,6 +241,7 @@ int graph_view(c2g_graph* base, c2g_graph** out) {
     g->in_edges = base->in_edges;
     g->in_seg = base->in_seg;
     g->in_segs = base->in_segs;
+    g->in_hubs = base->in_hubs;
     g->in_shift = base->in_shift;
     g->R = base->R;
     g->H = base->H;

@@ -932,21 +932,31 @@ static int batch_alloc(c2g_graph* g, int Q, size_t n_seeds) {
 // relaxations, and a wide batch amortises the pass: measured (push only / 0.3 / 0.1 / 0.03 of
 // E * Q): scale 22, 256 queries 137 / 60.3 / 53.2 / 44.3 ms; 500,003 uniform vertices, 256 queries
 // 27.4 / 22.3 / 21.6 / 21.3; scale 19, 64 queries 5.0 / 3.5 / 3.0 / 3.2; 685,230 uniform vertices, 31
-// queries 5.1 / 5.2 / - / 5.8.  Below a million lines the warps with the longest rows outlast the
-// rest of a pull (60,001 vertices, 128 queries 1.33 / 1.69 / 1.75 / 1.98 ms): those batches expand
-// only, unless the caller set another fraction.  After a launch's first pull the distances bound the rows
+// queries 5.1 / 5.2 / - / 5.8.  After a launch's first pull the distances bound the rows
 // of the next ones, whose passes get shorter (scale 22, 256 queries: 7.8 ms, then 4.0, 2.9, 2.6), so a
 // batch of one or two words goes on pulling down to the wide one's limit: scale 21, 64 queries 9.15 -> 7.95
 // ms, 32 6.60 -> 5.91; for 256 a lower limit is no gain (500,003 uniform vertices 25.0, a third of it 26.6).
+//
+// At the default fraction two kinds of batches expand only.  (1) Small ones, where the warps with the longest rows
+// outlast the rest of a pull: fewer than kPullMinLines lines, unless the queries together relax so much in a full
+// round that the push is the longer one all the same (expand only / pull: 65,536 vertices of scale 16, 250 queries, 239 M
+// relaxations 2.21 / 2.29 ms; 100,000 uniform vertices, 130 of degree 15, 195 M 3.26 / 3.60, 250, 375 M 5.58 / 4.74, 250 of degree
+// 40, 1.0 G 10.0 / 5.5; 60,000 of degree 60, 70, 252 M 2.51 / 2.70, 250, 900 M 7.35 / 3.92; two words, 60 queries, 210 -
+// 225 M: scale 18 1.94 / 1.60, 250,000 uniform 3.81 / 3.23, 30,000 1.59 / 1.39).  (2) One word on a graph without hubs,
+// whose rounds never get dense enough (in_hubs; 1M uniform vertices, 12 / 31 queries 5.5 / 7.0, 7.2 / 8.0; 2M 11.4 /
+// 14.5, 16.4 / 17.8; 4M 18.4 / 19.1, 24.4 / 26.3).
 constexpr size_t kPullMinLines = 1000000;
+constexpr unsigned long long kPullMinReach2 = 200000000ull, kPullMinReach4 = 300000000ull;  // of 2 and of more words
 
 // A resident batch goes by the words up to its last running slot, not by its slots (Q here): with all slots' pull
 // limits and words 11 queries in 256 slots pulled 8 words of which one was at work (scale 18: 0.92 ms with expansion
 // only, 1.46 so).
-static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, unsigned long long* next) {
+static void sssp_pull_min(const c2g_graph* g, int Q, int queries, unsigned long long* first, unsigned long long* next) {
     *first = *next = ~0ull;
     const float frac = g->sssp_cfg.batch_pull_frac;
-    const bool small = frac == kDefaultPullFrac && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines;
+    const unsigned long long reach = (unsigned long long)queries * (unsigned long long)g->E;
+    const bool small = frac == kDefaultPullFrac && (size_t)g->V * (size_t)(Q / 32) < kPullMinLines &&
+                       (Q <= 32 || reach < (Q <= 64 ? kPullMinReach2 : kPullMinReach4));
     if (!(frac >= 0.f) || small) return;
     const double width = Q <= 32 ? 1.0 : Q <= 64 ? 1.0 / 3.0 : 0.1, all = (double)frac * (double)g->E * (double)Q;
     *first = (unsigned long long)(width * all);
@@ -961,11 +971,12 @@ static void sssp_pull_min(const c2g_graph* g, int Q, unsigned long long* first, 
 static int sssp_pull_setup(c2g_graph* g, BatchWork* w, int Q, int Qrule, int queries, bool seeds, BatchParams& p) {
     p.pull_min = ~0ull;
     unsigned long long pull_min, pull_next;
-    sssp_pull_min(g, Qrule, &pull_min, &pull_next);
+    sssp_pull_min(g, Qrule, queries, &pull_min, &pull_next);
     if ((unsigned long long)queries * (unsigned long long)g->E <= pull_min) pull_min = ~0ull;
     int rc;
     if (pull_min != ~0ull && (rc = ensure_in_rows(g))) return rc;
     if (pull_min == ~0ull || !g->in_adj || (seeds && g->hw_negative)) return C2G_OK;
+    if (Qrule <= 32 && !g->in_hubs && g->sssp_cfg.batch_pull_frac == kDefaultPullFrac) return C2G_OK;
     p.in_row = g->in_row;
     p.in_adj = g->in_adj;
     p.in_seg = g->in_seg;

@@ -34,6 +34,7 @@ struct InStats {
     int wmin, wmax;
     unsigned n_long;             // rows longer than a warp
     unsigned n_seg;              // segments of rows longer than kInHead
+    unsigned n_hub;              // rows of more than 256 edges
     unsigned long long padded;   // padded edges of all rows
 };
 
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(kScanThreads) in_scan_rows(const int* __restri
     for (int k = 0; k < kScanItems; ++k) {
         const int v = base + k;
         const bool lng = pad && v < V && d[k] > 32;
+        if (lng && d[k] > 256) atomicAdd(&st->n_hub, 1u);
         if (lng && padded4(d[k]) > kInHead)
             atomicAdd(&st->n_seg, (unsigned)(padded4(d[k]) - kInHead + kInSegment - 1) / kInSegment);
         if (v < V) {
@@ -545,6 +547,7 @@ void in_rows_free(c2g_graph* g) {
     g->in_row = nullptr;
     g->in_seg = nullptr;
     g->in_segs = 0;
+    g->in_hubs = false;
     g->in_adj = nullptr;
 }
 
@@ -567,7 +570,7 @@ int build_in_rows(c2g_graph* g) {
     InStats* st = reinterpret_cast<InStats*>(tmp);
     int* indeg = reinterpret_cast<int*>(tmp + 256);
     int *cursor = indeg + V, *longs = cursor + V, *sums = longs + V;
-    InStats h{INT_MAX, INT_MIN, 0u, 0u, 0ull};
+    InStats h{INT_MAX, INT_MIN, 0u, 0u, 0u, 0ull};
     const int blocks = g->num_sms * 8;
     e = cudaMemsetAsync(indeg, 0, sizeof(int) * V, g->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, g->stream);
@@ -612,6 +615,7 @@ int build_in_rows(c2g_graph* g) {
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
         g->in_segs = h.n_seg;
+        g->in_hubs = h.n_hub > 0u;
         g->in_shift = shift;
         g->in_edges = (int64_t)h.padded;
     }

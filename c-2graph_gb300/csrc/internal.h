@@ -181,6 +181,7 @@ struct c2g_graph {
     int64_t in_edges = 0;       // padded edges
     int2* in_seg = nullptr;     // (vertex, first edge): rows behind their first kInHead edges, kInSegment edges each
     unsigned in_segs = 0;
+    bool in_hubs = false;       // some row has more than 256 edges
     int in_shift = 0;           // weights are ordered up to their low in_shift bits
     int32_t* mark_f = nullptr;  // pull-tile owner markers over row (the adjoint's gradient pass)
     // the reverse CSR's row starts by chunk of 32 in-edges (batched push, label propagation): start

@@ -221,8 +221,8 @@ int c2g_sssp_batch_get_tile(const c2g_graph* g, int32_t* big_steps, int32_t* min
  * slots, a tenth for more and for every round after a launch's first pull) pulls: each target takes the minimum over its in-edges from
  * sources that improved in the previous round, in ascending order of weight up to the
  * first that cannot improve any query of the word.  frac < 0: expand (push) only; 0: pull
- * every round; 0.3, the default: the library decides, as for any fraction but that a batch
- * with fewer than a million (vertex, 32-query word) pairs expands only.  Graphs with a weight below 0 or above 147483648
+ * every round; 0.3, the default: the library decides, as for any fraction but that small
+ * batches and those of one word on graphs without hubs expand only.  Graphs with a weight below 0 or above 147483648
  * always expand.  Distances do not depend on the setting. */
 int c2g_sssp_batch_set_pull(c2g_graph* g, float frac);
 int c2g_sssp_batch_get_pull(const c2g_graph* g, float* frac);
