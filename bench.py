@@ -376,7 +376,8 @@ def run_ours(args, rank, world, local_rank):
             "metric": METRIC, "value": value, "unit": "queries/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_dev / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "int32 (SSSP); PPR: f64 residual state (res, msg, pushed residual), f32 weights and pr",
+            "dtype": "int32 (SSSP); PPR: f64 residual state (res, msg, pushed residual), message sums of pull rounds "
+                     "as f32 pairs (47 bits), f32 weights and pr",
             "data": "synthetic R-MAT (seeded); no public dataset",
             "config": dict(step_config(args, V, int(so["vlist"][-1]), int(po["vlist"][-1]), nS, nP, world),
                            path="batched, one persistent launch per kind", ppr_pull_ratio=pull_ratio,
@@ -398,7 +399,9 @@ def run_ours(args, rank, world, local_rank):
                 "batched_vs_per_query": value / per_query_qps,
                 "per_query_qps": per_query_qps,
                 "per_query_sssp_ms": ms_sssp_pq, "per_query_ppr_ms": ms_ppr_pq,
-                # single-query relaxation against the HBM roofline (algorithmic bytes / time)
+                # single-query relaxation: algorithmic bytes over time, beside the HBM peak.  The bytes model the
+                # push (frontier out-edges); pull rounds read less, so these are no DRAM rates (nor are the
+                # batched relaxations and GB/s below)
                 "per_query_sssp_alg_gbs": pq_sb / (pq_s / 1000.0) / 1e9 if pq_s else None,
                 "per_query_sssp_roofline_frac": pq_sb / (pq_s / 1000.0) / 1e9 / peak if pq_s else None,
                 "per_query_ppr_alg_gbs": pq_pb / (pq_p / 1000.0) / 1e9 if pq_p else None,

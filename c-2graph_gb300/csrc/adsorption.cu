@@ -23,7 +23,7 @@
 // take 0.55 ms an iteration at scale 22, 7.6 TB/s into the SMs (a third of the rows from
 // DRAM).  Before, a group found each row's end in the row pointer (a dependent load per
 // row), wrote sums to memory for a vertex pass, and an iteration took 1.40 ms.  30 iterations
-// at scale 22: 16.6 ms with 2 rows ahead and 8 blocks per SM; 17.0 with 7; 18.0 with 4 rows
+// at scale 22: 16.1 ms with 2 rows ahead and 8 blocks per SM (16.6 while it spilled, as the others did); 17.0 with 7; 18.0 with 4 rows
 // ahead and 8 blocks, 17.8 with 6, 21.5 with 8 rows and 4 blocks: more warps, each with fewer
 // rows in registers.  What bounds a small one is the chain of loads through a stretch.
 // Per iteration: (8 + 64) bytes per edge (in-edge record + source label row) and
@@ -466,7 +466,7 @@ extern "C" int c2g_adsorption(c2g_graph* g, int32_t n_labels, const int32_t* see
         stats->vertices_popped = (int64_t)g->V * iterations;
         stats->n_seeds = n_labels;
         stats->device_ms = ms;
-        stats->alg_bytes = ((8.0 + 64.0) * (double)g->E + (64.0 + 64.0 + 12.0) * (double)g->V) * iterations;
+        stats->alg_bytes = ((8.0 + 64.0) * (double)g->E + (64.0 + 16.0) * (double)g->V) * iterations;
     }
     return C2G_OK;
 }

@@ -71,10 +71,12 @@ typedef struct c2g_stats {
     int32_t source;          /* source actually traversed                              */
     int32_t iterations;      /* frontier rounds executed (reference iteration_num)     */
     int64_t vertices_popped; /* sum over rounds of frontier vertices expanded          */
-    int64_t edges_relaxed;   /* sum over rounds of frontier out-edges relaxed/pushed   */
+    int64_t edges_relaxed;   /* sum over rounds of frontier out-edges (times queries), whether
+                              * the round pushed them or pulled and skipped some       */
     int64_t touched;         /* PPR: sum over rounds of vertices that got a message    */
     int64_t n_seeds;         /* seed entries applied before the first round            */
-    double  alg_bytes;       /* algorithmic bytes of the call (byte model per path)    */
+    double  alg_bytes;       /* algorithmic bytes of the call: a model of the push per path,
+                              * not traffic (pull rounds read less)                    */
     float   device_ms;       /* device time of the traversal launch (CUDA events)      */
     int32_t status_flags;    /* C2G_FLAG_* bits, 0 when clean                          */
     int32_t reserved;
@@ -272,7 +274,8 @@ int c2g_ppr_set_config(c2g_graph* g, int32_t pull_div, int32_t dense_div);
 
 /* Round shapes of the batched push (c2g_ppr_batch; no counterpart in the reference, which
  * runs one query per launch).  A round whose frontier makes more
- * than ratio * E (query, edge) pushes pulls over the reverse CSR (built on first use):
+ * than ratio * E (query, edge) pushes pulls over the reverse CSR (built with a graph that has
+ * float weights only, else on first use):
  * each target gathers its in-neighbours' pushed residuals and sums the messages as FP32
  * pairs (about 47 bits of relative precision) before they meet the FP64 residual.
  * ratio < 0: push only; 0: pull every round; 8, the default: the library decides, 8 but in
