@@ -79,7 +79,7 @@ extern "C" int c2g_sssp_autotune(c2g_graph* g, int32_t n, const int32_t* sources
 // Autotuner of the batched SSSP's expansion tiles (c2g_sssp_batch_set_tile) and round
 // shape (c2g_sssp_batch_set_pull): the size of the big tiles and the per-warp tile count
 // above which a round walks them, then, at the chosen tiles, the relaxation share above
-// which a round pulls over the reverse CSR.  Big tiles cut the tile-queue traffic and the
+// which a round pulls over the in-edges in weight order.  Big tiles cut the tile-queue traffic and the
 // owner lookups of long rounds; small ones balance the short rounds; pull rounds pay in
 // the rounds where most queries of most active words are active.  Which settings are best
 // depends on the batch (queries, graph, weights), so c2g_sssp_batch_autotune times each

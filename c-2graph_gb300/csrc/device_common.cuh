@@ -44,7 +44,6 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-// L2-coherent loads (bypass L1): for arrays written by other CTAs in the same launch.
 // Copies from global to shared memory that hold no registers; a wait leaves the newest N groups running.
 __device__ __forceinline__ void cp_async4(void* s, const void* g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
@@ -61,6 +60,7 @@ __device__ __forceinline__ void cp_async_wait_but() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// L2-coherent loads (bypass L1): for arrays written by other CTAs in the same launch.
 __device__ __forceinline__ int ldcg(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ unsigned ldcg(const unsigned* p) { return __ldcg(p); }
 __device__ __forceinline__ float ldcg(const float* p) { return __ldcg(p); }

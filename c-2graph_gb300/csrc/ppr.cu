@@ -7,12 +7,14 @@
 //   then every vertex v that got a message: res[v] += msg[v]; msg[v] = 0;
 //        if res[v] > rmax: pr[v] += alpha*res[v] and v joins the next frontier.
 //
-// Precision: edge weights and pr are FP32; the residual state (res, msg, the residual a
-// frontier vertex pushes) is FP64.  res > rmax is a threshold: FP32 residuals of vertices
+// Precision: edge weights and pr are FP32; the residual state (res, msg, the residual that a push
+// round pushes) is FP64.  Pull rounds take the pushed residuals as float pairs (cut to 47 bits) and sum their
+// messages as float pairs before they meet the FP64 residual: over 40 drawn queries, batches and gradients the L1 error of
+// each output against 64 bits is that of the all-FP64 push to six digits.  res > rmax is a threshold: FP32 residuals of vertices
 // sitting at rmax land on the other side of it than FP64 ones, each such flip moves
 // about rmax of mass and cascades downstream, so FP32 residual bookkeeping drifts past
 // L1 1e-6 of the FP64 result as graphs grow.  With FP64 residuals the decisions match the
-// FP64 push up to summation order.
+// FP64 push up to summation order and the pairs' 2^-47.
 //
 // Round shapes, chosen per round from the frontier's out-edge count T:
 //   * push (T small): edge-tiled walk over the frontier's out-edges, FP64 atomicAdd into
