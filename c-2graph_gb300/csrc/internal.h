@@ -41,7 +41,7 @@ struct TraversalCtl {
     unsigned listctr[3];         // PPR touched-list counters per round slot
     unsigned dctr[3];            // PPR activated vertices without out-edges, per slot
     unsigned farctr[3];          // SSSP far piles (rotating: current, target, free)
-    int farmin[3];  // by slot; single PPR: not 0 when a residual pushed in the slot's round is too large for pulls
+    int farmin[3];  // by slot; single PPR, after a push round: not 0 when a pushed residual is too large for pulls
     unsigned bar_count, bar_pad;  // GridBarrier
     int flags;                    // C2G_FLAG_*
     int iterations;

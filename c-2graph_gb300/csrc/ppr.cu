@@ -157,10 +157,13 @@ __device__ __forceinline__ void ppr_push(const PprParams& p, int buf, int slot, 
     if (track) list_stage_flush(tst, p.touched, &p.ctl->listctr[slot], (unsigned)p.V, &p.ctl->flags);
 }
 
-// Pulls end when a pushed residual passes kPullMaxQ.  The rounds' word for it is ctl->farmin[slot], kept by
+// Pulls end when a pushed residual passes kPullMaxQ.  The rounds' word for it is kept by
 // round slot like the counts: a round reads its own slot's and whoever finds such a residual writes the
 // next round's, so nothing that a round reads is written while it runs (a pull round has one barrier, at its
-// end).  A round that finds it set hands it on, so that it stays.
+// end).  A pull writes it beside the next round's counts (kPullsEnd in ctl->pcount: a load of its own costs a round of a
+// million edges 3%), a push into ctl->farmin, where a round that finds it set hands it on, so that it stays.
+constexpr unsigned long long kPullsEnd = 1ull << 63;
+__device__ __forceinline__ unsigned pull_frontier(unsigned long long c) { return (unsigned)((c & ~kPullsEnd) >> 32); }
 
 // The float pair of a pushed residual (fp64_mul.h), and its value.
 __device__ __forceinline__ float2 ppr_pair(double q) {
@@ -348,7 +351,7 @@ __device__ __forceinline__ void pull_totals(TraversalCtl* ctl, int nslot, PullTo
     if (threadIdx.x == 0) {
         if (share.count) atomicAdd(&ctl->pcount[nslot], share.count);
         if (share.dangling) atomicAdd(&ctl->dctr[nslot], share.dangling);
-        if (share.qmax > kPullMaxQ) atomicMax(&ctl->farmin[nslot], share.qmax);
+        if (share.qmax > kPullMaxQ) atomicOr(&ctl->pcount[nslot], kPullsEnd);
         share = PullTotals{0ull, 0u, 0};
     }
 }
@@ -425,8 +428,8 @@ __device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur
             pr0 = ldcg(p.pr + rec.x);
         }
         const unsigned long long c = ldcg(&ctl->pcount[slot]);
-        const unsigned F = (unsigned)(c >> 32), T = (unsigned)c, D = ldcg(&ctl->dctr[slot]);
-        if (F == 0 || T == 0 || iters >= p.max_iter || ldcg(&ctl->farmin[slot]) != 0) return true;  // grid-uniform
+        const unsigned F = pull_frontier(c), T = (unsigned)c, D = ldcg(&ctl->dctr[slot]);
+        if (F == 0 || T == 0 || iters >= p.max_iter || (c & kPullsEnd)) return true;  // grid-uniform
         ++iters;
         if (gtid == 0) {
             ctl->qctr[fslot] = 0ull;
@@ -434,7 +437,6 @@ __device__ __forceinline__ bool ppr_rounds_one_step(const PprParams& p, int& cur
             ctl->listctr[fslot] = 0u;
             ctl->dctr[fslot] = 0u;
             ctl->pcount[fslot] = 0ull;
-            ctl->farmin[fslot] = 0;
             ctl->popped += F + D;
             ctl->relaxed += T;
             ctl->touched += (unsigned)p.V;
@@ -636,7 +638,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
     for (;;) {
         const int buf = cur & 1, slot = cur % 3, nslot = (cur + 1) % 3, fslot = (cur + 2) % 3;
         const unsigned long long c = counted ? ldcg(&ctl->pcount[slot]) : ldcg(&ctl->qctr[slot]);
-        const unsigned F = (unsigned)(c >> 32), T = (unsigned)c;
+        const unsigned F = pull_frontier(c), T = (unsigned)c;
         const unsigned D = ldcg(&ctl->dctr[slot]);
         if (F == 0 && D == 0) break;
         if (cur == 1) F1 = F;
@@ -651,7 +653,7 @@ __global__ void __launch_bounds__(kPprThreads, kPprBlocksPerSm) ppr_persistent(c
             break;
         }
         // grid-uniform; float pairs hold the pushed residuals and their sums below kPullMaxQ
-        const bool large = ldcg(&ctl->farmin[slot]) != 0;
+        const bool large = counted ? (c & kPullsEnd) != 0 : ldcg(&ctl->farmin[slot]) != 0;
         const bool pull = T > (counted ? p.pull_next : p.pull_min) && !large;
         // Pop the activated vertices without out-edges: their residual is dropped.  A pull does so
         // for every vertex with in-edges.
@@ -881,7 +883,7 @@ static int ppr_alloc(c2g_graph* g) {
 // above E / 5 and 6.05 with pulls only.  On small graphs a pull is about as short as the two
 // barriers and dependent atomics of the emptiest push round: up to kPullAlwaysEdges every round pulls, and up to
 // kPullMostEdges every round but those of a few thousand edges, which are all there is of a local query (large
-// rmax); the last ones of any other pull on up to kPullTailEdges.  us a query, pulls above E / 3, E / 200, always:
+// rmax); up to kPullTailEdges only those of at most E / kTailPullDiv before the first pull.  us a query, pulls above E / 3, E / 200, always:
 // 1.2M edges (100,000 uniform vertices), rmax 1e-3 102 / 102 / 75, 1e-7 1273 / 1043 / 900; 2.1M (150,000) 90 /
 // 90 / 80, 1358 / 1198 / 1132; 3.7M (scale 18) 110 / 106 / 124, 1770 / 1747 / 1798; 3.9M (299,999) 92 / 93 /
 // 118, 1553 / 1460 / 1518; rmax 0.1 37 / 37 / 34, 32 / 32 / 36, 38 / 38 / 57, 38 / 38 / 58.
@@ -892,7 +894,7 @@ static int ppr_alloc(c2g_graph* g) {
 // frontier.
 constexpr int64_t kPushPullDiv = 3;
 constexpr int64_t kPullAlwaysEdges = 1600000, kPullTailEdges = 2500000, kPullMostEdges = 4000000;
-constexpr int64_t kMostPullDiv = 200;
+constexpr int64_t kMostPullDiv = 200, kTailPullDiv = 1000;
 
 static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& rows, unsigned* pull_min,
                         unsigned* pull_next) {
@@ -907,7 +909,9 @@ static int ppr_pull_min(c2g_graph* g, const c2g_ppr_params& pp, const RowLists& 
         *pull_min = *pull_next = (unsigned)(g->E / div);
         return C2G_OK;
     }
-    const unsigned min = (unsigned)(g->E / (g->E <= kPullMostEdges ? kMostPullDiv : kPushPullDiv));
+    const unsigned min = (unsigned)(g->E / (g->E <= kPullTailEdges   ? kTailPullDiv
+                                            : g->E <= kPullMostEdges ? kMostPullDiv
+                                                                     : kPushPullDiv));
     *pull_min = g->E <= kPullAlwaysEdges ? 0u : min;
     *pull_next = g->E <= kPullTailEdges ? 0u : min;
     return C2G_OK;

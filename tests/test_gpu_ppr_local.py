@@ -1,6 +1,6 @@
 """Local queries of the single push, whose frontier stays small (large rmax), and default ones, on graphs around the
 sizes where the rule for pull rounds changes: a local query's rounds push above 1.6M edges and pull below, and the
-last rounds of a default one pull below 2.5M and push above.
+last rounds of a default one all pull below 2.5M.
 
 Tolerance: L1 1e-6 of the mass in the graph, the bar of the other push tests."""
 import numpy as np
