@@ -304,7 +304,8 @@ int c2g_ppr_default_params(const c2g_graph* g, int adsorption, c2g_ppr_params* o
  * transposed push on the reverse CSR with threshold rmax_backward (no counterpart in the
  * reference; the forward push it differentiates replaces calcuatePPR).  Repeated targets
  * count with their multiplicity.  grad has E entries; pi_out / lambda_out (V entries,
- * may be NULL) return the two vectors; loss (may be NULL) returns L. */
+ * may be NULL) return the two vectors; loss (may be NULL) returns L.  A call whose pushes
+ * fail leaves them as they were. */
 int c2g_ppr_adjoint(c2g_graph* g, int32_t source, const c2g_ppr_params* params, int32_t n_targets,
                     const int32_t* targets, float rmax_backward, float* grad, float* pi_out,
                     float* lambda_out, double* loss, int on_device, c2g_stats* stats);
